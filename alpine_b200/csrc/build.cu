@@ -1,20 +1,24 @@
 // GPU BVH builder (see build.cuh).
 //
-// Binary phase: level-synchronous top-down binned SAH over primitive
-// references. Every level processes all active tasks (node ranges) at once:
-//   * big tasks (> kSmallMax references) are binned by blocks of kChunk
-//     references with shared-memory bins merged into per-task global bins,
-//     split by one warp per task, and partitioned stably by chunk;
-//   * small tasks are binned, split and partitioned by one warp each with
-//     warp-private shared-memory bins.
-// Children are compacted in a deterministic order with prefix sums, so a build
-// is a pure function of its input (the float min/max merges and integer counts
-// are order independent).
+// Binary phase: top-down binned SAH (32 bins) over primitive references.
+//   * Big tasks (nodes of more than kSmallMax references) go level by level,
+//     three launches a level. k_bin: blocks of kChunk references with
+//     shared-memory bins, merged into per-task global bins. k_split: one block
+//     per task picks the split plane, places the task's chunks and creates the
+//     children. k_scatter: the stable partition by chunk, which also gathers
+//     the children's centroid bounds.
+//   * A node of at most kSmallMax references is finished by one block in
+//     shared memory (k_subtree): every level below it, the leaves, and the
+//     collapse's cost program over the subtree.
+// Node ids and the order of the task lists depend on scheduling; the tree, the
+// order of the references in its leaves and everything derived from them do
+// not (float min/max merges, integer counts and stable partitions are order
+// independent), so a build is a pure function of its input.
 //
-// Wide phase: breadth-first collapse to 8 slots, quantised child boxes,
-// octant-ordered slots, triangle records in leaf order
-// (src/accelerators/wide_bvh.cpp:430-472 packs TriangleN likewise). Which
-// binary nodes fill a wide node's slots is chosen either
+// Wide phase: breadth-first collapse to 8 slots, two launches a level, eight
+// lanes per wide node, quantised child boxes, octant-ordered slots, triangle
+// records in leaf order (src/accelerators/wide_bvh.cpp:430-472 packs TriangleN
+// likewise). Which binary nodes fill a wide node's slots is chosen either
 //   * SAH-optimally (the default): a bottom-up dynamic program over the
 //     binary tree gives every node its least SAH cost when it may occupy
 //     1..8 slots of its parent (the method of Ylitie, Karras and Laine,
@@ -23,8 +27,12 @@
 //     collapse follows its choices; or
 //   * greedily, as the reference does (src/accelerators/wide_bvh.cpp:200-243):
 //     open the internal child of largest surface area until 8 slots are used.
+//
+// Every count stays in device memory, so a build is a fixed sequence of
+// launches that waits on nothing. build() enqueues the levels it expects and
+// reads the counters back once, at the end (it continues where they fell
+// short); enqueue() captures the sequence in a CUDA graph.
 #include "build.cuh"
-#include "scan.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -35,33 +43,26 @@
 namespace ag {
 namespace {
 
-constexpr uint32_t kSmallMax = 512;  // tasks up to this size are handled by one warp
-constexpr uint32_t kChunk = 1024;    // references per block for big tasks
+constexpr uint32_t kSmallMax = 512;  // nodes up to this size are finished by one block
+constexpr uint32_t kChunk = 1024;    // references per block of a big task
 constexpr int kChunkThreads = 256;   // kChunk / 4
-constexpr int kBinWords = 13;        // lo3 hi3 clo3 chi3 count
+constexpr int kBinWords = 7;         // lo3 hi3 count
 constexpr int kAxisBinWords = kSahBins * kBinWords;
 constexpr int kTaskBinWords = 3 * kAxisBinWords;
-constexpr int kSmallWarps = 4;       // warps per block in the small-task kernel
+constexpr int kChunkCounts = 3 * kSahBins;
 constexpr uint32_t kMaxLevels = 1024;
+constexpr uint32_t kMaxWideLevels = 64;
 
-struct alignas(16) Task {
-    float clo[3];
+// A big task. The centroid bounds are order-preserving integers (f2ord),
+// gathered by the parent's k_scatter.
+struct alignas(16) BigTask {
+    uint32_t clo[3];
     uint32_t node;
-    float chi[3];
+    uint32_t chi[3];
     uint32_t begin;
     uint32_t count;
-    uint32_t pad[3];
-};
-
-struct alignas(16) Cand {
-    float lo[3];
-    uint32_t begin;
-    float hi[3];
-    uint32_t count;
-    float clo[3];
-    uint32_t big;    // 1 when count > kSmallMax
-    float chi[3];
-    uint32_t chunks; // ceil(count / kChunk) for big candidates, else 0
+    uint32_t chunk0;  // its first entry of the level's chunk list
+    uint32_t pad[2];
 };
 
 struct BigSplit {
@@ -69,31 +70,40 @@ struct BigSplit {
     int bin;
     int mode;  // 0 = SAH bin split, 1 = median (all centroids coincide)
     uint32_t nL;
+    uint32_t child[2];  // big-task index of each child in the next level, kNoTask for a small one
+};
+constexpr uint32_t kNoTask = 0xffffffffu;
+
+// A node of at most kSmallMax references, finished by k_subtree.
+struct SmallTask {
+    uint32_t node, begin, count, level;
 };
 
-enum Counter { kCntTasks = 0, kCntBig, kCntChunks, kCntInt, kCntTri, kCntSlots, kCntBounds = 8, kCntWords = 32 };
-
-// Device-driven build (Builder::enqueue): the state the host loop keeps,
-// held in counter words instead, so that no kernel needs a host value.
-enum DevCounter {
-    kDevTasks = 20,  // tasks of the current binary level
-    kDevBig,         // big tasks of the current level
-    kDevChunks,      // chunks of the big tasks
-    kDevNodes,       // binary nodes so far (first id of the next level)
-    kDevLevels,      // binary levels that had tasks
-    kDevItems,       // wide nodes of the current collapse level
-    kDevWide,        // wide nodes so far
-    kDevTris,        // triangle records placed so far
-    kDevDepth,       // collapse levels that had items
-    kDevRootAreaInv, // float bits: 1 / half-area of the root box
-    kDevFailed,      // nonzero: the binary phase met a task it could not split (the build stops)
+// Counter words. The kLevel* arrays hold one word per binary level, the
+// kWide* arrays one per collapse level.
+enum Counter {
+    kCntBounds = 0,        // 12 words: box and centroid bounds of all primitives (f2ord)
+    kCntNodes = 12,        // binary node ids handed out
+    kCntRealNodes,         // binary nodes of the tree (id ranges of subtrees have gaps)
+    kCntSmall,             // entries of the small-task list
+    kCntTicket,            // next small task to be taken by k_subtree
+    kCntLevels,            // binary levels
+    kCntFailed,            // kFail* bits: the tree was not finished; the collapse is skipped
+    kCntSlots,             // filled child slots
+    kCntRootAreaInv,       // float bits: 1 / half-area of the root box
+    kCntSah,               // float bits: SAH cost of the wide tree
+    kCntWords = 32
 };
-static_assert((int)kDevFailed < (int)kCntWords, "counter words");
-
-// Work-item count of a level kernel: the host's count, or, in a
-// device-driven build, mult times the count a previous kernel left in
-// device memory.
-AG_D uint32_t level_count(const uint32_t* dn, uint32_t n, uint32_t mult = 1u) { return dn ? *dn * mult : n; }
+constexpr uint32_t kLevelBig = kCntWords;                             // big tasks
+constexpr uint32_t kLevelChunks = kLevelBig + kMaxLevels + 2;         // their chunks
+constexpr uint32_t kLevelNodes = kLevelChunks + kMaxLevels + 2;       // first node id
+constexpr uint32_t kWideItems = kLevelNodes + kMaxLevels + 2;         // wide nodes of the level
+constexpr uint32_t kWideTris = kWideItems + kMaxWideLevels + 2;       // triangle records placed by the level
+constexpr uint32_t kWideNodeBase = kWideTris + kMaxWideLevels + 2;    // first wide node of the next level
+constexpr uint32_t kWideTriBase = kWideNodeBase + kMaxWideLevels + 2; // first triangle record of the level
+constexpr uint32_t kFailLevels = 1u;    // big tasks left after the levels run, or a tree deeper than the cap
+constexpr uint32_t kFailCapacity = 2u;  // a list was full (never in a consistent build)
+constexpr uint32_t kAllWords = kWideTriBase + kMaxWideLevels + 2;
 
 // --------------------------------------------------------------------------
 // Binning arithmetic. Every kernel must compute identical bin indices, so all
@@ -112,15 +122,19 @@ AG_D int bin_of(float c, float clo, float scale)
 
 AG_D void bin_init_word(uint32_t* w, int k)
 {
-    int f = k % kBinWords;
-    // min words (lo, clo) start at the largest key, max words (hi, chi) at 0.
-    *w = (f < 3 || (f >= 6 && f < 9)) ? 0xffffffffu : 0u;
+    *w = k % kBinWords < 3 ? 0xffffffffu : 0u;  // min words start at the largest key, max words and counts at 0
 }
 
+// Half area of a box and the SAH cost of a split. Explicitly rounded, so that
+// every kernel that evaluates the same split gets the same cost.
 AG_D float area_of(float lx, float ly, float lz, float hx, float hy, float hz)
 {
-    float ex = hx - lx, ey = hy - ly, ez = hz - lz;
-    return ex * ey + ey * ez + ez * ex;
+    const float ex = __fsub_rn(hx, lx), ey = __fsub_rn(hy, ly), ez = __fsub_rn(hz, lz);
+    return __fmaf_rn(ez, ex, __fmaf_rn(ey, ez, __fmul_rn(ex, ey)));
+}
+AG_D float split_cost(uint32_t nL, float areaL, uint32_t nR, float areaR)
+{
+    return __fmaf_rn(float(nR), areaR, __fmul_rn(float(nL), areaL));
 }
 
 // Inclusive warp scans for union-of-boxes and counts.
@@ -146,30 +160,19 @@ AG_D float scan_max(float v)
     }
     return v;
 }
-template <bool kForward>
 AG_D uint32_t scan_add(uint32_t v)
 {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = kForward ? __shfl_up_sync(0xffffffffu, v, o) : __shfl_down_sync(0xffffffffu, v, o);
-        bool ok = kForward ? (lane_id() >= (uint32_t)o) : (lane_id() + o < 32);
-        if (ok) v += y;
+        uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane_id() >= (uint32_t)o) v += y;
     }
     return v;
 }
 
-AG_D float warp_min(float v)
-{
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-AG_D float warp_max(float v)
-{
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
+// Minimum / maximum of a float over the warp (no NaN among the values).
+AG_D float warp_min(float v) { return ord2f(__reduce_min_sync(0xffffffffu, f2ord(v))); }
+AG_D float warp_max(float v) { return ord2f(__reduce_max_sync(0xffffffffu, f2ord(v))); }
 
 // Result of a warp-wide split search over the bins of one task.
 struct SplitChoice {
@@ -177,46 +180,39 @@ struct SplitChoice {
     int axis;
     int bin;
     uint32_t nL;
-    float L[12];  // lo3 hi3 clo3 chi3 of the left child
-    float R[12];
+    float L[6];  // lo3 hi3 of the left child
+    float R[6];
 };
 
-// Evaluate all 31 split planes of one axis from bins held one per lane
-// (lane = bin). `v` holds the lane's bin: lo3 hi3 clo3 chi3 as floats (empty
-// bins: lo = +FLT_MAX, hi = -FLT_MAX) and `cnt`. Updates `best` when a cheaper
-// split is found (ties keep the earlier axis / lower bin).
-AG_D void eval_axis(int axis, const float v[12], uint32_t cnt, bool withCentroids, SplitChoice& best)
+AG_D void split_reset(SplitChoice& c)
 {
-    float Lv[12], Rv[12];
+    c.cost = FLT_MAX;
+    c.axis = -1;
+    c.bin = 0;
+    c.nL = 0;
+}
+
+// Evaluate all 31 split planes of one axis from bins held one per lane
+// (lane = bin). `v` holds the lane's bin: lo3 hi3 as floats (empty bins:
+// lo = +FLT_MAX, hi = -FLT_MAX) and `cnt`; total is the task's count. Updates
+// `best` when a cheaper split is found (ties keep the earlier axis / lower bin).
+AG_D void eval_axis(int axis, const float v[6], uint32_t cnt, uint32_t total, SplitChoice& best)
+{
+    float Lv[6], Rn[6];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         Lv[k] = scan_min<true>(v[k]);
         Lv[3 + k] = scan_max<true>(v[3 + k]);
-        Rv[k] = scan_min<false>(v[k]);
-        Rv[3 + k] = scan_max<false>(v[3 + k]);
+        // right side of the plane after bin k is bins k+1..31
+        Rn[k] = __shfl_down_sync(0xffffffffu, scan_min<false>(v[k]), 1);
+        Rn[3 + k] = __shfl_down_sync(0xffffffffu, scan_max<false>(v[3 + k]), 1);
     }
-    if (withCentroids) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            Lv[6 + k] = scan_min<true>(v[6 + k]);
-            Lv[9 + k] = scan_max<true>(v[9 + k]);
-            Rv[6 + k] = scan_min<false>(v[6 + k]);
-            Rv[9 + k] = scan_max<false>(v[9 + k]);
-        }
-    }
-    uint32_t cL = scan_add<true>(cnt);
-    uint32_t cR = scan_add<false>(cnt);
-    // right side of the plane after bin k is bins k+1..31
-    float Rn[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) Rn[k] = __shfl_down_sync(0xffffffffu, Rv[k], 1);
-    uint32_t cRn = __shfl_down_sync(0xffffffffu, cR, 1);
-    bool valid = lane_id() < 31 && cL > 0 && cRn > 0;
+    const uint32_t cL = scan_add(cnt);
+    const uint32_t cR = total - cL;
     float cost = FLT_MAX;
-    if (valid) {
-        cost = float(cL) * area_of(Lv[0], Lv[1], Lv[2], Lv[3], Lv[4], Lv[5]) +
-               float(cRn) * area_of(Rn[0], Rn[1], Rn[2], Rn[3], Rn[4], Rn[5]);
-    }
+    if (lane_id() < 31 && cL > 0 && cR > 0)
+        cost = split_cost(cL, area_of(Lv[0], Lv[1], Lv[2], Lv[3], Lv[4], Lv[5]), cR,
+                          area_of(Rn[0], Rn[1], Rn[2], Rn[3], Rn[4], Rn[5]));
     // warp argmin (cost, then lowest lane)
     float bc = cost;
     int bl = (int)lane_id();
@@ -232,66 +228,78 @@ AG_D void eval_axis(int axis, const float v[12], uint32_t cnt, bool withCentroid
         best.bin = bl;
         best.nL = __shfl_sync(0xffffffffu, cL, bl);
 #pragma unroll
-        for (int k = 0; k < 12; ++k) {
+        for (int k = 0; k < 6; ++k) {
             best.L[k] = __shfl_sync(0xffffffffu, Lv[k], bl);
             best.R[k] = __shfl_sync(0xffffffffu, Rn[k], bl);
         }
     }
 }
 
-AG_D void load_bin(const uint32_t* b, float v[12], uint32_t& cnt)
+AG_D void load_bin(const uint32_t* b, float v[6], uint32_t& cnt)
 {
-    cnt = b[12];
+    cnt = b[6];
 #pragma unroll
-    for (int k = 0; k < 12; ++k) {
-        bool isMin = (k < 3) || (k >= 6 && k < 9);
-        v[k] = cnt ? ord2f(b[k]) : (isMin ? FLT_MAX : -FLT_MAX);
-    }
+    for (int k = 0; k < 6; ++k) v[k] = cnt ? ord2f(b[k]) : (k < 3 ? FLT_MAX : -FLT_MAX);
 }
 
-AG_D void bin_accumulate(uint32_t* bin, float4 lo, float4 hi, float cx, float cy, float cz)
+AG_D void bin_accumulate(uint32_t* bin, const uint32_t ord[6])
 {
-    atomicMin(bin + 0, f2ord(lo.x));
-    atomicMin(bin + 1, f2ord(lo.y));
-    atomicMin(bin + 2, f2ord(lo.z));
-    atomicMax(bin + 3, f2ord(hi.x));
-    atomicMax(bin + 4, f2ord(hi.y));
-    atomicMax(bin + 5, f2ord(hi.z));
-    atomicMin(bin + 6, f2ord(cx));
-    atomicMin(bin + 7, f2ord(cy));
-    atomicMin(bin + 8, f2ord(cz));
-    atomicMax(bin + 9, f2ord(cx));
-    atomicMax(bin + 10, f2ord(cy));
-    atomicMax(bin + 11, f2ord(cz));
-    atomicAdd(bin + 12, 1u);
+    atomicMin(bin + 0, ord[0]);
+    atomicMin(bin + 1, ord[1]);
+    atomicMin(bin + 2, ord[2]);
+    atomicMax(bin + 3, ord[3]);
+    atomicMax(bin + 4, ord[4]);
+    atomicMax(bin + 5, ord[5]);
+    atomicAdd(bin + 6, 1u);
 }
 
-AG_D void write_cand(Cand* c, const float* b, uint32_t begin, uint32_t count)
+// Primitive boxes: {lo.xyz, hi.x}, {hi.y, hi.z, 0, 0}, one 32-byte sector each.
+AG_D void load_box(const float4* __restrict__ boxes, uint32_t p, float lo[3], float hi[3])
 {
-    Cand o;
-    o.lo[0] = b[0]; o.lo[1] = b[1]; o.lo[2] = b[2];
-    o.hi[0] = b[3]; o.hi[1] = b[4]; o.hi[2] = b[5];
-    o.clo[0] = b[6]; o.clo[1] = b[7]; o.clo[2] = b[8];
-    o.chi[0] = b[9]; o.chi[1] = b[10]; o.chi[2] = b[11];
-    o.begin = begin;
-    o.count = count;
-    o.big = count > kSmallMax ? 1u : 0u;
-    o.chunks = o.big ? (count + kChunk - 1) / kChunk : 0u;
-    *c = o;
+    const float4 a = boxes[2ull * p];
+    const float2 b = *reinterpret_cast<const float2*>(boxes + 2ull * p + 1);
+    lo[0] = a.x; lo[1] = a.y; lo[2] = a.z;
+    hi[0] = a.w; hi[1] = b.x; hi[2] = b.y;
+}
+
+AG_D void write_node(BinNode* __restrict__ bnodes, uint32_t id, const float box[6], uint32_t begin, uint32_t count)
+{
+    BinNode b;
+    b.lo = mk3(box[0], box[1], box[2]);
+    b.hi = mk3(box[3], box[4], box[5]);
+    b.begin = begin;
+    b.count = count;
+    b.left = -1;
+    b.right = -1;
+    b.pad[0] = b.pad[1] = 0u;
+    bnodes[id] = b;
 }
 
 // --------------------------------------------------------------------------
-// Preparation: primitive boxes and root bounds.
-// Primitives 0 .. ntris-1 are triangles, ntris .. n-1 spheres (centre +
-// radius): their box is centre -+ radius.
-__global__ void k_prep_prims(const float* __restrict__ verts, const uint32_t* __restrict__ idx, uint32_t ntris,
-                             const float4* __restrict__ spheres, uint32_t n, float4* __restrict__ primLo,
-                             float4* __restrict__ primHi, uint32_t* __restrict__ refs, uint32_t* __restrict__ bounds)
+// Preparation: counters, primitive boxes and root bounds.
+__global__ void k_begin(uint32_t* __restrict__ cnt)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kAllWords; i += gridDim.x * blockDim.x)
+        cnt[i] = (i < 3 || (i >= 6 && i < 9)) ? 0xffffffffu : 0u;  // the bounds' min words, else 0
+}
+
+// Primitives 0 .. ntris-1 are triangles, ntris .. n-1 spheres (centre +
+// radius): their box is centre -+ radius. The root's bounds are reduced per
+// block before the 12 atomics: one set of atomics per warp took 256 of the
+// 262 us of this kernel on 1M triangles.
+constexpr int kPrepThreads = 256;
+__global__ void __launch_bounds__(kPrepThreads) k_prep_prims(const float* __restrict__ verts,
+                                                             const uint32_t* __restrict__ idx, uint32_t ntris,
+                                                             const float4* __restrict__ spheres, uint32_t n,
+                                                             float4* __restrict__ boxes, uint32_t* __restrict__ refs,
+                                                             uint32_t* __restrict__ bounds)
+{
+    __shared__ uint32_t sb[12];
+    if (threadIdx.x < 12) sb[threadIdx.x] = (threadIdx.x < 3 || (threadIdx.x >= 6 && threadIdx.x < 9)) ? 0xffffffffu : 0u;
+    __syncthreads();
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     float c[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, cmx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    if (i < n) {
+    for (uint32_t i = blockIdx.x * kPrepThreads + threadIdx.x; i < n; i += gridDim.x * kPrepThreads) {
         float l[3], h[3];
         if (i < ntris) {
             const uint32_t* t = idx + 3ull * i;
@@ -313,272 +321,315 @@ __global__ void k_prep_prims(const float* __restrict__ verts, const uint32_t* __
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            lo[k] = l[k];
-            hi[k] = h[k];
-            c[k] = cmx[k] = centroid(l[k], h[k]);
+            const float ck = centroid(l[k], h[k]);
+            lo[k] = fminf(lo[k], l[k]);
+            hi[k] = fmaxf(hi[k], h[k]);
+            c[k] = fminf(c[k], ck);
+            cmx[k] = fmaxf(cmx[k], ck);
         }
-        primLo[i] = make_float4(l[0], l[1], l[2], 0.0f);
-        primHi[i] = make_float4(h[0], h[1], h[2], 0.0f);
+        boxes[2ull * i] = make_float4(l[0], l[1], l[2], h[0]);
+        boxes[2ull * i + 1] = make_float4(h[1], h[2], 0.0f, 0.0f);
         refs[i] = i;
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        lo[k] = warp_min(lo[k]);
-        hi[k] = warp_max(hi[k]);
-        c[k] = warp_min(c[k]);
-        cmx[k] = warp_max(cmx[k]);
-    }
-    if (lane_id() == 0) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            atomicMin(bounds + k, f2ord(lo[k]));
-            atomicMax(bounds + 3 + k, f2ord(hi[k]));
-            atomicMin(bounds + 6 + k, f2ord(c[k]));
-            atomicMax(bounds + 9 + k, f2ord(cmx[k]));
+        const uint32_t a = __reduce_min_sync(0xffffffffu, f2ord(lo[k])), b = __reduce_max_sync(0xffffffffu, f2ord(hi[k]));
+        const uint32_t d = __reduce_min_sync(0xffffffffu, f2ord(c[k])), e = __reduce_max_sync(0xffffffffu, f2ord(cmx[k]));
+        if (lane_id() == 0) {
+            atomicMin(sb + k, a);
+            atomicMax(sb + 3 + k, b);
+            atomicMin(sb + 6 + k, d);
+            atomicMax(sb + 9 + k, e);
         }
     }
+    __syncthreads();
+    const uint32_t w = threadIdx.x;
+    if (w < 12) {
+        if (w < 3 || (w >= 6 && w < 9)) atomicMin(bounds + w, sb[w]);
+        else atomicMax(bounds + w, sb[w]);
+    }
 }
 
-__global__ void k_init_bounds(uint32_t* bounds)
+__global__ void k_root(uint32_t n, uint32_t* __restrict__ cnt, BigTask* __restrict__ big, BinNode* __restrict__ bnodes,
+                       SmallTask* __restrict__ small, uint32_t* __restrict__ chunkTask, uint32_t* __restrict__ bins)
 {
-    int k = threadIdx.x;
-    if (k < 12) bounds[k] = (k < 3 || (k >= 6 && k < 9)) ? 0xffffffffu : 0u;
-}
-
-__global__ void k_root(uint32_t n, const uint32_t* __restrict__ bounds, Task* tasks, BinNode* bnodes,
-                       uint32_t* bigList, uint32_t* chunkOff, uint32_t* chunkTask, uint32_t nChunks)
-{
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t chunks = n > kSmallMax ? (n + kChunk - 1) / kChunk : 0u;
     if (i == 0) {
-        Task t;
-        for (int k = 0; k < 3; ++k) {
-            t.clo[k] = ord2f(bounds[6 + k]);
-            t.chi[k] = ord2f(bounds[9 + k]);
+        const uint32_t* bounds = cnt + kCntBounds;
+        float box[6];
+        for (int k = 0; k < 6; ++k) box[k] = ord2f(bounds[k]);
+        write_node(bnodes, 0, box, 0, n);
+        if (chunks) {
+            BigTask t{};
+            for (int k = 0; k < 3; ++k) {
+                t.clo[k] = bounds[6 + k];
+                t.chi[k] = bounds[9 + k];
+            }
+            t.node = 0;
+            t.begin = 0;
+            t.count = n;
+            t.chunk0 = 0;
+            big[0] = t;
+        } else {
+            small[0] = SmallTask{0u, 0u, n, 0u};
         }
-        t.node = 0;
-        t.begin = 0;
-        t.count = n;
-        tasks[0] = t;
-        BinNode b;
-        b.lo = mk3(ord2f(bounds[0]), ord2f(bounds[1]), ord2f(bounds[2]));
-        b.hi = mk3(ord2f(bounds[3]), ord2f(bounds[4]), ord2f(bounds[5]));
-        b.begin = 0;
-        b.count = n;
-        b.left = -1;
-        b.right = -1;
-        bnodes[0] = b;
-        bigList[0] = 0;
-        chunkOff[0] = 0;
+        cnt[kLevelBig] = chunks ? 1u : 0u;
+        cnt[kLevelChunks] = chunks;
+        cnt[kCntSmall] = chunks ? 0u : 1u;
+        cnt[kCntNodes] = 1u;
+        cnt[kCntRealNodes] = 1u;
     }
-    if (i < nChunks) chunkTask[i] = 0;
+    if (i < chunks) chunkTask[i] = 0;
+    if (chunks && i < (uint32_t)kTaskBinWords) bin_init_word(bins + i, (int)i);
 }
 
 // --------------------------------------------------------------------------
-// Big tasks.
-__global__ void k_bins_clear(uint32_t* bins, uint32_t numBig, const uint32_t* dBig)
-{
-    const uint32_t nb = level_count(dBig, numBig);
-    for (uint32_t bi = blockIdx.x; bi < nb; bi += gridDim.x) {
-        uint32_t* b = bins + size_t(bi) * kTaskBinWords;
-        for (int k = threadIdx.x; k < kTaskBinWords; k += blockDim.x) bin_init_word(b + k, k);
-    }
-}
-
-struct ChunkRange {
-    uint32_t bi, t, begin, end, local;
-};
-
-AG_D ChunkRange chunk_range(uint32_t c, const Task* tasks, const uint32_t* bigList, const uint32_t* chunkOff,
-                            const uint32_t* chunkTask, Task& task)
-{
-    ChunkRange r;
-    r.bi = chunkTask[c];
-    r.t = bigList[r.bi];
-    task = tasks[r.t];
-    r.local = c - chunkOff[r.bi];
-    r.begin = task.begin + r.local * kChunk;
-    r.end = min(task.begin + task.count, r.begin + kChunk);
-    return r;
-}
-
-__global__ void __launch_bounds__(kChunkThreads) k_bin_big(const Task* __restrict__ tasks, const uint32_t* __restrict__ refs,
-                                                           const float4* __restrict__ primLo, const float4* __restrict__ primHi,
-                                                           const uint32_t* __restrict__ bigList, const uint32_t* __restrict__ chunkOff,
-                                                           const uint32_t* __restrict__ chunkTask, uint32_t* __restrict__ bigBins,
-                                                           uint32_t numChunks, const uint32_t* __restrict__ dChunks)
+// Big tasks, level by level. The lists are double-buffered by level parity.
+// One block per chunk of 1,024 references; the chunk's bin counts are kept
+// (16 bits each), so that k_split can place the chunks of the partition
+// without another pass over the references. Bound by the shared-memory
+// atomics (21 a reference; with the centroid bounds among the bins' words it
+// was 39).
+__global__ void __launch_bounds__(kChunkThreads) k_bin(const BigTask* __restrict__ tasks, const uint32_t* __restrict__ refs,
+                                                       const float4* __restrict__ boxes,
+                                                       const uint32_t* __restrict__ chunkTask,
+                                                       uint32_t* __restrict__ bins, uint16_t* __restrict__ chunkCnt,
+                                                       uint32_t* __restrict__ cnt, uint32_t level, uint32_t capChunks)
 {
     __shared__ uint32_t sb[kTaskBinWords];
-    const uint32_t nc = level_count(dChunks, numChunks);
+    // the next level's nodes start where the ids handed out so far end
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt[kLevelNodes + level + 1] = cnt[kCntNodes];
+    const uint32_t nc = cnt[kCntFailed] ? 0u : min(cnt[kLevelChunks + level], capChunks);
     for (uint32_t cb = blockIdx.x; cb < nc; cb += gridDim.x) {
-        for (int k = threadIdx.x; k < kTaskBinWords; k += blockDim.x) bin_init_word(sb + k, k);
+        for (int k = threadIdx.x; k < kTaskBinWords; k += kChunkThreads) bin_init_word(sb + k, k);
         __syncthreads();
-        Task task;
-        ChunkRange r = chunk_range(cb, tasks, bigList, chunkOff, chunkTask, task);
-        float sc[3];
+        const uint32_t bi = chunkTask[cb];
+        const BigTask task = tasks[bi];
+        float clo[3], sc[3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) sc[a] = axis_scale(task.clo[a], task.chi[a]);
-        for (uint32_t i = r.begin + threadIdx.x; i < r.end; i += blockDim.x) {
-            uint32_t p = refs[i];
-            float4 lo = primLo[p], hi = primHi[p];
-            float cx = centroid(lo.x, hi.x), cy = centroid(lo.y, hi.y), cz = centroid(lo.z, hi.z);
-            float cc[3] = {cx, cy, cz};
+        for (int a = 0; a < 3; ++a) {
+            clo[a] = ord2f(task.clo[a]);
+            sc[a] = axis_scale(clo[a], ord2f(task.chi[a]));
+        }
+        const uint32_t begin = task.begin + (cb - task.chunk0) * kChunk, end = min(task.begin + task.count, begin + kChunk);
+        for (uint32_t i = begin + threadIdx.x; i < end; i += kChunkThreads) {
+            float lo[3], hi[3];
+            load_box(boxes, refs[i], lo, hi);
+            uint32_t ord[6];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                ord[k] = f2ord(lo[k]);
+                ord[3 + k] = f2ord(hi[k]);
+            }
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (sc[a] == 0.0f) continue;
-                int b = bin_of(cc[a], task.clo[a], sc[a]);
-                bin_accumulate(sb + a * kAxisBinWords + b * kBinWords, lo, hi, cx, cy, cz);
+                bin_accumulate(sb + a * kAxisBinWords + bin_of(centroid(lo[a], hi[a]), clo[a], sc[a]) * kBinWords, ord);
             }
         }
         __syncthreads();
-        uint32_t* g = bigBins + size_t(r.bi) * kTaskBinWords;
-        for (int k = threadIdx.x; k < kTaskBinWords; k += blockDim.x) {
-            int binBase = k - k % kBinWords;
-            if (sb[binBase + 12] == 0) continue;  // empty bin: nothing to merge
-            int f = k % kBinWords;
-            if (f == 12) atomicAdd(g + k, sb[k]);
-            else if (f < 3 || (f >= 6 && f < 9)) atomicMin(g + k, sb[k]);
+        uint32_t* g = bins + size_t(bi) * kTaskBinWords;
+        for (int k = threadIdx.x; k < kTaskBinWords; k += kChunkThreads) {
+            const int f = k % kBinWords;
+            const uint32_t filled = sb[k - f + 6];
+            if (f == 6) chunkCnt[size_t(cb) * kChunkCounts + k / kBinWords] = (uint16_t)filled;
+            if (filled == 0) continue;  // empty bin: nothing to merge
+            if (f == 6) atomicAdd(g + k, filled);
+            else if (f < 3) atomicMin(g + k, sb[k]);
             else atomicMax(g + k, sb[k]);
         }
         __syncthreads();  // sb is cleared again for the next chunk
     }
 }
 
-__global__ void k_split_big(const Task* __restrict__ tasks, const uint32_t* __restrict__ bigList,
-                            const uint32_t* __restrict__ bigBins, BigSplit* __restrict__ splits,
-                            Cand* __restrict__ cands, uint32_t* __restrict__ candFlag, uint32_t numBig,
-                            const uint32_t* __restrict__ dBig)
+// One block per big task: the split (a warp per axis), the children, and the
+// position of every chunk's left references in the partition.
+constexpr int kSplitThreads = 256;
+__global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* __restrict__ tasks, const uint32_t* __restrict__ bins,
+                                                         const uint16_t* __restrict__ chunkCnt,
+                                                         uint32_t* __restrict__ chunkLeft, BigSplit* __restrict__ splits,
+                                                         BinNode* __restrict__ bnodes, BigTask* __restrict__ next,
+                                                         uint32_t* __restrict__ nextChunkTask,
+                                                         uint32_t* __restrict__ nextBins, SmallTask* __restrict__ small,
+                                                         uint32_t* __restrict__ cnt, uint32_t level, uint32_t capBig,
+                                                         uint32_t capChunks, uint32_t capPrims,
+                                                         uint32_t* __restrict__ status)
 {
-    const uint32_t nb = level_count(dBig, numBig);
+    __shared__ SplitChoice axisBest[3];
+    __shared__ BigSplit split;
+    __shared__ uint32_t childChunk0[2], childChunks[2], warpSums[kSplitThreads / 32];
+    const uint32_t nb = cnt[kCntFailed] & kFailCapacity ? 0u : min(cnt[kLevelBig + level], capBig);
+    const uint32_t warp = threadIdx.x >> 5;
     for (uint32_t bi = blockIdx.x; bi < nb; bi += gridDim.x) {
-        uint32_t t = bigList[bi];
-        Task task = tasks[t];
-        SplitChoice best;
-        best.cost = FLT_MAX;
-        best.axis = -1;
-        best.bin = 0;
-        best.nL = 0;
-        for (int a = 0; a < 3; ++a) {
-            if (axis_scale(task.clo[a], task.chi[a]) == 0.0f) continue;
-            float v[12];
-            uint32_t cnt;
-            load_bin(bigBins + size_t(bi) * kTaskBinWords + a * kAxisBinWords + lane_id() * kBinWords, v, cnt);
-            eval_axis(a, v, cnt, true, best);
-        }
-        if (lane_id() == 0) {
-            BigSplit s;
-            if (best.axis >= 0) {
-                s.axis = best.axis;
-                s.bin = best.bin;
-                s.mode = 0;
-                s.nL = best.nL;
-                write_cand(cands + 2 * t, best.L, task.begin, best.nL);
-                write_cand(cands + 2 * t + 1, best.R, task.begin + best.nL, task.count - best.nL);
-            } else {
-                // All centroids coincide: split by position. The children inherit
-                // the parent's node box (a NaN in lo marks this for k_compact) and
-                // its point-sized centroid box.
-                float pb[12];
-                const float nan = __uint_as_float(0x7fc00000u);
-                for (int k = 0; k < 3; ++k) {
-                    pb[k] = nan;
-                    pb[3 + k] = nan;
-                    pb[6 + k] = task.clo[k];
-                    pb[9 + k] = task.chi[k];
-                }
-                s.axis = 0;
-                s.bin = 0;
-                s.mode = 1;
-                s.nL = task.count / 2;
-                write_cand(cands + 2 * t, pb, task.begin, s.nL);
-                write_cand(cands + 2 * t + 1, pb, task.begin + s.nL, task.count - s.nL);
+        const BigTask task = tasks[bi];
+        if (warp < 3) {
+            SplitChoice best;
+            split_reset(best);
+            if (axis_scale(ord2f(task.clo[warp]), ord2f(task.chi[warp])) != 0.0f) {
+                float v[6];
+                uint32_t c;
+                load_bin(bins + size_t(bi) * kTaskBinWords + warp * kAxisBinWords + lane_id() * kBinWords, v, c);
+                eval_axis((int)warp, v, c, task.count, best);
             }
-            splits[bi] = s;
-            candFlag[2 * t] = 1;
-            candFlag[2 * t + 1] = 1;
+            if (lane_id() == 0) axisBest[warp] = best;
         }
-    }
-}
-
-AG_D bool goes_left(const BigSplit& s, const Task& task, uint32_t i, uint32_t p, const float4* primLo,
-                    const float4* primHi)
-{
-    if (s.mode == 1) return (i - task.begin) < s.nL;
-    float lo = comp(make_float3(primLo[p].x, primLo[p].y, primLo[p].z), s.axis);
-    float hi = comp(make_float3(primHi[p].x, primHi[p].y, primHi[p].z), s.axis);
-    float c = centroid(lo, hi);
-    return bin_of(c, task.clo[s.axis], axis_scale(task.clo[s.axis], task.chi[s.axis])) <= s.bin;
-}
-
-__global__ void __launch_bounds__(kChunkThreads) k_part_count(const Task* __restrict__ tasks, const uint32_t* __restrict__ refs,
-                                                              const float4* __restrict__ primLo, const float4* __restrict__ primHi,
-                                                              const uint32_t* __restrict__ bigList, const uint32_t* __restrict__ chunkOff,
-                                                              const uint32_t* __restrict__ chunkTask, const BigSplit* __restrict__ splits,
-                                                              uint32_t* __restrict__ chunkLeft, uint32_t numChunks,
-                                                              const uint32_t* __restrict__ dChunks)
-{
-    __shared__ uint32_t ws[kChunkThreads / 32];
-    const uint32_t nc = level_count(dChunks, numChunks);
-    for (uint32_t cb = blockIdx.x; cb < nc; cb += gridDim.x) {
-        Task task;
-        ChunkRange r = chunk_range(cb, tasks, bigList, chunkOff, chunkTask, task);
-        BigSplit s = splits[r.bi];
-        uint32_t c = 0;
-        for (uint32_t i = r.begin + threadIdx.x; i < r.end; i += blockDim.x) c += goes_left(s, task, i, refs[i], primLo, primHi);
-#pragma unroll
-        for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        if (lane_id() == 0) ws[threadIdx.x >> 5] = c;
         __syncthreads();
         if (threadIdx.x == 0) {
-            uint32_t s2 = 0;
-            for (int w = 0; w < kChunkThreads / 32; ++w) s2 += ws[w];
-            chunkLeft[cb] = s2;
+            SplitChoice best = axisBest[0];
+            for (int a = 1; a < 3; ++a)
+                if (axisBest[a].cost < best.cost) best = axisBest[a];
+            BigSplit s;
+            s.axis = best.axis >= 0 ? best.axis : 0;
+            s.bin = best.bin;
+            s.mode = best.axis >= 0 ? 0 : 1;
+            s.nL = best.axis >= 0 ? best.nL : task.count / 2;
+            if (best.axis < 0) {  // all centroids coincide: split by position, the children keep the parent's box
+                const BinNode p = bnodes[task.node];
+                const float box[6] = {p.lo.x, p.lo.y, p.lo.z, p.hi.x, p.hi.y, p.hi.z};
+                for (int k = 0; k < 6; ++k) best.L[k] = best.R[k] = box[k];
+            }
+            s.child[0] = s.child[1] = kNoTask;
+            childChunks[0] = childChunks[1] = 0u;
+            childChunk0[0] = childChunk0[1] = 0u;
+            const uint32_t id = atomicAdd(cnt + kCntNodes, 2u);
+            atomicAdd(cnt + kCntRealNodes, 2u);
+            atomicMax(cnt + kCntLevels, level + 1u);
+            // capacities: never exceeded by a consistent build; checked so that
+            // inconsistent input cannot write past the buffers
+            bool ok = id + 1u < 2u * capPrims;
+            if (ok) {
+                bnodes[task.node].left = (int32_t)id;
+                bnodes[task.node].right = (int32_t)id + 1;
+                const uint32_t begin[2] = {task.begin, task.begin + s.nL}, count[2] = {s.nL, task.count - s.nL};
+                for (uint32_t k = 0; k < 2; ++k) {
+                    write_node(bnodes, id + k, k ? best.R : best.L, begin[k], count[k]);
+                    if (count[k] > kSmallMax) {
+                        const uint32_t chunks = (count[k] + kChunk - 1) / kChunk;
+                        const uint32_t ci = atomicAdd(cnt + kLevelBig + level + 1, 1u);
+                        const uint32_t c0 = atomicAdd(cnt + kLevelChunks + level + 1, chunks);
+                        if (ci >= capBig || c0 + chunks > capChunks) { ok = false; continue; }
+                        BigTask t{};
+                        for (int a = 0; a < 3; ++a) {
+                            t.clo[a] = 0xffffffffu;  // gathered by k_scatter
+                            t.chi[a] = 0u;
+                        }
+                        t.node = id + k;
+                        t.begin = begin[k];
+                        t.count = count[k];
+                        t.chunk0 = c0;
+                        next[ci] = t;
+                        s.child[k] = ci;
+                        childChunk0[k] = c0;
+                        childChunks[k] = chunks;
+                    } else {
+                        const uint32_t si = atomicAdd(cnt + kCntSmall, 1u);
+                        if (si >= capPrims) { ok = false; continue; }
+                        small[si] = SmallTask{id + k, begin[k], count[k], level + 1u};
+                    }
+                }
+            }
+            if (!ok) {
+                atomicOr(status, kErrBadIndex);
+                atomicOr(cnt + kCntFailed, kFailCapacity);
+            }
+            split = s;
+            splits[bi] = s;
         }
-        __syncthreads();  // ws is written again for the next chunk
+        __syncthreads();
+        const BigSplit s = split;
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (s.child[k] != kNoTask) {
+                for (uint32_t c = threadIdx.x; c < childChunks[k]; c += kSplitThreads)
+                    nextChunkTask[childChunk0[k] + c] = s.child[k];
+                uint32_t* b = nextBins + size_t(s.child[k]) * kTaskBinWords;
+                for (int w = threadIdx.x; w < kTaskBinWords; w += kSplitThreads) bin_init_word(b + w, w);
+            }
+        // left references before each chunk
+        const uint32_t chunks = (task.count + kChunk - 1) / kChunk;
+        uint32_t run = 0;
+        for (uint32_t base = 0; base < chunks; base += kSplitThreads) {
+            const uint32_t c = base + threadIdx.x;
+            uint32_t left = 0;
+            if (c < chunks && s.mode == 0) {
+                const uint16_t* p = chunkCnt + size_t(task.chunk0 + c) * kChunkCounts + s.axis * kSahBins;
+                for (int b = 0; b <= s.bin; ++b) left += p[b];
+            }
+            const uint32_t inc = scan_add(left);
+            if (lane_id() == 31) warpSums[warp] = inc;
+            __syncthreads();
+            uint32_t before = 0, all = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < kSplitThreads / 32; ++w) {
+                if (w < warp) before += warpSums[w];
+                all += warpSums[w];
+            }
+            if (c < chunks) chunkLeft[task.chunk0 + c] = s.mode == 0 ? run + before + inc - left : min(c * kChunk, s.nL);
+            run += all;
+            __syncthreads();  // warpSums is written again
+        }
     }
 }
 
-__global__ void __launch_bounds__(kChunkThreads) k_part_scatter(const Task* __restrict__ tasks, const uint32_t* __restrict__ refs,
-                                                                uint32_t* __restrict__ refsNext,
-                                                                const float4* __restrict__ primLo, const float4* __restrict__ primHi,
-                                                                const uint32_t* __restrict__ bigList, const uint32_t* __restrict__ chunkOff,
-                                                                const uint32_t* __restrict__ chunkTask, const BigSplit* __restrict__ splits,
-                                                                const uint32_t* __restrict__ chunkLeftOff,
-                                                                uint32_t* __restrict__ status, uint32_t numChunks,
-                                                                const uint32_t* __restrict__ dChunks)
+// Stable partition, one block per chunk, four consecutive references a
+// thread; also the centroid bounds of the big children.
+__global__ void __launch_bounds__(kChunkThreads) k_scatter(BigTask* __restrict__ next, const BigTask* __restrict__ tasks,
+                                                           const uint32_t* __restrict__ refs,
+                                                           uint32_t* __restrict__ refsNext,
+                                                           const float4* __restrict__ boxes,
+                                                           const uint32_t* __restrict__ chunkTask,
+                                                           const BigSplit* __restrict__ splits,
+                                                           const uint32_t* __restrict__ chunkLeft,
+                                                           const uint32_t* __restrict__ cnt, uint32_t level,
+                                                           uint32_t capChunks, uint32_t* __restrict__ status)
 {
-    __shared__ uint32_t wl[kChunkThreads / 32], wv[kChunkThreads / 32];
-    const uint32_t nc = level_count(dChunks, numChunks);
+    __shared__ uint32_t wl[kChunkThreads / 32], wv[kChunkThreads / 32], cb12[12];
+    const uint32_t nc = cnt[kCntFailed] ? 0u : min(cnt[kLevelChunks + level], capChunks);
     for (uint32_t cb = blockIdx.x; cb < nc; cb += gridDim.x) {
-        Task task;
-        ChunkRange r = chunk_range(cb, tasks, bigList, chunkOff, chunkTask, task);
-        BigSplit s = splits[r.bi];
-        uint32_t leftBefore = chunkLeftOff[cb] - chunkLeftOff[chunkOff[r.bi]];
-        uint32_t rightBefore = r.local * kChunk - leftBefore;
-        // each thread owns 4 consecutive references: stable order inside the chunk
-        uint32_t base = r.begin + threadIdx.x * 4;
+        const uint32_t bi = chunkTask[cb];
+        const BigTask task = tasks[bi];
+        const BigSplit s = splits[bi];
+        const uint32_t local = cb - task.chunk0, begin = task.begin + local * kChunk;
+        const uint32_t end = min(task.begin + task.count, begin + kChunk);
+        const uint32_t leftBefore = chunkLeft[cb], rightBefore = local * kChunk - leftBefore;
+        const float clo = ord2f(task.clo[s.axis]);
+        const float scale = axis_scale(clo, ord2f(task.chi[s.axis]));
+        if (threadIdx.x < 12) cb12[threadIdx.x] = threadIdx.x % 6 < 3 ? 0xffffffffu : 0u;
+        const uint32_t base = begin + threadIdx.x * 4;
         uint32_t p[4];
         bool f[4];
         uint32_t nl = 0;
+        uint32_t bb[12] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u, 0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            uint32_t i = base + k;
+            const uint32_t i = base + k;
             f[k] = false;
             p[k] = 0;
-            if (i < r.end) {
+            if (i < end) {
                 p[k] = refs[i];
-                f[k] = goes_left(s, task, i, p[k], primLo, primHi);
+                float lo[3], hi[3];
+                load_box(boxes, p[k], lo, hi);
+                const float c[3] = {centroid(lo[0], hi[0]), centroid(lo[1], hi[1]), centroid(lo[2], hi[2])};
+                const float ca = s.axis == 0 ? c[0] : (s.axis == 1 ? c[1] : c[2]);
+                f[k] = s.mode == 1 ? (i - task.begin) < s.nL : bin_of(ca, clo, scale) <= s.bin;
                 nl += f[k];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const uint32_t o = f2ord(c[a]);
+                    if (f[k]) {
+                        bb[a] = min(bb[a], o);
+                        bb[3 + a] = max(bb[3 + a], o);
+                    } else {
+                        bb[6 + a] = min(bb[6 + a], o);
+                        bb[9 + a] = max(bb[9 + a], o);
+                    }
+                }
             }
         }
-        uint32_t nvalid = base < r.end ? min(4u, r.end - base) : 0u;
+        const uint32_t nvalid = base < end ? min(4u, end - base) : 0u;
         // block exclusive scan of (left count, valid count)
-        uint32_t il = nl, iv = nvalid;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t yl = __shfl_up_sync(0xffffffffu, il, o);
-            uint32_t yv = __shfl_up_sync(0xffffffffu, iv, o);
-            if (lane_id() >= (uint32_t)o) { il += yl; iv += yv; }
-        }
+        const uint32_t il = scan_add(nl), iv = scan_add(nvalid);
         if (lane_id() == 31) { wl[threadIdx.x >> 5] = il; wv[threadIdx.x >> 5] = iv; }
         __syncthreads();
         uint32_t pl = 0, pv = 0;
@@ -587,276 +638,56 @@ __global__ void __launch_bounds__(kChunkThreads) k_part_scatter(const Task* __re
         uint32_t rightRank = (pv + iv - nvalid) - leftRank;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            uint32_t i = base + k;
-            if (i >= r.end) break;
-            uint32_t dst = f[k] ? task.begin + leftBefore + leftRank++ : task.begin + s.nL + rightBefore + rightRank++;
+            const uint32_t i = base + k;
+            if (i >= end) break;
+            const uint32_t dst = f[k] ? task.begin + leftBefore + leftRank++ : task.begin + s.nL + rightBefore + rightRank++;
             if (dst >= task.begin + task.count) { atomicOr(status, kErrBadIndex); continue; }
             refsNext[dst] = p[k];
         }
-        __syncthreads();  // wl / wv are written again for the next chunk
-    }
-}
-
-// --------------------------------------------------------------------------
-// Small tasks: one warp does bin + split + partition.
-// Task t by one warp; sb: the warp's bins in shared memory.
-AG_D void small_task(uint32_t t, const Task* __restrict__ tasks, const uint32_t* __restrict__ refs,
-                     uint32_t* __restrict__ refsNext, const float4* __restrict__ primLo,
-                     const float4* __restrict__ primHi, const BinNode* __restrict__ bnodes, Cand* __restrict__ cands,
-                     uint32_t* __restrict__ candFlag, uint32_t* __restrict__ order, uint32_t* __restrict__ status,
-                     uint32_t* sb, uint32_t* failed)
-{
-    Task task = tasks[t];
-    if (task.count > kSmallMax) {  // handled by the big-task kernels
-        // A device-driven build runs those kernels on its first levels only
-        // (failed != null below them): the task gets no children, and the
-        // build is stopped and reported.
-        if (failed && lane_id() == 0) {
-            candFlag[2 * t] = 0;
-            candFlag[2 * t + 1] = 0;
-            atomicOr(failed, 1u);
-            atomicOr(status, kErrBuildDepth);
-        }
-        return;
-    }
-    uint32_t lane = lane_id();
-    const uint32_t b0 = task.begin, n = task.count;
-
-    auto make_leaf = [&]() {
-        for (uint32_t i = lane; i < n; i += 32) order[b0 + i] = refs[b0 + i];
-        if (lane == 0) { candFlag[2 * t] = 0; candFlag[2 * t + 1] = 0; }
-    };
-    if (n <= 1) { make_leaf(); return; }
-
-    // centroid bounds of this task
-    float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (uint32_t i = lane; i < n; i += 32) {
-        uint32_t p = refs[b0 + i];
-        float4 lo = primLo[p], hi = primHi[p];
-        float c[3] = {centroid(lo.x, hi.x), centroid(lo.y, hi.y), centroid(lo.z, hi.z)};
 #pragma unroll
-        for (int k = 0; k < 3; ++k) { clo[k] = fminf(clo[k], c[k]); chi[k] = fmaxf(chi[k], c[k]); }
-    }
-    float sc[3];
+        for (int side = 0; side < 2; ++side) {
+            if (s.child[side] == kNoTask) continue;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        clo[k] = warp_min(clo[k]);
-        chi[k] = warp_max(chi[k]);
-        sc[k] = axis_scale(clo[k], chi[k]);
-    }
-
-    __syncwarp();  // the warp's previous task has finished reading sb
-    for (int k = lane; k < kTaskBinWords; k += 32) bin_init_word(sb + k, k);
-    __syncwarp();
-    for (uint32_t i = lane; i < n; i += 32) {
-        uint32_t p = refs[b0 + i];
-        float4 lo = primLo[p], hi = primHi[p];
-        float cx = centroid(lo.x, hi.x), cy = centroid(lo.y, hi.y), cz = centroid(lo.z, hi.z);
-        float cc[3] = {cx, cy, cz};
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            if (sc[a] == 0.0f) continue;
-            bin_accumulate(sb + a * kAxisBinWords + bin_of(cc[a], clo[a], sc[a]) * kBinWords, lo, hi, cx, cy, cz);
-        }
-    }
-    __syncwarp();
-    SplitChoice best;
-    best.cost = FLT_MAX;
-    best.axis = -1;
-    best.bin = 0;
-    best.nL = 0;
-    for (int a = 0; a < 3; ++a) {
-        if (sc[a] == 0.0f) continue;
-        float v[12];
-        uint32_t cnt;
-        load_bin(sb + a * kAxisBinWords + lane * kBinWords, v, cnt);
-        eval_axis(a, v, cnt, false, best);
-    }
-    const BinNode node = bnodes[task.node];
-    float nodeArea = area_of(node.lo.x, node.lo.y, node.lo.z, node.hi.x, node.hi.y, node.hi.z);
-    // SAH with unit traversal and intersection costs.
-    float leafCost = float(n) * nodeArea;
-    float splitCost = nodeArea + best.cost;
-    if (n <= (uint32_t)kMaxLeafTris && (best.axis < 0 || leafCost <= splitCost)) { make_leaf(); return; }
-
-    uint32_t nL;
-    float Lb[12], Rb[12];
-    bool median = best.axis < 0;
-    if (!median) {
-        nL = best.nL;
-        for (int k = 0; k < 12; ++k) { Lb[k] = best.L[k]; Rb[k] = best.R[k]; }
-    } else {
-        nL = n / 2;
-        // bounds of each half by warp reduction
-        float l0[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
-        float l1[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
-        for (uint32_t i = lane; i < n; i += 32) {
-            uint32_t p = refs[b0 + i];
-            float4 lo = primLo[p], hi = primHi[p];
-            float* d = i < nL ? l0 : l1;
-            d[0] = fminf(d[0], lo.x); d[1] = fminf(d[1], lo.y); d[2] = fminf(d[2], lo.z);
-            d[3] = fmaxf(d[3], hi.x); d[4] = fmaxf(d[4], hi.y); d[5] = fmaxf(d[5], hi.z);
-        }
-        for (int k = 0; k < 3; ++k) {
-            Lb[k] = warp_min(l0[k]); Lb[3 + k] = warp_max(l0[3 + k]);
-            Rb[k] = warp_min(l1[k]); Rb[3 + k] = warp_max(l1[3 + k]);
-        }
-        for (int k = 0; k < 3; ++k) { Lb[6 + k] = Rb[6 + k] = clo[k]; Lb[9 + k] = Rb[9 + k] = chi[k]; }
-    }
-    // stable partition into refsNext
-    uint32_t leftSeen = 0, rightSeen = 0;
-    for (uint32_t base = 0; base < n; base += 32) {
-        uint32_t i = base + lane;
-        bool valid = i < n;
-        uint32_t p = valid ? refs[b0 + i] : 0;
-        bool left = false;
-        if (valid) {
-            if (median) left = i < nL;
-            else {
-                float4 lo = primLo[p], hi = primHi[p];
-                float c = centroid(comp(make_float3(lo.x, lo.y, lo.z), best.axis), comp(make_float3(hi.x, hi.y, hi.z), best.axis));
-                left = bin_of(c, clo[best.axis], sc[best.axis]) <= best.bin;
+            for (int a = 0; a < 6; ++a) {
+                const uint32_t v = a < 3 ? __reduce_min_sync(0xffffffffu, bb[6 * side + a])
+                                         : __reduce_max_sync(0xffffffffu, bb[6 * side + a]);
+                if (lane_id() == 0) {
+                    if (a < 3) atomicMin(cb12 + 6 * side + a, v);
+                    else atomicMax(cb12 + 6 * side + a, v);
+                }
             }
         }
-        uint32_t bl = __ballot_sync(0xffffffffu, valid && left);
-        uint32_t br = __ballot_sync(0xffffffffu, valid && !left);
-        if (valid) {
-            uint32_t dst = left ? b0 + leftSeen + __popc(bl & lanemask_lt())
-                                : b0 + nL + rightSeen + __popc(br & lanemask_lt());
-            if (dst < b0 + n) refsNext[dst] = p;
-            else atomicOr(status, kErrBadIndex);
+        __syncthreads();
+        const uint32_t w = threadIdx.x;
+        if (w < 12 && s.child[w / 6] != kNoTask) {
+            BigTask* t = next + s.child[w / 6];
+            if (w % 6 < 3) atomicMin(t->clo + w % 6, cb12[w]);
+            else atomicMax(t->chi + w % 6 - 3, cb12[w]);
         }
-        leftSeen += __popc(bl);
-        rightSeen += __popc(br);
-    }
-    if (lane == 0) {
-        write_cand(cands + 2 * t, Lb, b0, nL);
-        write_cand(cands + 2 * t + 1, Rb, b0 + nL, n - nL);
-        candFlag[2 * t] = 1;
-        candFlag[2 * t + 1] = 1;
-    }
-}
-
-__global__ void __launch_bounds__(32 * kSmallWarps) k_small(const Task* __restrict__ tasks, uint32_t numTasks,
-                                                          const uint32_t* __restrict__ refs, uint32_t* __restrict__ refsNext,
-                                                          const float4* __restrict__ primLo, const float4* __restrict__ primHi,
-                                                          const BinNode* __restrict__ bnodes, Cand* __restrict__ cands,
-                                                          uint32_t* __restrict__ candFlag, uint32_t* __restrict__ order,
-                                                          uint32_t* __restrict__ status, const uint32_t* __restrict__ dTasks,
-                                                          uint32_t* __restrict__ failed)
-{
-    __shared__ uint32_t sbins[kSmallWarps][kTaskBinWords];
-    const uint32_t w = threadIdx.x >> 5;
-    const uint32_t nt = level_count(dTasks, numTasks);
-    for (uint32_t t = blockIdx.x * kSmallWarps + w; t < nt; t += gridDim.x * kSmallWarps)
-        small_task(t, tasks, refs, refsNext, primLo, primHi, bnodes, cands, candFlag, order, status, sbins[w],
-                   failed);
-}
-
-// --------------------------------------------------------------------------
-// Compaction of the children into the next level's task list.
-__global__ void k_cand_keys(const Cand* __restrict__ cands, const uint32_t* __restrict__ candFlag, uint32_t nHost,
-                            uint32_t* __restrict__ bigFlag, uint32_t* __restrict__ chunkCnt,
-                            const uint32_t* __restrict__ dTasks)
-{
-    const uint32_t n = level_count(dTasks, nHost, 2u);
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        bool v = candFlag[j] != 0;
-        bigFlag[j] = v ? cands[j].big : 0u;
-        chunkCnt[j] = v ? cands[j].chunks : 0u;
-    }
-}
-
-__global__ void k_compact(const Task* __restrict__ tasks, const Cand* __restrict__ cands,
-                          const uint32_t* __restrict__ candFlag, const uint32_t* __restrict__ candPos,
-                          const uint32_t* __restrict__ bigPos, const uint32_t* __restrict__ chunkOffSparse, uint32_t nHost,
-                          uint32_t nodeBaseHost, Task* __restrict__ next, BinNode* __restrict__ bnodes,
-                          uint32_t* __restrict__ bigList, uint32_t* __restrict__ chunkOff, uint32_t* __restrict__ chunkTask,
-                          const uint32_t* __restrict__ dTasks, const uint32_t* __restrict__ dNodes, uint32_t capTasks,
-                          uint32_t capBig, uint32_t capChunks, uint32_t* __restrict__ status)
-{
-    const uint32_t n = level_count(dTasks, nHost, 2u);
-    const uint32_t nodeBase = level_count(dNodes, nodeBaseHost);
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        if (!candFlag[j]) continue;
-        Cand c = cands[j];
-        uint32_t p = candPos[j];
-        uint32_t node = nodeBase + p;
-        // capacities: never exceeded by a consistent build; checked so that
-        // inconsistent input cannot write past the buffers
-        if (p >= capTasks || node >= 2u * capTasks ||
-            (c.big && (bigPos[j] >= capBig || chunkOffSparse[j] + c.chunks > capChunks))) {
-            atomicOr(status, kErrBadIndex);
-            continue;
-        }
-        uint32_t parent = tasks[j >> 1].node;
-        if (j & 1) bnodes[parent].right = (int32_t)node;
-        else bnodes[parent].left = (int32_t)node;
-        BinNode b;
-        if (c.lo[0] != c.lo[0]) {  // median split of coincident centroids: inherit parent box
-            b.lo = bnodes[parent].lo;
-            b.hi = bnodes[parent].hi;
-        } else {
-            b.lo = mk3(c.lo[0], c.lo[1], c.lo[2]);
-            b.hi = mk3(c.hi[0], c.hi[1], c.hi[2]);
-        }
-        b.begin = c.begin;
-        b.count = c.count;
-        b.left = -1;
-        b.right = -1;
-        bnodes[node] = b;
-        Task t;
-        for (int k = 0; k < 3; ++k) { t.clo[k] = c.clo[k]; t.chi[k] = c.chi[k]; }
-        t.node = node;
-        t.begin = c.begin;
-        t.count = c.count;
-        next[p] = t;
-        if (c.big) {
-            uint32_t bi = bigPos[j];
-            bigList[bi] = p;
-            uint32_t off = chunkOffSparse[j];
-            chunkOff[bi] = off;
-            for (uint32_t k = 0; k < c.chunks; ++k) chunkTask[off + k] = bi;
-        }
+        __syncthreads();  // the shared words are written again for the next chunk
     }
 }
 
 // --------------------------------------------------------------------------
-// Collapse to the wide layout.
-AG_D float bn_area(const BinNode& b) { return area_of(b.lo.x, b.lo.y, b.lo.z, b.hi.x, b.hi.y, b.hi.z); }
-
-// SAH cost program of the collapse, one binary level per launch from the
-// deepest up. For binary node x of area A, count n and children l, r:
+// SAH cost program of the collapse. For binary node x of area A, count n and
+// children l, r:
 //   leaf(x)    = A * triCost * n                       (n <= kMaxLeafTris)
 //   D(x, j)    = min over k in 1..j-1 of C(l, k) + C(r, j - k)
 //   C(x, 1)    = leaf(x) if n <= kMaxLeafTris, else A + D(x, 8)  (x in one slot:
 //                a leaf, or an internal child whose own wide node tests 8 slots)
 //   C(x, j)    = min(C(x, j - 1), D(x, j))             (x spread over at most j slots)
-// with a wide-node visit costing 1 per unit area. cost[8x + j - 1] holds
-// C(x, j) for j = 1..7 and cost[8x + 7] = A + D(x, 8); nibble j - 1 of
-// choice[x] holds the k of D(x, j) when it was taken (0: x keeps j - 1
-// slots; nibble 7: the split of x's own wide node). A binary leaf costs
-// leaf(x) for every j.
-AG_D void collapse_cost_node(const BinNode* __restrict__ bnodes, uint32_t x, float triCost, float* __restrict__ cost,
-                             uint32_t* __restrict__ choice)
+// with a wide-node visit costing 1 per unit area. C[j - 1] holds C(x, j) for
+// j = 1..7; nibble j - 1 of the choice holds the k of D(x, j) when it was
+// taken (0: x keeps j - 1 slots; nibble 7: the split of x's own wide node). A
+// binary leaf costs leaf(x) for every j.
+constexpr int kCosts = 7;
+AG_D float leaf_cost(float area, uint32_t count, float triCost)
 {
-    const BinNode b = bnodes[x];
-    const float A = bn_area(b);
-    float* C = cost + 8ull * x;
-    if (b.left < 0) {
-        const float leaf = b.count <= (uint32_t)kMaxLeafTris ? A * triCost * float(b.count) : INFINITY;
-        for (int j = 0; j < 8; ++j) C[j] = leaf;
-        choice[x] = 0;
-        return;
-    }
-    float L[7], R[7];
-    const float* cl = cost + 8ull * (uint32_t)b.left;
-    const float* cr = cost + 8ull * (uint32_t)b.right;
-#pragma unroll
-    for (int j = 0; j < 7; ++j) {
-        L[j] = cl[j];
-        R[j] = cr[j];
-    }
+    return count <= (uint32_t)kMaxLeafTris ? __fmul_rn(__fmul_rn(area, triCost), float(count)) : INFINITY;
+}
+AG_D uint32_t collapse_cost(const float L[kCosts], const float R[kCosts], float A, uint32_t count, float triCost,
+                            float C[kCosts])
+{
     float D[9];
     uint32_t K[9];
 #pragma unroll
@@ -865,7 +696,7 @@ AG_D void collapse_cost_node(const BinNode* __restrict__ bnodes, uint32_t x, flo
         uint32_t bk = 1;
 #pragma unroll
         for (int k = 1; k < j; ++k) {
-            const float v = L[k - 1] + R[j - k - 1];
+            const float v = __fadd_rn(L[k - 1], R[j - k - 1]);
             if (v < best) {
                 best = v;
                 bk = (uint32_t)k;
@@ -874,8 +705,7 @@ AG_D void collapse_cost_node(const BinNode* __restrict__ bnodes, uint32_t x, flo
         D[j] = best;
         K[j] = bk;
     }
-    const float node = A + D[8];
-    float prev = b.count <= (uint32_t)kMaxLeafTris ? A * triCost * float(b.count) : node;
+    float prev = count <= (uint32_t)kMaxLeafTris ? leaf_cost(A, count, triCost) : __fadd_rn(A, D[8]);
     C[0] = prev;
     uint32_t ch = K[8] << 28;
 #pragma unroll
@@ -886,135 +716,705 @@ AG_D void collapse_cost_node(const BinNode* __restrict__ bnodes, uint32_t x, flo
         }
         C[j - 1] = prev;
     }
-    C[7] = node;
-    choice[x] = ch;
+    return ch;
 }
 
-// One binary level per launch: nodes [first, first + count), or, in a
-// device-driven build, [levelStart[level], levelStart[level + 1]).
-__global__ void k_collapse_cost(const BinNode* __restrict__ bnodes, uint32_t firstHost, uint32_t countHost,
-                                float triCost, float* __restrict__ cost, uint32_t* __restrict__ choice,
-                                const uint32_t* __restrict__ levelStart, uint32_t level)
+// --------------------------------------------------------------------------
+// Small nodes: one block finishes the subtree of a node of at most kSmallMax
+// references in shared memory: every split below it, the leaves, the order of
+// its references, and its part of the cost program. Against one launch (and
+// its counts, scans and compaction) per level this removed half of a build's
+// time and most of its launches.
+//
+// A level's nodes above kDirectMax references are split by one warp each,
+// with shared-memory bins. The others are split without bins, one thread per
+// reference: a thread takes the plane after its own reference's bin as its
+// candidate on each axis, sums the two sides over the node's references, and
+// the node's cheapest candidate wins (a 64-bit shared-memory minimum over
+// cost, axis, bin). Planes between two references' bins need no candidate of
+// their own: they cut the same sets as the plane after the lower bin, which
+// the bin search prefers as well. At eight references this takes about 400
+// instructions for four nodes; the bin search takes 1,500 for each.
+constexpr int kSubThreads = 256;
+constexpr uint32_t kSubWarps = kSubThreads / 32;
+constexpr uint32_t kDirectMax = 32;
+constexpr uint32_t kNoChild = 0xffffu;
+constexpr int kSubRounds = (int)kSmallMax / kSubThreads;
+static_assert(kSmallMax % kSubThreads == 0 && kDirectMax <= 32, "left bits of a node span at most two words");
+
+struct SubSmem {
+    unsigned long long key[kSmallMax];  // per node of the level: its cheapest candidate
+    union {
+        uint32_t bins[kSubWarps][kTaskBinWords];
+        float cost[(kSmallMax - 1) * kCosts];  // per internal node, once the tree is built
+    };
+    float box[6][kSmallMax];            // lo3 hi3 of the subtree's primitives
+    uint32_t prim[kSmallMax];           // their ids
+    uint32_t pbin[kSmallMax];           // per position: bins on the three axes, and which axes have an extent
+    float area[2 * kSmallMax];          // per node of the subtree
+    uint32_t leftBits[kSmallMax / 32];
+    uint32_t ticket, idBase, nodeTop, levelEnd;
+    uint16_t perm[2][kSmallMax];        // per position: the primitive there (index into box, prim)
+    uint16_t posNode[2][kSmallMax];     // per position: the node it belongs to
+    uint16_t begin[2 * kSmallMax], count[2 * kSmallMax], left[2 * kSmallMax];
+    uint16_t levelStart[kSmallMax + 2];
+};
+
+AG_D void sub_box(const SubSmem& s, uint32_t j, float lo[3], float hi[3])
 {
-    const uint32_t first = levelStart ? levelStart[level] : firstHost;
-    const uint32_t count = levelStart ? levelStart[level + 1] - first : countHost;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x)
-        collapse_cost_node(bnodes, first + t, triCost, cost, choice);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = s.box[k][j];
+        hi[k] = s.box[3 + k][j];
+    }
 }
 
-// The slots of one wide node per thread. choice (the cost program's
-// decisions) selects the SAH-optimal distribution; null selects the greedy
-// rule. Slots are then assigned to octants.
-AG_D void collapse_decide_item(uint32_t i, const uint2* __restrict__ items, const BinNode* __restrict__ bnodes,
-                               const uint32_t* __restrict__ choice, int32_t* __restrict__ slots,
-                               uint32_t* __restrict__ intCount, uint32_t* __restrict__ triCount,
-                               uint32_t* __restrict__ slotTotal)
+AG_D void box_reset(float b[6])
 {
-    uint32_t b = items[i].x;
-    int32_t ent[kWidth];
-    int n = 0;
-    const BinNode root = bnodes[b];
-    if (root.count <= (uint32_t)kMaxLeafTris || root.left < 0) {
-        ent[n++] = (int32_t)b;
-    } else if (choice) {
-        // follow the cost program: (node, slots it may use), root split first
-        int32_t stN[kWidth];
-        uint32_t stJ[kWidth];
-        int sp = 0;
-        const uint32_t k8 = min(max(choice[b] >> 28, 1u), 7u);  // 1..7 by construction; clamped so j stays <= 8
-        stN[sp] = root.right;
-        stJ[sp++] = 8u - k8;
-        stN[sp] = root.left;
-        stJ[sp++] = k8;
-        while (sp > 0) {
-            const int32_t x = stN[--sp];
-            uint32_t j = stJ[sp];
-            const BinNode c = bnodes[x];
-            uint32_t k = 0;
-            if (c.left >= 0)
-                while (j > 1 && (k = (choice[x] >> (4 * (j - 1))) & 0xfu) == 0u) --j;
-            if (j <= 1 || c.left < 0 || k == 0u || k >= j || sp + 2 > kWidth || n + sp + 2 > kWidth) {
-                ent[n++] = x;  // one slot (the last tests only guard malformed input)
-                continue;
-            }
-            stN[sp] = c.right;
-            stJ[sp++] = j - k;
-            stN[sp] = c.left;
-            stJ[sp++] = k;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        b[k] = FLT_MAX;
+        b[3 + k] = -FLT_MAX;
+    }
+}
+AG_D void box_add(float b[6], const float lo[3], const float hi[3])
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        b[k] = fminf(b[k], lo[k]);
+        b[3 + k] = fmaxf(b[3 + k], hi[k]);
+    }
+}
+
+// Two children of node nd (nL of its references go left); returns the first's
+// local id. The subtree's nodes are 0 (the root, id rootNode) and 1, 2, ...
+// (ids idBase, idBase + 1, ...).
+AG_D uint32_t sub_children(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t rootNode, uint32_t globalBegin,
+                           uint32_t nd, uint32_t nL, const float L[6], const float R[6])
+{
+    const uint32_t ch = atomicAdd(&s.nodeTop, 2u);
+    const uint32_t b = s.begin[nd], n = s.count[nd];
+    s.left[nd] = (uint16_t)ch;
+    s.begin[ch] = (uint16_t)b;
+    s.count[ch] = (uint16_t)nL;
+    s.left[ch] = (uint16_t)kNoChild;
+    s.area[ch] = area_of(L[0], L[1], L[2], L[3], L[4], L[5]);
+    s.begin[ch + 1] = (uint16_t)(b + nL);
+    s.count[ch + 1] = (uint16_t)(n - nL);
+    s.left[ch + 1] = (uint16_t)kNoChild;
+    s.area[ch + 1] = area_of(R[0], R[1], R[2], R[3], R[4], R[5]);
+    const uint32_t id = s.idBase + ch - 1, parent = nd == 0 ? rootNode : s.idBase + nd - 1;
+    bnodes[parent].left = (int32_t)id;
+    bnodes[parent].right = (int32_t)id + 1;
+    write_node(bnodes, id, L, globalBegin + b, nL);
+    write_node(bnodes, id + 1, R, globalBegin + b + nL, n - nL);
+    return ch;
+}
+
+// Split of a node above kDirectMax references by one warp. cur: the
+// permutation's current buffer; the children's references go to the other.
+AG_D void sub_split_warp(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t rootNode, uint32_t globalBegin, uint32_t nd,
+                         uint32_t* bins, int cur)
+{
+    const uint32_t lane = lane_id(), b = s.begin[nd], n = s.count[nd];
+    float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    for (uint32_t i = lane; i < n; i += 32) {
+        float lo[3], hi[3];
+        sub_box(s, s.perm[cur][b + i], lo, hi);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float c = centroid(lo[k], hi[k]);
+            clo[k] = fminf(clo[k], c);
+            chi[k] = fmaxf(chi[k], c);
         }
-    } else {
-        ent[n++] = root.left;
-        ent[n++] = root.right;
-        // Open children until all 8 slots are used: first those too large for
-        // a leaf slot, then small internal ones (tighter leaf boxes are free
-        // since every slot box is tested anyway).
-        for (int phase = 0; phase < 2; ++phase) {
-            while (n < kWidth) {
-                int pick = -1;
-                float pa = -1.0f;
-                for (int k = 0; k < n; ++k) {
-                    const BinNode& c = bnodes[ent[k]];
-                    if (c.left < 0) continue;
-                    bool large = c.count > (uint32_t)kMaxLeafTris;
-                    if (phase == 0 ? !large : large) continue;
-                    float a = bn_area(c);
-                    if (a > pa) { pa = a; pick = k; }
+    }
+    float sc[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        clo[k] = warp_min(clo[k]);
+        chi[k] = warp_max(chi[k]);
+        sc[k] = axis_scale(clo[k], chi[k]);
+    }
+    __syncwarp();  // the warp's previous node has finished reading the bins
+    for (int k = lane; k < kTaskBinWords; k += 32) bin_init_word(bins + k, k);
+    __syncwarp();
+    for (uint32_t i = lane; i < n; i += 32) {
+        float lo[3], hi[3];
+        sub_box(s, s.perm[cur][b + i], lo, hi);
+        uint32_t ord[6];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            ord[k] = f2ord(lo[k]);
+            ord[3 + k] = f2ord(hi[k]);
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            if (sc[a] != 0.0f)
+                bin_accumulate(bins + a * kAxisBinWords + bin_of(centroid(lo[a], hi[a]), clo[a], sc[a]) * kBinWords, ord);
+    }
+    __syncwarp();
+    SplitChoice best;
+    split_reset(best);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (sc[a] == 0.0f) continue;
+        float v[6];
+        uint32_t c;
+        load_bin(bins + a * kAxisBinWords + lane * kBinWords, v, c);
+        eval_axis(a, v, c, n, best);
+    }
+    const bool median = best.axis < 0;  // all centroids coincide
+    if (median) {
+        best.nL = n / 2;
+        box_reset(best.L);
+        box_reset(best.R);
+        for (uint32_t i = lane; i < n; i += 32) {
+            float lo[3], hi[3];
+            sub_box(s, s.perm[cur][b + i], lo, hi);
+            if (i < best.nL) box_add(best.L, lo, hi);
+            else box_add(best.R, lo, hi);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            best.L[k] = warp_min(best.L[k]);
+            best.L[3 + k] = warp_max(best.L[3 + k]);
+            best.R[k] = warp_min(best.R[k]);
+            best.R[3 + k] = warp_max(best.R[3 + k]);
+        }
+    }
+    uint32_t ch = 0;
+    if (lane == 0) ch = sub_children(s, bnodes, rootNode, globalBegin, nd, best.nL, best.L, best.R);
+    ch = __shfl_sync(0xffffffffu, ch, 0);
+    // stable partition
+    uint32_t leftSeen = 0, rightSeen = 0;
+    for (uint32_t base = 0; base < n; base += 32) {
+        const uint32_t i = base + lane;
+        const bool valid = i < n;
+        uint32_t j = 0;
+        bool left = false;
+        if (valid) {
+            j = s.perm[cur][b + i];
+            if (median) {
+                left = i < best.nL;
+            } else {
+                const int a = best.axis;
+                const float cl = a == 0 ? clo[0] : (a == 1 ? clo[1] : clo[2]);
+                const float ss = a == 0 ? sc[0] : (a == 1 ? sc[1] : sc[2]);
+                left = bin_of(centroid(s.box[a][j], s.box[3 + a][j]), cl, ss) <= best.bin;
+            }
+        }
+        const uint32_t bl = __ballot_sync(0xffffffffu, valid && left);
+        const uint32_t br = __ballot_sync(0xffffffffu, valid && !left);
+        if (valid) {
+            const uint32_t dst = left ? leftSeen + __popc(bl & lanemask_lt()) : best.nL + rightSeen + __popc(br & lanemask_lt());
+            if (dst < n) {
+                s.perm[cur ^ 1][b + dst] = (uint16_t)j;
+                s.posNode[cur ^ 1][b + dst] = (uint16_t)(left ? ch : ch + 1);
+            }
+        }
+        leftSeen += __popc(bl);
+        rightSeen += __popc(br);
+    }
+}
+
+// levels: the binary levels that the big-task kernels ran; big tasks left
+// after them mean that the tree cannot be finished here (kCntFailed).
+__global__ void __launch_bounds__(kSubThreads, 3) k_subtree(const SmallTask* __restrict__ small,
+                                                            const uint32_t* __restrict__ refs0,
+                                                            const uint32_t* __restrict__ refs1,
+                                                            const float4* __restrict__ boxes,
+                                                            BinNode* __restrict__ bnodes, uint32_t* __restrict__ order,
+                                                            float* __restrict__ cost, uint32_t* __restrict__ choice,
+                                                            float triCost, bool sah, uint32_t* __restrict__ cnt,
+                                                            uint32_t levels, uint32_t capPrims)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    SubSmem& s = *reinterpret_cast<SubSmem*>(smem);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    if (cnt[kLevelBig + levels] != 0u) {
+        if (blockIdx.x == 0 && tid == 0) atomicOr(cnt + kCntFailed, kFailLevels);
+        return;
+    }
+    const uint32_t numSmall = cnt[kCntFailed] & kFailCapacity ? 0u : min(cnt[kCntSmall], capPrims);
+    for (;;) {
+        if (tid == 0) s.ticket = atomicAdd(cnt + kCntTicket, 1u);
+        __syncthreads();
+        const uint32_t ticket = s.ticket;
+        if (ticket >= numSmall) break;
+        const SmallTask task = small[ticket];
+        const uint32_t n = min(task.count, kSmallMax), b0 = task.begin;
+        const uint32_t* refs = (task.level & 1u) ? refs1 : refs0;
+        for (uint32_t p = tid; p < n; p += kSubThreads) {
+            const uint32_t prim = refs[b0 + p];
+            float lo[3], hi[3];
+            load_box(boxes, prim, lo, hi);
+            s.prim[p] = prim;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                s.box[k][p] = lo[k];
+                s.box[3 + k][p] = hi[k];
+            }
+            s.perm[0][p] = (uint16_t)p;
+            s.posNode[0][p] = 0;
+        }
+        if (tid == 0) {
+            // ids of the 2 n - 2 nodes below the root (fewer are used when leaves hold several references)
+            s.idBase = n > 1 ? atomicAdd(cnt + kCntNodes, 2u * n - 2u) : 0u;
+            s.nodeTop = 1;
+            s.begin[0] = 0;
+            s.count[0] = (uint16_t)n;
+            s.left[0] = (uint16_t)kNoChild;
+            const BinNode r = bnodes[task.node];
+            s.area[0] = area_of(r.lo.x, r.lo.y, r.lo.z, r.hi.x, r.hi.y, r.hi.z);
+        }
+        __syncthreads();
+        if (s.idBase + 2u * n - 2u > 2u * capPrims) {  // never in a consistent build
+            if (tid == 0) atomicOr(cnt + kCntFailed, kFailCapacity);
+            __syncthreads();
+            continue;
+        }
+        uint32_t ls = 0, le = 1, lev = 0;
+        int cur = 0;
+        while (ls < le) {
+            if (tid == 0) s.levelStart[lev] = (uint16_t)ls;
+            for (uint32_t nd = ls + warp; nd < le; nd += kSubWarps)
+                if (s.count[nd] > kDirectMax) sub_split_warp(s, bnodes, task.node, b0, nd, s.bins[warp], cur);
+            // bins of every reference of the other nodes
+#pragma unroll
+            for (int r = 0; r < kSubRounds; ++r) {
+                const uint32_t p = r * kSubThreads + tid;
+                if (p >= n) break;
+                const uint32_t nd = s.posNode[cur][p], c = s.count[nd], b = s.begin[nd];
+                if (nd < ls || c < 2u || c > kDirectMax) continue;
+                float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, own[3];
+                for (uint32_t i = b; i < b + c; ++i) {
+                    float lo[3], hi[3];
+                    sub_box(s, s.perm[cur][i], lo, hi);
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        const float ck = centroid(lo[k], hi[k]);
+                        clo[k] = fminf(clo[k], ck);
+                        chi[k] = fmaxf(chi[k], ck);
+                        if (i == p) own[k] = ck;
+                    }
                 }
-                if (pick < 0) break;
-                const BinNode& c = bnodes[ent[pick]];
-                ent[pick] = c.left;
-                ent[n++] = c.right;
+                uint32_t v = 0;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float sc = axis_scale(clo[k], chi[k]);
+                    if (sc != 0.0f) v |= ((uint32_t)bin_of(own[k], clo[k], sc) << (8 * k)) | (1u << (24 + k));
+                }
+                s.pbin[p] = v;
+                if (p == b) s.key[nd - ls] = ~0ull;
+            }
+            __syncthreads();
+            // each reference's candidate planes
+#pragma unroll 1
+            for (int r = 0; r < kSubRounds; ++r) {
+                const uint32_t p = r * kSubThreads + tid;
+                if (p >= n) break;
+                const uint32_t nd = s.posNode[cur][p], c = s.count[nd], b = s.begin[nd];
+                if (nd < ls || c < 2u || c > kDirectMax) continue;
+                const uint32_t own = s.pbin[p];
+                float L[3][6], R[3][6];
+                uint32_t nL[3] = {0u, 0u, 0u};
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    box_reset(L[a]);
+                    box_reset(R[a]);
+                }
+                for (uint32_t i = b; i < b + c; ++i) {
+                    const uint32_t v = s.pbin[i];
+                    float lo[3], hi[3];
+                    sub_box(s, s.perm[cur][i], lo, hi);
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        if (((v >> (8 * a)) & 0xffu) <= ((own >> (8 * a)) & 0xffu)) {
+                            box_add(L[a], lo, hi);
+                            ++nL[a];
+                        } else {
+                            box_add(R[a], lo, hi);
+                        }
+                    }
+                }
+                float bestCost = FLT_MAX;
+                int axis = -1;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    if (!(own & (1u << (24 + a))) || nL[a] >= c) continue;
+                    const float sc = split_cost(nL[a], area_of(L[a][0], L[a][1], L[a][2], L[a][3], L[a][4], L[a][5]),
+                                                c - nL[a], area_of(R[a][0], R[a][1], R[a][2], R[a][3], R[a][4], R[a][5]));
+                    if (sc < bestCost) {
+                        bestCost = sc;
+                        axis = a;
+                    }
+                }
+                if (axis >= 0)
+                    atomicMin(&s.key[nd - ls], ((unsigned long long)__float_as_uint(bestCost) << 32) | ((uint32_t)axis << 24) |
+                                                   (((own >> (8 * axis)) & 0xffu) << 16) | p);
+            }
+            __syncthreads();
+            // the winner (or, without a candidate, the first reference) makes the leaf or the children
+#pragma unroll 1
+            for (int r = 0; r < kSubRounds; ++r) {
+                const uint32_t p = r * kSubThreads + tid;
+                if (p >= n) break;
+                const uint32_t nd = s.posNode[cur][p], c = s.count[nd], b = s.begin[nd];
+                if (nd < ls || c < 2u || c > kDirectMax) continue;
+                const unsigned long long key = s.key[nd - ls];
+                const bool found = key != ~0ull;
+                if (p != (found ? (uint32_t)(key & 0xffffu) : b)) continue;
+                // SAH with unit traversal and intersection costs
+                const float area = s.area[nd], splitCost = __uint_as_float((uint32_t)(key >> 32));
+                if (c <= (uint32_t)kMaxLeafTris && (!found || __fmul_rn(float(c), area) <= __fadd_rn(area, splitCost)))
+                    continue;  // a leaf
+                const uint32_t sh = 8u * ((uint32_t)(key >> 24) & 0xffu), bin = (uint32_t)(key >> 16) & 0xffu;
+                float L[6], R[6];
+                uint32_t nL = 0;
+                box_reset(L);
+                box_reset(R);
+                for (uint32_t i = b; i < b + c; ++i) {
+                    float lo[3], hi[3];
+                    sub_box(s, s.perm[cur][i], lo, hi);
+                    if (found ? ((s.pbin[i] >> sh) & 0xffu) <= bin : (i - b) < c / 2u) {
+                        box_add(L, lo, hi);
+                        ++nL;
+                    } else {
+                        box_add(R, lo, hi);
+                    }
+                }
+                sub_children(s, bnodes, task.node, b0, nd, nL, L, R);
+            }
+            __syncthreads();
+            // stable partition of the split nodes' references
+#pragma unroll
+            for (int r = 0; r < kSubRounds; ++r) {
+                const uint32_t p = r * kSubThreads + tid;
+                bool lf = false;
+                if (p < n) {
+                    const uint32_t nd = s.posNode[cur][p], c = s.count[nd];
+                    if (nd >= ls && c <= kDirectMax && s.left[nd] != kNoChild) {
+                        const unsigned long long key = s.key[nd - ls];
+                        lf = key != ~0ull ? ((s.pbin[p] >> (8u * ((uint32_t)(key >> 24) & 0xffu))) & 0xffu) <=
+                                                ((uint32_t)(key >> 16) & 0xffu)
+                                          : p - s.begin[nd] < c / 2u;
+                    }
+                }
+                const uint32_t w = __ballot_sync(0xffffffffu, lf);
+                if (lane_id() == 0) s.leftBits[p >> 5] = w;
+            }
+            if (tid == 0) s.levelEnd = s.nodeTop;
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < kSubRounds; ++r) {
+                const uint32_t p = r * kSubThreads + tid;
+                if (p >= n) break;
+                const uint32_t nd = s.posNode[cur][p], c = s.count[nd], j = s.perm[cur][p];
+                uint32_t dst = p, to = nd;
+                if (nd >= ls && s.left[nd] != kNoChild) {
+                    if (c > kDirectMax) continue;  // its warp has moved it
+                    const uint32_t b = s.begin[nd], w0 = b >> 5, w1 = p >> 5, ch = s.left[nd];
+                    const uint32_t upTo = (1u << (p & 31u)) - 1u, from = 0xffffffffu << (b & 31u);
+                    const uint32_t rank = w0 == w1 ? __popc(s.leftBits[w0] & from & upTo)
+                                                   : __popc(s.leftBits[w0] & from) + __popc(s.leftBits[w1] & upTo);
+                    const bool lf = (s.leftBits[w1] >> (p & 31u)) & 1u;
+                    dst = lf ? b + rank : b + s.count[ch] + (p - b - rank);
+                    to = lf ? ch : ch + 1u;
+                }
+                s.perm[cur ^ 1][dst] = (uint16_t)j;
+                s.posNode[cur ^ 1][dst] = (uint16_t)to;
+            }
+            __syncthreads();
+            ls = le;
+            le = s.levelEnd;
+            cur ^= 1;
+            ++lev;
+        }
+        if (tid == 0) {
+            s.levelStart[lev] = (uint16_t)ls;
+            atomicMax(cnt + kCntLevels, task.level + lev);
+            atomicAdd(cnt + kCntRealNodes, s.nodeTop - 1u);
+        }
+        for (uint32_t p = tid; p < n; p += kSubThreads) order[b0 + p] = s.prim[s.perm[cur][p]];
+        __syncthreads();
+        if (sah) {  // the cost program, deepest level first (the bins' memory now holds the costs)
+            for (uint32_t l = lev; l-- > 0;) {
+                for (uint32_t nd = s.levelStart[l] + tid; nd < s.levelStart[l + 1]; nd += kSubThreads) {
+                    const uint32_t ch = s.left[nd], id = nd == 0 ? task.node : s.idBase + nd - 1;
+                    float C[kCosts];
+                    uint32_t pick = 0;
+                    if (ch == kNoChild) {
+                        const float leaf = leaf_cost(s.area[nd], s.count[nd], triCost);
+#pragma unroll
+                        for (int j = 0; j < kCosts; ++j) C[j] = leaf;
+                    } else {
+                        float side[2][kCosts];
+#pragma unroll
+                        for (uint32_t k = 0; k < 2; ++k) {
+                            const uint32_t x = ch + k, xc = s.left[x];
+                            const float leaf = leaf_cost(s.area[x], s.count[x], triCost);
+#pragma unroll
+                            for (int j = 0; j < kCosts; ++j)
+                                side[k][j] = xc == kNoChild ? leaf : s.cost[((xc - 1u) >> 1) * kCosts + j];
+                        }
+                        pick = collapse_cost(side[0], side[1], s.area[nd], s.count[nd], triCost, C);
+#pragma unroll
+                        for (int j = 0; j < kCosts; ++j) s.cost[((ch - 1u) >> 1) * kCosts + j] = C[j];
+                    }
+                    choice[id] = pick;
+                    if (nd == 0)
+#pragma unroll
+                        for (int j = 0; j < kCosts; ++j) cost[8ull * id + j] = C[j];
+                }
+                __syncthreads();
             }
         }
     }
-    atomicAdd(slotTotal, (uint32_t)n);
-    // Octant slot assignment: slot s prefers the child whose centre lies
-    // toward corner s of the parent box (bit k of s set = + side of axis k).
-    float3 pc = 0.5f * (root.lo + root.hi);
-    float3 cen[kWidth];
-    for (int k = 0; k < n; ++k) {
-        const BinNode& c = bnodes[ent[k]];
-        cen[k] = 0.5f * (c.lo + c.hi) - pc;
-    }
-    int32_t slot[kWidth];
-    for (int s = 0; s < kWidth; ++s) slot[s] = -1;
-    uint32_t usedChild = 0, usedSlot = 0;
-    for (int it = 0; it < n; ++it) {
-        float bestV = -FLT_MAX;
-        int bc = -1, bs = -1;
-        for (int k = 0; k < n; ++k) {
-            if (usedChild & (1u << k)) continue;
-            for (int s = 0; s < kWidth; ++s) {
-                if (usedSlot & (1u << s)) continue;
-                float v = ((s & 1) ? cen[k].x : -cen[k].x) + ((s & 2) ? cen[k].y : -cen[k].y) +
-                          ((s & 4) ? cen[k].z : -cen[k].z);
-                if (v > bestV) { bestV = v; bc = k; bs = s; }
-            }
-        }
-        usedChild |= 1u << bc;
-        usedSlot |= 1u << bs;
-        slot[bs] = ent[bc];
-    }
-    uint32_t ni = 0, nt = 0;
-    for (int s = 0; s < kWidth; ++s) {
-        slots[size_t(i) * kWidth + s] = slot[s];
-        if (slot[s] < 0) continue;
-        uint32_t cnt = bnodes[slot[s]].count;
-        if (cnt <= (uint32_t)kMaxLeafTris) nt += cnt;
-        else ni += 1;
-    }
-    intCount[i] = ni;
-    triCount[i] = nt;
 }
 
-__global__ void k_collapse_decide(const uint2* __restrict__ items, uint32_t numItems, const BinNode* __restrict__ bnodes,
-                                  const uint32_t* __restrict__ choice, int32_t* __restrict__ slots,
-                                  uint32_t* __restrict__ intCount, uint32_t* __restrict__ triCount,
-                                  uint32_t* __restrict__ slotTotal, const uint32_t* __restrict__ dItems)
+AG_D float bn_area(const BinNode& b) { return area_of(b.lo.x, b.lo.y, b.lo.z, b.hi.x, b.hi.y, b.hi.z); }
+
+// One block: the cost program over the big nodes (deepest level first), then
+// the collapse's start. A tree that was not finished, or is deeper than
+// maxLevels, leaves the collapse without items (the previous tree stays in
+// place); status (may be null) then gets kErrBuildDepth.
+constexpr int kTopThreads = 1024;
+__global__ void __launch_bounds__(kTopThreads) k_top(const BinNode* __restrict__ bnodes, float* __restrict__ cost,
+                                                     uint32_t* __restrict__ choice, float triCost, bool sah,
+                                                     uint2* __restrict__ items, uint32_t* __restrict__ cnt,
+                                                     uint32_t levels, uint32_t maxLevels, uint32_t* __restrict__ status)
 {
-    const uint32_t n = level_count(dItems, numItems);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        collapse_decide_item(i, items, bnodes, choice, slots, intCount, triCount, slotTotal);
+    if (cnt[kCntFailed] != 0u || cnt[kCntLevels] > maxLevels) {
+        if (threadIdx.x == 0) {
+            cnt[kCntFailed] |= kFailLevels;
+            if (status) atomicOr(status, kErrBuildDepth);
+        }
+        return;
+    }
+    if (sah)
+        for (uint32_t l = levels; l-- > 0;) {
+            const uint32_t end = cnt[kLevelNodes + l + 1];
+            for (uint32_t x = cnt[kLevelNodes + l] + threadIdx.x; x < end; x += kTopThreads) {
+                const BinNode b = bnodes[x];
+                if (b.count <= kSmallMax) continue;  // done by k_subtree
+                float C[kCosts], L[kCosts], R[kCosts];
+#pragma unroll
+                for (int j = 0; j < kCosts; ++j) {
+                    L[j] = cost[8ull * (uint32_t)b.left + j];
+                    R[j] = cost[8ull * (uint32_t)b.right + j];
+                }
+                choice[x] = collapse_cost(L, R, bn_area(b), b.count, triCost, C);
+#pragma unroll
+                for (int j = 0; j < kCosts; ++j) cost[8ull * x + j] = C[j];
+            }
+            __syncthreads();
+        }
+    if (threadIdx.x == 0) {
+        const float area = bn_area(bnodes[0]);
+        cnt[kCntRootAreaInv] = __float_as_uint(area > 0.0f ? __fdiv_rn(1.0f, area) : 0.0f);
+        items[0] = make_uint2(0u, 0u);
+        cnt[kWideItems] = 1u;
+        cnt[kWideNodeBase] = 1u;
+        cnt[kWideTriBase] = 0u;
+    }
+}
+
+// --------------------------------------------------------------------------
+// Collapse to the wide layout: eight lanes per wide node.
+constexpr int kWideThreads = 256;
+constexpr uint32_t kWideItemsPerBlock = kWideThreads / 8;
+
+// The slots of one wide node per group of eight lanes: lane g of a group
+// stands for the g-th of the node's entries, left to right. choice (the cost
+// program's decisions) selects the SAH-optimal distribution; null selects the
+// greedy rule. The entries are then assigned to octants, and the block's
+// counts kept for k_wide_emit's prefix sums.
+__global__ void __launch_bounds__(kWideThreads) k_wide_decide(const uint2* __restrict__ items,
+                                                              const BinNode* __restrict__ bnodes,
+                                                              const uint32_t* __restrict__ choice,
+                                                              int32_t* __restrict__ slots, uint2* __restrict__ itemOff,
+                                                              uint2* __restrict__ blockSum, uint32_t* __restrict__ cnt,
+                                                              uint32_t level, uint32_t capItems)
+{
+    __shared__ uint32_t sInt[kWideItemsPerBlock], sTri[kWideItemsPerBlock], sSlots[kWideItemsPerBlock];
+    const uint32_t n = min(cnt[kWideItems + level], capItems);
+    const uint32_t g = threadIdx.x & 7u, gshift = lane_id() & 24u;
+    constexpr uint32_t kAll = 0xffffffffu;
+    for (uint32_t blk = blockIdx.x; blk * kWideItemsPerBlock < n; blk += gridDim.x) {
+        const uint32_t local = threadIdx.x >> 3, i = blk * kWideItemsPerBlock + local;
+        const bool valid = i < n;
+        const uint32_t node = valid ? items[i].x : 0u;
+        const BinNode root = bnodes[node];
+        const bool single = root.count <= (uint32_t)kMaxLeafTris || root.left < 0;  // a tree of one leaf
+        int32_t ent = -1;
+        uint32_t count = 0;
+        int32_t entLeft = -1, entRight = -1;
+        auto load_entry = [&]() {
+            const BinNode* b = bnodes + ent;
+            const int2 lr = *reinterpret_cast<const int2*>(&b->left);
+            entLeft = lr.x;
+            entRight = lr.y;
+            count = b->count;
+        };
+        if (valid && single && g == 0) ent = (int32_t)node;
+        if (choice) {
+            // an entry owns j consecutive lanes from its own; splitting it hands the last j - k to the right child
+            uint32_t j = 1;
+            if (valid && !single) {
+                const uint32_t k8 = min(max(choice[node] >> 28, 1u), 7u);  // 1..7 by construction
+                if (g == 0) { ent = root.left; j = k8; }
+                if (g == k8) { ent = root.right; j = 8u - k8; }
+            }
+            bool open = ent >= 0 && j > 1u;
+            while (__any_sync(kAll, open)) {
+                int32_t give = -1;
+                uint32_t giveSlots = 0, target = 8u;
+                if (open) {
+                    load_entry();
+                    const uint32_t ch = choice[ent];
+                    uint32_t k = 0;
+                    if (entLeft >= 0)
+                        while (j > 1u && (k = (ch >> (4 * (j - 1))) & 0xfu) == 0u) --j;
+                    if (entLeft < 0 || j <= 1u || k == 0u || k >= j) {
+                        open = false;
+                    } else {
+                        give = entRight;
+                        giveSlots = j - k;
+                        target = g + k;
+                        ent = entLeft;
+                        j = k;
+                        open = j > 1u;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const uint32_t t = __shfl_sync(kAll, target, q, 8), gs = __shfl_sync(kAll, giveSlots, q, 8);
+                    const int32_t e = __shfl_sync(kAll, give, q, 8);
+                    if (t == g) {
+                        ent = e;
+                        j = gs;
+                        open = j > 1u;
+                    }
+                }
+            }
+        } else {
+            // Open children until all 8 slots are used: first those too large for
+            // a leaf slot, then small internal ones (tighter leaf boxes are free
+            // since every slot box is tested anyway).
+            uint32_t used = valid && !single ? 2u : 8u;
+            float area = -1.0f;
+            auto load_full = [&]() {
+                load_entry();
+                const float a = bn_area(bnodes[ent]);
+                area = entLeft >= 0 && a >= 0.0f ? a : -1.0f;
+            };
+            if (valid && !single && g < 2) {
+                ent = g ? root.right : root.left;
+                load_full();
+            }
+            for (int phase = 0; phase < 2; ++phase) {
+                bool active = used < 8u;
+                while (__any_sync(kAll, active)) {
+                    const bool large = count > (uint32_t)kMaxLeafTris;
+                    float a = active && ent >= 0 && (phase == 0 ? large : !large) ? area : -1.0f;
+                    uint32_t bl = g;
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) {
+                        const float oa = __shfl_xor_sync(kAll, a, o, 8);
+                        const uint32_t ol = __shfl_xor_sync(kAll, bl, o, 8);
+                        if (oa > a || (oa == a && ol < bl)) { a = oa; bl = ol; }
+                    }
+                    const int32_t r = __shfl_sync(kAll, entRight, bl, 8);
+                    if (!(a >= 0.0f)) active = false;
+                    if (active) {
+                        if (g == bl) { ent = entLeft; load_full(); }
+                        if (g == used) { ent = r; load_full(); }
+                        active = ++used < 8u;
+                    }
+                }
+            }
+        }
+        // Octant slot assignment: slot s prefers the child whose centre lies
+        // toward corner s of the parent box (bit k of s set = + side of axis k).
+        float v[kWidth];
+        {
+            float3 cen = mk3(0.0f, 0.0f, 0.0f);
+            if (ent >= 0) {
+                const BinNode c = bnodes[ent];
+                count = c.count;
+                cen = 0.5f * (c.lo + c.hi) - 0.5f * (root.lo + root.hi);
+            }
+#pragma unroll
+            for (int s = 0; s < kWidth; ++s)
+                v[s] = ((s & 1) ? cen.x : -cen.x) + ((s & 2) ? cen.y : -cen.y) + ((s & 4) ? cen.z : -cen.z);
+        }
+        uint32_t mySlot = 8u, usedSlots = 0;
+        bool open = ent >= 0;
+        while (__any_sync(kAll, open)) {
+            float bv = -FLT_MAX;
+            uint32_t bs = 8u;
+#pragma unroll
+            for (uint32_t s = 0; s < kWidth; ++s) {
+                if (usedSlots & (1u << s)) continue;
+                if (bs == 8u) bs = s;  // a free slot even when the centre is not a number
+                if (v[s] > bv) { bv = v[s]; bs = s; }
+            }
+            // the group's largest value, the first entry on ties
+            uint32_t pick = open ? (g << 4) | bs : 0xffu;
+            if (!open) bv = -INFINITY;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const float ov = __shfl_xor_sync(kAll, bv, o, 8);
+                const uint32_t op = __shfl_xor_sync(kAll, pick, o, 8);
+                if (ov > bv || (ov == bv && op < pick)) { bv = ov; pick = op; }
+            }
+            if (pick != 0xffu) {
+                usedSlots |= 1u << (pick & 0xfu);
+                if (pick >> 4 == g) {
+                    mySlot = pick & 0xfu;
+                    open = false;
+                }
+            }
+        }
+        // from entries (by lane) to slots (by lane)
+        int32_t slot = -1;
+        uint32_t slotCount = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t sq = __shfl_sync(kAll, mySlot, q, 8), cq = __shfl_sync(kAll, count, q, 8);
+            const int32_t e = __shfl_sync(kAll, ent, q, 8);
+            if (sq == g) {
+                slot = e;
+                slotCount = cq;
+            }
+        }
+        if (valid) slots[size_t(i) * kWidth + g] = slot;
+        const bool leaf = slot >= 0 && slotCount <= (uint32_t)kMaxLeafTris;
+        const uint32_t ni = __popc((__ballot_sync(kAll, slot >= 0 && !leaf) >> gshift) & 0xffu);
+        const uint32_t ns = __popc((__ballot_sync(kAll, slot >= 0) >> gshift) & 0xffu);
+        uint32_t nt = leaf ? slotCount : 0u;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) nt += __shfl_xor_sync(kAll, nt, o, 8);
+        if (g == 0) {
+            sInt[local] = ni;
+            sTri[local] = nt;
+            sSlots[local] = ns;
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const uint32_t a = sInt[threadIdx.x], t = sTri[threadIdx.x], sl = sSlots[threadIdx.x];
+            const uint32_t ia = scan_add(a), it = scan_add(t), is = scan_add(sl);
+            const uint32_t item = blk * kWideItemsPerBlock + threadIdx.x;
+            if (item < n) itemOff[item] = make_uint2(ia - a, it - t);
+            if (threadIdx.x == 31) {
+                blockSum[blk] = make_uint2(ia, it);
+                if (ia) atomicAdd(cnt + kWideItems + level + 1, ia);
+                if (it) atomicAdd(cnt + kWideTris + level, it);
+                atomicAdd(cnt + kCntSlots, is);
+            }
+        }
+        __syncthreads();  // the sums are written again for the next block of items
+    }
 }
 
 __host__ __device__ inline uint32_t quant_exponent(float extent)
@@ -1030,204 +1430,171 @@ __host__ __device__ inline uint32_t quant_exponent(float extent)
     return (uint32_t)biased;
 }
 
-AG_D void collapse_emit_item(uint32_t i, const uint2* __restrict__ items, const BinNode* __restrict__ bnodes,
-                             const int32_t* __restrict__ slots, const uint32_t* __restrict__ intOff,
-                             const uint32_t* __restrict__ triOff, uint32_t wideBase, uint32_t triBase0,
-                             const uint32_t* __restrict__ order, const float* __restrict__ verts,
-                             const uint32_t* __restrict__ idx, uint32_t ntris, const float4* __restrict__ spheres,
-                             WideNode* __restrict__ nodes, TriRecord* __restrict__ tris, uint2* __restrict__ itemsNext,
-                             float* sahAccum, float rootAreaInv, uint32_t nodeCap, uint32_t triCap,
-                             uint32_t* __restrict__ status)
+// Writes one wide node per group of eight lanes, a lane per slot, with its
+// triangle records and the next level's items. The places of a block's items
+// follow from the sums of the blocks before it, so the layout is breadth
+// first and does not depend on scheduling.
+__global__ void __launch_bounds__(kWideThreads) k_wide_emit(const uint2* __restrict__ items,
+                                                            const BinNode* __restrict__ bnodes,
+                                                            const int32_t* __restrict__ slots,
+                                                            const uint2* __restrict__ itemOff,
+                                                            const uint2* __restrict__ blockSum,
+                                                            const uint32_t* __restrict__ order,
+                                                            const float* __restrict__ verts,
+                                                            const uint32_t* __restrict__ idx, uint32_t ntris,
+                                                            const float4* __restrict__ spheres,
+                                                            WideNode* __restrict__ nodes, TriRecord* __restrict__ tris,
+                                                            uint2* __restrict__ itemsNext, uint32_t* __restrict__ cnt,
+                                                            uint32_t level, uint32_t nodeCap, uint32_t triCap,
+                                                            uint32_t* __restrict__ status)
 {
-    uint2 it = items[i];
-    const BinNode nb = bnodes[it.x];
-    WideNode w;
-    w.px = nb.lo.x;
-    w.py = nb.lo.y;
-    w.pz = nb.lo.z;
-    uint32_t E[3] = {quant_exponent(nb.hi.x - nb.lo.x), quant_exponent(nb.hi.y - nb.lo.y),
-                     quant_exponent(nb.hi.z - nb.lo.z)};
-    float q[3], invq[3];
-    for (int k = 0; k < 3; ++k) {
-        q[k] = __uint_as_float(E[k] << 23);
-        invq[k] = __uint_as_float((254u - E[k]) << 23);  // exact 1/q
+    __shared__ __align__(16) uint8_t rec[kWideItemsPerBlock][sizeof(WideNode)];
+    __shared__ uint32_t sums[2][kWideThreads / 32];
+    __shared__ float sahSums[kWideThreads / 32];
+    constexpr uint32_t kAll = 0xffffffffu;
+    const uint32_t n = min(cnt[kWideItems + level], nodeCap);
+    if (n == 0) return;
+    const uint32_t nodeBase = cnt[kWideNodeBase + level], triBase0 = cnt[kWideTriBase + level];
+    const float ria = __uint_as_float(cnt[kCntRootAreaInv]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        cnt[kWideNodeBase + level + 1] = nodeBase + cnt[kWideItems + level + 1];
+        cnt[kWideTriBase + level + 1] = triBase0 + cnt[kWideTris + level];
     }
-    float p[3] = {w.px, w.py, w.pz};
-    uint32_t imask = 0;
-    uint32_t childBase = wideBase + intOff[i];
-    uint32_t triBase = triBase0 + triOff[i];
-    uint8_t meta[8], qlo[3][8], qhi[3][8];
-    uint32_t rank = 0, toff = 0;
-    float sah = bn_area(nb) * rootAreaInv;  // one node visit
-    for (int s = 0; s < kWidth; ++s) {
-        int32_t e = slots[size_t(i) * kWidth + s];
-        if (e < 0) {
-            meta[s] = 0;
-            for (int k = 0; k < 3; ++k) { qlo[k][s] = 0xff; qhi[k][s] = 0; }
-            continue;
+    const uint32_t g = threadIdx.x & 7u, gshift = lane_id() & 24u, local = threadIdx.x >> 3, warp = threadIdx.x >> 5;
+    uint32_t summed = 0;               // blocks of items whose sums are in the two bases
+    uint32_t intBase = 0, triBase = 0;
+    float sah = 0.0f;
+    for (uint32_t blk = blockIdx.x; blk * kWideItemsPerBlock < n; blk += gridDim.x) {
+        uint32_t a = 0, t = 0;
+        for (uint32_t b = summed + threadIdx.x; b < blk; b += kWideThreads) {
+            const uint2 v = blockSum[b];
+            a += v.x;
+            t += v.y;
         }
-        const BinNode c = bnodes[e];
-        float clo[3] = {c.lo.x, c.lo.y, c.lo.z}, chi[3] = {c.hi.x, c.hi.y, c.hi.z};
+        a = __reduce_add_sync(kAll, a);
+        t = __reduce_add_sync(kAll, t);
+        if (lane_id() == 0) { sums[0][warp] = a; sums[1][warp] = t; }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kWideThreads / 32; ++w) {
+            intBase += sums[0][w];
+            triBase += sums[1][w];
+        }
+        summed = blk;
+        __syncthreads();  // sums are written again
+        const uint32_t i = blk * kWideItemsPerBlock + local;
+        const bool valid = i < n;
+        const uint2 it = valid ? items[i] : make_uint2(0u, 0u);
+        const uint2 off = valid ? itemOff[i] : make_uint2(0u, 0u);
+        const int32_t e = valid ? slots[size_t(i) * kWidth + g] : -1;
+        const BinNode nb = bnodes[it.x];
+        const float p[3] = {nb.lo.x, nb.lo.y, nb.lo.z};
+        const uint32_t E[3] = {quant_exponent(nb.hi.x - nb.lo.x), quant_exponent(nb.hi.y - nb.lo.y),
+                               quant_exponent(nb.hi.z - nb.lo.z)};
+        BinNode c = nb;
+        if (e >= 0) c = bnodes[e];
+        const bool leaf = e >= 0 && c.count <= (uint32_t)kMaxLeafTris, inner = e >= 0 && !leaf;
+        const uint32_t imask = (__ballot_sync(kAll, inner) >> gshift) & 0xffu;
+        const uint32_t rank = __popc(imask & ((1u << g) - 1u));
+        uint32_t toff = leaf ? c.count : 0u;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kAll, toff, o, 8);
+            if (g >= (uint32_t)o) toff += y;
+        }
+        if (leaf) toff -= c.count;  // triangles of the slots before this one
+        const uint32_t childBase = nodeBase + intBase + off.x, triAt = triBase0 + triBase + off.y;
+        uint8_t* r = rec[local];
+        uint8_t meta = 0;
+        if (leaf) meta = (uint8_t)((((1u << c.count) - 1u) << 5) | toff);
+        if (inner) meta = (uint8_t)(0x20u | (24u + g));
+        r[24 + g] = meta;
+        const float clo[3] = {c.lo.x, c.lo.y, c.lo.z}, chi[3] = {c.hi.x, c.hi.y, c.hi.z};
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
-            float fl = floorf((clo[k] - p[k]) * invq[k]);
-            float fh = ceilf((chi[k] - p[k]) * invq[k]);
+            const float q = __uint_as_float(E[k] << 23), invq = __uint_as_float((254u - E[k]) << 23);  // exact 1/q
+            const float fl = floorf((clo[k] - p[k]) * invq), fh = ceilf((chi[k] - p[k]) * invq);
             int l = (int)fmaxf(0.0f, fminf(255.0f, fl));
             int h = (int)fmaxf(0.0f, fminf(255.0f, fh));
-            while (l > 0 && p[k] + float(l) * q[k] > clo[k]) --l;
-            while (h < 255 && p[k] + float(h) * q[k] < chi[k]) ++h;
-            qlo[k][s] = (uint8_t)l;
-            qhi[k][s] = (uint8_t)h;
+            while (l > 0 && p[k] + float(l) * q > clo[k]) --l;
+            while (h < 255 && p[k] + float(h) * q < chi[k]) ++h;
+            r[32 + 8 * k + g] = e >= 0 ? (uint8_t)l : 0xffu;
+            r[56 + 8 * k + g] = e >= 0 ? (uint8_t)h : 0u;
         }
-        if (c.count <= (uint32_t)kMaxLeafTris) {
-            meta[s] = (uint8_t)((((1u << c.count) - 1u) << 5) | toff);
+        if (g == 0) {
+            float* f = reinterpret_cast<float*>(r);
+            uint32_t* u = reinterpret_cast<uint32_t*>(r);
+            f[0] = p[0];
+            f[1] = p[1];
+            f[2] = p[2];
+            u[3] = E[0] | (E[1] << 8) | (E[2] << 16) | (imask << 24);
+            u[4] = childBase;
+            u[5] = triAt;
+            if (valid) sah += bn_area(nb) * ria;  // one node visit
+        }
+        __syncwarp();
+        if (valid && g < sizeof(WideNode) / 16) {
+            if (it.y < nodeCap)
+                reinterpret_cast<uint4*>(nodes + it.y)[g] = reinterpret_cast<const uint4*>(r)[g];
+            else
+                atomicOr(status, kErrBadIndex);
+        }
+        __syncwarp();
+        if (inner) {
+            const uint32_t at = intBase + off.x + rank;
+            if (at < nodeCap) itemsNext[at] = make_uint2((uint32_t)e, childBase + rank);
+            else atomicOr(status, kErrBadIndex);
+        }
+        if (leaf) {
+            sah += bn_area(c) * ria * float(c.count);
             for (uint32_t k = 0; k < c.count; ++k) {
-                uint32_t prim = order[c.begin + k];
+                const uint32_t prim = order[c.begin + k], at = triAt + toff + k;
+                TriRecord tr;
                 if (prim >= ntris) {  // a sphere record
                     const float4 sp = spheres[prim - ntris];
-                    TriRecord r;
-                    r.v0 = make_float4(sp.x, sp.y, sp.z, __uint_as_float(kSpherePrim | (prim - ntris)));
-                    r.e0 = make_float4(fabsf(sp.w), 0.0f, 0.0f, __uint_as_float(kSphereTag));
-                    r.e1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (triBase + toff + k < triCap) tris[triBase + toff + k] = r;
-                    else atomicOr(status, kErrBadIndex);
-                    continue;
+                    tr.v0 = make_float4(sp.x, sp.y, sp.z, __uint_as_float(kSpherePrim | (prim - ntris)));
+                    tr.e0 = make_float4(fabsf(sp.w), 0.0f, 0.0f, __uint_as_float(kSphereTag));
+                    tr.e1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                } else {
+                    const uint32_t* ti = idx + 3ull * prim;
+                    float v0[3], v1[3], v2[3];
+#pragma unroll
+                    for (int x = 0; x < 3; ++x) {
+                        v0[x] = verts[3ull * ti[0] + x];
+                        v1[x] = verts[3ull * ti[1] + x];
+                        v2[x] = verts[3ull * ti[2] + x];
+                    }
+                    tr.v0 = make_float4(v0[0], v0[1], v0[2], __uint_as_float(prim));
+                    tr.e0 = make_float4(__fsub_rn(v1[0], v0[0]), __fsub_rn(v1[1], v0[1]), __fsub_rn(v1[2], v0[2]), 0.0f);
+                    tr.e1 = make_float4(__fsub_rn(v2[0], v0[0]), __fsub_rn(v2[1], v0[1]), __fsub_rn(v2[2], v0[2]), 0.0f);
                 }
-                const uint32_t* ti = idx + 3ull * prim;
-                float v0[3], v1[3], v2[3];
-                for (int a = 0; a < 3; ++a) {
-                    v0[a] = verts[3ull * ti[0] + a];
-                    v1[a] = verts[3ull * ti[1] + a];
-                    v2[a] = verts[3ull * ti[2] + a];
-                }
-                TriRecord r;
-                r.v0 = make_float4(v0[0], v0[1], v0[2], __uint_as_float(prim));
-                r.e0 = make_float4(__fsub_rn(v1[0], v0[0]), __fsub_rn(v1[1], v0[1]), __fsub_rn(v1[2], v0[2]), 0.0f);
-                r.e1 = make_float4(__fsub_rn(v2[0], v0[0]), __fsub_rn(v2[1], v0[1]), __fsub_rn(v2[2], v0[2]), 0.0f);
-                if (triBase + toff + k < triCap) tris[triBase + toff + k] = r;
+                if (at < triCap) tris[at] = tr;
                 else atomicOr(status, kErrBadIndex);
             }
-            toff += c.count;
-            sah += bn_area(c) * rootAreaInv * float(c.count);
-        } else {
-            meta[s] = (uint8_t)(0x20u | (24u + s));
-            imask |= 1u << s;
-            itemsNext[intOff[i] + rank] = make_uint2((uint32_t)e, childBase + rank);
-            ++rank;
         }
     }
-    w.e_imask = E[0] | (E[1] << 8) | (E[2] << 16) | (imask << 24);
-    w.childBase = childBase;
-    w.triBase = triBase;
-    w.meta[0] = meta[0] | (meta[1] << 8) | (meta[2] << 16) | ((uint32_t)meta[3] << 24);
-    w.meta[1] = meta[4] | (meta[5] << 8) | (meta[6] << 16) | ((uint32_t)meta[7] << 24);
-    for (int k = 0; k < 3; ++k) {
-        w.qlo[k][0] = qlo[k][0] | (qlo[k][1] << 8) | (qlo[k][2] << 16) | ((uint32_t)qlo[k][3] << 24);
-        w.qlo[k][1] = qlo[k][4] | (qlo[k][5] << 8) | (qlo[k][6] << 16) | ((uint32_t)qlo[k][7] << 24);
-        w.qhi[k][0] = qhi[k][0] | (qhi[k][1] << 8) | (qhi[k][2] << 16) | ((uint32_t)qhi[k][3] << 24);
-        w.qhi[k][1] = qhi[k][4] | (qhi[k][5] << 8) | (qhi[k][6] << 16) | ((uint32_t)qhi[k][7] << 24);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sah += __shfl_xor_sync(kAll, sah, o);
+    if (lane_id() == 0) sahSums[warp] = sah;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float s = 0.0f;
+        for (int w = 0; w < kWideThreads / 32; ++w) s += sahSums[w];
+        if (s != 0.0f) atomicAdd(reinterpret_cast<float*>(cnt + kCntSah), s);
     }
-    if (it.y < nodeCap) nodes[it.y] = w;
-    else atomicOr(status, kErrBadIndex);
-    atomicAdd(sahAccum, sah);
 }
 
-// One collapse level: the counts and bases are the host's, or, in a
-// device-driven build, counter words (dDev != null: items, wide nodes and
-// triangle records so far, and the root's inverse area).
-__global__ void k_collapse_emit(const uint2* __restrict__ items, uint32_t numItems, const BinNode* __restrict__ bnodes,
-                                const int32_t* __restrict__ slots, const uint32_t* __restrict__ intOff,
-                                const uint32_t* __restrict__ triOff, uint32_t wideBase, uint32_t triBase0,
-                                const uint32_t* __restrict__ order, const float* __restrict__ verts,
-                                const uint32_t* __restrict__ idx, uint32_t ntris, const float4* __restrict__ spheres,
-                                WideNode* __restrict__ nodes,
-                                TriRecord* __restrict__ tris, uint2* __restrict__ itemsNext, float* sahAccum,
-                                float rootAreaInv, uint32_t nodeCap, uint32_t triCap, uint32_t* __restrict__ status,
-                                const uint32_t* __restrict__ dDev)
+// End of a device-driven build: a tree that needed more collapse levels than
+// were enqueued, or is deeper than the traversal stack, is reported.
+__global__ void k_end(const uint32_t* __restrict__ cnt, uint32_t n, uint32_t wideLevels, uint32_t* __restrict__ status)
 {
-    const uint32_t n = dDev ? dDev[kDevItems] : numItems;
-    const uint32_t wb = dDev ? dDev[kDevWide] : wideBase;
-    const uint32_t tb = dDev ? dDev[kDevTris] : triBase0;
-    const float ria = dDev ? __uint_as_float(dDev[kDevRootAreaInv]) : rootAreaInv;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        collapse_emit_item(i, items, bnodes, slots, intOff, triOff, wb, tb, order, verts, idx, ntris, spheres, nodes,
-                           tris, itemsNext, sahAccum, ria, nodeCap, triCap, status);
-}
-
-// --------------------------------------------------------------------------
-// Device-driven build: the host loop's bookkeeping as single-thread kernels.
-__global__ void k_dev_begin(uint32_t n, uint32_t* __restrict__ dv, uint32_t* __restrict__ levelStart)
-{
-    const uint32_t big = n > kSmallMax ? 1u : 0u;
-    dv[kDevTasks] = 1u;
-    dv[kDevBig] = big;
-    dv[kDevChunks] = big ? (n + kChunk - 1) / kChunk : 0u;
-    dv[kDevNodes] = 1u;
-    dv[kDevLevels] = 0u;
-    dv[kDevFailed] = 0u;
-    levelStart[0] = 0u;
-}
-
-// After binary level L: the next level's counts (the scans' totals) become
-// current, the next level's nodes start at the node count so far. Counts
-// beyond the buffers' capacities (impossible for a consistent build) stop
-// the build with an error instead of reaching past the buffers.
-__global__ void k_dev_level_end(uint32_t* __restrict__ dv, uint32_t* __restrict__ levelStart, uint32_t L,
-                                uint32_t capTasks, uint32_t capBig, uint32_t capChunks, uint32_t* __restrict__ status)
-{
-    if (dv[kDevTasks] > 0u) dv[kDevLevels] += 1u;
-    levelStart[L + 1] = dv[kDevNodes];
-    uint32_t t = dv[kCntTasks], b = dv[kCntBig], c = dv[kCntChunks];
-    if (t > capTasks || b > capBig || c > capChunks || dv[kDevNodes] + t > 2u * capTasks) {
-        atomicOr(status, kErrBadIndex);
-        dv[kDevFailed] = 1u;
+    if (cnt[kCntFailed] != 0u) return;  // reported by k_top
+    uint32_t depth = 0, tris = 0;
+    for (uint32_t l = 0; l < wideLevels; ++l) {
+        if (cnt[kWideItems + l] != 0u) ++depth;
+        tris += cnt[kWideTris + l];
     }
-    if (dv[kDevFailed]) t = b = c = 0u;  // the build stops; the collapse is skipped
-    dv[kDevNodes] += t;
-    dv[kDevTasks] = t;
-    dv[kDevBig] = b;
-    dv[kDevChunks] = c;
-}
-
-// Before the collapse: the root item, the counters, the root's inverse area
-// (in the host build's order of rounded operations). Tasks left over mean
-// the level cap was too small: the collapse is then skipped (the previous
-// tree stays in place) and the status word says so.
-__global__ void k_dev_collapse_begin(uint32_t* __restrict__ dv, const BinNode* __restrict__ bnodes,
-                                     uint2* __restrict__ items, float* __restrict__ sahAccum,
-                                     uint32_t* __restrict__ status)
-{
-    const bool failed = dv[kDevTasks] != 0u || dv[kDevFailed] != 0u;
-    if (failed) atomicOr(status, kErrBuildDepth);
-    items[0] = make_uint2(0u, 0u);
-    dv[kDevItems] = failed ? 0u : 1u;
-    dv[kDevWide] = 1u;
-    dv[kDevTris] = 0u;
-    dv[kDevDepth] = 0u;
-    dv[kCntSlots] = 0u;
-    *sahAccum = 0.0f;
-    const BinNode rb = bnodes[0];
-    const float ex = __fsub_rn(rb.hi.x, rb.lo.x), ey = __fsub_rn(rb.hi.y, rb.lo.y), ez = __fsub_rn(rb.hi.z, rb.lo.z);
-    const float area = __fadd_rn(__fadd_rn(__fmul_rn(ex, ey), __fmul_rn(ey, ez)), __fmul_rn(ez, ex));
-    dv[kDevRootAreaInv] = __float_as_uint(area > 0.0f ? __fdiv_rn(1.0f, area) : 0.0f);
-}
-
-__global__ void k_dev_wide_end(uint32_t* __restrict__ dv, uint32_t capItems, uint32_t* __restrict__ status)
-{
-    if (dv[kDevItems] > 0u) dv[kDevDepth] += 1u;
-    uint32_t items = dv[kCntInt];
-    if (items > capItems || dv[kDevWide] + items > capItems) {
-        atomicOr(status, kErrBadIndex);
-        items = 0u;
-    }
-    dv[kDevItems] = items;
-    dv[kDevWide] += items;
-    dv[kDevTris] += dv[kCntTri];
-}
-
-__global__ void k_dev_end(const uint32_t* __restrict__ dv, uint32_t n, uint32_t* __restrict__ status)
-{
-    const bool skipped = dv[kDevWide] == 1u && dv[kDevTris] == 0u && dv[kDevDepth] == 0u;
-    if (dv[kDevItems] != 0u || dv[kDevDepth] > (uint32_t)kTraversalStack || (!skipped && dv[kDevTris] != n))
+    if (cnt[kWideItems + wideLevels] != 0u || depth > (uint32_t)kTraversalStack || tris != n)
         atomicOr(status, kErrBuildDepth);
 }
 
@@ -1245,7 +1612,25 @@ size_t carve_bytes(size_t count)
     return (count * sizeof(T) + 255) & ~size_t(255);
 }
 
-inline unsigned blocks_for(size_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
+inline unsigned blocks_for(size_t n, int threads, size_t cap = 0x7fffffff)
+{
+    const size_t b = (n + threads - 1) / threads;
+    return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
+}
+
+// Capacities of the big-task lists: at most N / (kSmallMax + 1) tasks on a
+// level, and one partial chunk for each.
+inline size_t max_big(size_t N) { return N / kSmallMax + 2; }
+inline size_t max_chunks(size_t N) { return N / kChunk + max_big(N) + 2; }
+
+// Collapse levels enqueued before the depth is known: log8 of the primitives,
+// doubled for uneven trees. A level without items costs two empty launches.
+inline uint32_t expected_levels(uint32_t n, uint32_t per)
+{
+    uint32_t bits = 0;
+    while (bits < 31 && (n >> bits) > per) ++bits;
+    return bits;
+}
 
 }  // namespace
 
@@ -1264,82 +1649,50 @@ void Builder::release()
     hostCounters_ = nullptr;
     ev0_ = ev1_ = nullptr;
     cap_ = 0;
+    bigLevels_ = wideLevels_ = 0;
 }
 
 int Builder::reserve(uint32_t n, char* err, size_t errLen)
 {
     if (n <= cap_ && mem_) return 0;
     release();
-    size_t N = n ? n : 1;
-    size_t maxBig = N / kSmallMax + 2;
-    size_t maxChunks = N / kChunk + maxBig + 2;
-    size_t bytes = 0;
-    bytes += 2 * carve_bytes<float4>(N);           // primLo, primHi
-    bytes += 3 * carve_bytes<uint32_t>(N);         // refs x2, order
-    bytes += carve_bytes<BinNode>(2 * N);          // bnodes
-    bytes += 2 * carve_bytes<Task>(N);             // tasks x2
-    bytes += carve_bytes<Cand>(2 * N);             // cands
-    bytes += 4 * carve_bytes<uint32_t>(2 * N);     // candFlag, candPos, bigFlag, bigPos
-    bytes += 2 * carve_bytes<uint32_t>(2 * N);     // chunk counts (sparse) + offsets
-    bytes += carve_bytes<uint32_t>(maxBig);        // bigList
-    bytes += carve_bytes<uint32_t>(maxBig);        // chunkOff
-    bytes += 3 * carve_bytes<uint32_t>(maxChunks); // chunkTask, chunkLeft, chunkLeftOff
-    bytes += carve_bytes<uint32_t>(maxBig * kTaskBinWords);
-    bytes += carve_bytes<BigSplit>(maxBig);
-    bytes += 2 * carve_bytes<uint2>(N + 1);        // items x2
-    bytes += carve_bytes<int32_t>((N + 1) * kWidth);
-    bytes += carve_bytes<float>(2 * N * 8);        // collapse costs
-    bytes += carve_bytes<uint32_t>(2 * N);         // collapse choices
-    bytes += 4 * carve_bytes<uint32_t>(N + 1);     // intCount, intOff, triCount, triOff
-    bytes += carve_bytes<uint32_t>(kCntWords);
-    const size_t scanWords = std::max(scan_scratch_words(2 * N + 2), scan3_scratch_words(2 * N + 2));
-    bytes += carve_bytes<uint32_t>(scanWords);
-    bytes += carve_bytes<float>(1);
-    bytes += carve_bytes<uint32_t>(kMaxLevels + 2);  // level starts of a device-driven build
-    if (cudaMalloc(&mem_, bytes) != cudaSuccess) {
-        snprintf(err, errLen, "BVH build: cudaMalloc of %zu bytes failed", bytes);
-        mem_ = nullptr;
-        cudaGetLastError();
-        return -5;
+    const size_t N = n ? n : 1;
+    const size_t maxBig = max_big(N), maxChunks = max_chunks(N);
+    char* p = nullptr;
+    // the same carving twice: sizes from a null base, then the pointers
+    for (int pass = 0; pass < 2; ++pass) {
+        boxes_ = carve<float4>(p, 2 * N);
+        for (int k = 0; k < 2; ++k) {
+            refs_[k] = carve<uint32_t>(p, N);
+            tasks_[k] = carve<BigTask>(p, maxBig);
+            chunkTask_[k] = carve<uint32_t>(p, maxChunks);
+            bins_[k] = carve<uint32_t>(p, maxBig * kTaskBinWords);
+            items_[k] = reinterpret_cast<uint32_t*>(carve<uint2>(p, N + 1));
+        }
+        order_ = carve<uint32_t>(p, N);
+        bnodes_ = carve<BinNode>(p, 2 * N);
+        small_ = carve<SmallTask>(p, N);
+        chunkCnt_ = carve<uint16_t>(p, maxChunks * kChunkCounts);
+        chunkLeft_ = carve<uint32_t>(p, maxChunks);
+        splits_ = carve<BigSplit>(p, maxBig);
+        slots_ = carve<int32_t>(p, (N + 1) * kWidth);
+        itemOff_ = carve<uint2>(p, N + 1);
+        blockSum_ = carve<uint2>(p, (N + 1) / kWideItemsPerBlock + 1);
+        collapseCost_ = carve<float>(p, 2 * N * 8);
+        collapseChoice_ = carve<uint32_t>(p, 2 * N);
+        counters_ = carve<uint32_t>(p, kAllWords);
+        if (pass == 0) {
+            const size_t bytes = (size_t)(uintptr_t)p;
+            if (cudaMalloc(&mem_, bytes) != cudaSuccess) {
+                snprintf(err, errLen, "BVH build: cudaMalloc of %zu bytes failed", bytes);
+                mem_ = nullptr;
+                cudaGetLastError();
+                return -5;
+            }
+            p = static_cast<char*>(mem_);
+        }
     }
-    memBytes_ = bytes;
-    char* p = static_cast<char*>(mem_);
-    primLo_ = carve<float4>(p, N);
-    primHi_ = carve<float4>(p, N);
-    refs_[0] = carve<uint32_t>(p, N);
-    refs_[1] = carve<uint32_t>(p, N);
-    order_ = carve<uint32_t>(p, N);
-    bnodes_ = carve<BinNode>(p, 2 * N);
-    tasks_[0] = carve<Task>(p, N);
-    tasks_[1] = carve<Task>(p, N);
-    cands_ = carve<Cand>(p, 2 * N);
-    candFlag_ = carve<uint32_t>(p, 2 * N);
-    candPos_ = carve<uint32_t>(p, 2 * N);
-    bigFlag_ = carve<uint32_t>(p, 2 * N);
-    bigPos_ = carve<uint32_t>(p, 2 * N);
-    bigChunks_ = carve<uint32_t>(p, 2 * N);
-    chunkOffSparse_ = carve<uint32_t>(p, 2 * N);
-    bigList_ = carve<uint32_t>(p, maxBig);
-    chunkOff_ = carve<uint32_t>(p, maxBig);
-    chunkTask_ = carve<uint32_t>(p, maxChunks);
-    chunkLeft_ = carve<uint32_t>(p, maxChunks);
-    chunkLeftOff_ = carve<uint32_t>(p, maxChunks);
-    bigBins_ = carve<uint32_t>(p, maxBig * kTaskBinWords);
-    bigSplit_ = carve<BigSplit>(p, maxBig);
-    items_[0] = reinterpret_cast<uint32_t*>(carve<uint2>(p, N + 1));
-    items_[1] = reinterpret_cast<uint32_t*>(carve<uint2>(p, N + 1));
-    slots_ = reinterpret_cast<uint32_t*>(carve<int32_t>(p, (N + 1) * kWidth));
-    collapseCost_ = carve<float>(p, 2 * N * 8);
-    collapseChoice_ = carve<uint32_t>(p, 2 * N);
-    intCount_ = carve<uint32_t>(p, N + 1);
-    intOff_ = carve<uint32_t>(p, N + 1);
-    triCount_ = carve<uint32_t>(p, N + 1);
-    triOff_ = carve<uint32_t>(p, N + 1);
-    counters_ = carve<uint32_t>(p, kCntWords);
-    scanScratch_ = carve<uint32_t>(p, scanWords);
-    sahAccum_ = carve<float>(p, 1);
-    levelStartDev_ = carve<uint32_t>(p, kMaxLevels + 2);
-    if (cudaMallocHost(&hostCounters_, kCntWords * sizeof(uint32_t)) != cudaSuccess) {
+    if (cudaMallocHost(&hostCounters_, kAllWords * sizeof(uint32_t)) != cudaSuccess) {
         snprintf(err, errLen, "BVH build: cudaMallocHost failed");
         cudaGetLastError();
         release();
@@ -1349,6 +1702,87 @@ int Builder::reserve(uint32_t n, char* err, size_t errLen)
     cudaEventCreate(&ev1_);
     cap_ = n;
     return 0;
+}
+
+void Builder::launch_begin(const Input& in, cudaStream_t st)
+{
+    const uint32_t n = in.ntris + in.nspheres;
+    k_begin<<<4, 1024, 0, st>>>(counters_);
+    k_prep_prims<<<blocks_for(n, kPrepThreads, 148 * 8), kPrepThreads, 0, st>>>(
+        in.verts, in.idx, in.ntris, in.spheres, n, boxes_, refs_[0], counters_ + kCntBounds);
+    const size_t rootThreads = std::max<size_t>(n > kSmallMax ? (n + kChunk - 1) / kChunk : 1, kTaskBinWords);
+    k_root<<<blocks_for(rootThreads, 256), 256, 0, st>>>(n, counters_, static_cast<BigTask*>(tasks_[0]), bnodes_,
+                                                         static_cast<SmallTask*>(small_), chunkTask_[0], bins_[0]);
+}
+
+// Binary levels [first, last) of the big tasks.
+void Builder::launch_big_levels(const Input& in, uint32_t first, uint32_t last, cudaStream_t st)
+{
+    const uint32_t n = in.ntris + in.nspheres;
+    const uint32_t capBig = (uint32_t)max_big(n), capChunks = (uint32_t)max_chunks(n);
+    BigSplit* splits = static_cast<BigSplit*>(splits_);
+    for (uint32_t L = first; L < last; ++L) {
+        const int a = L & 1u, b = a ^ 1;
+        BigTask *cur = static_cast<BigTask*>(tasks_[a]), *next = static_cast<BigTask*>(tasks_[b]);
+        // level L has at most 2^L tasks; the kernels loop, so any grid covers them
+        const size_t tasks = std::min<size_t>(L < 20 ? size_t(1) << L : capBig, n / (kSmallMax + 1) + 1);
+        const unsigned gTasks = blocks_for(tasks, 1, 148 * 8), gChunks = blocks_for(n / kChunk + tasks, 1, 148 * 8);
+        k_bin<<<gChunks, kChunkThreads, 0, st>>>(cur, refs_[a], boxes_, chunkTask_[a], bins_[a], chunkCnt_, counters_, L,
+                                                 capChunks);
+        k_split<<<gTasks, kSplitThreads, 0, st>>>(cur, bins_[a], chunkCnt_, chunkLeft_, splits, bnodes_, next,
+                                                  chunkTask_[b], bins_[b], static_cast<SmallTask*>(small_), counters_, L,
+                                                  capBig, capChunks, n, in.status);
+        k_scatter<<<gChunks, kChunkThreads, 0, st>>>(next, cur, refs_[a], refs_[b], boxes_, chunkTask_[a], splits,
+                                                     chunkLeft_, counters_, L, capChunks, in.status);
+    }
+}
+
+// The subtrees, the top of the cost program and the collapse's start.
+void Builder::launch_subtrees(const Input& in, uint32_t levels, uint32_t maxLevels, bool report, cudaStream_t st)
+{
+    const uint32_t n = in.ntris + in.nspheres;
+    const bool sah = collapse_ == kCollapseSah;
+    cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SubSmem));
+    k_subtree<<<blocks_for(n, 64, 148 * 3), kSubThreads, sizeof(SubSmem), st>>>(
+        static_cast<const SmallTask*>(small_), refs_[0], refs_[1], boxes_, bnodes_, order_, collapseCost_,
+        collapseChoice_, triCost_, sah, counters_, levels, n);
+    k_top<<<1, kTopThreads, 0, st>>>(bnodes_, collapseCost_, collapseChoice_, triCost_, sah,
+                                     reinterpret_cast<uint2*>(items_[0]), counters_, levels, maxLevels,
+                                     report ? in.status : nullptr);
+}
+
+// Collapse levels [first, last).
+void Builder::launch_wide_levels(const Input& in, uint32_t first, uint32_t last, cudaStream_t st)
+{
+    const uint32_t n = in.ntris + in.nspheres;
+    uint2 *off = static_cast<uint2*>(itemOff_), *sums = static_cast<uint2*>(blockSum_);
+    for (uint32_t D = first; D < last; ++D) {
+        uint2 *cur = reinterpret_cast<uint2*>(items_[D & 1u]), *next = reinterpret_cast<uint2*>(items_[(D & 1u) ^ 1u]);
+        // level D has at most 8^D wide nodes
+        const size_t items = std::min<size_t>(D < 7 ? size_t(1) << (3 * D) : n + 1, n + 1);
+        const unsigned grid = blocks_for(items, (int)kWideItemsPerBlock, 148 * 8);
+        k_wide_decide<<<grid, kWideThreads, 0, st>>>(cur, bnodes_, collapse_ == kCollapseSah ? collapseChoice_ : nullptr,
+                                                     slots_, off, sums, counters_, D, n + 1);
+        k_wide_emit<<<grid, kWideThreads, 0, st>>>(cur, bnodes_, slots_, off, sums, order_, in.verts, in.idx, in.ntris,
+                                                   in.spheres, in.nodes, in.tris, next, counters_, D, n + 1, n, in.status);
+    }
+}
+
+// Statistics from the counter words of a finished build.
+BuildStats Builder::stats_of(const uint32_t* h) const
+{
+    BuildStats s;
+    s.binaryNodes = h[kCntRealNodes];
+    s.binaryLevels = h[kCntLevels];
+    for (uint32_t L = 0; L < kMaxLevels && h[kLevelBig + L]; ++L) s.bigLevels = L + 1;
+    for (uint32_t D = 0; D <= kMaxWideLevels; ++D) {
+        s.wideNodes += h[kWideItems + D];
+        s.triCount += h[kWideTris + D];
+        if (h[kWideItems + D]) s.wideDepth = D + 1;
+    }
+    s.sahCost = __builtin_bit_cast(float, h[kCntSah]);
+    s.childSlots = h[kCntSlots];
+    return s;
 }
 
 int Builder::build(const float* verts, const uint32_t* idx, uint32_t ntris, const float4* spheres, uint32_t nspheres,
@@ -1362,285 +1796,83 @@ int Builder::build(const float* verts, const uint32_t* idx, uint32_t ntris, cons
         return 0;
     }
     if (int rc = reserve(n, err, errLen)) return rc;
-    const size_t N = n;
-    const size_t maxBig = N / kSmallMax + 2;              // as reserve() sizes the buffers
-    const size_t maxChunks = N / kChunk + maxBig + 2;
-    uint32_t* chunkOffSparse = chunkOffSparse_;
-    Task* tasks[2] = {static_cast<Task*>(tasks_[0]), static_cast<Task*>(tasks_[1])};
-    Cand* cands = static_cast<Cand*>(cands_);
-    BigSplit* splits = static_cast<BigSplit*>(bigSplit_);
-    uint32_t* bounds = counters_ + kCntBounds;
-
+    const Input in{verts, idx, ntris, spheres, nspheres, nodes, tris, deviceStatus};
+    // levels enqueued at first: the last build's with a margin, or those of a
+    // balanced tree with one
+    uint32_t levels = n > kSmallMax ? (bigLevels_ ? bigLevels_ + 1u : expected_levels(n, kSmallMax) + 3u) : 0u;
+    uint32_t wide = wideLevels_ ? wideLevels_ + 1u : 4u + expected_levels(n, 1) / 3u;
+    levels = std::min(levels, kMaxLevels);
+    wide = std::min(wide, kMaxWideLevels);
+    uint32_t* h = hostCounters_;
+    auto read_counters = [&]() -> int {
+        cudaEventRecord(ev1_, st);
+        cudaMemcpyAsync(h, counters_, kAllWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+        if (cudaStreamSynchronize(st) == cudaSuccess) return 0;
+        snprintf(err, errLen, "BVH build: %s", cudaGetErrorString(cudaGetLastError()));
+        return -2;
+    };
     cudaEventRecord(ev0_, st);
-    k_init_bounds<<<1, 32, 0, st>>>(bounds);
-    k_prep_prims<<<blocks_for(N, 256), 256, 0, st>>>(verts, idx, ntris, spheres, n, primLo_, primHi_, refs_[0], bounds);
-    uint32_t numTasks = 1;
-    uint32_t numBig = n > kSmallMax ? 1u : 0u;
-    uint32_t totalChunks = numBig ? (n + kChunk - 1) / kChunk : 0u;
-    k_root<<<blocks_for(totalChunks + 1, 256), 256, 0, st>>>(n, bounds, tasks[0], bnodes_, bigList_, chunkOff_,
-                                                             chunkTask_, totalChunks);
-    uint32_t nodeCount = 1;
-    int cur = 0;
-    uint32_t level = 0;
-    bigLevels_ = 0;
-    levelCounts_.clear();
-    wideCounts_.clear();
-    ++buildGeneration_;
-    levelStart_.assign(1, 0u);  // binary node ids of level L: [levelStart_[L], levelStart_[L + 1])
-    while (numTasks > 0) {
-        if (++level > kMaxLevels) {
+    launch_begin(in, st);
+    launch_big_levels(in, 0, levels, st);
+    launch_subtrees(in, levels, kMaxLevels, false, st);
+    launch_wide_levels(in, 0, wide, st);
+    if (int rc = read_counters()) return rc;
+    while (h[kLevelBig + levels] != 0u && !(h[kCntFailed] & kFailCapacity)) {  // big tasks below the levels enqueued: nothing after them has run
+        if (levels >= kMaxLevels) {
             snprintf(err, errLen, "BVH build: more than %u levels", kMaxLevels);
             return -4;
         }
-        Task* tk = tasks[cur];
-        levelCounts_.push_back({numTasks, numBig, totalChunks});
-        if (numBig > 0) {
-            bigLevels_ = level;
-            k_bins_clear<<<numBig, 256, 0, st>>>(bigBins_, numBig, nullptr);
-            k_bin_big<<<totalChunks, kChunkThreads, 0, st>>>(tk, refs_[cur], primLo_, primHi_, bigList_, chunkOff_,
-                                                             chunkTask_, bigBins_, totalChunks, nullptr);
-            k_split_big<<<numBig, 32, 0, st>>>(tk, bigList_, bigBins_, splits, cands, candFlag_, numBig, nullptr);
-            k_part_count<<<totalChunks, kChunkThreads, 0, st>>>(tk, refs_[cur], primLo_, primHi_, bigList_, chunkOff_,
-                                                                chunkTask_, splits, chunkLeft_, totalChunks, nullptr);
-            exclusive_scan(chunkLeft_, chunkLeftOff_, totalChunks, nullptr, scanScratch_, st);
-            k_part_scatter<<<totalChunks, kChunkThreads, 0, st>>>(tk, refs_[cur], refs_[cur ^ 1], primLo_, primHi_,
-                                                                  bigList_, chunkOff_, chunkTask_, splits,
-                                                                  chunkLeftOff_, deviceStatus, totalChunks, nullptr);
-        }
-        k_small<<<blocks_for(numTasks, kSmallWarps), 32 * kSmallWarps, 0, st>>>(
-            tk, numTasks, refs_[cur], refs_[cur ^ 1], primLo_, primHi_, bnodes_, cands, candFlag_, order_,
-            deviceStatus, nullptr, nullptr);
-        const uint32_t nc = 2 * numTasks;
-        k_cand_keys<<<blocks_for(nc, 256), 256, 0, st>>>(cands, candFlag_, nc, bigFlag_, bigChunks_, nullptr);
-        exclusive_scan(candFlag_, candPos_, nc, counters_ + kCntTasks, scanScratch_, st);
-        exclusive_scan(bigFlag_, bigPos_, nc, counters_ + kCntBig, scanScratch_, st);
-        exclusive_scan(bigChunks_, chunkOffSparse, nc, counters_ + kCntChunks, scanScratch_, st);
-        k_compact<<<blocks_for(nc, 256), 256, 0, st>>>(tk, cands, candFlag_, candPos_, bigPos_, chunkOffSparse, nc,
-                                                       nodeCount, tasks[cur ^ 1], bnodes_, bigList_, chunkOff_,
-                                                       chunkTask_, nullptr, nullptr, n, (uint32_t)maxBig,
-                                                       (uint32_t)maxChunks, deviceStatus);
-        cudaMemcpyAsync(hostCounters_, counters_, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-        if (cudaStreamSynchronize(st) != cudaSuccess) {
-            snprintf(err, errLen, "BVH build: %s", cudaGetErrorString(cudaGetLastError()));
-            return -2;
-        }
-        numTasks = hostCounters_[kCntTasks];
-        numBig = hostCounters_[kCntBig];
-        totalChunks = hostCounters_[kCntChunks];
-        levelStart_.push_back(nodeCount);
-        nodeCount += numTasks;
-        cur ^= 1;
+        const uint32_t more = std::min(kMaxLevels, levels + std::max(8u, levels / 2));
+        cudaMemsetAsync(counters_ + kCntFailed, 0, sizeof(uint32_t), st);
+        launch_big_levels(in, levels, more, st);
+        levels = more;
+        launch_subtrees(in, levels, kMaxLevels, false, st);
+        launch_wide_levels(in, 0, wide, st);
+        if (int rc = read_counters()) return rc;
     }
-    levelStart_.push_back(nodeCount);
-    local.binaryNodes = nodeCount;
-    local.binaryLevels = level;
-    local.bigLevels = bigLevels_;
-
-    // SAH cost program of the collapse, deepest level first
-    const bool sahCollapse = collapse_ == kCollapseSah;
-    if (sahCollapse)
-        for (size_t L = levelStart_.size() - 1; L-- > 0;) {
-            const uint32_t first = levelStart_[L], cnt = levelStart_[L + 1] - first;
-            if (cnt) k_collapse_cost<<<blocks_for(cnt, 128), 128, 0, st>>>(bnodes_, first, cnt, triCost_,
-                                                                          collapseCost_, collapseChoice_, nullptr, 0u);
-        }
-
-    // Wide collapse.
-    BinNode rb;
-    cudaMemcpyAsync(&rb, bnodes_, sizeof(BinNode), cudaMemcpyDeviceToHost, st);
-    uint2 rootItem = make_uint2(0, 0);
-    cudaMemcpyAsync(items_[0], &rootItem, sizeof(uint2), cudaMemcpyHostToDevice, st);
-    cudaMemsetAsync(sahAccum_, 0, sizeof(float), st);
-    cudaMemsetAsync(counters_ + kCntSlots, 0, sizeof(uint32_t), st);
-    cudaStreamSynchronize(st);
-    float rootArea = (rb.hi.x - rb.lo.x) * (rb.hi.y - rb.lo.y) + (rb.hi.y - rb.lo.y) * (rb.hi.z - rb.lo.z) +
-                     (rb.hi.z - rb.lo.z) * (rb.hi.x - rb.lo.x);
-    float rootAreaInv = rootArea > 0.0f ? 1.0f / rootArea : 0.0f;
-    uint32_t numItems = 1, wideCount = 1, triCount = 0, depth = 0;
-    int ci = 0;
-    while (numItems > 0) {
-        if (++depth > 64) {
-            snprintf(err, errLen, "BVH collapse: more than 64 wide levels");
+    if (h[kCntLevels] > kMaxLevels) {
+        snprintf(err, errLen, "BVH build: more than %u levels", kMaxLevels);
+        return -4;
+    }
+    while (h[kWideItems + wide] != 0u) {
+        if (wide >= kMaxWideLevels) {
+            snprintf(err, errLen, "BVH collapse: more than %u wide levels", kMaxWideLevels);
             return -4;
         }
-        const uint2* items = reinterpret_cast<const uint2*>(items_[ci]);
-        uint2* itemsNext = reinterpret_cast<uint2*>(items_[ci ^ 1]);
-        int32_t* slots = reinterpret_cast<int32_t*>(slots_);
-        wideCounts_.push_back(numItems);
-        k_collapse_decide<<<blocks_for(numItems, 128), 128, 0, st>>>(
-            items, numItems, bnodes_, sahCollapse ? collapseChoice_ : nullptr, slots, intCount_, triCount_,
-            counters_ + kCntSlots, nullptr);
-        exclusive_scan(intCount_, intOff_, numItems, counters_ + kCntInt, scanScratch_, st);
-        exclusive_scan(triCount_, triOff_, numItems, counters_ + kCntTri, scanScratch_, st);
-        k_collapse_emit<<<blocks_for(numItems, 128), 128, 0, st>>>(items, numItems, bnodes_, slots, intOff_, triOff_,
-                                                                    wideCount, triCount, order_, verts, idx, ntris,
-                                                                    spheres, nodes,
-                                                                    tris, itemsNext, sahAccum_, rootAreaInv, n + 1, n,
-                                                                    deviceStatus, nullptr);
-        cudaMemcpyAsync(hostCounters_ + kCntInt, counters_ + kCntInt, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                        st);
-        if (cudaStreamSynchronize(st) != cudaSuccess) {
-            snprintf(err, errLen, "BVH collapse: %s", cudaGetErrorString(cudaGetLastError()));
-            return -2;
-        }
-        numItems = hostCounters_[kCntInt];
-        wideCount += numItems;
-        triCount += hostCounters_[kCntTri];
-        ci ^= 1;
+        const uint32_t more = std::min(kMaxWideLevels, wide + 8u);
+        launch_wide_levels(in, wide, more, st);
+        wide = more;
+        if (int rc = read_counters()) return rc;
     }
-    cudaEventRecord(ev1_, st);
-    float sah = 0.0f;
-    cudaMemcpyAsync(&sah, sahAccum_, sizeof(float), cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(hostCounters_ + kCntSlots, counters_ + kCntSlots, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) {
-        snprintf(err, errLen, "BVH build: %s", cudaGetErrorString(cudaGetLastError()));
-        return -2;
-    }
-    float ms = 0.0f;
-    cudaEventElapsedTime(&ms, ev0_, ev1_);
-    local.wideNodes = wideCount;
-    local.wideDepth = depth;
-    local.triCount = triCount;
-    local.sahCost = sah;
-    local.buildMs = ms;
-    local.childSlots = hostCounters_[kCntSlots];
-    if (triCount != n) {
-        snprintf(err, errLen, "BVH build: %u triangles placed, expected %u", triCount, n);
+    local = stats_of(h);
+    bigLevels_ = local.bigLevels;
+    wideLevels_ = local.wideDepth;
+    cudaEventElapsedTime(&local.buildMs, ev0_, ev1_);
+    if (h[kCntFailed] != 0u || local.triCount != n) {
+        snprintf(err, errLen, "BVH build: %u primitives placed, expected %u", local.triCount, n);
         return -3;
     }
-    if (depth > (uint32_t)kTraversalStack) {
-        snprintf(err, errLen, "BVH build: wide depth %u exceeds the traversal stack (%d)", depth, kTraversalStack);
+    if (local.wideDepth > (uint32_t)kTraversalStack) {
+        snprintf(err, errLen, "BVH build: wide depth %u exceeds the traversal stack (%d)", local.wideDepth,
+                 kTraversalStack);
         return -4;
     }
     if (stats) *stats = local;
     return 0;
 }
 
-
-namespace {
-// Grids of the device-driven build: the counts are not known when the
-// launches are made, so each kernel loops over its work items on at most
-// this many blocks (a few waves of the 148 SMs).
-constexpr unsigned kDevChunkBlocks = 148 * 4;
-constexpr unsigned kDevThreadBlocks = 148 * 8;
-inline unsigned dev_blocks(size_t n, int threads, unsigned cap)
+void Builder::enqueue_launches(const Input& in, uint32_t maxLevels, uint32_t maxWideLevels, cudaStream_t st)
 {
-    const size_t b = (n + threads - 1) / threads;
-    return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
-}
-}  // namespace
-
-void Builder::enqueue_launches(const float* verts, const uint32_t* idx, uint32_t ntris, const float4* spheres,
-                               uint32_t n, WideNode* nodes, TriRecord* tris, uint32_t* deviceStatus, cudaStream_t st,
-                               uint32_t maxLevels, uint32_t maxWideLevels)
-{
-    const size_t N = n;
-    const size_t maxBig = N / kSmallMax + 2;
-    const size_t maxChunks = N / kChunk + maxBig + 2;
-    Task* tasks[2] = {static_cast<Task*>(tasks_[0]), static_cast<Task*>(tasks_[1])};
-    Cand* cands = static_cast<Cand*>(cands_);
-    BigSplit* splits = static_cast<BigSplit*>(bigSplit_);
-    uint32_t* bounds = counters_ + kCntBounds;
-    uint32_t* dv = counters_;
-    const uint32_t rootChunks = n > kSmallMax ? (n + kChunk - 1) / kChunk : 0u;
-
-    k_init_bounds<<<1, 32, 0, st>>>(bounds);
-    k_prep_prims<<<blocks_for(N, 256), 256, 0, st>>>(verts, idx, ntris, spheres, n, primLo_, primHi_, refs_[0], bounds);
-    k_root<<<blocks_for(rootChunks + 1, 256), 256, 0, st>>>(n, bounds, tasks[0], bnodes_, bigList_, chunkOff_,
-                                                            chunkTask_, rootChunks);
-    k_dev_begin<<<1, 1, 0, st>>>(n, dv, levelStartDev_);
-    // Grids: the kernels loop over their work items, so any grid is correct.
-    // Each level's grid is sized for 1.5 times the count the last host-driven
-    // build had there (animated geometry keeps them close), capped by the
-    // buffers' capacities, instead of the capacity itself: far fewer idle
-    // blocks are dispatched.
-    auto expect = [](uint32_t recorded, size_t cap) {
-        return std::min(cap, size_t(recorded) + recorded / 2 + 32);
-    };
-    auto level_expect = [&](uint32_t L) {
-        return L < levelCounts_.size() ? levelCounts_[L] : (levelCounts_.empty() ? LevelCounts{1, 1, 1} : levelCounts_.back());
-    };
-    // tasks above kSmallMax references occur on the top levels only: the
-    // big-task kernels run on the levels where the last host-driven build had
-    // them, plus a margin (k_small reports a big task met past them)
-    const uint32_t bigCap = std::min(maxLevels, bigLevels_ + 2u);
-    int cur = 0;
-    for (uint32_t L = 0; L < maxLevels; ++L) {
-        Task* tk = tasks[cur];
-        const bool bigLevel = L < bigCap;
-        const LevelCounts e = level_expect(L);
-        const unsigned gBig = dev_blocks(expect(e.big, maxBig), 1, kDevChunkBlocks);
-        const unsigned gChunks = dev_blocks(expect(e.chunks, maxChunks), 1, kDevChunkBlocks);
-        const unsigned gSmall = dev_blocks(expect(e.tasks, N), kSmallWarps, kDevThreadBlocks);
-        const unsigned gCand = dev_blocks(2 * expect(e.tasks, N), 256, kDevThreadBlocks);
-        if (bigLevel) {
-            k_bins_clear<<<gBig, 256, 0, st>>>(bigBins_, 0u, dv + kDevBig);
-            k_bin_big<<<gChunks, kChunkThreads, 0, st>>>(tk, refs_[cur], primLo_, primHi_, bigList_, chunkOff_,
-                                                         chunkTask_, bigBins_, 0u, dv + kDevChunks);
-            k_split_big<<<gBig, 32, 0, st>>>(tk, bigList_, bigBins_, splits, cands, candFlag_, 0u, dv + kDevBig);
-            k_part_count<<<gChunks, kChunkThreads, 0, st>>>(tk, refs_[cur], primLo_, primHi_, bigList_, chunkOff_,
-                                                            chunkTask_, splits, chunkLeft_, 0u, dv + kDevChunks);
-            {
-                const uint32_t* in[] = {chunkLeft_};
-                uint32_t* out[] = {chunkLeftOff_};
-                exclusive_scan_count(1, in, out, dv + kDevChunks, 1u, maxChunks, nullptr, scanScratch_, st,
-                                     expect(e.chunks, maxChunks));
-            }
-            k_part_scatter<<<gChunks, kChunkThreads, 0, st>>>(tk, refs_[cur], refs_[cur ^ 1], primLo_, primHi_,
-                                                              bigList_, chunkOff_, chunkTask_, splits, chunkLeftOff_,
-                                                              deviceStatus, 0u, dv + kDevChunks);
-        }
-        k_small<<<gSmall, 32 * kSmallWarps, 0, st>>>(tk, 0u, refs_[cur], refs_[cur ^ 1], primLo_, primHi_, bnodes_,
-                                                     cands, candFlag_, order_, deviceStatus, dv + kDevTasks,
-                                                     bigLevel ? nullptr : dv + kDevFailed);
-        k_cand_keys<<<gCand, 256, 0, st>>>(cands, candFlag_, 0u, bigFlag_, bigChunks_, dv + kDevTasks);
-        {
-            const uint32_t* in[] = {candFlag_, bigFlag_, bigChunks_};
-            uint32_t* out[] = {candPos_, bigPos_, chunkOffSparse_};
-            uint32_t* tot[] = {counters_ + kCntTasks, counters_ + kCntBig, counters_ + kCntChunks};
-            exclusive_scan_count(3, in, out, dv + kDevTasks, 2u, 2 * N, tot, scanScratch_, st,
-                                 2 * expect(e.tasks, N));
-        }
-        k_compact<<<gCand, 256, 0, st>>>(tk, cands, candFlag_, candPos_, bigPos_, chunkOffSparse_, 0u, 0u,
-                                         tasks[cur ^ 1], bnodes_, bigList_, chunkOff_, chunkTask_, dv + kDevTasks,
-                                         dv + kDevNodes, n, (uint32_t)maxBig, (uint32_t)maxChunks, deviceStatus);
-        k_dev_level_end<<<1, 1, 0, st>>>(dv, levelStartDev_, L, n, (uint32_t)maxBig, (uint32_t)maxChunks,
-                                         deviceStatus);
-        cur ^= 1;
-    }
-
-    k_dev_collapse_begin<<<1, 1, 0, st>>>(dv, bnodes_, reinterpret_cast<uint2*>(items_[0]), sahAccum_, deviceStatus);
-    const bool sahCollapse = collapse_ == kCollapseSah;
-    if (sahCollapse) {
-        for (uint32_t L = maxLevels; L-- > 0;) {
-            // the nodes of binary level L are the tasks split at level L
-            const unsigned gCost = dev_blocks(expect(level_expect(L).tasks, N), 128, kDevThreadBlocks);
-            k_collapse_cost<<<gCost, 128, 0, st>>>(bnodes_, 0u, 0u, triCost_, collapseCost_, collapseChoice_,
-                                                   levelStartDev_, L);
-        }
-    }
-    int ci = 0;
-    for (uint32_t D = 0; D < maxWideLevels; ++D) {
-        const uint32_t we = D < wideCounts_.size() ? wideCounts_[D] : (wideCounts_.empty() ? 1u : wideCounts_.back());
-        const unsigned gItems = dev_blocks(expect(we, N + 1), 128, kDevThreadBlocks);
-        const uint2* items = reinterpret_cast<const uint2*>(items_[ci]);
-        uint2* itemsNext = reinterpret_cast<uint2*>(items_[ci ^ 1]);
-        int32_t* slots = reinterpret_cast<int32_t*>(slots_);
-        k_collapse_decide<<<gItems, 128, 0, st>>>(items, 0u, bnodes_, sahCollapse ? collapseChoice_ : nullptr, slots,
-                                                  intCount_, triCount_, counters_ + kCntSlots, dv + kDevItems);
-        {
-            const uint32_t* in[] = {intCount_, triCount_};
-            uint32_t* out[] = {intOff_, triOff_};
-            uint32_t* tot[] = {counters_ + kCntInt, counters_ + kCntTri};
-            exclusive_scan_count(2, in, out, dv + kDevItems, 1u, N + 1, tot, scanScratch_, st, expect(we, N + 1));
-        }
-        k_collapse_emit<<<gItems, 128, 0, st>>>(items, 0u, bnodes_, slots, intOff_, triOff_, 0u, 0u, order_, verts, idx,
-                                                ntris, spheres, nodes, tris, itemsNext, sahAccum_, 0.0f, n + 1, n,
-                                                deviceStatus, dv);
-        k_dev_wide_end<<<1, 1, 0, st>>>(dv, n + 1, deviceStatus);
-        ci ^= 1;
-    }
-    k_dev_end<<<1, 1, 0, st>>>(dv, n, deviceStatus);
+    const uint32_t n = in.ntris + in.nspheres;
+    // tasks above kSmallMax references occur on the top levels only: their
+    // kernels run on the levels where the last build() had them, plus a margin
+    // (k_subtree reports a big task left after them)
+    const uint32_t levels = n > kSmallMax ? std::min(maxLevels, bigLevels_ + 2u) : 0u;
+    launch_begin(in, st);
+    launch_big_levels(in, 0, levels, st);
+    launch_subtrees(in, levels, maxLevels, true, st);
+    launch_wide_levels(in, 0, maxWideLevels, st);
+    k_end<<<1, 1, 0, st>>>(counters_, n, maxWideLevels, in.status);
 }
 
 int Builder::enqueue(const float* verts, const uint32_t* idx, uint32_t ntris, const float4* spheres,
@@ -1653,14 +1885,13 @@ int Builder::enqueue(const float* verts, const uint32_t* idx, uint32_t ntris, co
         snprintf(err, errLen, "BVH enqueue: no buffers for %u primitives (run a build of this size first)", n);
         return -6;
     }
-    if (maxLevels == 0 || maxLevels > kMaxLevels || maxWideLevels == 0 || maxWideLevels > 64) {
-        snprintf(err, errLen, "BVH enqueue: level caps must be 1-%u (binary) and 1-64 (wide)", kMaxLevels);
+    if (maxLevels == 0 || maxLevels > kMaxLevels || maxWideLevels == 0 || maxWideLevels > kMaxWideLevels) {
+        snprintf(err, errLen, "BVH enqueue: level caps must be 1-%u (binary) and 1-%u (wide)", kMaxLevels, kMaxWideLevels);
         return -6;
     }
     const uint64_t key[] = {(uint64_t)(uintptr_t)verts, (uint64_t)(uintptr_t)idx, (uint64_t)(uintptr_t)spheres,
                             (uint64_t)(uintptr_t)nodes, (uint64_t)(uintptr_t)tris, (uint64_t)(uintptr_t)deviceStatus,
-                            (uint64_t)(uintptr_t)mem_, ntris, nspheres, maxLevels, maxWideLevels, bigLevels_,
-                            buildGeneration_, collapse_,
+                            (uint64_t)(uintptr_t)mem_, ntris, nspheres, maxLevels, maxWideLevels, bigLevels_, collapse_,
                             (uint64_t)__builtin_bit_cast(uint32_t, triCost_)};
     const std::vector<uint64_t> k(key, key + sizeof key / sizeof key[0]);
     if (!graphExec_ || k != graphKey_) {
@@ -1671,7 +1902,8 @@ int Builder::enqueue(const float* verts, const uint32_t* idx, uint32_t ntris, co
                      cudaGetErrorString(cudaGetLastError()));
             return -2;
         }
-        enqueue_launches(verts, idx, ntris, spheres, n, nodes, tris, deviceStatus, st, maxLevels, maxWideLevels);
+        enqueue_launches(Input{verts, idx, ntris, spheres, nspheres, nodes, tris, deviceStatus}, maxLevels, maxWideLevels,
+                         st);
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(st, &g);
         if (e == cudaSuccess) e = cudaGraphInstantiate(&graphExec_, g, 0);
@@ -1702,26 +1934,15 @@ int Builder::enqueued_stats(cudaStream_t st, BuildStats* stats, char* err, size_
         snprintf(err, errLen, "BVH stats: no device-driven build yet");
         return -6;
     }
-    uint32_t h[kCntWords];
-    float sah = 0.0f;
-    cudaMemcpyAsync(h, counters_, sizeof h, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&sah, sahAccum_, sizeof(float), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(hostCounters_, counters_, kAllWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) {
         snprintf(err, errLen, "BVH stats: %s", cudaGetErrorString(cudaGetLastError()));
         return -2;
     }
-    BuildStats s;
-    s.binaryNodes = h[kDevNodes];
-    s.binaryLevels = h[kDevLevels];
-    s.wideNodes = h[kDevWide];
-    s.wideDepth = h[kDevDepth];
-    s.triCount = h[kDevTris];
-    s.sahCost = sah;
-    s.childSlots = h[kCntSlots];
+    *stats = stats_of(hostCounters_);
     float ms = 0.0f;
-    if (graphLaunches_ && cudaEventElapsedTime(&ms, ev0_, ev1_) == cudaSuccess) s.buildMs = ms;
+    if (graphLaunches_ && cudaEventElapsedTime(&ms, ev0_, ev1_) == cudaSuccess) stats->buildMs = ms;
     cudaGetLastError();
-    *stats = s;
     return 0;
 }
 

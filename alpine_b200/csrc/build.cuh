@@ -45,15 +45,14 @@ public:
               WideNode* nodes, TriRecord* tris, uint32_t* deviceStatus, cudaStream_t stream, BuildStats* stats,
               char* err, size_t errLen);
 
-    // Device-driven build: the same tree as build(), bit for bit, with every
-    // count kept in device memory, so that nothing waits on the host and the
-    // sequence of launches is fixed. It runs maxLevels binary levels and
-    // maxWideLevels collapse levels (a level past the tree's depth costs a
-    // few short launches), captured in a CUDA graph on the first call and
-    // replayed until the arguments change or a build() records new per-level
-    // counts (they size the grids and pick the levels that run the big-task
-    // kernels). Needs buffers for ntris + nspheres primitives (a build() of
-    // at least that size first). A tree deeper than the binary cap, or a big
+    // Device-driven build: the same tree as build(), bit for bit, as a fixed
+    // sequence of launches that nothing waits for. The tree may have maxLevels
+    // binary levels and maxWideLevels collapse levels (a collapse level past
+    // the tree's depth costs two short launches). The sequence is captured in
+    // a CUDA graph on the first call and replayed until the arguments change
+    // or a build() finds big tasks on another number of levels (they pick the
+    // levels that run the big-task kernels). Needs buffers for ntris + nspheres
+    // primitives (a build() of at least that size first). A tree deeper than the binary cap, or a big
     // task below the big-task levels, leaves the previous tree in place; one
     // deeper than the wide cap leaves it partly rewritten; all three set
     // kErrBuildDepth in deviceStatus. Returns 0, or a negative code with a
@@ -77,59 +76,53 @@ public:
     float triangle_cost() const { return triCost_; }
 
 private:
-    int reserve(uint32_t ntris, char* err, size_t errLen);
+    struct Input {
+        const float* verts;
+        const uint32_t* idx;
+        uint32_t ntris;
+        const float4* spheres;
+        uint32_t nspheres;
+        WideNode* nodes;
+        TriRecord* tris;
+        uint32_t* status;
+    };
+    int reserve(uint32_t n, char* err, size_t errLen);
     void release();
-    void enqueue_launches(const float* verts, const uint32_t* idx, uint32_t ntris, const float4* spheres, uint32_t n,
-                          WideNode* nodes, TriRecord* tris, uint32_t* deviceStatus, cudaStream_t stream,
-                          uint32_t maxLevels, uint32_t maxWideLevels);
+    void launch_begin(const Input& in, cudaStream_t st);
+    void launch_big_levels(const Input& in, uint32_t first, uint32_t last, cudaStream_t st);
+    void launch_subtrees(const Input& in, uint32_t levels, uint32_t maxLevels, bool report, cudaStream_t st);
+    void launch_wide_levels(const Input& in, uint32_t first, uint32_t last, cudaStream_t st);
+    void enqueue_launches(const Input& in, uint32_t maxLevels, uint32_t maxWideLevels, cudaStream_t st);
+    BuildStats stats_of(const uint32_t* counters) const;
 
     uint32_t cap_ = 0;
     uint32_t collapse_ = kCollapseSah;
     float triCost_ = kCollapseTriCost;
     void* mem_ = nullptr;  // one allocation carved into the arrays below
-    size_t memBytes_ = 0;
-    float4* primLo_ = nullptr;
-    float4* primHi_ = nullptr;
+    // binary phase; index 0 / 1 by level parity
+    float4* boxes_ = nullptr;
     uint32_t* refs_[2] = {nullptr, nullptr};
-    uint32_t* order_ = nullptr;
-    BinNode* bnodes_ = nullptr;
     void* tasks_[2] = {nullptr, nullptr};
-    void* cands_ = nullptr;
-    uint32_t* candFlag_ = nullptr;
-    uint32_t* candPos_ = nullptr;
-    uint32_t* bigFlag_ = nullptr;
-    uint32_t* bigPos_ = nullptr;
-    uint32_t* bigList_ = nullptr;
-    uint32_t* bigChunks_ = nullptr;
-    uint32_t* chunkOffSparse_ = nullptr;
-    uint32_t* chunkOff_ = nullptr;
-    uint32_t* chunkTask_ = nullptr;
+    uint32_t* chunkTask_[2] = {nullptr, nullptr};
+    uint32_t* bins_[2] = {nullptr, nullptr};
+    uint16_t* chunkCnt_ = nullptr;
     uint32_t* chunkLeft_ = nullptr;
-    uint32_t* chunkLeftOff_ = nullptr;
-    uint32_t* bigBins_ = nullptr;
-    void* bigSplit_ = nullptr;
-    uint32_t* items_[2] = {nullptr, nullptr};
-    uint32_t* slots_ = nullptr;
-    std::vector<uint32_t> levelStart_;   // first binary node id of each level (host)
-    float* collapseCost_ = nullptr;      // 8 per binary node (k_collapse_cost)
+    void* splits_ = nullptr;
+    void* small_ = nullptr;
+    BinNode* bnodes_ = nullptr;
+    uint32_t* order_ = nullptr;
+    float* collapseCost_ = nullptr;      // 8 per binary node
     uint32_t* collapseChoice_ = nullptr; // 1 per binary node
-    uint32_t* intCount_ = nullptr;
-    uint32_t* intOff_ = nullptr;
-    uint32_t* triCount_ = nullptr;
-    uint32_t* triOff_ = nullptr;
-    uint32_t* counters_ = nullptr;  // small device scalars
+    // collapse; items_ by level parity
+    uint32_t* items_[2] = {nullptr, nullptr};
+    int32_t* slots_ = nullptr;
+    void* itemOff_ = nullptr;
+    void* blockSum_ = nullptr;
+    uint32_t* counters_ = nullptr;      // counts of all levels (device)
     uint32_t* hostCounters_ = nullptr;  // pinned mirror
-    uint32_t* scanScratch_ = nullptr;
-    float* sahAccum_ = nullptr;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
-    uint32_t* levelStartDev_ = nullptr;  // first binary node id of each level (device-driven build)
-    uint32_t bigLevels_ = 0;             // leading binary levels with big tasks in the last build()
-    struct LevelCounts {
-        uint32_t tasks, big, chunks;
-    };
-    std::vector<LevelCounts> levelCounts_;  // per binary level of the last build(): sizes enqueue()'s grids
-    std::vector<uint32_t> wideCounts_;      // wide nodes per collapse level of the last build()
-    uint64_t buildGeneration_ = 0;          // build() calls so far (part of the graph key)
+    uint32_t bigLevels_ = 0;   // leading binary levels with big tasks in the last build()
+    uint32_t wideLevels_ = 0;  // collapse levels of the last build()
     cudaGraphExec_t graphExec_ = nullptr;  // the captured device-driven build
     std::vector<uint64_t> graphKey_;
     uint32_t graphCaptures_ = 0, graphLaunches_ = 0;
