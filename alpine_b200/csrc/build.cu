@@ -726,49 +726,51 @@ AG_D uint32_t collapse_cost(const float L[kCosts], const float R[kCosts], float 
 // its counts, scans and compaction) per level this removed half of a build's
 // time and most of its launches.
 //
-// A level's nodes above kDirectMax references are split by one warp each,
-// with shared-memory bins. The others are split without bins, one thread per
-// reference: a thread takes the plane after its own reference's bin as its
-// candidate on each axis, sums the two sides over the node's references, and
-// the node's cheapest candidate wins (a 64-bit shared-memory minimum over
-// cost, axis, bin). Planes between two references' bins need no candidate of
-// their own: they cut the same sets as the plane after the lower bin, which
-// the bin search prefers as well. At eight references this takes about 400
-// instructions for four nodes; the bin search takes 1,500 for each.
-constexpr int kSubThreads = 256;
+// One thread per reference; the references' boxes move with the partition, so
+// that a node's are consecutive. Nodes above kDirectMax references are split
+// with shared-memory bins, kBinNodes of them at a time, a warp per node and
+// axis for the search. The others are split without bins: a thread takes the
+// plane after its own reference's bin as its candidate on each axis, sums the
+// two sides over the node's references, and the node's cheapest candidate
+// wins (a 64-bit shared-memory minimum over cost, axis, bin). Planes between
+// two references' bins need no candidate of their own: they cut the same sets
+// as the plane after the lower bin, which the bin search prefers as well. At
+// eight references this takes about 400 instructions for four nodes; the bin
+// search takes 1,500 for each.
+//
+// The kernel is a chain of short steps between block barriers, about 12 levels
+// deep, and its time on a small scene is that chain's.
+constexpr int kSubThreads = (int)kSmallMax;
 constexpr uint32_t kSubWarps = kSubThreads / 32;
 constexpr uint32_t kDirectMax = 32;
+constexpr uint32_t kBinNodes = 8;
 constexpr uint32_t kNoChild = 0xffffu;
-constexpr int kSubRounds = (int)kSmallMax / kSubThreads;
-static_assert(kSmallMax % kSubThreads == 0 && kDirectMax <= 32, "left bits of a node span at most two words");
 
 struct SubSmem {
+    float4 pa[kSmallMax];               // per position: lo.xyz, hi.x
+    float4 pb[kSmallMax];               // hi.y, hi.z, bits: bins on the three axes and which have an extent, primitive id
     unsigned long long key[kSmallMax];  // per node of the level: its cheapest candidate
     union {
-        uint32_t bins[kSubWarps][kTaskBinWords];
+        uint32_t bins[kBinNodes][kTaskBinWords];
         float cost[(kSmallMax - 1) * kCosts];  // per internal node, once the tree is built
     };
-    float box[6][kSmallMax];            // lo3 hi3 of the subtree's primitives
-    uint32_t prim[kSmallMax];           // their ids
-    uint32_t pbin[kSmallMax];           // per position: bins on the three axes, and which axes have an extent
+    SplitChoice axisBest[kBinNodes][3];
+    uint32_t cbounds[kBinNodes][6];     // centroid bounds (f2ord) of the nodes being binned
     float area[2 * kSmallMax];          // per node of the subtree
     uint32_t leftBits[kSmallMax / 32];
-    uint32_t ticket, idBase, nodeTop, levelEnd;
-    uint16_t perm[2][kSmallMax];        // per position: the primitive there (index into box, prim)
-    uint16_t posNode[2][kSmallMax];     // per position: the node it belongs to
+    uint32_t ticket, idBase, nodeTop, levelEnd, binCount;
+    uint16_t binNode[kSmallMax / kDirectMax];  // the level's nodes above kDirectMax references
+    uint16_t binSlot[kSmallMax];        // per node of the level: its entry there
+    uint16_t posNode[kSmallMax];        // per position: the node it belongs to
     uint16_t begin[2 * kSmallMax], count[2 * kSmallMax], left[2 * kSmallMax];
     uint16_t levelStart[kSmallMax + 2];
 };
 
-AG_D void sub_box(const SubSmem& s, uint32_t j, float lo[3], float hi[3])
+AG_D void sub_box(const float4& a, const float4& b, float lo[3], float hi[3])
 {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = s.box[k][j];
-        hi[k] = s.box[3 + k][j];
-    }
+    lo[0] = a.x; lo[1] = a.y; lo[2] = a.z;
+    hi[0] = a.w; hi[1] = b.x; hi[2] = b.y;
 }
-
 AG_D void box_reset(float b[6])
 {
 #pragma unroll
@@ -786,11 +788,22 @@ AG_D void box_add(float b[6], const float lo[3], const float hi[3])
     }
 }
 
-// Two children of node nd (nL of its references go left); returns the first's
-// local id. The subtree's nodes are 0 (the root, id rootNode) and 1, 2, ...
-// (ids idBase, idBase + 1, ...).
-AG_D uint32_t sub_children(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t rootNode, uint32_t globalBegin,
-                           uint32_t nd, uint32_t nL, const float L[6], const float R[6])
+// A node's split as its key: cost, axis, bin, candidate's position.
+AG_D unsigned long long split_key(float cost, uint32_t axis, uint32_t bin, uint32_t p)
+{
+    return ((unsigned long long)__float_as_uint(cost) << 32) | (axis << 24) | (bin << 16) | p;
+}
+constexpr unsigned long long kNoSplit = ~0ull;  // all centroids coincide: split by position
+AG_D bool key_left(unsigned long long key, uint32_t pbin, uint32_t local, uint32_t count)
+{
+    if (key == kNoSplit) return local < count / 2u;
+    return ((pbin >> (8u * ((uint32_t)(key >> 24) & 0xffu))) & 0xffu) <= ((uint32_t)(key >> 16) & 0xffu);
+}
+
+// Two children of node nd (nL of its references go left). The subtree's nodes
+// are 0 (the root, id rootNode) and 1, 2, ... (ids idBase, idBase + 1, ...).
+AG_D void sub_children(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t rootNode, uint32_t globalBegin, uint32_t nd,
+                       uint32_t nL, const float L[6], const float R[6])
 {
     const uint32_t ch = atomicAdd(&s.nodeTop, 2u);
     const uint32_t b = s.begin[nd], n = s.count[nd];
@@ -808,118 +821,115 @@ AG_D uint32_t sub_children(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t ro
     bnodes[parent].right = (int32_t)id + 1;
     write_node(bnodes, id, L, globalBegin + b, nL);
     write_node(bnodes, id + 1, R, globalBegin + b + nL, n - nL);
-    return ch;
 }
 
-// Split of a node above kDirectMax references by one warp. cur: the
-// permutation's current buffer; the children's references go to the other.
-AG_D void sub_split_warp(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t rootNode, uint32_t globalBegin, uint32_t nd,
-                         uint32_t* bins, int cur)
+// Boxes of the two halves of a node whose centroids coincide.
+AG_D void median_boxes(const SubSmem& s, uint32_t b, uint32_t c, float L[6], float R[6])
 {
-    const uint32_t lane = lane_id(), b = s.begin[nd], n = s.count[nd];
-    float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (uint32_t i = lane; i < n; i += 32) {
+    box_reset(L);
+    box_reset(R);
+    for (uint32_t i = 0; i < c; ++i) {
         float lo[3], hi[3];
-        sub_box(s, s.perm[cur][b + i], lo, hi);
+        sub_box(s.pa[b + i], s.pb[b + i], lo, hi);
+        if (i < c / 2u) box_add(L, lo, hi);
+        else box_add(R, lo, hi);
+    }
+}
+
+// Splits the level's nodes above kDirectMax references (binNode). bin: this
+// thread's entry of the list, kNoTask if it has none. Called by the whole block.
+AG_D void sub_split_bins(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t rootNode, uint32_t globalBegin, uint32_t ls,
+                         uint32_t bin)
+{
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, total = s.binCount;
+    for (uint32_t first = 0; first < total; first += kBinNodes) {
+        const uint32_t nodes = min(kBinNodes, total - first);
+        const bool mine = bin - first < nodes;  // (wraps for kNoTask and entries of other rounds)
+        const uint32_t slot = mine ? bin - first : 0u;
+        for (uint32_t k = tid; k < nodes * kTaskBinWords; k += kSubThreads) bin_init_word(&s.bins[0][0] + k, (int)k);
+        if (tid < nodes * 6) (&s.cbounds[0][0])[tid] = tid % 6 < 3 ? 0xffffffffu : 0u;
+        __syncthreads();
+        float lo[3], hi[3], c[3] = {0.0f, 0.0f, 0.0f};
+        uint32_t cmin[3], cmax[3];
+        sub_box(s.pa[tid], s.pb[tid], lo, hi);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const float c = centroid(lo[k], hi[k]);
-            clo[k] = fminf(clo[k], c);
-            chi[k] = fmaxf(chi[k], c);
+            c[k] = centroid(lo[k], hi[k]);
+            const bool nan = c[k] != c[k];  // no bound, as with fminf / fmaxf
+            cmin[k] = nan ? f2ord(FLT_MAX) : f2ord(c[k]);
+            cmax[k] = nan ? f2ord(-FLT_MAX) : f2ord(c[k]);
         }
-    }
-    float sc[3];
+        const uint32_t slot0 = __shfl_sync(0xffffffffu, slot, 0);
+        if (__all_sync(0xffffffffu, mine && slot == slot0)) {  // one set of atomics for the warp
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        clo[k] = warp_min(clo[k]);
-        chi[k] = warp_max(chi[k]);
-        sc[k] = axis_scale(clo[k], chi[k]);
-    }
-    __syncwarp();  // the warp's previous node has finished reading the bins
-    for (int k = lane; k < kTaskBinWords; k += 32) bin_init_word(bins + k, k);
-    __syncwarp();
-    for (uint32_t i = lane; i < n; i += 32) {
-        float lo[3], hi[3];
-        sub_box(s, s.perm[cur][b + i], lo, hi);
-        uint32_t ord[6];
+            for (int k = 0; k < 3; ++k) {
+                const uint32_t a = __reduce_min_sync(0xffffffffu, cmin[k]), b = __reduce_max_sync(0xffffffffu, cmax[k]);
+                if (lane_id() == 0) {
+                    atomicMin(&s.cbounds[slot][k], a);
+                    atomicMax(&s.cbounds[slot][3 + k], b);
+                }
+            }
+        } else if (mine) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            ord[k] = f2ord(lo[k]);
-            ord[3 + k] = f2ord(hi[k]);
+            for (int k = 0; k < 3; ++k) {
+                atomicMin(&s.cbounds[slot][k], cmin[k]);
+                atomicMax(&s.cbounds[slot][3 + k], cmax[k]);
+            }
         }
+        __syncthreads();
+        if (mine) {
+            uint32_t ord[6], v = 0;
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-            if (sc[a] != 0.0f)
-                bin_accumulate(bins + a * kAxisBinWords + bin_of(centroid(lo[a], hi[a]), clo[a], sc[a]) * kBinWords, ord);
-    }
-    __syncwarp();
-    SplitChoice best;
-    split_reset(best);
+            for (int k = 0; k < 3; ++k) {
+                ord[k] = f2ord(lo[k]);
+                ord[3 + k] = f2ord(hi[k]);
+            }
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (sc[a] == 0.0f) continue;
-        float v[6];
-        uint32_t c;
-        load_bin(bins + a * kAxisBinWords + lane * kBinWords, v, c);
-        eval_axis(a, v, c, n, best);
-    }
-    const bool median = best.axis < 0;  // all centroids coincide
-    if (median) {
-        best.nL = n / 2;
-        box_reset(best.L);
-        box_reset(best.R);
-        for (uint32_t i = lane; i < n; i += 32) {
-            float lo[3], hi[3];
-            sub_box(s, s.perm[cur][b + i], lo, hi);
-            if (i < best.nL) box_add(best.L, lo, hi);
-            else box_add(best.R, lo, hi);
+            for (int k = 0; k < 3; ++k) {
+                const float clo = ord2f(s.cbounds[slot][k]), sc = axis_scale(clo, ord2f(s.cbounds[slot][3 + k]));
+                if (sc == 0.0f) continue;
+                const uint32_t bk = (uint32_t)bin_of(c[k], clo, sc);
+                v |= (bk << (8 * k)) | (1u << (24 + k));
+                bin_accumulate(&s.bins[slot][k * kAxisBinWords + bk * kBinWords], ord);
+            }
+            s.pb[tid].z = __uint_as_float(v);
         }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            best.L[k] = warp_min(best.L[k]);
-            best.L[3 + k] = warp_max(best.L[3 + k]);
-            best.R[k] = warp_min(best.R[k]);
-            best.R[3 + k] = warp_max(best.R[3 + k]);
+        __syncthreads();
+        for (uint32_t pair = warp; pair < nodes * 3u; pair += kSubWarps) {
+            const uint32_t sl = pair / 3u, a = pair % 3u;
+            SplitChoice best;
+            split_reset(best);
+            if (axis_scale(ord2f(s.cbounds[sl][a]), ord2f(s.cbounds[sl][3 + a])) != 0.0f) {
+                float v[6];
+                uint32_t n;
+                load_bin(&s.bins[sl][a * kAxisBinWords + lane_id() * kBinWords], v, n);
+                eval_axis((int)a, v, n, s.count[s.binNode[first + sl]], best);
+            }
+            if (lane_id() == 0) s.axisBest[sl][a] = best;
         }
-    }
-    uint32_t ch = 0;
-    if (lane == 0) ch = sub_children(s, bnodes, rootNode, globalBegin, nd, best.nL, best.L, best.R);
-    ch = __shfl_sync(0xffffffffu, ch, 0);
-    // stable partition
-    uint32_t leftSeen = 0, rightSeen = 0;
-    for (uint32_t base = 0; base < n; base += 32) {
-        const uint32_t i = base + lane;
-        const bool valid = i < n;
-        uint32_t j = 0;
-        bool left = false;
-        if (valid) {
-            j = s.perm[cur][b + i];
-            if (median) {
-                left = i < best.nL;
+        __syncthreads();
+        if (lane_id() == 0 && warp < nodes) {  // a warp per node, so that their memory waits overlap
+            const uint32_t nd = s.binNode[first + warp];
+            int a = 0;
+            for (int k = 1; k < 3; ++k)
+                if (s.axisBest[warp][k].cost < s.axisBest[warp][a].cost) a = k;
+            const SplitChoice& best = s.axisBest[warp][a];
+            if (best.axis >= 0) {
+                s.key[nd - ls] = split_key(best.cost, (uint32_t)best.axis, (uint32_t)best.bin, 0u);
+                sub_children(s, bnodes, rootNode, globalBegin, nd, best.nL, best.L, best.R);
             } else {
-                const int a = best.axis;
-                const float cl = a == 0 ? clo[0] : (a == 1 ? clo[1] : clo[2]);
-                const float ss = a == 0 ? sc[0] : (a == 1 ? sc[1] : sc[2]);
-                left = bin_of(centroid(s.box[a][j], s.box[3 + a][j]), cl, ss) <= best.bin;
+                float L[6], R[6];
+                median_boxes(s, s.begin[nd], s.count[nd], L, R);
+                sub_children(s, bnodes, rootNode, globalBegin, nd, s.count[nd] / 2u, L, R);
             }
         }
-        const uint32_t bl = __ballot_sync(0xffffffffu, valid && left);
-        const uint32_t br = __ballot_sync(0xffffffffu, valid && !left);
-        if (valid) {
-            const uint32_t dst = left ? leftSeen + __popc(bl & lanemask_lt()) : best.nL + rightSeen + __popc(br & lanemask_lt());
-            if (dst < n) {
-                s.perm[cur ^ 1][b + dst] = (uint16_t)j;
-                s.posNode[cur ^ 1][b + dst] = (uint16_t)(left ? ch : ch + 1);
-            }
-        }
-        leftSeen += __popc(bl);
-        rightSeen += __popc(br);
+        __syncthreads();  // the bins are cleared again for the next nodes
     }
 }
 
 // levels: the binary levels that the big-task kernels ran; big tasks left
 // after them mean that the tree cannot be finished here (kCntFailed).
-__global__ void __launch_bounds__(kSubThreads, 3) k_subtree(const SmallTask* __restrict__ small,
+__global__ void __launch_bounds__(kSubThreads, 2) k_subtree(const SmallTask* __restrict__ small,
                                                             const uint32_t* __restrict__ refs0,
                                                             const uint32_t* __restrict__ refs1,
                                                             const float4* __restrict__ boxes,
@@ -930,7 +940,7 @@ __global__ void __launch_bounds__(kSubThreads, 3) k_subtree(const SmallTask* __r
 {
     extern __shared__ __align__(16) unsigned char smem[];
     SubSmem& s = *reinterpret_cast<SubSmem*>(smem);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x;
     if (cnt[kLevelBig + levels] != 0u) {
         if (blockIdx.x == 0 && tid == 0) atomicOr(cnt + kCntFailed, kFailLevels);
         return;
@@ -943,19 +953,13 @@ __global__ void __launch_bounds__(kSubThreads, 3) k_subtree(const SmallTask* __r
         if (ticket >= numSmall) break;
         const SmallTask task = small[ticket];
         const uint32_t n = min(task.count, kSmallMax), b0 = task.begin;
-        const uint32_t* refs = (task.level & 1u) ? refs1 : refs0;
-        for (uint32_t p = tid; p < n; p += kSubThreads) {
-            const uint32_t prim = refs[b0 + p];
-            float lo[3], hi[3];
-            load_box(boxes, prim, lo, hi);
-            s.prim[p] = prim;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                s.box[k][p] = lo[k];
-                s.box[3 + k][p] = hi[k];
-            }
-            s.perm[0][p] = (uint16_t)p;
-            s.posNode[0][p] = 0;
+        const bool live = tid < n;  // this thread has a position
+        if (live) {
+            const uint32_t prim = ((task.level & 1u) ? refs1 : refs0)[b0 + tid];
+            const float4 a = boxes[2ull * prim], b = boxes[2ull * prim + 1];
+            s.pa[tid] = a;
+            s.pb[tid] = make_float4(b.x, b.y, 0.0f, __uint_as_float(prim));
+            s.posNode[tid] = 0;
         }
         if (tid == 0) {
             // ids of the 2 n - 2 nodes below the root (fewer are used when leaves hold several references)
@@ -966,6 +970,7 @@ __global__ void __launch_bounds__(kSubThreads, 3) k_subtree(const SmallTask* __r
             s.left[0] = (uint16_t)kNoChild;
             const BinNode r = bnodes[task.node];
             s.area[0] = area_of(r.lo.x, r.lo.y, r.lo.z, r.hi.x, r.hi.y, r.hi.z);
+            s.binCount = 0;
         }
         __syncthreads();
         if (s.idBase + 2u * n - 2u > 2u * capPrims) {  // never in a consistent build
@@ -974,168 +979,141 @@ __global__ void __launch_bounds__(kSubThreads, 3) k_subtree(const SmallTask* __r
             continue;
         }
         uint32_t ls = 0, le = 1, lev = 0;
-        int cur = 0;
         while (ls < le) {
             if (tid == 0) s.levelStart[lev] = (uint16_t)ls;
-            for (uint32_t nd = ls + warp; nd < le; nd += kSubWarps)
-                if (s.count[nd] > kDirectMax) sub_split_warp(s, bnodes, task.node, b0, nd, s.bins[warp], cur);
-            // bins of every reference of the other nodes
-#pragma unroll
-            for (int r = 0; r < kSubRounds; ++r) {
-                const uint32_t p = r * kSubThreads + tid;
-                if (p >= n) break;
-                const uint32_t nd = s.posNode[cur][p], c = s.count[nd], b = s.begin[nd];
-                if (nd < ls || c < 2u || c > kDirectMax) continue;
-                float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, own[3];
+            uint32_t nd = 0, c = 0, b = 0;
+            if (live) {
+                nd = s.posNode[tid];
+                c = s.count[nd];
+                b = s.begin[nd];
+            }
+            const bool active = live && nd >= ls && c >= 2u, direct = active && c <= kDirectMax;
+            if (active && tid == b) {
+                s.key[nd - ls] = kNoSplit;
+                if (!direct) {
+                    const uint32_t at = atomicAdd(&s.binCount, 1u);
+                    s.binNode[at] = (uint16_t)nd;
+                    s.binSlot[nd - ls] = (uint16_t)at;
+                }
+            }
+            if (direct) {  // this reference's bins
+                float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, lo[3], hi[3];
                 for (uint32_t i = b; i < b + c; ++i) {
-                    float lo[3], hi[3];
-                    sub_box(s, s.perm[cur][i], lo, hi);
+                    sub_box(s.pa[i], s.pb[i], lo, hi);
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         const float ck = centroid(lo[k], hi[k]);
                         clo[k] = fminf(clo[k], ck);
                         chi[k] = fmaxf(chi[k], ck);
-                        if (i == p) own[k] = ck;
                     }
                 }
+                sub_box(s.pa[tid], s.pb[tid], lo, hi);
                 uint32_t v = 0;
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     const float sc = axis_scale(clo[k], chi[k]);
-                    if (sc != 0.0f) v |= ((uint32_t)bin_of(own[k], clo[k], sc) << (8 * k)) | (1u << (24 + k));
+                    if (sc != 0.0f) v |= ((uint32_t)bin_of(centroid(lo[k], hi[k]), clo[k], sc) << (8 * k)) | (1u << (24 + k));
                 }
-                s.pbin[p] = v;
-                if (p == b) s.key[nd - ls] = ~0ull;
+                s.pb[tid].z = __uint_as_float(v);
             }
             __syncthreads();
-            // each reference's candidate planes
+            if (s.binCount) sub_split_bins(s, bnodes, task.node, b0, ls, active && !direct ? s.binSlot[nd - ls] : kNoTask);
+            // this reference's candidate planes; the best one's two sides stay in registers
+            float bestL[6], bestR[6];
+            uint32_t bestN = 0;
+            unsigned long long key = kNoSplit;
+            if (direct) {
+                const uint32_t own = __float_as_uint(s.pb[tid].z);
+                float bestCost = FLT_MAX;
 #pragma unroll 1
-            for (int r = 0; r < kSubRounds; ++r) {
-                const uint32_t p = r * kSubThreads + tid;
-                if (p >= n) break;
-                const uint32_t nd = s.posNode[cur][p], c = s.count[nd], b = s.begin[nd];
-                if (nd < ls || c < 2u || c > kDirectMax) continue;
-                const uint32_t own = s.pbin[p];
-                float L[3][6], R[3][6];
-                uint32_t nL[3] = {0u, 0u, 0u};
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    box_reset(L[a]);
-                    box_reset(R[a]);
-                }
-                for (uint32_t i = b; i < b + c; ++i) {
-                    const uint32_t v = s.pbin[i];
-                    float lo[3], hi[3];
-                    sub_box(s, s.perm[cur][i], lo, hi);
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        if (((v >> (8 * a)) & 0xffu) <= ((own >> (8 * a)) & 0xffu)) {
-                            box_add(L[a], lo, hi);
-                            ++nL[a];
+                for (uint32_t a = 0; a < 3; ++a) {
+                    if (!(own & (1u << (24 + a)))) continue;
+                    const uint32_t sh = 8u * a, ob = (own >> sh) & 0xffu;
+                    float L[6], R[6];
+                    uint32_t nL = 0;
+                    box_reset(L);
+                    box_reset(R);
+                    for (uint32_t i = b; i < b + c; ++i) {
+                        const float4 pa = s.pa[i], pb = s.pb[i];
+                        float lo[3], hi[3];
+                        sub_box(pa, pb, lo, hi);
+                        if (((__float_as_uint(pb.z) >> sh) & 0xffu) <= ob) {
+                            box_add(L, lo, hi);
+                            ++nL;
                         } else {
-                            box_add(R[a], lo, hi);
+                            box_add(R, lo, hi);
+                        }
+                    }
+                    if (nL >= c) continue;
+                    const float sc = split_cost(nL, area_of(L[0], L[1], L[2], L[3], L[4], L[5]), c - nL,
+                                                area_of(R[0], R[1], R[2], R[3], R[4], R[5]));
+                    if (sc < bestCost) {
+                        bestCost = sc;
+                        key = split_key(sc, a, ob, tid);
+                        bestN = nL;
+#pragma unroll
+                        for (int k = 0; k < 6; ++k) {
+                            bestL[k] = L[k];
+                            bestR[k] = R[k];
                         }
                     }
                 }
-                float bestCost = FLT_MAX;
-                int axis = -1;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    if (!(own & (1u << (24 + a))) || nL[a] >= c) continue;
-                    const float sc = split_cost(nL[a], area_of(L[a][0], L[a][1], L[a][2], L[a][3], L[a][4], L[a][5]),
-                                                c - nL[a], area_of(R[a][0], R[a][1], R[a][2], R[a][3], R[a][4], R[a][5]));
-                    if (sc < bestCost) {
-                        bestCost = sc;
-                        axis = a;
-                    }
-                }
-                if (axis >= 0)
-                    atomicMin(&s.key[nd - ls], ((unsigned long long)__float_as_uint(bestCost) << 32) | ((uint32_t)axis << 24) |
-                                                   (((own >> (8 * axis)) & 0xffu) << 16) | p);
+                if (key != kNoSplit) atomicMin(&s.key[nd - ls], key);
             }
             __syncthreads();
             // the winner (or, without a candidate, the first reference) makes the leaf or the children
-#pragma unroll 1
-            for (int r = 0; r < kSubRounds; ++r) {
-                const uint32_t p = r * kSubThreads + tid;
-                if (p >= n) break;
-                const uint32_t nd = s.posNode[cur][p], c = s.count[nd], b = s.begin[nd];
-                if (nd < ls || c < 2u || c > kDirectMax) continue;
-                const unsigned long long key = s.key[nd - ls];
-                const bool found = key != ~0ull;
-                if (p != (found ? (uint32_t)(key & 0xffffu) : b)) continue;
-                // SAH with unit traversal and intersection costs
-                const float area = s.area[nd], splitCost = __uint_as_float((uint32_t)(key >> 32));
-                if (c <= (uint32_t)kMaxLeafTris && (!found || __fmul_rn(float(c), area) <= __fadd_rn(area, splitCost)))
-                    continue;  // a leaf
-                const uint32_t sh = 8u * ((uint32_t)(key >> 24) & 0xffu), bin = (uint32_t)(key >> 16) & 0xffu;
-                float L[6], R[6];
-                uint32_t nL = 0;
-                box_reset(L);
-                box_reset(R);
-                for (uint32_t i = b; i < b + c; ++i) {
-                    float lo[3], hi[3];
-                    sub_box(s, s.perm[cur][i], lo, hi);
-                    if (found ? ((s.pbin[i] >> sh) & 0xffu) <= bin : (i - b) < c / 2u) {
-                        box_add(L, lo, hi);
-                        ++nL;
-                    } else {
-                        box_add(R, lo, hi);
+            if (direct) {
+                const unsigned long long won = s.key[nd - ls];
+                if (won == kNoSplit ? tid == b && c > (uint32_t)kMaxLeafTris : won == key) {
+                    // SAH with unit traversal and intersection costs
+                    const float area = s.area[nd], splitCost = __uint_as_float((uint32_t)(won >> 32));
+                    if (won == kNoSplit) {
+                        bestN = c / 2u;
+                        median_boxes(s, b, c, bestL, bestR);
                     }
+                    if (won == kNoSplit || c > (uint32_t)kMaxLeafTris ||
+                        !(__fmul_rn(float(c), area) <= __fadd_rn(area, splitCost)))
+                        sub_children(s, bnodes, task.node, b0, nd, bestN, bestL, bestR);
                 }
-                sub_children(s, bnodes, task.node, b0, nd, nL, L, R);
             }
             __syncthreads();
             // stable partition of the split nodes' references
-#pragma unroll
-            for (int r = 0; r < kSubRounds; ++r) {
-                const uint32_t p = r * kSubThreads + tid;
-                bool lf = false;
-                if (p < n) {
-                    const uint32_t nd = s.posNode[cur][p], c = s.count[nd];
-                    if (nd >= ls && c <= kDirectMax && s.left[nd] != kNoChild) {
-                        const unsigned long long key = s.key[nd - ls];
-                        lf = key != ~0ull ? ((s.pbin[p] >> (8u * ((uint32_t)(key >> 24) & 0xffu))) & 0xffu) <=
-                                                ((uint32_t)(key >> 16) & 0xffu)
-                                          : p - s.begin[nd] < c / 2u;
-                    }
-                }
-                const uint32_t w = __ballot_sync(0xffffffffu, lf);
-                if (lane_id() == 0) s.leftBits[p >> 5] = w;
+            const bool split = active && s.left[nd] != kNoChild;
+            float4 pa, pb;
+            bool lf = false;
+            if (live) {
+                pa = s.pa[tid];
+                pb = s.pb[tid];
             }
-            if (tid == 0) s.levelEnd = s.nodeTop;
-            __syncthreads();
-#pragma unroll
-            for (int r = 0; r < kSubRounds; ++r) {
-                const uint32_t p = r * kSubThreads + tid;
-                if (p >= n) break;
-                const uint32_t nd = s.posNode[cur][p], c = s.count[nd], j = s.perm[cur][p];
-                uint32_t dst = p, to = nd;
-                if (nd >= ls && s.left[nd] != kNoChild) {
-                    if (c > kDirectMax) continue;  // its warp has moved it
-                    const uint32_t b = s.begin[nd], w0 = b >> 5, w1 = p >> 5, ch = s.left[nd];
-                    const uint32_t upTo = (1u << (p & 31u)) - 1u, from = 0xffffffffu << (b & 31u);
-                    const uint32_t rank = w0 == w1 ? __popc(s.leftBits[w0] & from & upTo)
-                                                   : __popc(s.leftBits[w0] & from) + __popc(s.leftBits[w1] & upTo);
-                    const bool lf = (s.leftBits[w1] >> (p & 31u)) & 1u;
-                    dst = lf ? b + rank : b + s.count[ch] + (p - b - rank);
-                    to = lf ? ch : ch + 1u;
-                }
-                s.perm[cur ^ 1][dst] = (uint16_t)j;
-                s.posNode[cur ^ 1][dst] = (uint16_t)to;
+            if (split) lf = key_left(s.key[nd - ls], __float_as_uint(pb.z), tid - b, c);
+            const uint32_t bits = __ballot_sync(0xffffffffu, lf);
+            if (lane_id() == 0) s.leftBits[tid >> 5] = bits;
+            if (tid == 0) {
+                s.levelEnd = s.nodeTop;
+                s.binCount = 0;
             }
             __syncthreads();
+            if (split) {
+                const uint32_t ch = s.left[nd], w0 = b >> 5, w1 = tid >> 5;
+                uint32_t rank = __popc(bits & ((1u << lane_id()) - 1u) & (w0 == w1 ? 0xffffffffu << (b & 31u) : 0xffffffffu));
+                if (w0 != w1) rank += __popc(s.leftBits[w0] & (0xffffffffu << (b & 31u)));
+                for (uint32_t w = w0 + 1; w < w1; ++w) rank += __popc(s.leftBits[w]);
+                const uint32_t dst = lf ? b + rank : b + s.count[ch] + (tid - b - rank);
+                s.pa[dst] = pa;
+                s.pb[dst] = pb;
+                s.posNode[dst] = (uint16_t)(lf ? ch : ch + 1u);
+            }
             ls = le;
             le = s.levelEnd;
-            cur ^= 1;
             ++lev;
+            __syncthreads();
         }
         if (tid == 0) {
             s.levelStart[lev] = (uint16_t)ls;
             atomicMax(cnt + kCntLevels, task.level + lev);
             atomicAdd(cnt + kCntRealNodes, s.nodeTop - 1u);
         }
-        for (uint32_t p = tid; p < n; p += kSubThreads) order[b0 + p] = s.prim[s.perm[cur][p]];
+        if (live) order[b0 + tid] = __float_as_uint(s.pb[tid].w);
         __syncthreads();
         if (sah) {  // the cost program, deepest level first (the bins' memory now holds the costs)
             for (uint32_t l = lev; l-- > 0;) {
@@ -1743,7 +1721,7 @@ void Builder::launch_subtrees(const Input& in, uint32_t levels, uint32_t maxLeve
     const uint32_t n = in.ntris + in.nspheres;
     const bool sah = collapse_ == kCollapseSah;
     cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SubSmem));
-    k_subtree<<<blocks_for(n, 64, 148 * 3), kSubThreads, sizeof(SubSmem), st>>>(
+    k_subtree<<<blocks_for(n, 64, 148 * 2), kSubThreads, sizeof(SubSmem), st>>>(
         static_cast<const SmallTask*>(small_), refs_[0], refs_[1], boxes_, bnodes_, order_, collapseCost_,
         collapseChoice_, triCost_, sah, counters_, levels, n);
     k_top<<<1, kTopThreads, 0, st>>>(bnodes_, collapseCost_, collapseChoice_, triCost_, sah,
