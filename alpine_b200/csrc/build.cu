@@ -16,7 +16,7 @@
 // independent), so a build is a pure function of its input.
 //
 // Wide phase: breadth-first collapse to 8 slots, two launches a level, eight
-// lanes per wide node, quantised child boxes, octant-ordered slots, triangle
+// lanes per wide node, 16-bit child boxes, octant-ordered slots, triangle
 // records in leaf order (src/accelerators/wide_bvh.cpp:430-472 packs TriangleN
 // likewise). Which binary nodes fill a wide node's slots is chosen either
 //   * SAH-optimally (the default): a bottom-up dynamic program over the
@@ -1395,17 +1395,19 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_decide(const uint2* __res
     }
 }
 
-__host__ __device__ inline uint32_t quant_exponent(float extent)
+// A plane word of bvh.cuh: the box [lo, hi] of one axis as offsets from the
+// node's origin, rounded outwards to the top 16 bits of a float.
+AG_D uint32_t plane_word(float lo, float hi, float origin)
 {
-    // smallest power of two q with 255 * q >= extent (biased exponent byte)
-    if (!(extent > 0.0f)) return 1u;
-    int e;
-    frexpf(extent / 255.0f, &e);
-    float q = ldexpf(1.0f, e);
-    if (255.0f * q < extent * 1.000001f) { e += 1; q *= 2.0f; }
-    int biased = e + 127;
-    biased = biased < 1 ? 1 : (biased > 253 ? 253 : biased);
-    return (uint32_t)biased;
+    float dl = __fsub_rd(lo, origin), dh = __fsub_ru(hi, origin);
+    dl = dl >= 0.0f ? dl : 0.0f;                      // (NaN: the origin)
+    constexpr float kNoBound = 1.7014118346046923e38f;  // 2^127: finite with any lower half
+    dh = dh <= kNoBound ? fmaxf(dh, 0.0f) : kNoBound;   // (infinite or NaN: no bound)
+    const uint32_t l16 = __float_as_uint(dl) >> 16;   // truncated: rounded down
+    const uint32_t hb = __float_as_uint(dh);
+    uint32_t h16 = hb >> 16;                          // read with the lower half below it
+    if (((h16 << 16) | l16) < hb) ++h16;
+    return (h16 << 16) | l16;
 }
 
 // Writes one wide node per group of eight lanes, a lane per slot, with its
@@ -1467,8 +1469,6 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_emit(const uint2* __restr
         const int32_t e = valid ? slots[size_t(i) * kWidth + g] : -1;
         const BinNode nb = bnodes[it.x];
         const float p[3] = {nb.lo.x, nb.lo.y, nb.lo.z};
-        const uint32_t E[3] = {quant_exponent(nb.hi.x - nb.lo.x), quant_exponent(nb.hi.y - nb.lo.y),
-                               quant_exponent(nb.hi.z - nb.lo.z)};
         BinNode c = nb;
         if (e >= 0) c = bnodes[e];
         const bool leaf = e >= 0 && c.count <= (uint32_t)kMaxLeafTris, inner = e >= 0 && !leaf;
@@ -1487,25 +1487,18 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_emit(const uint2* __restr
         if (leaf) meta = (uint8_t)((((1u << c.count) - 1u) << 5) | toff);
         if (inner) meta = (uint8_t)(0x20u | (24u + g));
         r[24 + g] = meta;
-        const float clo[3] = {c.lo.x, c.lo.y, c.lo.z}, chi[3] = {c.hi.x, c.hi.y, c.hi.z};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float q = __uint_as_float(E[k] << 23), invq = __uint_as_float((254u - E[k]) << 23);  // exact 1/q
-            const float fl = floorf((clo[k] - p[k]) * invq), fh = ceilf((chi[k] - p[k]) * invq);
-            int l = (int)fmaxf(0.0f, fminf(255.0f, fl));
-            int h = (int)fmaxf(0.0f, fminf(255.0f, fh));
-            while (l > 0 && p[k] + float(l) * q > clo[k]) --l;
-            while (h < 255 && p[k] + float(h) * q < chi[k]) ++h;
-            r[32 + 8 * k + g] = e >= 0 ? (uint8_t)l : 0xffu;
-            r[56 + 8 * k + g] = e >= 0 ? (uint8_t)h : 0u;
-        }
+        uint32_t* u = reinterpret_cast<uint32_t*>(r);
+        // an empty slot's box is inside out: minimum 1e30, maximum -1e30
+        constexpr uint32_t kEmptyPlanes = 0xf1497149u;
+        u[8 + g] = e >= 0 ? plane_word(c.lo.x, c.hi.x, p[0]) : kEmptyPlanes;
+        u[16 + g] = e >= 0 ? plane_word(c.lo.y, c.hi.y, p[1]) : kEmptyPlanes;
+        u[24 + g] = e >= 0 ? plane_word(c.lo.z, c.hi.z, p[2]) : kEmptyPlanes;
         if (g == 0) {
             float* f = reinterpret_cast<float*>(r);
-            uint32_t* u = reinterpret_cast<uint32_t*>(r);
             f[0] = p[0];
             f[1] = p[1];
             f[2] = p[2];
-            u[3] = E[0] | (E[1] << 8) | (E[2] << 16) | (imask << 24);
+            u[3] = imask;
             u[4] = childBase;
             u[5] = triAt;
             if (valid) sah += bn_area(nb) * ria;  // one node visit

@@ -1,17 +1,24 @@
 // BVH layouts in HBM.
 //
-// Wide node (80 bytes, five 16-byte words, read with five 128-bit loads):
-//   word0: float px, py, pz          quantisation origin = node box minimum
-//          u8 ex, ey, ez             biased exponents: child box quantum 2^(e-127)
-//          u8 imask                  bit s set <=> slot s holds an internal child
-//   word1: u32 childBase             index of the first internal child node
-//          u32 triBase               index of the first triangle record
-//          u8 meta[8]                per slot: empty = 0;
+// Wide node (128 bytes, one cache line, read with four 256-bit loads):
+//   words 0-7:   float px, py, pz    origin = node box minimum
+//                u32 imask           bit s set <=> slot s holds an internal child
+//                u32 childBase       index of the first internal child node
+//                u32 triBase         index of the first triangle record
+//                u8 meta[8]          per slot: empty = 0;
 //                                    internal = 0x20 | (24 + slot);
 //                                    leaf = (unary count << 5) | triangle offset
-//   word2: u8 qlox[8], qloy[8]       child box minima, in quanta, rounded down
-//   word3: u8 qloz[8], qhix[8]
-//   word4: u8 qhiy[8], qhiz[8]       child box maxima, in quanta, rounded up
+//   words 8-31:  u32 planes[3][8]    per axis and slot the child's box, as offsets
+//                                    from the origin in the top 16 bits of a float:
+//                                    minimum (rounded down) in the lower half,
+//                                    maximum in the upper. The maximum is read as
+//                                    the whole word, so the lower half is part of
+//                                    its value; it is rounded up with that counted.
+// A word becomes the near or the far plane by one integer multiplication (by
+// 65536 or 1, chosen per ray and axis by the direction's sign). The 80-byte
+// node before it held the planes as bytes of a per-axis quantum, which took
+// 64 conversions and 12 selections a node on the conversion unit and the ALU;
+// see traverse.cuh for what that cost.
 // Internal children are stored contiguously from childBase in slot order, so
 // slot s lives at childBase + popc(imask & ((1 << s) - 1)). Leaf children hold
 // 1-3 triangles; the triangles of one node are contiguous from triBase (at
@@ -32,16 +39,17 @@
 
 namespace ag {
 
-struct alignas(16) WideNode {
+constexpr int kWidth = 8;
+
+struct alignas(128) WideNode {
     float px, py, pz;
-    uint32_t e_imask;     // ex | ey << 8 | ez << 16 | imask << 24
+    uint32_t imask;
     uint32_t childBase;
     uint32_t triBase;
     uint32_t meta[2];
-    uint32_t qlo[3][2];   // [axis][bytes 0-3, 4-7]
-    uint32_t qhi[3][2];
+    uint32_t planes[3][kWidth];
 };
-static_assert(sizeof(WideNode) == 80, "wide node is 80 bytes");
+static_assert(sizeof(WideNode) == 128, "wide node is 128 bytes");
 
 struct alignas(16) TriRecord {
     float4 v0;   // w = prim id (bits)
@@ -65,7 +73,6 @@ static_assert(sizeof(BinNode) == 48, "binary node is 48 bytes");
 constexpr uint32_t kSpherePrim = 0x80000000u;  // hit / record prim ids of spheres carry this bit
 constexpr uint32_t kSphereTag = 1u;            // e0.w bits of a sphere record
 
-constexpr int kWidth = 8;
 constexpr int kMaxLeafTris = 3;          // unary count field holds 1..3
 constexpr int kSahBins = 32;             // binned SAH resolution
 #ifndef AG_TRAVERSAL_STACK

@@ -159,7 +159,7 @@ struct alpine_gpu_ctx {
     uint32_t totalSamples = 0;
     ag::DeviceBuffer dWave;
     uint32_t waveCapacity = 0;
-    int traceBlock = 128;             // k_trace_dyn block size (autotuned)
+    int traceBlock = 64;              // k_trace_dyn block size (autotuned)
     // CUDA-graph replay of the render loop: the captured graph and the launch
     // configuration it was captured for
     cudaGraphExec_t graphExec = nullptr;

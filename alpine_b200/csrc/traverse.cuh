@@ -11,8 +11,8 @@
 // The binary-BVH rule (kBinary, src/accelerators/bvh_common.cpp:66-103) is
 // selectable per launch: |det| >= FLT_EPSILON, t, b1, b2 by IEEE division,
 // b1 <= 1 and b2 <= 1 - b1, with the reference's order of tests. Child
-// boxes are tested conservatively (quantised boxes are rounded outwards and
-// the exit distance is scaled by 1 + 4e-7 as bounding_box.ispc:29 does).
+// boxes are tested conservatively (their planes are rounded outwards and the
+// exit distance is scaled by 1 + 4e-7 as bounding_box.ispc:29 does).
 //
 // Traversal order: a node group {childBase, hits | imask} holds the pending
 // internal children of one node in bits 24-31 (position = slot ^ octant of
@@ -133,22 +133,27 @@ AG_D float safe_rcp(float d)
     return __frcp_rn(a);
 }
 
-AG_D uint4 ldg4(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
-
-// Exact float value of byte k of w, by the conversion unit (I2F, XU pipe) or
-// by placing the byte under the exponent of 2^23 (PRMT) and subtracting 2^23
-// (FADD), which runs on the ALU and FMA pipes. Bit i of AG_CVT_PRMT_MASK
-// selects the second form for plane group i (near x, y, z, far x, y, z), so
-// the 48 conversions of a node can be split between the pipes.
-#ifndef AG_CVT_PRMT_MASK
-#define AG_CVT_PRMT_MASK 0x12  // measured best on B200: y planes on ALU + FMA, the rest on XU
-#endif
-template <int kGroup>
-AG_D float byte_to_float(uint32_t w, uint32_t k)
+// 32 bytes by one 256-bit load (p 32-byte aligned).
+AG_D void ldg8(const void* p, uint32_t (&w)[8])
 {
-    if ((AG_CVT_PRMT_MASK >> kGroup) & 1)
-        return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u | k)) - 8388608.0f;
-    return float((w >> (8 * k)) & 0xffu);
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+        : "l"(p));
+}
+
+AG_D uint64_t pack2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+// x = a * m.lo + c.lo, y = b * m.hi + c.hi, each rounded once (a, b: float bits).
+AG_D void fma2(uint32_t a, uint32_t b, uint64_t m, uint64_t c, float& x, float& y)
+{
+    const uint64_t v = pack2(__uint_as_float(a), __uint_as_float(b));
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(v), "l"(m), "l"(c));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(r));
 }
 
 AG_D float max3f(float a, float b, float c)
@@ -164,46 +169,64 @@ AG_D float min3f(float a, float b, float c)
     return r;
 }
 
-// Intersects the 8 child boxes of a node; returns the hit mask (internal
-// children at bits 24 + (slot ^ oct), triangles at their offsets).
-AG_D uint32_t intersect_children(const uint4& w0, const uint4& w1, const uint4& w2, const uint4& w3, const uint4& w4,
-                                 float3 o, float3 id, uint32_t oct, float tmin, float tmax)
+// Per axis, the multipliers that bring a plane word's near and far half to the
+// top 16 bits (bvh.cuh): near = minimum for a positive direction.
+struct PlaneMul {
+    uint32_t nx, ny, nz, fx, fy, fz;
+};
+AG_D uint32_t plane_mul(bool upper)
 {
-    const float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
-    const uint32_t e = w0.w;
-    const float sx = __fmul_rn(__uint_as_float((e & 0xffu) << 23), id.x);
-    const float sy = __fmul_rn(__uint_as_float(((e >> 8) & 0xffu) << 23), id.y);
-    const float sz = __fmul_rn(__uint_as_float(((e >> 16) & 0xffu) << 23), id.z);
-    const float ox = __fmul_rn(__fsub_rn(px, o.x), id.x);
-    const float oy = __fmul_rn(__fsub_rn(py, o.y), id.y);
-    const float oz = __fmul_rn(__fsub_rn(pz, o.z), id.z);
-    // near / far planes per axis chosen by the direction sign
-    const bool nx = oct & 1u, ny = oct & 2u, nz = oct & 4u;
-    const uint32_t nearX[2] = {nx ? w3.z : w2.x, nx ? w3.w : w2.y};
-    const uint32_t farX[2] = {nx ? w2.x : w3.z, nx ? w2.y : w3.w};
-    const uint32_t nearY[2] = {ny ? w4.x : w2.z, ny ? w4.y : w2.w};
-    const uint32_t farY[2] = {ny ? w2.z : w4.x, ny ? w2.w : w4.y};
-    const uint32_t nearZ[2] = {nz ? w4.z : w3.x, nz ? w4.w : w3.y};
-    const uint32_t farZ[2] = {nz ? w3.x : w4.z, nz ? w3.y : w4.w};
-    const uint32_t meta[2] = {w1.z, w1.w};
+    // opaque: knowing that it is 1 or 65536, the compiler would select between
+    // the word and its shift, on the ALU that bounds the kernel
+    uint32_t m;
+    asm volatile("mov.u32 %0, %1;" : "=r"(m) : "r"(upper ? 1u : 65536u));
+    return m;
+}
+
+// Intersects the 8 child boxes of a node (its 32 words); returns the hit mask
+// (internal children at bits 24 + (slot ^ oct), triangles at their offsets).
+//
+// The traversal kernels are bound by instruction issue and the ALU (about 9 of
+// 32 lanes active, DRAM and L2 nearly idle). Against byte planes (64
+// conversions a node, I2F on the conversion unit and PRMT + FADD), the 16-bit
+// planes with the selecting multiplications on the FMA pipe, the packed FMAs
+// and byte-parallel meta decoding take 17 % fewer instructions. Measured on
+// B200, 2M rays, 1M-triangle soup: incoherent closest hit 3.01 to 2.66 ms,
+// primary 2.00 to 1.70 ms, incoherent any hit 2.52 to 2.18 ms; interior of 2M
+// triangles, incoherent 0.96 to 0.88 ms. The same with separate FMAs 2.77 ms,
+// with the halves selected instead of multiplied 2.96 ms, with an
+// unconditional hit mask 3.2 ms (incoherent closest hit).
+AG_D uint32_t intersect_children(const uint32_t (&hd)[8], const uint32_t (&X)[8], const uint32_t (&Y)[8],
+                                 const uint32_t (&Z)[8], float3 o, float3 id, uint32_t oct, const PlaneMul& mul,
+                                 float tmin, float tmax)
+{
+    const float ox = __fmul_rn(__fsub_rn(__uint_as_float(hd[0]), o.x), id.x);
+    const float oy = __fmul_rn(__fsub_rn(__uint_as_float(hd[1]), o.y), id.y);
+    const float oz = __fmul_rn(__fsub_rn(__uint_as_float(hd[2]), o.z), id.z);
+    const uint64_t idx2 = pack2(id.x, id.x), idy2 = pack2(id.y, id.y), idz2 = pack2(id.z, id.z);
+    const uint64_t ox2 = pack2(ox, ox), oy2 = pack2(oy, oy), oz2 = pack2(oz, oz);
     uint32_t hits = 0;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
+        // four meta bytes at once: internal slots (positions 24..31: bits 3 and
+        // 4 set) are permuted by the octant
+        const uint32_t meta = hd[6 + h];
+        const uint32_t inner = ((meta & (meta << 1)) & 0x10101010u) >> 4;
+        const uint32_t pos = (meta ^ (inner * oct)) & 0x1f1f1f1fu;
+        const uint32_t bits = (meta >> 5) & 0x07070707u;
 #pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) {
-            float tnx = fmaf(byte_to_float<0>(nearX[h], k), sx, ox);
-            float tny = fmaf(byte_to_float<1>(nearY[h], k), sy, oy);
-            float tnz = fmaf(byte_to_float<2>(nearZ[h], k), sz, oz);
-            float tfx = fmaf(byte_to_float<3>(farX[h], k), sx, ox);
-            float tfy = fmaf(byte_to_float<4>(farY[h], k), sy, oy);
-            float tfz = fmaf(byte_to_float<5>(farZ[h], k), sz, oz);
-            float tn = max3f(tnx, tny, fmaxf(tnz, tmin));
-            float tf = min3f(tfx, tfy, tfz) * kBoxExitScale;
+        for (int k = 0; k < 4; ++k) {
+            const int c = 4 * h + k;
+            float tnx, tny, tnz, tfx, tfy, tfz;
+            fma2(X[c] * mul.nx, X[c] * mul.fx, idx2, ox2, tnx, tfx);
+            fma2(Y[c] * mul.ny, Y[c] * mul.fy, idy2, oy2, tny, tfy);
+            fma2(Z[c] * mul.nz, Z[c] * mul.fz, idz2, oz2, tnz, tfz);
+            const float tn = max3f(tnx, tny, fmaxf(tnz, tmin));
+            const float tf = min3f(tfx, tfy, tfz) * kBoxExitScale;
             if (tn <= tf && tn <= tmax) {
-                uint32_t m = (meta[h] >> (8 * k)) & 0xffu;
-                uint32_t low = m & 0x1fu;
-                uint32_t pos = low >= 24u ? (low ^ oct) : low;
-                hits |= (m >> 5) << pos;
+                uint32_t b = __byte_perm(bits, 0u, 0x4440u | k);
+                asm("shf.l.wrap.b32 %0, %1, %2, %3;" : "=r"(b) : "r"(0u), "r"(b), "r"(pos >> (8 * k)));
+                hits |= b;
             }
         }
     }
@@ -215,6 +238,7 @@ struct RayState {
     float3 o, d, id;
     float tmin, tmax;
     uint32_t oct;
+    PlaneMul mul;
     uint2 ngroup, tgroup;
     int sp;
     uint32_t visits;
@@ -230,6 +254,12 @@ AG_D void ray_init(RayState& s, float3 o, float3 d, float tmin, float tmax)
     s.tmin = tmin;
     s.tmax = tmax;
     s.oct = (s.id.x < 0.0f ? 1u : 0u) | (s.id.y < 0.0f ? 2u : 0u) | (s.id.z < 0.0f ? 4u : 0u);
+    s.mul.nx = plane_mul(s.oct & 1u);
+    s.mul.ny = plane_mul(s.oct & 2u);
+    s.mul.nz = plane_mul(s.oct & 4u);
+    s.mul.fx = plane_mul(!(s.oct & 1u));
+    s.mul.fy = plane_mul(!(s.oct & 2u));
+    s.mul.fz = plane_mul(!(s.oct & 4u));
     s.ngroup = make_uint2(0u, (1u << (24u + s.oct)) | 1u);  // the root as slot 0 of a virtual parent
     s.tgroup = make_uint2(0u, 0u);
     s.sp = 0;
@@ -295,11 +325,15 @@ AG_D bool ray_step(const BvhView& bvh, RayState& s, uint2* stack, int stride, ui
     if (child >= bvh.nodeCount) { err |= kErrBadIndex; s.found = false; return true; }
     if (++s.visits > bvh.maxVisits) { err |= kErrIterations; s.found = false; return true; }
     ++nodeVisits;
-    const uint4* np = reinterpret_cast<const uint4*>(bvh.nodes + child);
-    uint4 w0 = ldg4(np), w1 = ldg4(np + 1), w2 = ldg4(np + 2), w3 = ldg4(np + 3), w4 = ldg4(np + 4);
-    uint32_t hits = intersect_children(w0, w1, w2, w3, w4, s.o, s.id, s.oct, s.tmin, s.tmax);
-    s.ngroup = make_uint2(w1.x, (hits & 0xff000000u) | (w0.w >> 24));
-    s.tgroup = make_uint2(w1.y, hits & 0x00ffffffu);
+    const uint32_t* np = reinterpret_cast<const uint32_t*>(bvh.nodes + child);
+    uint32_t hd[8], X[8], Y[8], Z[8];
+    ldg8(np, hd);
+    ldg8(np + 8, X);
+    ldg8(np + 16, Y);
+    ldg8(np + 24, Z);
+    const uint32_t hits = intersect_children(hd, X, Y, Z, s.o, s.id, s.oct, s.mul, s.tmin, s.tmax);
+    s.ngroup = make_uint2(hd[4], (hits & 0xff000000u) | hd[3]);
+    s.tgroup = make_uint2(hd[5], hits & 0x00ffffffu);
     return false;
 }
 

@@ -58,7 +58,7 @@ sys.path.insert(0, ROOT)
 METRIC = "traversal Mrays/s (closest+any hit) vs CPU host"
 UNIT = "Mrays/s"
 WORKLOAD = "traversal microbenchmark: 1,048,576-tri soup, 4,194,304 closest + 4,194,304 any-hit rays"
-NODE_BYTES = 80
+NODE_BYTES = 128
 TRI_BYTES = 48
 RAY_BYTES = 32
 HIT_BYTES = 16

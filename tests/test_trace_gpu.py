@@ -276,3 +276,28 @@ def test_full_size_traversal_workload(ctx):
     ob = oracle.OracleBvh(tris)
     ref = ob.closest(closest[sample])
     compare_closest(closest[sample], tris, hits[sample], *ref[:4])
+
+
+@pytest.mark.parametrize("kind", ["near", "far", "large", "thin", "infinite"])
+def test_child_box_planes(ctx, kind):
+    """The 16-bit planes of the child boxes never cut off a hit: small and
+    large coordinates, far from the origin, boxes without thickness on one
+    axis, and a triangle with infinite vertices among finite ones."""
+    n = 3000
+    verts, idx = scenes.triangle_soup(n, seed=91, mu=np.log(0.03))
+    scale, offset = {"near": (1.0, -0.5), "far": (1.0, 64.0), "large": (3.0e5, -1.0e5)}.get(kind, (1.0, 0.0))
+    verts = (verts * np.float32(scale) + np.float32(offset)).astype(np.float32)
+    if kind == "thin":  # every triangle in an axis-aligned plane
+        v = verts.reshape(n, 3, 3)
+        for a in range(3):
+            v[a::3, :, a] = v[a::3, :1, a]
+    if kind == "infinite":
+        verts[30:33] = [[np.inf, 0.2, 0.3], [0.1, np.inf, 0.3], [0.1, 0.2, np.inf]]
+    _load(ctx, verts, idx)
+    rays = np.concatenate([scenes.primary_rays(64, 32), scenes.incoherent_rays(4000, seed=92)])
+    rays[:, 0:3] = rays[:, 0:3] * np.float32(scale) + np.float32(offset)
+    if kind == "thin":  # and rays along the axes
+        rays[::2, 4:7] = np.eye(3, dtype=np.float32)[np.arange(len(rays[::2])) % 3]
+    tris = oracle.make_tris(verts, idx)
+    compare_closest(rays, tris, ctx.trace(rays), *oracle.closest_brute(rays, tris)[:4])
+    assert (ctx.occluded(rays) == oracle.any_brute(rays, tris)).all()
