@@ -16,10 +16,8 @@ constexpr int kInferWarps = 8;
 
 // Shared-memory strides, padded so that the mma fragment loads of a warp
 // (8 rows x 4 words) fall in 32 different banks: activation rows of 72 bf16
-// (36 words, rows 4 banks apart), weight rows of in + 8, and rows of 40 bf16
-// for the transposed [64][32] buffers (20 words).
+// (36 words, rows 4 banks apart) and weight rows of in + 8.
 constexpr int kLd = kHidden + 8;
-constexpr int kLdT = 32 + 8;
 __host__ __device__ constexpr int wld(int l) { return layer_in(l) + 8; }
 __host__ __device__ constexpr int wsm_offset(int l)
 {
@@ -37,121 +35,196 @@ AG_D uint32_t pack_bf2(float a, float b)
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// Packed [out][in] weights of every layer into the padded shared copy.
-AG_D void load_weights(const __nv_bfloat16* __restrict__ g, __nv_bfloat16* s)
-{
-    for (int l = 0; l < kLayers; ++l) {
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(g + layer_offset(l));
-        uint32_t* dst = reinterpret_cast<uint32_t*>(s + wsm_offset(l));
-        const int words = layer_in(l) / 2, rows = layer_out(l);
-        for (int i = threadIdx.x; i < rows * words; i += blockDim.x) dst[(i / words) * (wld(l) / 2) + i % words] = src[i];
-    }
-}
-
-// Encodes the 64 inputs of one query into a bf16 row. The corner loads of
-// kEncodeLevels levels are issued together, the trilinear weights formed
-// after them (2, 4 and 8 levels per round measured the same).
+// Encodes the 64 inputs of one query per lane into a bf16 row (16-byte
+// aligned, written 16 bytes at a time: with the padded row stride four-byte
+// stores had four lanes to a bank). Called by whole warps.
+//
+// Inference is bound by the L1 data pipe, which the corner gathers fill. The
+// two corners of a cell that differ in x are neighbours in the table (an even
+// x pairs with x + 1 in dense and hashed levels alike; an odd one does in
+// dense levels), three times out of four in the same 32-byte sector. So lanes
+// work in pairs: the even lane loads the corners at x, the odd lane those at
+// x + 1, of both lanes' queries in turn, and one wavefront serves both lanes
+// where each corner's load took its own. The values then change lanes by
+// shuffles and are summed in corner order as before.
+// The loads of kEncodeLevels levels are issued together.
 constexpr int kEncodeLevels = 4;
-static_assert(kLevels % kEncodeLevels == 0, "levels per round");
+static_assert(kLevels % kEncodeLevels == 0 && kEncodeLevels * kFeatures % 8 == 0, "levels per round");
 AG_D void encode_row(const Params& g, const Query& q, __nv_bfloat16* row)
 {
     const float3 p = normalise_position(g, mk3(q.pos[0], q.pos[1], q.pos[2]));
-#pragma unroll
-    // one corner's kFeatures fp16 values in one load
+    // one corner's kFeatures fp16 values
+    constexpr int kWords = kFeatures / 2;
+    const uint32_t odd = threadIdx.x & 1u;
+    const float3 other = mk3(__shfl_xor_sync(0xffffffffu, p.x, 1), __shfl_xor_sync(0xffffffffu, p.y, 1),
+                             __shfl_xor_sync(0xffffffffu, p.z, 1));
+    const float3 pe = odd ? other : p, po = odd ? p : other;  // the even and the odd lane's query
     using Corner = typename std::conditional<kFeatures == 4, uint2, uint32_t>::type;
+    uint4* out = reinterpret_cast<uint4*>(row);
+#pragma unroll
     for (int l0 = 0; l0 < kLevels; l0 += kEncodeLevels) {
-        Corner v[kEncodeLevels][8];
+        Corner ve[kEncodeLevels][4], vo[kEncodeLevels][4];  // corners 2 c + odd of the two queries
 #pragma unroll
-        for (int j = 0; j < kEncodeLevels; ++j)
+        for (int j = 0; j < kEncodeLevels; ++j) {
+            const __half* table = g.grid + (uint64_t)(l0 + j) * kTableSize * kFeatures;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                uint32_t idx;
+            for (int c = 0; c < 4; ++c) {
+                uint32_t ie, io;
                 float w;
-                grid_corner(g.res[l0 + j], p, c, idx, w);
-                v[j][c] = *reinterpret_cast<const Corner*>(g.grid + ((uint64_t)(l0 + j) * kTableSize + idx) * kFeatures);
+                grid_corner(g.res[l0 + j], pe, 2 * c + (int)odd, ie, w);
+                grid_corner(g.res[l0 + j], po, 2 * c + (int)odd, io, w);
+                ve[j][c] = *reinterpret_cast<const Corner*>(table + (uint64_t)ie * kFeatures);
+                vo[j][c] = *reinterpret_cast<const Corner*>(table + (uint64_t)io * kFeatures);
             }
+        }
+        uint32_t word[kEncodeLevels * kFeatures / 2];
 #pragma unroll
         for (int j = 0; j < kEncodeLevels; ++j) {
             float f[kFeatures] = {};
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                uint32_t idx;
-                float w;
-                grid_corner(g.res[l0 + j], p, c, idx, w);
-                const __half2* h = reinterpret_cast<const __half2*>(&v[j][c]);
+            for (int c = 0; c < 4; ++c) {
+                uint32_t even[kWords], oddv[kWords];  // this lane's query: corners 2 c and 2 c + 1
 #pragma unroll
-                for (int k = 0; k < kFeatures / 2; ++k) {  // one rounding per corner, in corner order
-                    f[2 * k] = __fmaf_rn(w, __low2float(h[k]), f[2 * k]);
-                    f[2 * k + 1] = __fmaf_rn(w, __high2float(h[k]), f[2 * k + 1]);
+                for (int k = 0; k < kWords; ++k) {
+                    const uint32_t e = reinterpret_cast<const uint32_t*>(&ve[j][c])[k];
+                    const uint32_t o = reinterpret_cast<const uint32_t*>(&vo[j][c])[k];
+                    const uint32_t keep = odd ? o : e;
+                    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? e : o, 1);
+                    even[k] = odd ? got : keep;
+                    oddv[k] = odd ? keep : got;
+                }
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    uint32_t idx;
+                    float w;
+                    grid_corner(g.res[l0 + j], p, 2 * c + x, idx, w);
+                    const __half2* h = reinterpret_cast<const __half2*>(x ? oddv : even);
+#pragma unroll
+                    for (int k = 0; k < kWords; ++k) {  // one rounding per corner, in corner order
+                        f[2 * k] = __fmaf_rn(w, __low2float(h[k]), f[2 * k]);
+                        f[2 * k + 1] = __fmaf_rn(w, __high2float(h[k]), f[2 * k + 1]);
+                    }
                 }
             }
 #pragma unroll
-            for (int k = 0; k < kFeatures; k += 2)
-                *reinterpret_cast<uint32_t*>(row + kFeatures * (l0 + j) + k) = pack_bf2(f[k], f[k + 1]);
+            for (int k = 0; k < kFeatures; k += 2) word[(kFeatures * j + k) / 2] = pack_bf2(f[k], f[k + 1]);
         }
+#pragma unroll
+        for (int k = 0; k < kEncodeLevels * kFeatures / 8; ++k)
+            out[kFeatures * l0 / 8 + k] = make_uint4(word[4 * k], word[4 * k + 1], word[4 * k + 2], word[4 * k + 3]);
     }
     float ex[8];
     extra_inputs(mk3(q.wo[0], q.wo[1], q.wo[2]), mk3(q.n[0], q.n[1], q.n[2]), q.rough, ex);
+    out[kGridDims / 8] = make_uint4(pack_bf2(ex[0], ex[1]), pack_bf2(ex[2], ex[3]), pack_bf2(ex[4], ex[5]), pack_bf2(ex[6], ex[7]));
 #pragma unroll
-    for (int k = 0; k < 8; k += 2) *reinterpret_cast<uint32_t*>(row + kGridDims + k) = pack_bf2(ex[k], ex[k + 1]);
-#pragma unroll
-    for (int k = kGridDims + 8; k < kIn; k += 2) *reinterpret_cast<uint32_t*>(row + k) = 0u;
+    for (int k = kGridDims / 8 + 1; k < kIn / 8; ++k) out[k] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// acc = X[32 x K] * Wl^T for one warp's 32 rows: X row-major (stride kLd),
-// Wl [N][K] row-major (stride ldw), fragments as mma m16n8k16 leaves them.
-template <int N, int K>
-AG_D void warp_layer(const __nv_bfloat16* X, const __nv_bfloat16* Wl, int ldw, float (&acc)[2][N / 8][4])
+// Packed [out][in] weights of every layer into the padded shared copy, 16
+// bytes at a time. outRow: the packed row that goes to row r of the output layer.
+template <typename OutRow>
+AG_D void load_weights(const __nv_bfloat16* __restrict__ g, __nv_bfloat16* s, OutRow outRow)
 {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
+    for (int l = 0; l < kLayers; ++l) {
+        const uint4* src = reinterpret_cast<const uint4*>(g + layer_offset(l));
+        uint4* dst = reinterpret_cast<uint4*>(s + wsm_offset(l));
+        constexpr int kChunks = kIn / 8;
+        for (int i = threadIdx.x; i < layer_out(l) * kChunks; i += blockDim.x) {
+            const int r = i / kChunks, k = i % kChunks;
+            dst[r * (wld(l) / 8) + k] = src[(l == kLayers - 1 ? outRow(r) : r) * kChunks + k];
+        }
+    }
+}
+
+// Four 8 x 8 bf16 matrices from shared memory (a row address per lane).
+AG_D void ldmatrix4(const __nv_bfloat16* p, uint32_t (&r)[4])
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+
+AG_D void ldmatrix4_trans(const __nv_bfloat16* p, uint32_t (&r)[4])
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+AG_D void stmatrix4_trans(__nv_bfloat16* p, const uint32_t (&r)[4])
+{
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(p)),
+                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+                 : "memory");
+}
+
+// The activations of one warp's 16 MT rows as mma A fragments in registers:
+// [m tile][k step of 16][4]. The accumulators of the n tiles 2j and 2j + 1 of
+// a layer are, rounded to bf16, exactly the fragments of k step j of the
+// next, so activations pass from layer to layer without shared memory (a
+// third of the inference kernel's L1 data-pipe traffic before).
+template <int MT>
+using Fragments = uint32_t[MT][kHidden / 16][4];
+
+template <int MT>
+AG_D void load_fragments(const __nv_bfloat16* X, Fragments<MT>& A)
+{
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-        for (int nt = 0; nt < N / 8; ++nt) {
-            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-            for (int ks = 0; ks < K / 16; ++ks) {
-                const __nv_bfloat16* a = X + (mt * 16 + g) * kLd + ks * 16 + 2 * t;
-                const __nv_bfloat16* b = Wl + (nt * 8 + g) * ldw + ks * 16 + 2 * t;
-                mma_bf16(c, ld32(a), ld32(a + 8 * kLd), ld32(a + 8), ld32(a + 8 * kLd + 8), ld32(b), ld32(b + 8));
+        for (int ks = 0; ks < kIn / 16; ++ks)
+            ldmatrix4(X + (mt * 16 + (lane & 15)) * kLd + ks * 16 + (lane >> 4) * 8, A[mt][ks]);
+}
+
+// acc[mt] = the n tile's 8 columns of A * Wl^T (k steps in ascending order).
+template <int MT>
+AG_D void fragment_tile(const Fragments<MT>& A, const __nv_bfloat16* Wl, int ldw, int nt, float (&acc)[MT][4])
+{
+    const int lane = threadIdx.x & 31;
+    const __nv_bfloat16* w = Wl + (nt * 8 + (lane & 7)) * ldw + (lane >> 3) * 8;
+    uint32_t B[2][4];
+    ldmatrix4(w, B[0]);
+    ldmatrix4(w + 32, B[1]);
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[mt][k] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < kHidden / 16; ++ks)
+            mma_bf16(acc[mt], A[mt][ks][0], A[mt][ks][1], A[mt][ks][2], A[mt][ks][3], B[ks / 2][2 * (ks & 1)],
+                     B[ks / 2][2 * (ks & 1) + 1]);
+    }
+}
+
+// One hidden layer in registers: A = bf16(relu(A * Wl^T)).
+template <int MT>
+AG_D void fragment_layer(Fragments<MT>& A, const __nv_bfloat16* Wl, int ldw)
+{
+    Fragments<MT> out;
+#pragma unroll
+    for (int j = 0; j < kHidden / 16; ++j)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float acc[MT][4];
+            fragment_tile<MT>(A, Wl, ldw, 2 * j + half, acc);
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                out[mt][j][2 * half] = pack_bf2(fmaxf(acc[mt][0], 0.0f), fmaxf(acc[mt][1], 0.0f));
+                out[mt][j][2 * half + 1] = pack_bf2(fmaxf(acc[mt][2], 0.0f), fmaxf(acc[mt][3], 0.0f));
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) acc[mt][nt][k] = c[k];
         }
-    }
-}
-
-// X = bf16(relu(acc)) (call after every lane has finished reading X).
-template <int N>
-AG_D void store_relu(__nv_bfloat16* X, const float (&acc)[2][N / 8][4])
-{
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < N / 8; ++nt) {
-            const int r = mt * 16 + g, col = nt * 8 + 2 * t;
-            *reinterpret_cast<uint32_t*>(X + r * kLd + col) =
-                pack_bf2(fmaxf(acc[mt][nt][0], 0.0f), fmaxf(acc[mt][nt][1], 0.0f));
-            *reinterpret_cast<uint32_t*>(X + (r + 8) * kLd + col) =
-                pack_bf2(fmaxf(acc[mt][nt][2], 0.0f), fmaxf(acc[mt][nt][3], 0.0f));
-        }
+        for (int j = 0; j < kHidden / 16; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) A[mt][j][k] = out[mt][j][k];
 }
-
-// Hidden layers of one warp's 32 rows in place; saved (optional) receives
-// the input of every layer ([kLayers][32][kLd]). Leaves the input of the
-// output layer in X.
-AG_D void hidden_layers(const __nv_bfloat16* W, __nv_bfloat16* X, __nv_bfloat16* saved)
-{
-    for (int l = 0; l < kLayers - 1; ++l) {
-        float acc[2][kHidden / 8][4];
-        warp_layer<kHidden, kHidden>(X, W + wsm_offset(l), wld(l), acc);
-        __syncwarp();
-        store_relu<kHidden>(saved ? saved + (l + 1) * 32 * kLd : X, acc);
-        if (saved) X = saved + (l + 1) * 32 * kLd;
-        __syncwarp();
-    }
-}
+static_assert(kIn == kHidden, "every layer has the same four k steps, the hidden layers the same shape");
 
 // The inference kernel's shared copy of the output layer has its rows (the
 // output units) permuted so that each lane's mma fragments hold whole lobes:
@@ -162,20 +235,6 @@ AG_D void hidden_layers(const __nv_bfloat16* W, __nv_bfloat16* X, __nv_bfloat16*
 __host__ __device__ constexpr int out_column_raw(int c)
 {
     return c >= 40 ? c : (2 * ((c % 8) / 2) + (2 * (c / 8) + c % 2) / 5) * 5 + (2 * (c / 8) + c % 2) % 5;
-}
-
-AG_D void load_weights_infer(const __nv_bfloat16* __restrict__ g, __nv_bfloat16* s)
-{
-    for (int l = 0; l < kLayers; ++l) {
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(g + layer_offset(l));
-        uint32_t* dst = reinterpret_cast<uint32_t*>(s + wsm_offset(l));
-        const int words = layer_in(l) / 2, rows = layer_out(l);
-        for (int i = threadIdx.x; i < rows * words; i += blockDim.x) {
-            const int r = i / words, k = i % words;
-            const int from = l == kLayers - 1 ? out_column_raw(r) : r;
-            dst[r * (wld(l) / 2) + k] = src[from * words + k];
-        }
-    }
 }
 
 // Writes the output tile of one warp's 32 queries (acc: the mma fragments of
@@ -201,12 +260,13 @@ AG_D void write_outputs(const float (&acc)[2][kOut / 8][4], uint32_t row0, uint3
                     r[j][v] = acc[mt][sIdx / 2][2 * h + sIdx % 2];
                 }
             if (!packed) {
-                if (gr < n)
+                if (gr < n) {  // ten consecutive values per lane
+                    float2* o = reinterpret_cast<float2*>(out + (uint64_t)gr * 40 + 2 * t4 * kRawPerLobe);
 #pragma unroll
-                    for (int j = 0; j < 2; ++j)
-#pragma unroll
-                        for (int v = 0; v < kRawPerLobe; ++v)
-                            out[(uint64_t)gr * 40 + (2 * t4 + j) * kRawPerLobe + v] = r[j][v];
+                    for (int v = 0; v < kRawPerLobe; ++v)
+                        o[v] = make_float2(r[2 * v / kRawPerLobe][2 * v % kRawPerLobe],
+                                           r[(2 * v + 1) / kRawPerLobe][(2 * v + 1) % kRawPerLobe]);
+                }
                 continue;
             }
             float mx = fmaxf(r[0][4], r[1][4]);
@@ -236,22 +296,29 @@ __global__ void __launch_bounds__(32 * kInferWarps, 2) k_infer(Params g, const Q
     __nv_bfloat16* W = reinterpret_cast<__nv_bfloat16*>(smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __nv_bfloat16* X = W + kWsm + warp * 32 * kLd;
-    load_weights_infer(g.W, W);
+    load_weights(g.W, W, [](int r) { return out_column_raw(r); });
     __syncthreads();
     const uint32_t chunks = (n + 31) / 32;
     for (uint32_t ch = blockIdx.x * kInferWarps + warp; ch < chunks; ch += gridDim.x * kInferWarps) {
         const uint32_t i = ch * 32 + lane;
-        if (i < n) {
-            encode_row(g, q[i], X + lane * kLd);
-        } else {
-            for (int k = 0; k < kIn; ++k) X[lane * kLd + k] = bf(0.0f);
-        }
+        encode_row(g, q[min(i, n - 1)], X + lane * kLd);  // (rows past n are not written out)
         __syncwarp();
-        hidden_layers(W, X, nullptr);
+        Fragments<2> A;
+        load_fragments<2>(X, A);
+        __syncwarp();  // X is free for the next chunk's encoding
+#pragma unroll 1
+        for (int l = 0; l < kLayers - 1; ++l) fragment_layer<2>(A, W + l * wsm_offset(1), wld(0));
         float acc[2][kOut / 8][4];
-        warp_layer<kOut, kHidden>(X, W + wsm_offset(kLayers - 1), wld(kLayers - 1), acc);
+#pragma unroll
+        for (int nt = 0; nt < kOut / 8; ++nt) {
+            float c[2][4];
+            fragment_tile<2>(A, W + wsm_offset(kLayers - 1), wld(kLayers - 1), nt, c);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) acc[mt][nt][k] = c[mt][k];
+        }
         write_outputs(acc, ch * 32, n, raw, packed, nMax);
-        __syncwarp();
     }
 }
 
@@ -409,12 +476,7 @@ __global__ void __launch_bounds__(kTcRows, 4) k_infer_tc(Params g, const Query* 
         const uint32_t i = tile * kTcRows + tid;
         {
             __align__(16) __nv_bfloat16 row[kIn];
-            if (i < n) {
-                encode_row(g, q[i], row);
-            } else {
-#pragma unroll
-                for (int k = 0; k < kIn; ++k) row[k] = bf(0.0f);
-            }
+            encode_row(g, q[min(i, n - 1)], row);  // (rows past n are not written out)
 #pragma unroll
             for (int c = 0; c < kIn / 8; ++c)
                 *reinterpret_cast<uint4*>(at + tc_offset(tid, 8 * c)) = *reinterpret_cast<const uint4*>(row + 8 * c);
@@ -492,42 +554,172 @@ __global__ void __launch_bounds__(kTcRows, 4) k_infer_tc(Params g, const Query* 
 
 // Training, in two kernels per slice of at most kTrainSlice samples.
 //
-// k_train_rows: one warp per 32 samples runs the encoding and the forward
-// pass (keeping every layer's input in shared memory), the mixture's output
-// gradient, and the backward data pass through the layers (dX = dY W_l,
-// then ReLU'). It scatters the grid gradients with float2 atomics, and
-// writes, for the weight gradients, every layer's input X_l and output
-// gradient dY_l transposed: XT[l][k][s] and DT[l][m][s] (bf16, s = sample
-// of the slice, rows kTrainSlice long).
+// k_train_rows: one warp per 16 samples runs the encoding and the forward
+// pass, the mixture's output gradient, and the backward data pass through the
+// layers (dX = dY W_l, then ReLU'). It scatters the grid gradients with
+// float4 atomics, and writes, for the weight gradients, every layer's input
+// X_l and output gradient dY_l transposed: XT[l][k][s] and DT[l][m][s] (bf16,
+// s = sample of the slice, rows kTrainSlice long).
+//
+// A step is one slice, about 110 samples per SM, so the kernel is one chain of
+// dependent steps and its time is that chain's latency. Seven warps a block
+// and one block per SM cover a slice; two lanes share a sample where the work
+// is per sample; activations and gradients stay in registers as mma
+// fragments, ReLU' as a bit per element, and the backward weights are the
+// forward ones read transposed (ldmatrix.trans). Measured on B200, 16,384
+// samples: 106 us with one warp per 32 samples and the layers' inputs in
+// shared memory, 47 us so.
 //
 // k_dw: dW_l = dY_l^T X_l over the slice, one warp per (layer, 16-row tile
 // of dW_l, split of the samples), with the mma tiles reading XT and DT
 // directly; each split writes its own partial dW, summed in fixed order by
 // k_reduce_dw. Sample i of the slice is s[offset + i * stride].
 constexpr uint32_t kTrainSlice = 16384;
-constexpr int kTrainRowWarps = 2;
+constexpr int kTrainRowWarps = 7;
+constexpr uint32_t kTrainRows = 16;  // samples per warp
 constexpr uint32_t kDwSplits = 32;
 constexpr int kDwTasks = (kLayers - 1) * (kHidden / 16) + kOut / 16;  // (layer, 16-row tile) pairs: 19
+static_assert(kTrainSlice % kTrainRows == 0, "whole warps per slice");
 
-// Columns 0..cols-1 of a warp's [32][kLd] bf16 tile, transposed into dst
-// (dst[c * ld + r], rows of the tile are consecutive samples): two columns
-// per instruction, each lane storing a pair of samples.
-AG_D void store_transposed(const __nv_bfloat16* src, int cols, __nv_bfloat16* dst, uint32_t ld)
+// Per warp: rows of inputs, then of output gradients; outputs (fp32, odd
+// stride: a lane reads a whole row), then grid-feature gradients; a transposed
+// tile on its way out.
+constexpr int kLdOut = kOut + 1, kLdT = kTrainRows + 8;
+struct TrainWarp {
+    __nv_bfloat16 rows[kTrainRows * kLd];
+    __nv_bfloat16 tile[kHidden * kLdT];
+    float out[kTrainRows * kLdOut];
+};
+static_assert(sizeof(TrainWarp) % 16 == 0 && kWsm % 8 == 0, "16-byte rows");
+static_assert(kGridDims < kLdOut, "grid-feature gradients fit the output rows");
+
+size_t train_rows_smem() { return (size_t)kWsm * 2 + kTrainRowWarps * sizeof(TrainWarp); }
+
+// The encoding of 16 samples, two lanes each (encode_row's pairs, with one
+// query per pair): the even lane sums the lower levels, the odd lane the upper.
+AG_D void encode_row_pair(const Params& g, const Query& q, __nv_bfloat16* row)
 {
-    const int lane = threadIdx.x & 31, pr = lane & 15, half = lane >> 4;
-    for (int c0 = 0; c0 < cols; c0 += 2) {
-        const int c = c0 + half;
-        __nv_bfloat162 v;
-        v.x = src[(2 * pr) * kLd + c];
-        v.y = src[(2 * pr + 1) * kLd + c];
-        *reinterpret_cast<__nv_bfloat162*>(dst + (uint64_t)c * ld + 2 * pr) = v;
+    const float3 p = normalise_position(g, mk3(q.pos[0], q.pos[1], q.pos[2]));
+    constexpr int kWords = kFeatures / 2, kHalf = kLevels / 2;
+    const uint32_t odd = threadIdx.x & 1u;
+    using Corner = typename std::conditional<kFeatures == 4, uint2, uint32_t>::type;
+    uint4* out = reinterpret_cast<uint4*>(row);
+    Corner v[kLevels][4];  // corners 2 c + odd
+#pragma unroll
+    for (int l = 0; l < kLevels; ++l)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            uint32_t idx;
+            float w;
+            grid_corner(g.res[l], p, 2 * c + (int)odd, idx, w);
+            v[l][c] = *reinterpret_cast<const Corner*>(g.grid + ((uint64_t)l * kTableSize + idx) * kFeatures);
+        }
+    uint32_t word[kHalf * kFeatures / 2];
+#pragma unroll
+    for (int j = 0; j < kHalf; ++j) {
+        const uint32_t res = odd ? g.res[kHalf + j] : g.res[j];
+        float f[kFeatures] = {};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            uint32_t even[kWords], oddv[kWords];
+#pragma unroll
+            for (int k = 0; k < kWords; ++k) {
+                const uint32_t low = reinterpret_cast<const uint32_t*>(&v[j][c])[k];
+                const uint32_t high = reinterpret_cast<const uint32_t*>(&v[kHalf + j][c])[k];
+                const uint32_t keep = odd ? high : low;
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? low : high, 1);
+                even[k] = odd ? got : keep;
+                oddv[k] = odd ? keep : got;
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                uint32_t idx;
+                float w;
+                grid_corner(res, p, 2 * c + x, idx, w);
+                const __half2* h = reinterpret_cast<const __half2*>(x ? oddv : even);
+#pragma unroll
+                for (int k = 0; k < kWords; ++k) {  // one rounding per corner, in corner order
+                    f[2 * k] = __fmaf_rn(w, __low2float(h[k]), f[2 * k]);
+                    f[2 * k + 1] = __fmaf_rn(w, __high2float(h[k]), f[2 * k + 1]);
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kFeatures; k += 2) word[(kFeatures * j + k) / 2] = pack_bf2(f[k], f[k + 1]);
+    }
+    constexpr int kChunks = kHalf * kFeatures / 8;
+#pragma unroll
+    for (int k = 0; k < kChunks; ++k)
+        out[odd * kChunks + k] = make_uint4(word[4 * k], word[4 * k + 1], word[4 * k + 2], word[4 * k + 3]);
+    if (odd) {
+        float ex[8];
+        extra_inputs(mk3(q.wo[0], q.wo[1], q.wo[2]), mk3(q.n[0], q.n[1], q.n[2]), q.rough, ex);
+        out[kGridDims / 8] =
+            make_uint4(pack_bf2(ex[0], ex[1]), pack_bf2(ex[2], ex[3]), pack_bf2(ex[4], ex[5]), pack_bf2(ex[6], ex[7]));
+    } else {
+#pragma unroll
+        for (int k = kGridDims / 8 + 1; k < kIn / 8; ++k) out[k] = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
-size_t train_rows_smem()
+// A warp's 16 rows (A fragments) transposed to dst: column c of the rows at
+// dst[c * kTrainSlice], KS k steps of 16 columns. tile: the warp's scratch.
+template <int KS>
+AG_D void store_transposed(const Fragments<1>& A, __nv_bfloat16* tile, __nv_bfloat16* dst)
 {
-    // padded weights + per warp: G0 [32][kLd] followed by the inputs of the kLayers layers
-    return (size_t)kWsm * 2 + (size_t)kTrainRowWarps * (kLayers + 1) * 32 * kLd * 2;
+    const int lane = threadIdx.x & 31;
+    __syncwarp();  // the tile's previous reader is done
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks)
+        stmatrix4_trans(tile + (ks * 16 + ((lane >> 4) & 1) * 8 + (lane & 7)) * kLdT + ((lane >> 3) & 1) * 8, A[0][ks]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < KS; ++i) {
+        const int c = (lane + 32 * i) >> 1, h = lane & 1;
+        *reinterpret_cast<uint4*>(dst + (uint64_t)c * kTrainSlice + 8 * h) =
+            *reinterpret_cast<const uint4*>(tile + c * kLdT + 8 * h);
+    }
+}
+
+// acc = the n tile's 8 columns of dY * Wl (dY: A fragments over KS k steps of
+// Wl's rows, in ascending order).
+template <int KS>
+AG_D void fragment_tile_back(const Fragments<1>& A, const __nv_bfloat16* Wl, int ldw, int nt, float (&acc)[4])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] = 0.0f;
+#pragma unroll
+    for (int ks = 0; ks < KS; ks += 2) {
+        uint32_t B[4];
+        // rows ks * 16 .. + 31 of Wl; past the last k step the first 16 again (unused)
+        const int r = ks + 1 < KS ? lane : lane & 15;
+        ldmatrix4_trans(Wl + (ks * 16 + r) * ldw + nt * 8, B);
+        mma_bf16(acc, A[0][ks][0], A[0][ks][1], A[0][ks][2], A[0][ks][3], B[0], B[1]);
+        if (ks + 1 < KS)
+            mma_bf16(acc, A[0][ks + 1][0], A[0][ks + 1][1], A[0][ks + 1][2], A[0][ks + 1][3], B[2], B[3]);
+    }
+}
+
+// dY_{l-1} = (dY_l W_l) * [X_l > 0] in registers; mask: a bit per element of X_l.
+template <int KS>
+AG_D void fragment_layer_back(Fragments<1>& A, const __nv_bfloat16* Wl, int ldw, uint32_t mask)
+{
+    Fragments<1> out;
+#pragma unroll
+    for (int nt = 0; nt < kHidden / 8; ++nt) {
+        float acc[4];
+        fragment_tile_back<KS>(A, Wl, ldw, nt, acc);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (!((mask >> (4 * nt + k)) & 1u)) acc[k] = 0.0f;
+        out[0][nt / 2][2 * (nt & 1)] = pack_bf2(acc[0], acc[1]);
+        out[0][nt / 2][2 * (nt & 1) + 1] = pack_bf2(acc[2], acc[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < kHidden / 16; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) A[0][j][k] = out[0][j][k];
 }
 
 __global__ void __launch_bounds__(32 * kTrainRowWarps) k_train_rows(Params g, const Sample* __restrict__ s, uint32_t n,
@@ -539,51 +731,56 @@ __global__ void __launch_bounds__(32 * kTrainRowWarps) k_train_rows(Params g, co
     extern __shared__ __align__(16) unsigned char smem[];
     __nv_bfloat16* W = reinterpret_cast<__nv_bfloat16*>(smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g4 = lane >> 2, t4 = lane & 3;
-    __nv_bfloat16* G0 = W + kWsm + warp * (kLayers + 1) * 32 * kLd;  // [32][kLd] gradient dY of the current layer
-    __nv_bfloat16* saved = G0 + 32 * kLd;                              // [kLayers][32][kLd] layer inputs
-    // outputs in fp32 over G0 and saved[0] (X_0 is in XT by then)
-    float* outF = reinterpret_cast<float*>(G0);                        // [32][kOut]
-    static_assert(32 * kOut * 4 <= 2 * 32 * kLd * 2, "output tile fits G0 + saved[0]");
-    // grid-feature gradients over saved[1] (X_1 has served its ReLU' by then)
-    float* dIn = reinterpret_cast<float*>(saved + 32 * kLd);           // [32][kGridDims]
-    static_assert(32 * kGridDims * 4 <= 32 * kLd * 2, "grid-feature gradients fit saved[1]");
-    load_weights(g.W, W);
+    TrainWarp& t = reinterpret_cast<TrainWarp*>(W + kWsm)[warp];
+    const uint32_t row0 = (blockIdx.x * kTrainRowWarps + warp) * kTrainRows;
+    const bool busy = row0 < n;
+    const int local = lane >> 1;              // this lane pair's sample
+    const bool valid = row0 + local < n;
+    Sample smp;
+    if (busy) {  // the samples and their grid entries are on their way while the weights are copied
+        smp = s[offset + (uint64_t)min(row0 + local, n - 1) * stride];
+        encode_row_pair(g, smp.q, t.rows + local * kLd);
+        __syncwarp();
+        if (!valid)  // rows past n add nothing to the weight gradients
+            for (int k = lane & 1; k < kIn; k += 2) t.rows[local * kLd + k] = bf(0.0f);
+    }
+    load_weights(g.W, W, [](int r) { return r; });
     __syncthreads();
     float lossSum = 0.0f;
-    const uint32_t ch = blockIdx.x * kTrainRowWarps + warp;
-    if (ch * 32 < n) {
-        const uint32_t row0 = ch * 32, i = row0 + lane;
-        const bool valid = i < n;
-        Sample smp;
-        if (valid) {
-            smp = s[offset + (uint64_t)i * stride];
-            encode_row(g, smp.q, saved + lane * kLd);
-        } else {
-            for (int k = 0; k < kIn; ++k) saved[lane * kLd + k] = bf(0.0f);
-        }
-        __syncwarp();
-        hidden_layers(W, saved, saved);
-        for (int l = 0; l < kLayers; ++l)
-            store_transposed(saved + l * 32 * kLd, kIn, XT + (uint64_t)l * kHidden * kTrainSlice + row0, kTrainSlice);
-        {
-            float acc[2][kOut / 8][4];
-            warp_layer<kOut, kHidden>(saved + (kLayers - 1) * 32 * kLd, W + wsm_offset(kLayers - 1),
-                                      wld(kLayers - 1), acc);
-            __syncwarp();  // X_0 (under outF) has been stored by every lane
+    if (busy) {
+        Fragments<1> A;
+        load_fragments<1>(t.rows, A);
+        uint32_t mask[kLayers - 1];
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
+        for (int l = 0; l < kLayers - 1; ++l) {
+            store_transposed<kIn / 16>(A, t.tile, XT + (uint64_t)l * kHidden * kTrainSlice + row0);
+            fragment_layer<1>(A, W + wsm_offset(l), wld(l));
+            mask[l] = 0u;  // [X_{l+1} > 0]: activations are not negative
 #pragma unroll
-                for (int nt = 0; nt < kOut / 8; ++nt) {
-                    const int r = mt * 16 + g4, col = nt * 8 + 2 * t4;
-                    *reinterpret_cast<float2*>(outF + r * kOut + col) = make_float2(acc[mt][nt][0], acc[mt][nt][1]);
-                    *reinterpret_cast<float2*>(outF + (r + 8) * kOut + col) = make_float2(acc[mt][nt][2], acc[mt][nt][3]);
+            for (int j = 0; j < kHidden / 16; ++j)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t bit = 4 * (2 * j + k / 2) + 2 * (k & 1);
+                    mask[l] |= ((A[0][j][k] & 0xffffu) ? 1u : 0u) << bit;
+                    mask[l] |= ((A[0][j][k] >> 16) ? 1u : 0u) << (bit + 1);
                 }
         }
+        store_transposed<kHidden / 16>(A, t.tile, XT + (uint64_t)(kLayers - 1) * kHidden * kTrainSlice + row0);
+#pragma unroll
+        for (int nt = 0; nt < kOut / 8; ++nt) {
+            float c[1][4];
+            fragment_tile<1>(A, W + wsm_offset(kLayers - 1), wld(kLayers - 1), nt, c);
+            const int col = nt * 8 + 2 * t4;
+            t.out[g4 * kLdOut + col] = c[0][0];
+            t.out[g4 * kLdOut + col + 1] = c[0][1];
+            t.out[(g4 + 8) * kLdOut + col] = c[0][2];
+            t.out[(g4 + 8) * kLdOut + col + 1] = c[0][3];
+        }
         __syncwarp();
-        // output gradient (lane = sample)
-        {
+        // output gradient (even lanes, one sample each)
+        if ((lane & 1) == 0) {
             float raw[40], grad[40];
-            for (int k = 0; k < 40; ++k) raw[k] = outF[lane * kOut + k];
+            for (int k = 0; k < 40; ++k) raw[k] = t.out[local * kLdOut + k];
             if (valid) {
                 const float3 dir = mk3(smp.dir[0], smp.dir[1], smp.dir[2]);
                 const float w = smp.weight * invBatch;
@@ -594,52 +791,57 @@ __global__ void __launch_bounds__(32 * kTrainRowWarps) k_train_rows(Params g, co
             } else {
                 for (int k = 0; k < 40; ++k) grad[k] = 0.0f;
             }
-            __syncwarp();  // every lane has read its outputs
-            for (int k = 0; k < kOut; ++k) G0[lane * kLd + k] = bf(k < 40 ? grad[k] : 0.0f);
+            uint4* o = reinterpret_cast<uint4*>(t.rows + local * kLd);
+#pragma unroll
+            for (int k = 0; k < 40; k += 8)
+                o[k / 8] = make_uint4(pack_bf2(grad[k], grad[k + 1]), pack_bf2(grad[k + 2], grad[k + 3]),
+                                      pack_bf2(grad[k + 4], grad[k + 5]), pack_bf2(grad[k + 6], grad[k + 7]));
+            o[5] = make_uint4(0u, 0u, 0u, 0u);  // outputs 40..47 are unused
         }
         __syncwarp();
-        store_transposed(G0, kOut, DT + (uint64_t)(kLayers - 1) * kHidden * kTrainSlice + row0, kTrainSlice);
-        // backward: G0 holds dY_l; dX_l = dY_l W_l, dY_{l-1} = dX_l * [X_l > 0]
-        for (int l = kLayers - 1; l >= 1; --l) {
-            const __nv_bfloat16* Xl = saved + l * 32 * kLd;
-            const __nv_bfloat16* WTl = g.WT + layer_offset(l);
-            float acc[2][kHidden / 8][4];
-            if (l == kLayers - 1) warp_layer<kHidden, kOut>(G0, WTl, kOut, acc);
-            else warp_layer<kHidden, kHidden>(G0, WTl, kHidden, acc);
-            __syncwarp();
+        // backward: A holds dY_l; the first three k steps are the output layer's 48 columns
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
+        for (int ks = 0; ks < kOut / 16; ++ks) ldmatrix4(t.rows + (lane & 15) * kLd + ks * 16 + (lane >> 4) * 8, A[0][ks]);
+        store_transposed<kOut / 16>(A, t.tile, DT + (uint64_t)(kLayers - 1) * kHidden * kTrainSlice + row0);
+        fragment_layer_back<kOut / 16>(A, W + wsm_offset(kLayers - 1), wld(kLayers - 1), mask[kLayers - 2]);
+        store_transposed<kHidden / 16>(A, t.tile, DT + (uint64_t)(kLayers - 2) * kHidden * kTrainSlice + row0);
 #pragma unroll
-                for (int nt = 0; nt < kHidden / 8; ++nt) {
-                    const int r = mt * 16 + g4, c = nt * 8 + 2 * t4;
-                    const __nv_bfloat162 x0 = *reinterpret_cast<const __nv_bfloat162*>(Xl + r * kLd + c);
-                    const __nv_bfloat162 x1 = *reinterpret_cast<const __nv_bfloat162*>(Xl + (r + 8) * kLd + c);
-                    *reinterpret_cast<uint32_t*>(G0 + r * kLd + c) =
-                        pack_bf2(fl(x0.x) > 0.0f ? acc[mt][nt][0] : 0.0f, fl(x0.y) > 0.0f ? acc[mt][nt][1] : 0.0f);
-                    *reinterpret_cast<uint32_t*>(G0 + (r + 8) * kLd + c) =
-                        pack_bf2(fl(x1.x) > 0.0f ? acc[mt][nt][2] : 0.0f, fl(x1.y) > 0.0f ? acc[mt][nt][3] : 0.0f);
-                }
-            __syncwarp();
-            store_transposed(G0, kHidden, DT + (uint64_t)(l - 1) * kHidden * kTrainSlice + row0, kTrainSlice);
+        for (int l = kLayers - 2; l >= 1; --l) {
+            fragment_layer_back<kHidden / 16>(A, W + wsm_offset(l), wld(l), mask[l - 1]);
+            store_transposed<kHidden / 16>(A, t.tile, DT + (uint64_t)(l - 1) * kHidden * kTrainSlice + row0);
         }
         // grid-feature gradients: dX0[s][k] = sum_m dY_0[s][m] W_0[m][k], k < kGridDims
-        warp_gemm<32, kGridDims, kHidden>(G0, kLd, g.WT + layer_offset(0), layer_out(0),
-                                          [&](int r, int c, float v) { dIn[r * kGridDims + c] = v; });
+#pragma unroll
+        for (int nt = 0; nt < kGridDims / 8; ++nt) {
+            float c[4];
+            fragment_tile_back<kHidden / 16>(A, W + wsm_offset(0), wld(0), nt, c);
+            const int col = nt * 8 + 2 * t4;
+            t.out[g4 * kLdOut + col] = c[0];
+            t.out[g4 * kLdOut + col + 1] = c[1];
+            t.out[(g4 + 8) * kLdOut + col] = c[2];
+            t.out[(g4 + 8) * kLdOut + col + 1] = c[3];
+        }
         __syncwarp();
-        if (valid) {
+        if (valid) {  // each lane of the pair half of the levels
             const float3 p = normalise_position(g, mk3(smp.q.pos[0], smp.q.pos[1], smp.q.pos[2]));
-            for (int lv = 0; lv < kLevels; ++lv) {
+            const int first = (lane & 1) * (kLevels / 2);
+#pragma unroll
+            for (int j = 0; j < kLevels / 2; ++j) {
+                const int lv = first + j;
+                const uint32_t res = (lane & 1) ? g.res[kLevels / 2 + j] : g.res[j];
                 float d[kFeatures];
 #pragma unroll
-                for (int k = 0; k < kFeatures; ++k) d[k] = dIn[lane * kGridDims + kFeatures * lv + k];
+                for (int k = 0; k < kFeatures; ++k) d[k] = t.out[local * kLdOut + kFeatures * lv + k];
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     uint32_t idx;
                     float w;
-                    grid_corner(g.res[lv], p, c, idx, w);
-                    float2* dst = reinterpret_cast<float2*>(dGrid + ((uint64_t)lv * kTableSize + idx) * kFeatures);
-#pragma unroll
-                    for (int k = 0; k < kFeatures / 2; ++k) atomicAdd(dst + k, make_float2(w * d[2 * k], w * d[2 * k + 1]));
+                    grid_corner(res, p, c, idx, w);
+                    float* dst = dGrid + ((uint64_t)lv * kTableSize + idx) * kFeatures;
+                    if constexpr (kFeatures == 4)
+                        atomicAdd(reinterpret_cast<float4*>(dst), make_float4(w * d[0], w * d[1], w * d[2], w * d[3]));
+                    else
+                        atomicAdd(reinterpret_cast<float2*>(dst), make_float2(w * d[0], w * d[1]));
                 }
             }
         }
@@ -851,7 +1053,7 @@ __global__ void k_reduce_dw(const float* __restrict__ partial, uint32_t blocks, 
 
 // Adam (Kingma & Ba 2015) on fp32 master parameters; writes the compute copies.
 __global__ void k_adam_weights(float* p, float* m, float* v, float* grad, uint32_t n, float lr, float b1, float b2,
-                               float eps, float c1, float c2, __nv_bfloat16* W, __nv_bfloat16* WT)
+                               float eps, float c1, float c2, __nv_bfloat16* W)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -863,13 +1065,7 @@ __global__ void k_adam_weights(float* p, float* m, float* v, float* grad, uint32
     float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     p[i] = pi;
     grad[i] = 0.0f;
-    // locate (layer, out, in) for the transposed copy
-    int l = 0;
-    while (l < kLayers - 1 && (int)i >= layer_offset(l + 1)) ++l;
-    int local = (int)i - layer_offset(l);
-    int o = local / layer_in(l), in = local % layer_in(l);
     W[i] = __float2bfloat16_rn(pi);
-    WT[layer_offset(l) + in * layer_out(l) + o] = __float2bfloat16_rn(pi);
 }
 
 // Adam on the grid, lazily: an entry is updated only in the steps in which
@@ -902,18 +1098,10 @@ __global__ void k_adam_grid(float* p, float* m, float* v, float* grad, uint64_t 
     reinterpret_cast<float4*>(grad)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
-__global__ void k_publish(const float* pw, uint32_t nw, __nv_bfloat16* W, __nv_bfloat16* WT, const float* pg,
-                          uint64_t ng, __half* h)
+__global__ void k_publish(const float* pw, uint32_t nw, __nv_bfloat16* W, const float* pg, uint64_t ng, __half* h)
 {
     uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < nw) {
-        int l = 0;
-        while (l < kLayers - 1 && (int)i >= layer_offset(l + 1)) ++l;
-        int local = (int)i - layer_offset(l);
-        int o = local / layer_in(l), in = local % layer_in(l);
-        W[i] = __float2bfloat16_rn(pw[i]);
-        WT[layer_offset(l) + in * layer_out(l) + o] = __float2bfloat16_rn(pw[i]);
-    }
+    if (i < nw) W[i] = __float2bfloat16_rn(pw[i]);
     if (i < ng) h[i] = __float2half_rn(pg[i]);
 }
 
@@ -955,7 +1143,7 @@ bool Guide::allocate()
     bytes += 4 * kGridParams * sizeof(float);             // grid master, m, v, grad
     bytes += kGridParams * sizeof(__half);                // grid compute copy
     bytes += 4 * (size_t)kWeightCount * sizeof(float);    // W master, m, v, grad
-    bytes += 2 * (size_t)kWeightCount * sizeof(__nv_bfloat16);
+    bytes += (size_t)kWeightCount * sizeof(__nv_bfloat16);
     bytes += (size_t)kDwSplits * kWeightCount * sizeof(float);        // per-split dW partials
     bytes += 2 * (size_t)kLayers * kHidden * kTrainSlice * sizeof(__nv_bfloat16);  // XT, DT
     bytes += 256 * 8;
@@ -980,7 +1168,6 @@ bool Guide::allocate()
     wV_ = (float*)take(kWeightCount * 4);
     wG_ = (float*)take(kWeightCount * 4);
     wB_ = (__nv_bfloat16*)take(kWeightCount * 2);
-    wT_ = (__nv_bfloat16*)take(kWeightCount * 2);
     partial_ = (float*)take((size_t)kDwSplits * kWeightCount * 4);
     xt_ = (__nv_bfloat16*)take((size_t)kLayers * kHidden * kTrainSlice * 2);
     dt_ = (__nv_bfloat16*)take((size_t)kLayers * kHidden * kTrainSlice * 2);
@@ -1020,7 +1207,7 @@ int Guide::reset(uint32_t seed, cudaStream_t st)
 void Guide::publish(cudaStream_t st)
 {
     uint64_t n = kGridParams > (uint64_t)kWeightCount ? kGridParams : (uint64_t)kWeightCount;
-    k_publish<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(wP_, kWeightCount, wB_, wT_, gridP_, kGridParams, gridH_);
+    k_publish<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(wP_, kWeightCount, wB_, gridP_, kGridParams, gridH_);
 }
 
 void Guide::set_scene_box(float3 lo, float3 hi)
@@ -1037,7 +1224,6 @@ Params Guide::params() const
     Params p;
     p.grid = gridH_;
     p.W = wB_;
-    p.WT = wT_;
     p.bmin = bmin_;
     p.invExtent = invExtent_;
     double b = std::exp((std::log((double)kMaxRes) - std::log((double)kMinRes)) / (kLevels - 1));
@@ -1079,7 +1265,7 @@ void Guide::accumulate_gradients(const Sample* s, uint32_t n, float invBatch, cu
     cudaFuncSetAttribute(k_train_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_rows_smem());
     for (uint32_t start = 0; start < n; start += kTrainSlice) {
         const uint32_t m = std::min(kTrainSlice, n - start);
-        const uint32_t chunks = (m + 31) / 32;
+        const uint32_t chunks = (m + kTrainRows - 1) / kTrainRows;
         k_train_rows<<<(chunks + kTrainRowWarps - 1) / kTrainRowWarps, 32 * kTrainRowWarps, train_rows_smem(), st>>>(
             params(), s, m, offset + start * stride, stride, invBatch, xt_, dt_, gridG_, loss_);
         if (gradKernel_ == kKernelTensorMemory) {
@@ -1101,7 +1287,7 @@ void Guide::apply_adam(float lr, cudaStream_t st)
     const float b1 = 0.9f, b2 = 0.99f, eps = 1e-8f;
     float c1 = 1.0f - (float)std::pow(b1, step_), c2 = 1.0f - (float)std::pow(b2, step_);
     k_adam_weights<<<(kWeightCount + 255) / 256, 256, 0, st>>>(wP_, wM_, wV_, wG_, kWeightCount, lr, b1, b2, eps, c1,
-                                                               c2, wB_, wT_);
+                                                               c2, wB_);
     static_assert(kGridParams % 4 == 0, "grid Adam reads gradients four at a time");
     k_adam_grid<<<(unsigned)((kGridParams / 4 + 255) / 256), 256, 0, st>>>(gridP_, gridM_, gridV_, gridG_, kGridParams / 4, lr,
                                                                         b1, b2, eps, c1, c2, gridH_);

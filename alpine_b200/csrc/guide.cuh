@@ -57,7 +57,6 @@ constexpr uint64_t kGridParams = (uint64_t)kLevels * kTableSize * kFeatures;
 struct Params {
     const __half* grid;            // [level][entry][feature] (inference copy)
     const __nv_bfloat16* W;        // packed [out][in] per layer
-    const __nv_bfloat16* WT;       // packed transposes [in][out] per layer
     float3 bmin;                   // scene box used to normalise positions
     float3 invExtent;
     uint32_t res[kLevels];         // grid resolution per level
@@ -291,34 +290,6 @@ AG_D void mma_bf16(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a
 }
 
 AG_D uint32_t ld32(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
-
-// D[M x N] (+)= A[M x K] * B, with A row-major in shared memory (lda
-// elements per row) and B given as Bt[N x K] row-major (ldb), i.e.
-// D[m][n] = sum_k A[m][k] * Bt[n][k]. M multiple of 16, N of 8, K of 16.
-// The warp calls `emit(m, n, value)` for every output element.
-template <int M, int N, int K, typename Emit>
-AG_D void warp_gemm(const __nv_bfloat16* A, int lda, const __nv_bfloat16* Bt, int ldb, Emit emit)
-{
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int mt = 0; mt < M / 16; ++mt) {
-#pragma unroll
-        for (int nt = 0; nt < N / 8; ++nt) {
-            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int ks = 0; ks < K / 16; ++ks) {
-                const __nv_bfloat16* a = A + (mt * 16 + g) * lda + ks * 16 + 2 * t;
-                const __nv_bfloat16* b = Bt + (nt * 8 + g) * ldb + ks * 16 + 2 * t;
-                mma_bf16(c, ld32(a), ld32(a + 8 * lda), ld32(a + 8), ld32(a + 8 * lda + 8), ld32(b), ld32(b + 8));
-            }
-            const int r = mt * 16 + g, col = nt * 8 + 2 * t;
-            emit(r, col, c[0]);
-            emit(r, col + 1, c[1]);
-            emit(r + 8, col, c[2]);
-            emit(r + 8, col + 1, c[3]);
-        }
-    }
-}
 
 }  // namespace guide
 }  // namespace ag

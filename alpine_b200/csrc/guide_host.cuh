@@ -77,7 +77,6 @@ private:
     float* wV_ = nullptr;
     float* wG_ = nullptr;
     __nv_bfloat16* wB_ = nullptr;
-    __nv_bfloat16* wT_ = nullptr;
     float* partial_ = nullptr;   // per-split weight gradients
     __nv_bfloat16* xt_ = nullptr;  // layer inputs of a training slice, transposed
     __nv_bfloat16* dt_ = nullptr;  // layer output gradients of a training slice, transposed
