@@ -81,6 +81,7 @@ struct WaveView {
     alpine_gpu_ray* shadowRays;
     uint8_t* shadowOcc;
     uint32_t* shadowCount;
+    uint32_t* tickets;         // work tickets of the bounce's closest-hit and any-hit traversals
     // persistent per-pixel reference RNG state (stream mode)
     uint4* pixelRng;
     // learned guiding (counter RNG only)
@@ -438,17 +439,26 @@ __global__ void __launch_bounds__(kThreads) k_guide_query(SceneView sc, WaveView
 
 // kSampler: the light sampler kind, or -1 to read it from the scene.
 // Resident blocks per SM: the shading kernel waits on instruction fetch and
-// memory, so more warps beat fewer spills (measured on B200: 14 blocks of
-// 128, 32 registers with spills to L1, +28-41 % samples/s over 6 blocks for
-// unguided shading; the guided kernel, with more live state, is best at 10).
+// memory, so warps count; since the queue is grouped by material its warps
+// diverge less, and fewer spills (48 registers at 10 blocks of 128, 32 at 14)
+// count more. Measured on B200, 10 against 14 blocks: room with a quad light,
+// 1M paths, 2,648 to 2,472 us a render, 48 lights 1,293 to 1,198 us. A guided
+// vertex without next-event estimation has the most live state: 8 against 10
+// blocks, guided interior 10,206 to 9,795 us. (9 blocks, and 8 for guided
+// shading with lights, are 2 to 4 % faster still, but there the compiler
+// contracts other multiply-adds, and a rounding can turn a path.)
 #ifndef AG_SHADE_MIN_BLOCKS
-#define AG_SHADE_MIN_BLOCKS 14
+#define AG_SHADE_MIN_BLOCKS 10
 #endif
 #ifndef AG_SHADE_MIN_BLOCKS_GUIDED
-#define AG_SHADE_MIN_BLOCKS_GUIDED 10
+#define AG_SHADE_MIN_BLOCKS_GUIDED 8
 #endif
+constexpr int shade_min_blocks(bool guided, int sampler)
+{
+    return guided && sampler == (int)kSamplerNone ? AG_SHADE_MIN_BLOCKS_GUIDED : AG_SHADE_MIN_BLOCKS;
+}
 template <bool kGuided, int kSampler>
-__global__ void __launch_bounds__(kThreads, kGuided ? AG_SHADE_MIN_BLOCKS_GUIDED : AG_SHADE_MIN_BLOCKS)
+__global__ void __launch_bounds__(kThreads, shade_min_blocks(kGuided, kSampler))
     k_shade(SceneView sc, WaveView w, bool streamRng)
 {
     const uint32_t n = *w.queueCount;

@@ -343,6 +343,7 @@ ag::WaveView carve_wave(alpine_gpu_ctx* c)
     w.queueCount = counters;
     w.queueCountNext = counters + 1;
     w.shadowCount = counters + 2;
+    w.tickets = counters + 3;
     w.shadeBins = counters + 16;  // 16 words: bin counts, bin cursors
     return w;
 }
@@ -426,6 +427,21 @@ __global__ void k_post(const float* a32, const double* a64, uint32_t pixels, uin
 }
 
 __global__ void k_set_word(uint32_t* p, uint32_t v) { *p = v; }
+
+// The counters of one bounce, zeroed by one launch: the next queue's and the
+// shadow queue's lengths, the traversals' tickets, the shading-order bins and
+// the number of guided vertices (guideCount may be null).
+__global__ void k_bounce_begin(uint32_t* next, uint32_t* shadow, uint32_t* tickets, uint32_t* bins, uint32_t* guideCount)
+{
+    const uint32_t i = threadIdx.x;
+    if (i < 2 * ag::kShadeBins) bins[i] = 0u;
+    if (i < 2) tickets[i] = 0u;
+    if (i == 0) {
+        *next = 0u;
+        *shadow = 0u;
+        if (guideCount) *guideCount = 0u;
+    }
+}
 
 // Turns the wave's recorded vertices into training samples and takes up to
 // `maxSteps` Adam steps; step i uses samples i, i + stride, i + 2 stride, ...
@@ -882,6 +898,8 @@ static int render_enqueue(alpine_gpu_ctx* c, uint32_t spp)
             return c->fail(ALPINE_GPU_ERR_CUDA, "render: stream capture could not begin");
     }
     const uint32_t sampleOrigin = useGraph ? 0u : c->totalSamples;
+    // without lights no vertex casts a shadow ray
+    const bool shadows = sc.lights.kind != ag::kSamplerNone && sc.lights.count > 0;
     const bool shadeSort = o.shade_order == ALPINE_GPU_SHADE_ORDER_BY_MATERIAL;
     for (uint32_t done = 0; done < spp;) {
         const bool trainNow = trainEnabled && (o.guide_train_steps == 0 || c->guide.steps() < o.guide_train_steps);
@@ -922,10 +940,9 @@ static int render_enqueue(alpine_gpu_ctx* c, uint32_t spp)
             K.generate(sc, w, stream, st);
             for (uint32_t depth = 0; depth < sc.maxDepth; ++depth) {
                 w.depth = depth;
-                ag::launch_trace_dyn(bvh, w.rays, w.queueCount, w.numPaths, false, w.hits, c->dStatus, st,
+                k_bounce_begin<<<1, 32, 0, st>>>(w.queueCountNext, w.shadowCount, w.tickets, w.shadeBins, w.guideCount);
+                ag::launch_trace_dyn(bvh, w.rays, w.queueCount, w.numPaths, w.tickets, false, w.hits, c->dStatus, st,
                                      c->traceBlock);
-                cudaMemsetAsync(w.queueCountNext, 0, sizeof(uint32_t), st);
-                cudaMemsetAsync(w.shadowCount, 0, sizeof(uint32_t), st);
                 const bool guideHere = guiding && (o.guide_max_depth == 0 || depth < o.guide_max_depth);
                 ag::WaveView sw = w;
                 if (!guideHere) {  // unguided shading (pending training records still resolve)
@@ -933,20 +950,19 @@ static int render_enqueue(alpine_gpu_ctx* c, uint32_t spp)
                     sw.guideLobes = nullptr;
                 }
                 if (guideHere) {
-                    cudaMemsetAsync(w.guideCount, 0, sizeof(uint32_t), st);
                     K.guide_query(sc, w, w.numPaths, st);
                     if (sampleGuide)
                         c->guide.infer_queue(gw.query, w.guideCount, w.numPaths, gw.lobes, st, c->dStatus, true);
                 }
                 if (shadeSort) {  // group the queue by shade_key before shading
-                    cudaMemsetAsync(w.shadeBins, 0, 2 * ag::kShadeBins * sizeof(uint32_t), st);
                     K.sort(sc, sw, w.numPaths, w.shadeBins, w.shadeKeys, w.shadeOrderBuf, st);
                     sw.shadeOrder = w.shadeOrderBuf;
                 }
                 K.shade(sc, sw, stream, w.numPaths, st);
-                ag::launch_trace_dyn(bvh, w.shadowRays, w.shadowCount, 2 * w.numPaths, true, w.shadowOcc,
-                                     c->dStatus, st, c->traceBlock);
-                K.resolve(w, w.numPaths, st);
+                if (shadows)
+                    ag::launch_trace_dyn(bvh, w.shadowRays, w.shadowCount, 2 * w.numPaths, w.tickets + 1, true,
+                                         w.shadowOcc, c->dStatus, st, c->traceBlock);
+                if (shadows || w.trainSlot) K.resolve(w, w.numPaths, st);
                 std::swap(w.rays, w.raysNext);
                 std::swap(w.queuePath, w.queuePathNext);
                 std::swap(w.queueCount, w.queueCountNext);
