@@ -127,3 +127,42 @@ def test_animation_errors():
     with pytest.raises(RuntimeError):
         ctx.add_animation_channel(sid, [1.0, 0.0], [[0.0], [1.0]])  # decreasing times
     ctx.close()
+
+
+def test_many_meshes_morph_in_one_launch():
+    """Meshes of sizes around a block of the launch, with and without normals,
+    one to three targets, one without a channel, and one with two channels
+    (the last one's weights hold): bit-identical to separately rounded FP32."""
+    rng = np.random.default_rng(5)
+    ctx = gpu.Context(0)
+    try:
+        expect = []
+        for k, n in enumerate([3, 85, 86, 171, 700, 4]):
+            v = rng.normal(size=(n, 3)).astype(np.float32)
+            idx = np.arange(3, dtype=np.uint32).reshape(1, 3)
+            nrm = rng.normal(size=(n, 3)).astype(np.float32) if k % 2 else None
+            sid = ctx.add_mesh(v, idx)
+            ctx.set_triangle_attributes(sid, nrm, np.zeros(1, np.uint32))
+            t = 1 + k % 3
+            d = rng.normal(size=(t, n, 3)).astype(np.float32)
+            dn = rng.normal(size=(t, n, 3)).astype(np.float32) if k % 2 else None
+            ctx.set_morph_targets(sid, d, dn)
+            w = rng.normal(size=(2, t)).astype(np.float32)
+            for weights in ([] if k == 4 else [w + 1, w] if k == 2 else [w]):
+                ctx.add_animation_channel(sid, [0.0, 1.0], weights)
+            ev, en = v.copy(), nrm
+            if k != 4:
+                for j in range(t):
+                    ev = ev + d[j] * w[1, j]
+                    if dn is not None:
+                        en = en + dn[j] * w[1, j]
+            expect.append((sid, n, ev, en))
+        for _ in range(2):
+            ctx.update_scene(1.0)
+            for sid, n, ev, en in expect:
+                gv, gn = ctx.get_vertices(sid, n)
+                assert gv.tobytes() == ev.tobytes()
+                if en is not None:
+                    assert gn.tobytes() == en.tobytes()
+    finally:
+        ctx.close()
