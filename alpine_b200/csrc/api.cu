@@ -18,21 +18,6 @@ std::string cuda_msg(const char* what, cudaError_t e)
     return std::string(what) + ": " + cudaGetErrorString(e);
 }
 
-// Reads and clears the device status word (stream must be idle).
-int check_status(alpine_gpu_ctx* c)
-{
-    cudaError_t e = cudaMemcpyAsync(c->hStatus, c->dStatus, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) return c->fail(ALPINE_GPU_ERR_CUDA, cuda_msg("status readback", e));
-    if (*c->hStatus) {
-        uint32_t bits = *c->hStatus;
-        cudaMemsetAsync(c->dStatus, 0, sizeof(uint32_t), c->stream);
-        cudaStreamSynchronize(c->stream);
-        return c->fail(ALPINE_GPU_ERR_LIMIT, ag::status_msg(bits));
-    }
-    return ALPINE_GPU_OK;
-}
-
 int upload_geometry_now(alpine_gpu_ctx* c)
 {
     if (!c->geometryDirty) return ALPINE_GPU_OK;
@@ -93,6 +78,24 @@ int host_query(alpine_gpu_ctx* c, const alpine_gpu_ray* rays, uint64_t n, void* 
     if (int rc = require_bvh(c)) return rc;
     if (n == 0) return ALPINE_GPU_OK;
     const size_t outSize = kAny ? 1 : sizeof(alpine_gpu_hit);
+    if (n <= ag::kDirectRays) {
+        // A small batch is all latency: the rays are copied by the host into
+        // page-locked memory that the kernel reads over the link, the results
+        // come back the same way, and one wait covers them and the status word.
+        // 256 rays: 56 us with copies and two waits, 32 us so (B200); above
+        // about 4,096 rays the copy engines win.
+        char* hits = c->hDirect + ag::kDirectRays * sizeof(alpine_gpu_ray);
+        std::memcpy(c->hDirect, rays, n * sizeof(alpine_gpu_ray));
+        if (kAny) ag::launch_occluded(view(c), c->hDirect, n, reinterpret_cast<uint8_t*>(hits), c->dStatus, c->stream);
+        else ag::launch_trace(view(c), c->hDirect, n, hits, c->dStatus, c->stream);
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(c->hStatus, c->dStatus, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e != cudaSuccess) return c->fail(ALPINE_GPU_ERR_CUDA, cuda_msg(kAny ? "occluded" : "trace", e));
+        std::memcpy(out, hits, n * outSize);
+        return c->report_status();
+    }
     if (!c->dRays.reserve(n * sizeof(alpine_gpu_ray)) || !c->dOut.reserve(n * outSize))
         return c->fail(ALPINE_GPU_ERR_OUT_OF_MEMORY, "ray staging: cudaMalloc failed");
     ag::BvhView v = view(c);
@@ -144,11 +147,10 @@ int host_query(alpine_gpu_ctx* c, const alpine_gpu_ray* rays, uint64_t n, void* 
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(out, c->dOut.ptr, n * outSize, cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return c->fail(ALPINE_GPU_ERR_CUDA, cuda_msg(kAny ? "occluded" : "trace", e));
-    return check_status(c);
+    return c->check_device_status();
 }
 
 template <bool kAny>
@@ -195,6 +197,8 @@ int alpine_gpu_create(const alpine_gpu_config* cfg, alpine_gpu_ctx** out)
     // 16 device words: [0] status bits, [4] the sample base of a replayed render
     if (e == cudaSuccess) e = cudaMalloc(&c->dStatus, 16 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMallocHost(&c->hStatus, 16 * sizeof(uint32_t));
+    if (e == cudaSuccess)
+        e = cudaMallocHost(&c->hDirect, ag::kDirectRays * (sizeof(alpine_gpu_ray) + sizeof(alpine_gpu_hit)));
     if (e == cudaSuccess) e = cudaMemset(c->dStatus, 0, 16 * sizeof(uint32_t));
     if (e == cudaSuccess) c->dSampleBase = c->dStatus + 4;
     if (e != cudaSuccess) {
@@ -222,6 +226,7 @@ void alpine_gpu_destroy(alpine_gpu_ctx* c)
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->dStatus) cudaFree(c->dStatus);
     if (c->hStatus) cudaFreeHost(c->hStatus);
+    if (c->hDirect) cudaFreeHost(c->hDirect);
     delete c;
 }
 
@@ -355,7 +360,7 @@ int alpine_gpu_build(alpine_gpu_ctx* c, alpine_gpu_bvh_stats* stats)
     c->stats.big_levels = bs.bigLevels;
     c->syncBuildPrims = (uint32_t)prims;
     if (stats) *stats = c->stats;
-    return check_status(c);
+    return c->check_device_status();
 }
 
 int alpine_gpu_build_async(alpine_gpu_ctx* c, uint32_t max_binary_levels, uint32_t max_wide_levels)
@@ -394,7 +399,7 @@ int alpine_gpu_read_build_stats(alpine_gpu_ctx* c, alpine_gpu_bvh_stats* stats, 
     cudaSetDevice(c->device);
     if (graph_captures) *graph_captures = c->builder.graph_captures();
     if (graph_launches) *graph_launches = c->builder.graph_launches();
-    if (!stats) return check_status(c);
+    if (!stats) return c->check_device_status();
     ag::BuildStats bs;
     char err[256] = {0};
     if (int rc = c->builder.enqueued_stats(c->stream, &bs, err, sizeof err))
@@ -407,7 +412,7 @@ int alpine_gpu_read_build_stats(alpine_gpu_ctx* c, alpine_gpu_bvh_stats* stats, 
     stats->sah_cost = bs.sahCost;
     stats->build_ms = bs.buildMs;
     stats->child_slots = bs.childSlots;
-    return check_status(c);
+    return c->check_device_status();
 }
 
 int alpine_gpu_trace(alpine_gpu_ctx* c, const alpine_gpu_ray* rays, uint64_t n, alpine_gpu_hit* hits)
@@ -452,7 +457,7 @@ int alpine_gpu_traversal_stats(alpine_gpu_ctx* c, const alpine_gpu_ray* rays, ui
     if (e != cudaSuccess) return c->fail(ALPINE_GPU_ERR_CUDA, cuda_msg("traversal_stats", e));
     *nodeVisits = h[0];
     *triVisits = h[1];
-    return check_status(c);
+    return c->check_device_status();
 }
 
 int alpine_gpu_set_traversal_options(alpine_gpu_ctx* c, const alpine_gpu_traversal_options* o)
@@ -487,7 +492,7 @@ int alpine_gpu_synchronize(alpine_gpu_ctx* c)
     if (!c) return ALPINE_GPU_ERR_INVALID_ARGUMENT;
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return c->fail(ALPINE_GPU_ERR_CUDA, cuda_msg("synchronize", e));
-    return check_status(c);
+    return c->check_device_status();
 }
 
 }  // extern "C"

@@ -43,6 +43,9 @@ struct DeviceBuffer {
 
 constexpr int kCopyStreams = 8;  // host-query pipeline streams: copies in, 6 traversal streams, copies out
 constexpr int kPipeChunks = 32;  // host-query pipeline: at most this many chunks per call
+// Host queries of at most this many rays go through page-locked memory that
+// the kernel reads and writes itself: no copies are enqueued.
+constexpr uint64_t kDirectRays = 4096;
 
 // Human-readable description of DeviceError bits.
 inline std::string status_msg(uint32_t bits)
@@ -120,6 +123,7 @@ struct alpine_gpu_ctx {
 
     // staging for host-memory queries
     ag::DeviceBuffer dRays, dOut;
+    char* hDirect = nullptr;  // page-locked: kDirectRays rays, then as many hits
 
     // rendering: per-triangle material/normal flags and per-vertex normals
     std::vector<uint32_t> triInfo;  // material id | kTriHasNormals | kTriMorphedNormals
@@ -199,12 +203,18 @@ struct alpine_gpu_ctx {
     uint32_t guideWaveIndex = 0;     // waves rendered with guiding (record selection hash)
     uint32_t guideLastLossSteps = 0;  // Adam steps behind the loss sum in hStatus[2]
 
-    // Reads and clears the device status word (stream must be idle).
+    // Waits for the stream and reads and clears the device status word.
     int check_device_status()
     {
         cudaError_t e = cudaMemcpyAsync(hStatus, dStatus, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return fail(ALPINE_GPU_ERR_CUDA, std::string("status readback: ") + cudaGetErrorString(e));
+        return report_status();
+    }
+
+    // The status word that a copy has brought to hStatus (stream idle).
+    int report_status()
+    {
         if (*hStatus) {
             uint32_t bits = *hStatus;
             cudaMemsetAsync(dStatus, 0, sizeof(uint32_t), stream);

@@ -1146,6 +1146,7 @@ bool Guide::allocate()
     bytes += (size_t)kWeightCount * sizeof(__nv_bfloat16);
     bytes += (size_t)kDwSplits * kWeightCount * sizeof(float);        // per-split dW partials
     bytes += 2 * (size_t)kLayers * kHidden * kTrainSlice * sizeof(__nv_bfloat16);  // XT, DT
+    bytes += kWorkspace;
     bytes += 256 * 8;
     if (cudaMalloc(&mem_, bytes) != cudaSuccess) {
         cudaGetLastError();
@@ -1172,6 +1173,7 @@ bool Guide::allocate()
     xt_ = (__nv_bfloat16*)take((size_t)kLayers * kHidden * kTrainSlice * 2);
     dt_ = (__nv_bfloat16*)take((size_t)kLayers * kHidden * kTrainSlice * 2);
     loss_ = (float*)take(256);
+    work_ = take(kWorkspace);
     return true;
 }
 

@@ -145,29 +145,39 @@ int alpine_gpu_guide_gradients(alpine_gpu_ctx* c, const float* samples, uint32_t
 {
     if (!c || (n && !samples)) return ALPINE_GPU_ERR_INVALID_ARGUMENT;
     if (int rc = ensure_guide(c)) return rc;
-    DeviceBuffer ds, di, dg;
-    if (!ds.reserve((size_t)n * sizeof(G::Sample)) || !di.reserve((size_t)grid_count * 8 + 8) ||
-        !dg.reserve((size_t)grid_count * 4 + 4))
+    // samples, indices and gathered gradients in one workspace. The gradient
+    // buffers are clean between calls (reset, Adam and this call leave them so).
+    auto round256 = [](size_t b) { return (b + 255) & ~size_t(255); };
+    const size_t sb = round256((size_t)n * sizeof(G::Sample)), ib = round256((size_t)grid_count * 8);
+    const size_t bytes = sb + ib + (size_t)grid_count * 4;
+    DeviceBuffer large;
+    if (bytes > G::Guide::kWorkspace && !large.reserve(bytes))
         return c->fail(ALPINE_GPU_ERR_OUT_OF_MEMORY, "guide_gradients buffers");
+    char* work = static_cast<char*>(large.ptr ? large.ptr : c->guide.workspace());
+    G::Sample* ds = reinterpret_cast<G::Sample*>(work);
+    uint64_t* di = reinterpret_cast<uint64_t*>(work + sb);
+    float* dg = reinterpret_cast<float*>(work + sb + ib);
     cudaStream_t st = c->stream;
-    cudaError_t e = cudaMemcpyAsync(ds.ptr, samples, (size_t)n * sizeof(G::Sample), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->guide.weight_grad(), 0, G::kWeightCount * 4, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->guide.grid_grad(), 0, G::kGridParams * 4, st);
+    cudaError_t e = cudaMemcpyAsync(ds, samples, (size_t)n * sizeof(G::Sample), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
-        c->guide.accumulate_gradients(ds.as<G::Sample>(), n, n ? 1.0f / (float)n : 0.0f, st, 0, 1, c->dStatus);
+        c->guide.accumulate_gradients(ds, n, n ? 1.0f / (float)n : 0.0f, st, 0, 1, c->dStatus);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess && dW) e = cudaMemcpyAsync(dW, c->guide.weight_grad(), G::kWeightCount * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && grid_count && grid_index && grid_grad) {
-        e = cudaMemcpyAsync(di.ptr, grid_index, (size_t)grid_count * 8, cudaMemcpyHostToDevice, st);
-        k_gather<<<(grid_count + 255) / 256, 256, 0, st>>>(c->guide.grid_grad(), di.as<uint64_t>(), grid_count, dg.as<float>());
-        if (e == cudaSuccess) e = cudaMemcpyAsync(grid_grad, dg.ptr, (size_t)grid_count * 4, cudaMemcpyDeviceToHost, st);
+    // the index copy and the gather's launch while the gradients are computed
+    const bool gather = grid_count && grid_index && grid_grad;
+    if (e == cudaSuccess && gather) {
+        e = cudaMemcpyAsync(di, grid_index, (size_t)grid_count * 8, cudaMemcpyHostToDevice, st);
+        k_gather<<<(grid_count + 255) / 256, 256, 0, st>>>(c->guide.grid_grad(), di, grid_count, dg);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    // leave clean gradient buffers behind
+    if (e == cudaSuccess && dW) e = cudaMemcpyAsync(dW, c->guide.weight_grad(), G::kWeightCount * 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && gather) e = cudaMemcpyAsync(grid_grad, dg, (size_t)grid_count * 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaEventRecord(c->pipeStart, st);
+    // clean gradient buffers for the next call on the stream, not waited for
     cudaMemsetAsync(c->guide.weight_grad(), 0, G::kWeightCount * 4, st);
     cudaMemsetAsync(c->guide.grid_grad(), 0, G::kGridParams * 4, st);
-    cudaStreamSynchronize(st);
+    const cudaError_t e2 = e == cudaSuccess ? cudaEventSynchronize(c->pipeStart) : cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return c->fail(ALPINE_GPU_ERR_CUDA, std::string("guide_gradients: ") + cudaGetErrorString(e));
     (void)loss;
     return ALPINE_GPU_OK;
@@ -177,11 +187,14 @@ int alpine_gpu_guide_train(alpine_gpu_ctx* c, const float* samples, uint32_t n, 
 {
     if (!c || (n && !samples)) return ALPINE_GPU_ERR_INVALID_ARGUMENT;
     if (int rc = ensure_guide(c)) return rc;
-    DeviceBuffer ds;
-    if (!ds.reserve((size_t)n * sizeof(G::Sample))) return c->fail(ALPINE_GPU_ERR_OUT_OF_MEMORY, "guide_train buffer");
-    cudaError_t e = cudaMemcpyAsync(ds.ptr, samples, (size_t)n * sizeof(G::Sample), cudaMemcpyHostToDevice, c->stream);
+    const size_t bytes = (size_t)n * sizeof(G::Sample);
+    DeviceBuffer large;
+    if (bytes > G::Guide::kWorkspace && !large.reserve(bytes))
+        return c->fail(ALPINE_GPU_ERR_OUT_OF_MEMORY, "guide_train buffer");
+    G::Sample* ds = static_cast<G::Sample*>(large.ptr ? large.ptr : c->guide.workspace());
+    cudaError_t e = cudaMemcpyAsync(ds, samples, bytes, cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess) return c->fail(ALPINE_GPU_ERR_CUDA, "guide_train upload");
-    float l = c->guide.train_step(ds.as<G::Sample>(), n, lr, c->stream);
+    float l = c->guide.train_step(ds, n, lr, c->stream);
     e = cudaGetLastError();
     if (e != cudaSuccess) return c->fail(ALPINE_GPU_ERR_CUDA, std::string("guide_train: ") + cudaGetErrorString(e));
     if (loss) *loss = l;

@@ -52,6 +52,11 @@ public:
     // Recomputes the BF16 / FP16 compute copies from the FP32 masters.
     void publish(cudaStream_t st);
 
+    // Device workspace of host-buffer calls (samples, indices, gathered
+    // values), part of the guide's one allocation. Larger calls allocate.
+    static constexpr size_t kWorkspace = 8u << 20;
+    void* workspace() const { return work_; }
+
     float* weight_master() const { return wP_; }
     float* weight_grad() const { return wG_; }
     float* grid_master() const { return gridP_; }
@@ -81,6 +86,7 @@ private:
     __nv_bfloat16* xt_ = nullptr;  // layer inputs of a training slice, transposed
     __nv_bfloat16* dt_ = nullptr;  // layer output gradients of a training slice, transposed
     float* loss_ = nullptr;
+    void* work_ = nullptr;
     float3 bmin_ = make_float3(0.0f, 0.0f, 0.0f);
     float3 invExtent_ = make_float3(1.0f, 1.0f, 1.0f);
 };
