@@ -129,6 +129,8 @@ struct IntegratorKernels {
     // order: the queue entries grouped by bin
     void (*sort)(const SceneView&, const WaveView&, uint32_t maxQueue, uint32_t* bins, uint8_t* keys,
                  uint32_t* order, cudaStream_t);
+    // the light BVH's records for this integrator's descent
+    void (*light_records)(const LightPair* pairs, uint32_t count, LightRecord* out, cudaStream_t);
 };
 
 const IntegratorKernels& integrator_fast();
@@ -235,6 +237,13 @@ AG_D bool sample_material(const Material& m, float3 wo, float u0, float u1, Bsdf
     return mat_sample(m, wo, u0, u1, out);
 }
 #endif
+
+__global__ void __launch_bounds__(kThreads) k_light_records(const LightPair* __restrict__ pairs, uint32_t count,
+                                                            LightRecord* __restrict__ out)
+{
+    const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
+    if (i < count) out[i] = light_record(pairs[i]);
+}
 
 __global__ void __launch_bounds__(kThreads) k_generate(SceneView sc, WaveView w, bool streamRng)
 {
@@ -832,6 +841,11 @@ void sort(const SceneView& sc, const WaveView& w, uint32_t maxQueue, uint32_t* b
     if (!maxQueue) return;
     k_shade_bins<<<grid(maxQueue), kThreads, 0, st>>>(sc, w, bins, keys);
     k_shade_scatter<<<grid(maxQueue), kThreads, 0, st>>>(w, bins, keys, order);
+}
+
+void light_records(const LightPair* pairs, uint32_t count, LightRecord* out, cudaStream_t st)
+{
+    if (count) k_light_records<<<grid(count), kThreads, 0, st>>>(pairs, count, out);
 }
 
 }  // namespace AG_INTEGRATOR_NS

@@ -10,7 +10,7 @@ const IntegratorKernels& integrator_exact()
 {
     static const IntegratorKernels k = {exact::generate, exact::shade, exact::resolve, exact::accumulate,
                                               exact::guide_query, exact::train_finalize,
-                                              exact::sort};
+                                              exact::sort, exact::light_records};
     return k;
 }
 }  // namespace ag

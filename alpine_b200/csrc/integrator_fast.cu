@@ -7,7 +7,7 @@ const IntegratorKernels& integrator_fast()
 {
     static const IntegratorKernels k = {fast::generate, fast::shade, fast::resolve, fast::accumulate,
                                               fast::guide_query, fast::train_finalize,
-                                              fast::sort};
+                                              fast::sort, fast::light_records};
     return k;
 }
 }  // namespace ag

@@ -701,8 +701,15 @@ int alpine_gpu_build_light_sampler(alpine_gpu_ctx* c, int type)
             pairs[i].lo1 = make_float4(b.bmin.x, b.bmin.y, b.bmin.z, b.power);
             pairs[i].hi1 = make_float4(b.bmax.x, b.bmax.y, b.bmax.z, ref(n.right));
         }
-        if (!upload(c->dLightNodes, nodes, c->stream) || !upload(c->dLightPairs, pairs, c->stream))
+        const size_t rb = pairs.size() * sizeof(ag::LightRecord);
+        if (!upload(c->dLightNodes, nodes, c->stream) || !upload(c->dLightPairs, pairs, c->stream) ||
+            !c->dLightRecords[0].reserve(rb) || !c->dLightRecords[1].reserve(rb))
             return c->fail(ALPINE_GPU_ERR_CUDA, "light BVH upload failed");
+        const uint32_t count = (uint32_t)pairs.size();
+        ag::integrator_fast().light_records(c->dLightPairs.as<ag::LightPair>(), count,
+                                            c->dLightRecords[0].as<ag::LightRecord>(), c->stream);
+        ag::integrator_exact().light_records(c->dLightPairs.as<ag::LightPair>(), count,
+                                             c->dLightRecords[1].as<ag::LightRecord>(), c->stream);
         c->lightNodeCount = (uint32_t)nodes.size();
     }
     if (cudaStreamSynchronize(c->stream) != cudaSuccess)
@@ -845,7 +852,7 @@ static int render_enqueue(alpine_gpu_ctx* c, uint32_t spp)
     sc.lights.lights = c->dLights.as<ag::Light>();
     sc.lights.alias = c->dAlias.as<ag::AliasBin>();
     sc.lights.nodes = c->dLightNodes.as<ag::LightNode>();
-    sc.lights.pairs = c->dLightPairs.as<ag::LightPair>();
+    sc.lights.records = c->dLightRecords[stream ? 1 : 0].as<ag::LightRecord>();
     sc.background = c->background;
     sc.cam = c->camera;
     sc.width = c->cfg.width;
