@@ -23,6 +23,7 @@
 #include "../../include/alpine_gpu.h"
 #include "bvh.cuh"
 #include "guide.cuh"
+#include "shade_key.cuh"
 #include "shading.cuh"
 
 namespace ag {
@@ -109,26 +110,26 @@ struct WaveView {
     uint32_t* shadeBins;
 };
 
-// Shading-queue bins (shade_key): a miss; a Dielectric with its Lambertian
-// lobe only; a Dielectric with both lobes; a Conductor; plus kShadeGuided for
-// a vertex the guide samples. Threads of one warp then mostly take the same
-// branches of the shading kernel.
-constexpr uint32_t kShadeBins = 8;
-constexpr uint32_t kShadeGuided = 4;
+// The key source of a scene and wave (keys null without a shading order).
+inline ShadeKeys shade_keys(const SceneView& sc, const WaveView& w, bool sorted)
+{
+    return ShadeKeys{sc.triInfo, sc.sphereMaterial, sc.materials, sc.sphereCount, sc.materialCount,
+                     sorted ? w.shadeKeys : nullptr, w.shadeBins};
+}
 
 struct IntegratorKernels {
     void (*generate)(const SceneView&, const WaveView&, bool streamRng, cudaStream_t);
     void (*shade)(const SceneView&, const WaveView&, bool streamRng, uint32_t maxQueue, cudaStream_t);
     void (*resolve)(const WaveView&, uint32_t maxQueue, cudaStream_t);
     void (*accumulate)(const WaveView&, float* accum, double* accum64, bool streamRng, cudaStream_t);
-    // guiding: queries of the current queue; recorded vertices -> training samples
-    void (*guide_query)(const SceneView&, const WaveView&, uint32_t maxQueue, cudaStream_t);
+    // guiding: queries of the current queue (and, when `sorted`, its shading
+    // keys); recorded vertices -> training samples
+    void (*guide_query)(const SceneView&, const WaveView&, bool sorted, uint32_t maxQueue, cudaStream_t);
     void (*train_finalize)(const WaveView&, guide::Sample* out, uint32_t* outCount, cudaStream_t);
-    // shading order of the current queue: bins[0..7] counts, bins[8..15]
-    // cursors (both zeroed by the caller), keys: one byte per queue entry,
-    // order: the queue entries grouped by bin
-    void (*sort)(const SceneView&, const WaveView&, uint32_t maxQueue, uint32_t* bins, uint8_t* keys,
-                 uint32_t* order, cudaStream_t);
+    // shading order of the current queue from its keys and their counts
+    // (shade_key.cuh): shadeBins[0..7] counts, [8..15] cursors (zeroed by the
+    // caller); shadeOrderBuf: the queue entries grouped by bin
+    void (*sort)(const WaveView&, uint32_t maxQueue, cudaStream_t);
     // the light BVH's records for this integrator's descent
     void (*light_records)(const LightPair* pairs, uint32_t count, LightRecord* out, cudaStream_t);
 };
@@ -415,12 +416,15 @@ AG_D bool guided_continuation(const Material& mat, float3 wo, const float* lobes
 // (a hit, the view direction above the shading surface, material alpha >=
 // guideMinRough), compacted: shading position, roughness, direction towards
 // the previous vertex and shading normal.
-__global__ void __launch_bounds__(kThreads) k_guide_query(SceneView sc, WaveView w)
+__global__ void __launch_bounds__(kThreads) k_guide_query(SceneView sc, WaveView w, ShadeKeys sk)
 {
+    __shared__ uint32_t hist[kShadeBins];
+    if (threadIdx.x < kShadeBins) hist[threadIdx.x] = 0;
+    __syncthreads();
     const uint32_t n = *w.queueCount;
-    uint32_t q = blockIdx.x * kThreads + threadIdx.x;
-    if (q >= n) return;
-    const uint4 h = w.hits[q];
+    const uint32_t q = blockIdx.x * kThreads + threadIdx.x;
+    uint4 h = make_uint4(0xffffffffu, 0u, 0u, 0u);
+    if (q < n) h = w.hits[q];
     bool guided = false;
     guide::Query gq = {};
     if (h.x != 0xffffffffu) {
@@ -443,7 +447,15 @@ __global__ void __launch_bounds__(kThreads) k_guide_query(SceneView sc, WaveView
     }
     const uint32_t slot = warp_append(w.guideCount, guided);
     if (guided) w.guideQuery[slot] = gq;
-    w.guideSlot[q] = guided ? (int)slot : -1;
+    if (q < n) w.guideSlot[q] = guided ? (int)slot : -1;
+    if (!sk.keys) return;
+    if (q < n) {
+        const uint32_t key = shade_key(sk, h.x, guided && w.guideLobes);
+        sk.keys[q] = (uint8_t)key;
+        bin_rank(hist, key);
+    }
+    __syncthreads();
+    if (threadIdx.x < kShadeBins && hist[threadIdx.x]) atomicAdd(sk.counts + threadIdx.x, hist[threadIdx.x]);
 }
 
 // kSampler: the light sampler kind, or -1 to read it from the scene.
@@ -623,54 +635,9 @@ __global__ void __launch_bounds__(kThreads, shade_min_blocks(kGuided, kSampler))
     w.rng[p] = rng.save();
 }
 
-AG_D uint32_t shade_key(const SceneView& sc, const WaveView& w, uint32_t q)
-{
-    const uint32_t prim = w.hits[q].x;
-    uint32_t key = 0;
-    if (prim != 0xffffffffu) {
-        uint32_t mid = (prim & kSpherePrim) ? sc.sphereMaterial[min(prim & ~kSpherePrim, sc.sphereCount - 1u)]
-                                            : __ldg(sc.triInfo + prim) & kTriMaterialMask;
-        if (mid >= sc.materialCount) mid = 0;
-        const Material& m = sc.materials[mid];
-        key = m.kind == kMatConductor ? 3u : (m.lobes == 2u ? 2u : 1u);
-        if (w.guideSlot && w.guideLobes && w.guideSlot[q] >= 0) key |= kShadeGuided;
-    }
-    return key;
-}
-
-// Warp-aggregated rank of this thread among the block's threads with the
-// same key, added to hist[key] (shared memory).
-AG_D uint32_t bin_rank(uint32_t* hist, uint32_t key)
-{
-    const uint32_t am = __activemask();
-    const uint32_t peers = __match_any_sync(am, key);
-    const int leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(hist + key, __popc(peers));
-    base = __shfl_sync(am, base, leader);
-    return base + __popc(peers & lanemask_lt());
-}
-
-// Pass 1 of the shading-order counting sort: the key of every queue entry
-// and the global count of each bin.
-__global__ void __launch_bounds__(kThreads) k_shade_bins(SceneView sc, WaveView w, uint32_t* bins, uint8_t* keys)
-{
-    __shared__ uint32_t hist[kShadeBins];
-    if (threadIdx.x < kShadeBins) hist[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t n = *w.queueCount;
-    const uint32_t q = blockIdx.x * kThreads + threadIdx.x;
-    if (q < n) {
-        const uint32_t key = shade_key(sc, w, q);
-        keys[q] = (uint8_t)key;
-        bin_rank(hist, key);
-    }
-    __syncthreads();
-    if (threadIdx.x < kShadeBins && hist[threadIdx.x]) atomicAdd(bins + threadIdx.x, hist[threadIdx.x]);
-}
-
-// Pass 2: each block reserves a run in every bin it holds (bin start =
-// counts of the lower bins, then a cursor) and writes its entries there.
+// The shading order from the keys (shade_key.cuh): each block reserves a run
+// in every bin it holds (bin start = counts of the lower bins, then a cursor)
+// and writes its entries there.
 // The order inside a bin depends on scheduling; shading results do not.
 __global__ void __launch_bounds__(kThreads) k_shade_scatter(WaveView w, uint32_t* bins, const uint8_t* keys,
                                                             uint32_t* order)
@@ -827,22 +794,18 @@ void accumulate(const WaveView& w, float* accum, double* accum64, bool streamRng
 {
     if (w.numPixels) k_accumulate<<<grid(w.numPixels), kThreads, 0, st>>>(w, accum, accum64, streamRng);
 }
-void guide_query(const SceneView& sc, const WaveView& w, uint32_t maxQueue, cudaStream_t st)
+void guide_query(const SceneView& sc, const WaveView& w, bool sorted, uint32_t maxQueue, cudaStream_t st)
 {
-    if (maxQueue) k_guide_query<<<grid(maxQueue), kThreads, 0, st>>>(sc, w);
+    if (maxQueue) k_guide_query<<<grid(maxQueue), kThreads, 0, st>>>(sc, w, shade_keys(sc, w, sorted));
 }
 void train_finalize(const WaveView& w, guide::Sample* out, uint32_t* outCount, cudaStream_t st)
 {
     if (w.trainCap) k_train_finalize<<<grid(w.trainCap), kThreads, 0, st>>>(w, out, outCount);
 }
-void sort(const SceneView& sc, const WaveView& w, uint32_t maxQueue, uint32_t* bins, uint8_t* keys, uint32_t* order,
-          cudaStream_t st)
+void sort(const WaveView& w, uint32_t maxQueue, cudaStream_t st)
 {
-    if (!maxQueue) return;
-    k_shade_bins<<<grid(maxQueue), kThreads, 0, st>>>(sc, w, bins, keys);
-    k_shade_scatter<<<grid(maxQueue), kThreads, 0, st>>>(w, bins, keys, order);
+    if (maxQueue) k_shade_scatter<<<grid(maxQueue), kThreads, 0, st>>>(w, w.shadeBins, w.shadeKeys, w.shadeOrderBuf);
 }
-
 void light_records(const LightPair* pairs, uint32_t count, LightRecord* out, cudaStream_t st)
 {
     if (count) k_light_records<<<grid(count), kThreads, 0, st>>>(pairs, count, out);

@@ -948,27 +948,29 @@ static int render_enqueue(alpine_gpu_ctx* c, uint32_t spp)
             for (uint32_t depth = 0; depth < sc.maxDepth; ++depth) {
                 w.depth = depth;
                 k_bounce_begin<<<1, 32, 0, st>>>(w.queueCountNext, w.shadowCount, w.tickets, w.shadeBins, w.guideCount);
-                ag::launch_trace_dyn(bvh, w.rays, w.queueCount, w.numPaths, w.tickets, false, w.hits, c->dStatus, st,
-                                     c->traceBlock);
                 const bool guideHere = guiding && (o.guide_max_depth == 0 || depth < o.guide_max_depth);
+                // the shading keys come from the traversal, or, where they
+                // depend on the guide, from its query kernel
+                ag::launch_trace_dyn(bvh, w.rays, w.queueCount, w.numPaths, w.tickets, false, w.hits,
+                                     ag::shade_keys(sc, w, shadeSort && !guideHere), c->dStatus, st, c->traceBlock);
                 ag::WaveView sw = w;
                 if (!guideHere) {  // unguided shading (pending training records still resolve)
                     sw.guideQuery = nullptr;
                     sw.guideLobes = nullptr;
                 }
                 if (guideHere) {
-                    K.guide_query(sc, w, w.numPaths, st);
+                    K.guide_query(sc, w, shadeSort, w.numPaths, st);
                     if (sampleGuide)
                         c->guide.infer_queue(gw.query, w.guideCount, w.numPaths, gw.lobes, st, c->dStatus, true);
                 }
                 if (shadeSort) {  // group the queue by shade_key before shading
-                    K.sort(sc, sw, w.numPaths, w.shadeBins, w.shadeKeys, w.shadeOrderBuf, st);
+                    K.sort(sw, w.numPaths, st);
                     sw.shadeOrder = w.shadeOrderBuf;
                 }
                 K.shade(sc, sw, stream, w.numPaths, st);
                 if (shadows)
                     ag::launch_trace_dyn(bvh, w.shadowRays, w.shadowCount, 2 * w.numPaths, w.tickets + 1, true,
-                                         w.shadowOcc, c->dStatus, st, c->traceBlock);
+                                         w.shadowOcc, ag::ShadeKeys{}, c->dStatus, st, c->traceBlock);
                 if (shadows || w.trainSlot) K.resolve(w, w.numPaths, st);
                 std::swap(w.rays, w.raysNext);
                 std::swap(w.queuePath, w.queuePathNext);

@@ -70,13 +70,22 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceThreads / kTraceBlock) k_tr
 // empty. A grid over the queue's capacity cost 0.55 us per 1,000 blocks that
 // found nothing to do: 32 us for an empty queue of 3.7M entries, on every
 // bounce of a render whose queues run short.
+// With sk.keys a closest-hit launch also writes and counts the entries' shading
+// keys, which took a pass of their own over the hits.
 template <bool kAny, int kBlock, bool kBinary>
 __global__ void __launch_bounds__(kBlock, kTraceThreads / kBlock)
     k_trace_dyn(BvhView bvh, const float4* __restrict__ rays, const uint32_t* __restrict__ count, uint32_t cap,
-                uint32_t* __restrict__ ticket, void* __restrict__ out, uint32_t* __restrict__ status)
+                uint32_t* __restrict__ ticket, void* __restrict__ out, ShadeKeys sk, uint32_t* __restrict__ status)
 {
-    static_assert(kTraversalStack * kBlock * sizeof(uint2) <= 48 * 1024, "static shared memory");
-    __shared__ uint2 stack[kTraversalStack * kBlock];
+    // (the stacks of 256 rays take all the static shared memory a block may have)
+    extern __shared__ uint2 dynStack[];
+    __shared__ uint2 fixedStack[kBlock <= 128 ? kTraversalStack * kBlock : 1];
+    uint2* stack = kBlock <= 128 ? fixedStack : dynStack;
+    __shared__ uint32_t hist[kShadeBins];
+    if (!kAny) {
+        if (threadIdx.x < kShadeBins) hist[threadIdx.x] = 0;
+        __syncthreads();
+    }
     // a count above the capacity would be a queue overflow upstream: reported,
     // and no ray beyond the capacity is read
     if (blockIdx.x == 0 && threadIdx.x == 0 && *count > cap) atomicOr(status, kErrQueueOverflow);
@@ -92,6 +101,11 @@ __global__ void __launch_bounds__(kBlock, kTraceThreads / kBlock)
                                                   stack + threadIdx.x, kBlock, err, nv, tv);
             if (kAny) static_cast<uint8_t*>(out)[i] = hit ? 1 : 0;
             else static_cast<uint4*>(out)[i] = make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.b1), __float_as_uint(r.b2));
+            if (!kAny && sk.keys) {
+                const uint32_t key = shade_key(sk, r.prim, false);
+                sk.keys[i] = (uint8_t)key;
+                bin_rank(hist, key);
+            }
         }
         __syncwarp();
         uint32_t taken = 0;
@@ -99,6 +113,10 @@ __global__ void __launch_bounds__(kBlock, kTraceThreads / kBlock)
         base = first + __shfl_sync(0xffffffffu, taken, 0);
     }
     if (err) atomicOr(status, err);
+    if (!kAny && sk.keys) {
+        __syncthreads();
+        if (threadIdx.x < kShadeBins && hist[threadIdx.x]) atomicAdd(sk.counts + threadIdx.x, hist[threadIdx.x]);
+    }
 }
 
 template <bool kAny>
@@ -120,26 +138,35 @@ void launch(const BvhView& bvh, const void* rays, uint64_t n, void* out, uint32_
 namespace {
 template <int kBlock>
 void launch_dyn(const BvhView& bvh, const float4* r, const uint32_t* count, uint32_t maxCount, uint32_t* ticket, bool any,
-                void* out, uint32_t* status, cudaStream_t st)
+                void* out, const ShadeKeys& sk, uint32_t* status, cudaStream_t st)
 {
     const unsigned wave = 148u * (unsigned)(kTraceThreads / kBlock);  // resident blocks
     const unsigned blocks = std::min((maxCount + kBlock - 1) / kBlock, wave);
     const bool bin = bvh.triTest == kTriTestBinary;
-    if (any && bin) k_trace_dyn<true, kBlock, true><<<blocks, kBlock, 0, st>>>(bvh, r, count, maxCount, ticket, out, status);
-    else if (any) k_trace_dyn<true, kBlock, false><<<blocks, kBlock, 0, st>>>(bvh, r, count, maxCount, ticket, out, status);
-    else if (bin) k_trace_dyn<false, kBlock, true><<<blocks, kBlock, 0, st>>>(bvh, r, count, maxCount, ticket, out, status);
-    else k_trace_dyn<false, kBlock, false><<<blocks, kBlock, 0, st>>>(bvh, r, count, maxCount, ticket, out, status);
+    auto run = [&](auto kernel) {
+        size_t dyn = 0;
+        if (kBlock > 128) {
+            dyn = kTraversalStack * kBlock * sizeof(uint2);
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+        }
+        kernel<<<blocks, kBlock, dyn, st>>>(bvh, r, count, maxCount, ticket, out, sk, status);
+    };
+    if (any && bin) run(k_trace_dyn<true, kBlock, true>);
+    else if (any) run(k_trace_dyn<true, kBlock, false>);
+    else if (bin) run(k_trace_dyn<false, kBlock, true>);
+    else run(k_trace_dyn<false, kBlock, false>);
 }
 }  // namespace
 
 void launch_trace_dyn(const BvhView& bvh, const void* rays, const uint32_t* count, uint32_t maxCount,
-                      uint32_t* ticket, bool any, void* out, uint32_t* status, cudaStream_t st, int block)
+                      uint32_t* ticket, bool any, void* out, const ShadeKeys& sk, uint32_t* status, cudaStream_t st,
+                      int block)
 {
     if (maxCount == 0) return;
     const float4* r = static_cast<const float4*>(rays);
-    if (block == 64) launch_dyn<64>(bvh, r, count, maxCount, ticket, any, out, status, st);
-    else if (block == 256) launch_dyn<256>(bvh, r, count, maxCount, ticket, any, out, status, st);
-    else launch_dyn<128>(bvh, r, count, maxCount, ticket, any, out, status, st);
+    if (block == 64) launch_dyn<64>(bvh, r, count, maxCount, ticket, any, out, sk, status, st);
+    else if (block == 256) launch_dyn<256>(bvh, r, count, maxCount, ticket, any, out, sk, status, st);
+    else launch_dyn<128>(bvh, r, count, maxCount, ticket, any, out, sk, status, st);
 }
 
 void launch_trace_count(const BvhView& bvh, const void* rays, uint64_t n, bool any, unsigned long long* counts,

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "bvh.cuh"
+#include "shade_key.cuh"
 
 namespace ag {
 
@@ -21,9 +22,10 @@ void launch_occluded(const BvhView& bvh, const void* rays, uint64_t n, uint8_t* 
 // Queue variant: the number of rays is *count (device memory, read by the
 // kernel), at most maxCount. ticket: a device word that is 0 when the kernel
 // starts and used by this launch alone. any selects any-hit (uint8 results) or
-// closest. block: threads per block, 64, 128 or 256.
+// closest. sk: where a closest-hit launch puts the entries' shading keys and
+// counts (keys null: nowhere). block: threads per block, 64, 128 or 256.
 void launch_trace_dyn(const BvhView& bvh, const void* rays, const uint32_t* count, uint32_t maxCount,
-                      uint32_t* ticket, bool any, void* out, uint32_t* status, cudaStream_t st,
+                      uint32_t* ticket, bool any, void* out, const ShadeKeys& sk, uint32_t* status, cudaStream_t st,
                       int block = kTraceBlock);
 
 // Instrumented traversal: counts[0] += wide nodes fetched, counts[1] += triangles tested.
