@@ -171,8 +171,6 @@ AG_D uint32_t scan_add(uint32_t v)
 }
 
 // Minimum / maximum of a float over the warp (no NaN among the values).
-AG_D float warp_min(float v) { return ord2f(__reduce_min_sync(0xffffffffu, f2ord(v))); }
-AG_D float warp_max(float v) { return ord2f(__reduce_max_sync(0xffffffffu, f2ord(v))); }
 
 // Result of a warp-wide split search over the bins of one task.
 struct SplitChoice {
@@ -250,6 +248,23 @@ AG_D void bin_accumulate(uint32_t* bin, const uint32_t ord[6])
     atomicMax(bin + 3, ord[3]);
     atomicMax(bin + 4, ord[4]);
     atomicMax(bin + 5, ord[5]);
+    atomicAdd(bin + 6, 1u);
+}
+
+// The same, for bins that many references fall into: a bound that the bin
+// already covers needs no atomic. The bounds only ever widen, so a stale word
+// costs an atomic and changes nothing.
+AG_D void bin_widen(uint32_t* bin, const uint32_t ord[6])
+{
+    const volatile uint32_t* seen = bin;
+    uint32_t w[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) w[k] = seen[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (ord[k] < w[k]) atomicMin(bin + k, ord[k]);
+        if (ord[3 + k] > w[3 + k]) atomicMax(bin + 3 + k, ord[3 + k]);
+    }
     atomicAdd(bin + 6, 1u);
 }
 
@@ -388,9 +403,12 @@ __global__ void k_root(uint32_t n, uint32_t* __restrict__ cnt, BigTask* __restri
 // Big tasks, level by level. The lists are double-buffered by level parity.
 // One block per chunk of 1,024 references; the chunk's bin counts are kept
 // (16 bits each), so that k_split can place the chunks of the partition
-// without another pass over the references. Bound by the shared-memory
-// atomics (21 a reference; with the centroid bounds among the bins' words it
-// was 39).
+// without another pass over the references. 21 atomics a reference on the
+// shared bins bound it at first, and at the top the 1,024 blocks' merges into
+// one task's bins: most of a bin's later references widen nothing, so a plain
+// read comes before each atomic min / max, here and in the merge, and the four
+// references of a thread are fetched together. Root of 1M triangles: 43 to
+// 31 us, the level below 37 to 25 (B200).
 __global__ void __launch_bounds__(kChunkThreads) k_bin(const BigTask* __restrict__ tasks, const uint32_t* __restrict__ refs,
                                                        const float4* __restrict__ boxes,
                                                        const uint32_t* __restrict__ chunkTask,
@@ -413,9 +431,17 @@ __global__ void __launch_bounds__(kChunkThreads) k_bin(const BigTask* __restrict
             sc[a] = axis_scale(clo[a], ord2f(task.chi[a]));
         }
         const uint32_t begin = task.begin + (cb - task.chunk0) * kChunk, end = min(task.begin + task.count, begin + kChunk);
-        for (uint32_t i = begin + threadIdx.x; i < end; i += kChunkThreads) {
+        uint32_t p[kChunk / kChunkThreads];
+#pragma unroll
+        for (int r = 0; r < (int)kChunk / kChunkThreads; ++r) {
+            const uint32_t i = begin + r * kChunkThreads + threadIdx.x;
+            p[r] = i < end ? refs[i] : kNoTask;
+        }
+#pragma unroll
+        for (int r = 0; r < (int)kChunk / kChunkThreads; ++r) {
+            if (p[r] == kNoTask) break;
             float lo[3], hi[3];
-            load_box(boxes, refs[i], lo, hi);
+            load_box(boxes, p[r], lo, hi);
             uint32_t ord[6];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -425,7 +451,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_bin(const BigTask* __restrict
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (sc[a] == 0.0f) continue;
-                bin_accumulate(sb + a * kAxisBinWords + bin_of(centroid(lo[a], hi[a]), clo[a], sc[a]) * kBinWords, ord);
+                bin_widen(sb + a * kAxisBinWords + bin_of(centroid(lo[a], hi[a]), clo[a], sc[a]) * kBinWords, ord);
             }
         }
         __syncthreads();
@@ -435,9 +461,10 @@ __global__ void __launch_bounds__(kChunkThreads) k_bin(const BigTask* __restrict
             const uint32_t filled = sb[k - f + 6];
             if (f == 6) chunkCnt[size_t(cb) * kChunkCounts + k / kBinWords] = (uint16_t)filled;
             if (filled == 0) continue;  // empty bin: nothing to merge
+            const uint32_t mine = sb[k], seen = __ldcg(g + k);
             if (f == 6) atomicAdd(g + k, filled);
-            else if (f < 3) atomicMin(g + k, sb[k]);
-            else atomicMax(g + k, sb[k]);
+            else if (f < 3 && mine < seen) atomicMin(g + k, mine);
+            else if (f >= 3 && mine > seen) atomicMax(g + k, mine);
         }
         __syncthreads();  // sb is cleared again for the next chunk
     }
@@ -475,66 +502,79 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* __restri
             if (lane_id() == 0) axisBest[warp] = best;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < 2) {  // lane k takes child k; the counters' round trips overlap
+            const uint32_t k = threadIdx.x;
             SplitChoice best = axisBest[0];
+#pragma unroll
             for (int a = 1; a < 3; ++a)
                 if (axisBest[a].cost < best.cost) best = axisBest[a];
-            BigSplit s;
-            s.axis = best.axis >= 0 ? best.axis : 0;
-            s.bin = best.bin;
-            s.mode = best.axis >= 0 ? 0 : 1;
-            s.nL = best.axis >= 0 ? best.nL : task.count / 2;
-            if (best.axis < 0) {  // all centroids coincide: split by position, the children keep the parent's box
-                const BinNode p = bnodes[task.node];
-                const float box[6] = {p.lo.x, p.lo.y, p.lo.z, p.hi.x, p.hi.y, p.hi.z};
-                for (int k = 0; k < 6; ++k) best.L[k] = best.R[k] = box[k];
+            const bool median = best.axis < 0;
+            const uint32_t nL = median ? task.count / 2 : best.nL;
+            const uint32_t begin = k ? task.begin + nL : task.begin, count = k ? task.count - nL : nL;
+            const uint32_t chunks = count > kSmallMax ? (count + kChunk - 1) / kChunk : 0u;
+            uint32_t id = 0, ci = kNoTask, c0 = 0, si = 0;
+            if (k == 0) id = atomicAdd(cnt + kCntNodes, 2u);
+            if (chunks) {
+                ci = atomicAdd(cnt + kLevelBig + level + 1, 1u);
+                c0 = atomicAdd(cnt + kLevelChunks + level + 1, chunks);
+            } else {
+                si = atomicAdd(cnt + kCntSmall, 1u);
             }
-            s.child[0] = s.child[1] = kNoTask;
-            childChunks[0] = childChunks[1] = 0u;
-            childChunk0[0] = childChunk0[1] = 0u;
-            const uint32_t id = atomicAdd(cnt + kCntNodes, 2u);
-            atomicAdd(cnt + kCntRealNodes, 2u);
-            atomicMax(cnt + kCntLevels, level + 1u);
+            if (k == 0) {
+                atomicAdd(cnt + kCntRealNodes, 2u);
+                atomicMax(cnt + kCntLevels, level + 1u);
+            }
+            float box[6];
+#pragma unroll
+            for (int j = 0; j < 6; ++j) box[j] = k ? best.R[j] : best.L[j];
+            if (median) {  // all centroids coincide: split by position, the children keep the parent's box
+                const BinNode parent = bnodes[task.node];
+                box[0] = parent.lo.x; box[1] = parent.lo.y; box[2] = parent.lo.z;
+                box[3] = parent.hi.x; box[4] = parent.hi.y; box[5] = parent.hi.z;
+            }
+            id = __shfl_sync(3u, id, 0);
             // capacities: never exceeded by a consistent build; checked so that
             // inconsistent input cannot write past the buffers
-            bool ok = id + 1u < 2u * capPrims;
-            if (ok) {
-                bnodes[task.node].left = (int32_t)id;
-                bnodes[task.node].right = (int32_t)id + 1;
-                const uint32_t begin[2] = {task.begin, task.begin + s.nL}, count[2] = {s.nL, task.count - s.nL};
-                for (uint32_t k = 0; k < 2; ++k) {
-                    write_node(bnodes, id + k, k ? best.R : best.L, begin[k], count[k]);
-                    if (count[k] > kSmallMax) {
-                        const uint32_t chunks = (count[k] + kChunk - 1) / kChunk;
-                        const uint32_t ci = atomicAdd(cnt + kLevelBig + level + 1, 1u);
-                        const uint32_t c0 = atomicAdd(cnt + kLevelChunks + level + 1, chunks);
-                        if (ci >= capBig || c0 + chunks > capChunks) { ok = false; continue; }
-                        BigTask t{};
-                        for (int a = 0; a < 3; ++a) {
-                            t.clo[a] = 0xffffffffu;  // gathered by k_scatter
-                            t.chi[a] = 0u;
-                        }
-                        t.node = id + k;
-                        t.begin = begin[k];
-                        t.count = count[k];
-                        t.chunk0 = c0;
-                        next[ci] = t;
-                        s.child[k] = ci;
-                        childChunk0[k] = c0;
-                        childChunks[k] = chunks;
-                    } else {
-                        const uint32_t si = atomicAdd(cnt + kCntSmall, 1u);
-                        if (si >= capPrims) { ok = false; continue; }
-                        small[si] = SmallTask{id + k, begin[k], count[k], level + 1u};
-                    }
+            const bool nodes = id + 1u < 2u * capPrims;
+            const bool listed = chunks ? ci < capBig && c0 + chunks <= capChunks : si < capPrims;
+            if (nodes) {
+                if (k == 0) {
+                    bnodes[task.node].left = (int32_t)id;
+                    bnodes[task.node].right = (int32_t)id + 1;
                 }
+                write_node(bnodes, id + k, box, begin, count);
             }
-            if (!ok) {
+            if (nodes && listed) {
+                if (chunks) {
+                    BigTask t{};
+                    for (int a = 0; a < 3; ++a) {
+                        t.clo[a] = 0xffffffffu;  // gathered by k_scatter
+                        t.chi[a] = 0u;
+                    }
+                    t.node = id + k;
+                    t.begin = begin;
+                    t.count = count;
+                    t.chunk0 = c0;
+                    next[ci] = t;
+                } else {
+                    small[si] = SmallTask{id + k, begin, count, level + 1u};
+                }
+            } else {
                 atomicOr(status, kErrBadIndex);
                 atomicOr(cnt + kCntFailed, kFailCapacity);
             }
-            split = s;
-            splits[bi] = s;
+            const bool pass = nodes && listed && chunks;  // to the next level
+            split.child[k] = pass ? ci : kNoTask;
+            childChunk0[k] = c0;
+            childChunks[k] = pass ? chunks : 0u;
+            if (k == 0) {
+                split.axis = median ? 0 : best.axis;
+                split.bin = best.bin;
+                split.mode = median ? 1 : 0;
+                split.nL = nL;
+            }
+            __syncwarp(3u);
+            if (k == 0) splits[bi] = split;
         }
         __syncthreads();
         const BigSplit s = split;
@@ -553,8 +593,20 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* __restri
             const uint32_t c = base + threadIdx.x;
             uint32_t left = 0;
             if (c < chunks && s.mode == 0) {
-                const uint16_t* p = chunkCnt + size_t(task.chunk0 + c) * kChunkCounts + s.axis * kSahBins;
-                for (int b = 0; b <= s.bin; ++b) left += p[b];
+                // the row of the axis: 32 counts of 16 bits, 64 bytes
+                const uint4* p = reinterpret_cast<const uint4*>(chunkCnt + size_t(task.chunk0 + c) * kChunkCounts + s.axis * kSahBins);
+                uint4 q[kSahBins / 8];
+#pragma unroll
+                for (int k = 0; k < kSahBins / 8; ++k) q[k] = p[k];
+#pragma unroll
+                for (int k = 0; k < kSahBins / 8; ++k) {
+                    const uint32_t v[4] = {q[k].x, q[k].y, q[k].z, q[k].w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int b = 8 * k + 2 * j;
+                        left += (b <= s.bin ? v[j] & 0xffffu : 0u) + (b + 1 <= s.bin ? v[j] >> 16 : 0u);
+                    }
+                }
             }
             const uint32_t inc = scan_add(left);
             if (lane_id() == 31) warpSums[warp] = inc;
@@ -572,52 +624,62 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* __restri
     }
 }
 
-// Stable partition, one block per chunk, four consecutive references a
-// thread; also the centroid bounds of the big children.
-__global__ void __launch_bounds__(kChunkThreads) k_scatter(BigTask* __restrict__ next, const BigTask* __restrict__ tasks,
-                                                           const uint32_t* __restrict__ refs,
-                                                           uint32_t* __restrict__ refsNext,
-                                                           const float4* __restrict__ boxes,
-                                                           const uint32_t* __restrict__ chunkTask,
-                                                           const BigSplit* __restrict__ splits,
-                                                           const uint32_t* __restrict__ chunkLeft,
-                                                           const uint32_t* __restrict__ cnt, uint32_t level,
-                                                           uint32_t capChunks, uint32_t* __restrict__ status)
+// Stable partition, one block per chunk, four references a thread, a block's
+// width apart: whole sectors of references, and a reference's rank is a ballot
+// within its warp plus the counts of the 32 (round, warp) groups before it.
+// Also the centroid bounds of the big children. Bound by the latency of
+// reference -> box -> rank, so by the blocks in flight: 8 per SM hold the
+// 1,024 chunks of 1M references at once. With four consecutive references a
+// thread and 4 blocks per SM a level took 22 us, at 6 blocks 19 (B200).
+constexpr int kScatterRounds = (int)kChunk / kChunkThreads;
+static_assert(kScatterRounds * (kChunkThreads / 32) == 32, "one lane a group in the scan of the groups");
+__global__ void __launch_bounds__(kChunkThreads, 8) k_scatter(BigTask* __restrict__ next, const BigTask* __restrict__ tasks,
+                                                              const uint32_t* __restrict__ refs,
+                                                              uint32_t* __restrict__ refsNext,
+                                                              const float4* __restrict__ boxes,
+                                                              const uint32_t* __restrict__ chunkTask,
+                                                              const BigSplit* __restrict__ splits,
+                                                              const uint32_t* __restrict__ chunkLeft,
+                                                              const uint32_t* __restrict__ cnt, uint32_t level,
+                                                              uint32_t capChunks, uint32_t* __restrict__ status)
 {
-    __shared__ uint32_t wl[kChunkThreads / 32], wv[kChunkThreads / 32], cb12[12];
+    __shared__ uint32_t groupLeft[32], cb12[12];
     const uint32_t nc = cnt[kCntFailed] ? 0u : min(cnt[kLevelChunks + level], capChunks);
+    const uint32_t warp = threadIdx.x >> 5;
     for (uint32_t cb = blockIdx.x; cb < nc; cb += gridDim.x) {
         const uint32_t bi = chunkTask[cb];
-        const BigTask task = tasks[bi];
-        const BigSplit s = splits[bi];
-        const uint32_t local = cb - task.chunk0, begin = task.begin + local * kChunk;
-        const uint32_t end = min(task.begin + task.count, begin + kChunk);
-        const uint32_t leftBefore = chunkLeft[cb], rightBefore = local * kChunk - leftBefore;
-        const float clo = ord2f(task.clo[s.axis]);
-        const float scale = axis_scale(clo, ord2f(task.chi[s.axis]));
+        const BigTask& task = tasks[bi];
+        const BigSplit& s = splits[bi];
+        const uint32_t taskBegin = task.begin, taskCount = task.count, nL = s.nL;
+        const uint32_t first = (cb - task.chunk0) * kChunk;  // within the task
+        const uint32_t count = min(taskCount - first, kChunk);
+        const uint32_t leftBefore = chunkLeft[cb], rightBefore = first - leftBefore;
+        const int axis = s.axis, bin = s.bin;
+        const bool byPosition = s.mode == 1;
+        const float clo = ord2f(task.clo[axis]);
+        const float scale = axis_scale(clo, ord2f(task.chi[axis]));
         if (threadIdx.x < 12) cb12[threadIdx.x] = threadIdx.x % 6 < 3 ? 0xffffffffu : 0u;
-        const uint32_t base = begin + threadIdx.x * 4;
-        uint32_t p[4];
-        bool f[4];
-        uint32_t nl = 0;
+        uint32_t p[kScatterRounds];
+#pragma unroll
+        for (int r = 0; r < kScatterRounds; ++r) {
+            const uint32_t i = r * kChunkThreads + threadIdx.x;
+            p[r] = i < count ? refs[taskBegin + first + i] : kNoTask;
+        }
+        uint32_t leftMask[kScatterRounds];
         uint32_t bb[12] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u, 0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t i = base + k;
-            f[k] = false;
-            p[k] = 0;
-            if (i < end) {
-                p[k] = refs[i];
+        for (int r = 0; r < kScatterRounds; ++r) {
+            bool left = false;
+            if (p[r] != kNoTask) {
                 float lo[3], hi[3];
-                load_box(boxes, p[k], lo, hi);
+                load_box(boxes, p[r], lo, hi);
                 const float c[3] = {centroid(lo[0], hi[0]), centroid(lo[1], hi[1]), centroid(lo[2], hi[2])};
-                const float ca = s.axis == 0 ? c[0] : (s.axis == 1 ? c[1] : c[2]);
-                f[k] = s.mode == 1 ? (i - task.begin) < s.nL : bin_of(ca, clo, scale) <= s.bin;
-                nl += f[k];
+                const float ca = axis == 0 ? c[0] : (axis == 1 ? c[1] : c[2]);
+                left = byPosition ? first + r * kChunkThreads + threadIdx.x < nL : bin_of(ca, clo, scale) <= bin;
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     const uint32_t o = f2ord(c[a]);
-                    if (f[k]) {
+                    if (left) {
                         bb[a] = min(bb[a], o);
                         bb[3 + a] = max(bb[3 + a], o);
                     } else {
@@ -626,27 +688,25 @@ __global__ void __launch_bounds__(kChunkThreads) k_scatter(BigTask* __restrict__
                     }
                 }
             }
+            leftMask[r] = __ballot_sync(0xffffffffu, left);
+            if (lane_id() == 0) groupLeft[r * (kChunkThreads / 32) + warp] = __popc(leftMask[r]);
         }
-        const uint32_t nvalid = base < end ? min(4u, end - base) : 0u;
-        // block exclusive scan of (left count, valid count)
-        const uint32_t il = scan_add(nl), iv = scan_add(nvalid);
-        if (lane_id() == 31) { wl[threadIdx.x >> 5] = il; wv[threadIdx.x >> 5] = iv; }
         __syncthreads();
-        uint32_t pl = 0, pv = 0;
-        for (uint32_t w = 0; w < (threadIdx.x >> 5); ++w) { pl += wl[w]; pv += wv[w]; }
-        uint32_t leftRank = pl + il - nl;
-        uint32_t rightRank = (pv + iv - nvalid) - leftRank;
+        const uint32_t mine = groupLeft[lane_id()], before = scan_add(mine) - mine;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t i = base + k;
-            if (i >= end) break;
-            const uint32_t dst = f[k] ? task.begin + leftBefore + leftRank++ : task.begin + s.nL + rightBefore + rightRank++;
-            if (dst >= task.begin + task.count) { atomicOr(status, kErrBadIndex); continue; }
-            refsNext[dst] = p[k];
+        for (int r = 0; r < kScatterRounds; ++r) {
+            const uint32_t leftRank = __shfl_sync(0xffffffffu, before, r * (kChunkThreads / 32) + (int)warp) +
+                                      __popc(leftMask[r] & ((1u << lane_id()) - 1u));
+            if (p[r] == kNoTask) continue;
+            const uint32_t i = r * kChunkThreads + threadIdx.x;
+            const uint32_t at = leftMask[r] >> lane_id() & 1u ? leftBefore + leftRank : nL + rightBefore + i - leftRank;
+            if (at >= taskCount) { atomicOr(status, kErrBadIndex); continue; }
+            refsNext[taskBegin + at] = p[r];
         }
+        const uint32_t child[2] = {s.child[0], s.child[1]};
 #pragma unroll
         for (int side = 0; side < 2; ++side) {
-            if (s.child[side] == kNoTask) continue;
+            if (child[side] == kNoTask) continue;
 #pragma unroll
             for (int a = 0; a < 6; ++a) {
                 const uint32_t v = a < 3 ? __reduce_min_sync(0xffffffffu, bb[6 * side + a])
@@ -658,9 +718,9 @@ __global__ void __launch_bounds__(kChunkThreads) k_scatter(BigTask* __restrict__
             }
         }
         __syncthreads();
-        const uint32_t w = threadIdx.x;
-        if (w < 12 && s.child[w / 6] != kNoTask) {
-            BigTask* t = next + s.child[w / 6];
+        const uint32_t w = threadIdx.x, to = w < 6 ? child[0] : child[1];
+        if (w < 12 && to != kNoTask) {
+            BigTask* t = next + to;
             if (w % 6 < 3) atomicMin(t->clo + w % 6, cb12[w]);
             else atomicMax(t->chi + w % 6 - 3, cb12[w]);
         }
