@@ -170,8 +170,6 @@ AG_D uint32_t scan_add(uint32_t v)
     return v;
 }
 
-// Minimum / maximum of a float over the warp (no NaN among the values).
-
 // Result of a warp-wide split search over the bins of one task.
 struct SplitChoice {
     float cost;
@@ -269,7 +267,7 @@ AG_D void bin_widen(uint32_t* bin, const uint32_t ord[6])
 }
 
 // Primitive boxes: {lo.xyz, hi.x}, {hi.y, hi.z, 0, 0}, one 32-byte sector each.
-AG_D void load_box(const float4* __restrict__ boxes, uint32_t p, float lo[3], float hi[3])
+AG_D void load_box(const float4* boxes, uint32_t p, float lo[3], float hi[3])
 {
     const float4 a = boxes[2ull * p];
     const float2 b = *reinterpret_cast<const float2*>(boxes + 2ull * p + 1);
@@ -277,7 +275,7 @@ AG_D void load_box(const float4* __restrict__ boxes, uint32_t p, float lo[3], fl
     hi[0] = a.w; hi[1] = b.x; hi[2] = b.y;
 }
 
-AG_D void write_node(BinNode* __restrict__ bnodes, uint32_t id, const float box[6], uint32_t begin, uint32_t count)
+AG_D void write_node(BinNode* bnodes, uint32_t id, const float box[6], uint32_t begin, uint32_t count)
 {
     BinNode b;
     b.lo = mk3(box[0], box[1], box[2]);
@@ -291,9 +289,29 @@ AG_D void write_node(BinNode* __restrict__ bnodes, uint32_t id, const float box[
 }
 
 // --------------------------------------------------------------------------
-// Preparation: counters, primitive boxes and root bounds.
-__global__ void k_begin(uint32_t* __restrict__ cnt)
+// The kernels of a build form a chain in which each needs all of the one
+// before it, 30 to 70 launches of which many run for a few microseconds. They
+// are launched with programmatic stream serialisation: the blocks of the next
+// kernel are placed while this one runs, and chain_wait(), the first statement
+// of every kernel of the chain in every thread, holds them until it has
+// finished and its writes are visible. Only then is the kernel after them
+// allowed in, so at most one is waiting at a time, and each kernel's end
+// implies the end of all before it. The pointers of these kernels carry no
+// __restrict__: it would let the compiler take what the kernel before writes
+// for constant data. 1M triangles: 2,091 to 1,995 us; an animated frame of 8k
+// triangles: 488 to 404 us (B200).
+AG_D void chain_allow() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+AG_D void chain_wait()
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    chain_allow();
+}
+
+// --------------------------------------------------------------------------
+// Preparation: counters, primitive boxes and root bounds.
+__global__ void k_begin(uint32_t* cnt)
+{
+    chain_allow();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kAllWords; i += gridDim.x * blockDim.x)
         cnt[i] = (i < 3 || (i >= 6 && i < 9)) ? 0xffffffffu : 0u;  // the bounds' min words, else 0
 }
@@ -303,12 +321,13 @@ __global__ void k_begin(uint32_t* __restrict__ cnt)
 // block before the 12 atomics: one set of atomics per warp took 256 of the
 // 262 us of this kernel on 1M triangles.
 constexpr int kPrepThreads = 256;
-__global__ void __launch_bounds__(kPrepThreads) k_prep_prims(const float* __restrict__ verts,
-                                                             const uint32_t* __restrict__ idx, uint32_t ntris,
-                                                             const float4* __restrict__ spheres, uint32_t n,
-                                                             float4* __restrict__ boxes, uint32_t* __restrict__ refs,
-                                                             uint32_t* __restrict__ bounds)
+__global__ void __launch_bounds__(kPrepThreads) k_prep_prims(const float* verts,
+                                                             const uint32_t* idx, uint32_t ntris,
+                                                             const float4* spheres, uint32_t n,
+                                                             float4* boxes, uint32_t* refs,
+                                                             uint32_t* bounds)
 {
+    chain_wait();
     __shared__ uint32_t sb[12];
     if (threadIdx.x < 12) sb[threadIdx.x] = (threadIdx.x < 3 || (threadIdx.x >= 6 && threadIdx.x < 9)) ? 0xffffffffu : 0u;
     __syncthreads();
@@ -365,9 +384,10 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep_prims(const float* __rest
     }
 }
 
-__global__ void k_root(uint32_t n, uint32_t* __restrict__ cnt, BigTask* __restrict__ big, BinNode* __restrict__ bnodes,
-                       SmallTask* __restrict__ small, uint32_t* __restrict__ chunkTask, uint32_t* __restrict__ bins)
+__global__ void k_root(uint32_t n, uint32_t* cnt, BigTask* big, BinNode* bnodes,
+                       SmallTask* small, uint32_t* chunkTask, uint32_t* bins)
 {
+    chain_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t chunks = n > kSmallMax ? (n + kChunk - 1) / kChunk : 0u;
     if (i == 0) {
@@ -409,12 +429,13 @@ __global__ void k_root(uint32_t n, uint32_t* __restrict__ cnt, BigTask* __restri
 // read comes before each atomic min / max, here and in the merge, and the four
 // references of a thread are fetched together. Root of 1M triangles: 43 to
 // 31 us, the level below 37 to 25 (B200).
-__global__ void __launch_bounds__(kChunkThreads) k_bin(const BigTask* __restrict__ tasks, const uint32_t* __restrict__ refs,
-                                                       const float4* __restrict__ boxes,
-                                                       const uint32_t* __restrict__ chunkTask,
-                                                       uint32_t* __restrict__ bins, uint16_t* __restrict__ chunkCnt,
-                                                       uint32_t* __restrict__ cnt, uint32_t level, uint32_t capChunks)
+__global__ void __launch_bounds__(kChunkThreads) k_bin(const BigTask* tasks, const uint32_t* refs,
+                                                       const float4* boxes,
+                                                       const uint32_t* chunkTask,
+                                                       uint32_t* bins, uint16_t* chunkCnt,
+                                                       uint32_t* cnt, uint32_t level, uint32_t capChunks)
 {
+    chain_wait();
     __shared__ uint32_t sb[kTaskBinWords];
     // the next level's nodes start where the ids handed out so far end
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt[kLevelNodes + level + 1] = cnt[kCntNodes];
@@ -473,16 +494,17 @@ __global__ void __launch_bounds__(kChunkThreads) k_bin(const BigTask* __restrict
 // One block per big task: the split (a warp per axis), the children, and the
 // position of every chunk's left references in the partition.
 constexpr int kSplitThreads = 256;
-__global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* __restrict__ tasks, const uint32_t* __restrict__ bins,
-                                                         const uint16_t* __restrict__ chunkCnt,
-                                                         uint32_t* __restrict__ chunkLeft, BigSplit* __restrict__ splits,
-                                                         BinNode* __restrict__ bnodes, BigTask* __restrict__ next,
-                                                         uint32_t* __restrict__ nextChunkTask,
-                                                         uint32_t* __restrict__ nextBins, SmallTask* __restrict__ small,
-                                                         uint32_t* __restrict__ cnt, uint32_t level, uint32_t capBig,
+__global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* tasks, const uint32_t* bins,
+                                                         const uint16_t* chunkCnt,
+                                                         uint32_t* chunkLeft, BigSplit* splits,
+                                                         BinNode* bnodes, BigTask* next,
+                                                         uint32_t* nextChunkTask,
+                                                         uint32_t* nextBins, SmallTask* small,
+                                                         uint32_t* cnt, uint32_t level, uint32_t capBig,
                                                          uint32_t capChunks, uint32_t capPrims,
-                                                         uint32_t* __restrict__ status)
+                                                         uint32_t* status)
 {
+    chain_wait();
     __shared__ SplitChoice axisBest[3];
     __shared__ BigSplit split;
     __shared__ uint32_t childChunk0[2], childChunks[2], warpSums[kSplitThreads / 32];
@@ -633,16 +655,17 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* __restri
 // thread and 4 blocks per SM a level took 22 us, at 6 blocks 19 (B200).
 constexpr int kScatterRounds = (int)kChunk / kChunkThreads;
 static_assert(kScatterRounds * (kChunkThreads / 32) == 32, "one lane a group in the scan of the groups");
-__global__ void __launch_bounds__(kChunkThreads, 8) k_scatter(BigTask* __restrict__ next, const BigTask* __restrict__ tasks,
-                                                              const uint32_t* __restrict__ refs,
-                                                              uint32_t* __restrict__ refsNext,
-                                                              const float4* __restrict__ boxes,
-                                                              const uint32_t* __restrict__ chunkTask,
-                                                              const BigSplit* __restrict__ splits,
-                                                              const uint32_t* __restrict__ chunkLeft,
-                                                              const uint32_t* __restrict__ cnt, uint32_t level,
-                                                              uint32_t capChunks, uint32_t* __restrict__ status)
+__global__ void __launch_bounds__(kChunkThreads, 8) k_scatter(BigTask* next, const BigTask* tasks,
+                                                              const uint32_t* refs,
+                                                              uint32_t* refsNext,
+                                                              const float4* boxes,
+                                                              const uint32_t* chunkTask,
+                                                              const BigSplit* splits,
+                                                              const uint32_t* chunkLeft,
+                                                              const uint32_t* cnt, uint32_t level,
+                                                              uint32_t capChunks, uint32_t* status)
 {
+    chain_wait();
     __shared__ uint32_t groupLeft[32], cb12[12];
     const uint32_t nc = cnt[kCntFailed] ? 0u : min(cnt[kLevelChunks + level], capChunks);
     const uint32_t warp = threadIdx.x >> 5;
@@ -862,7 +885,7 @@ AG_D bool key_left(unsigned long long key, uint32_t pbin, uint32_t local, uint32
 
 // Two children of node nd (nL of its references go left). The subtree's nodes
 // are 0 (the root, id rootNode) and 1, 2, ... (ids idBase, idBase + 1, ...).
-AG_D void sub_children(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t rootNode, uint32_t globalBegin, uint32_t nd,
+AG_D void sub_children(SubSmem& s, BinNode* bnodes, uint32_t rootNode, uint32_t globalBegin, uint32_t nd,
                        uint32_t nL, const float L[6], const float R[6])
 {
     const uint32_t ch = atomicAdd(&s.nodeTop, 2u);
@@ -898,7 +921,7 @@ AG_D void median_boxes(const SubSmem& s, uint32_t b, uint32_t c, float L[6], flo
 
 // Splits the level's nodes above kDirectMax references (binNode). bin: this
 // thread's entry of the list, kNoTask if it has none. Called by the whole block.
-AG_D void sub_split_bins(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t rootNode, uint32_t globalBegin, uint32_t ls,
+AG_D void sub_split_bins(SubSmem& s, BinNode* bnodes, uint32_t rootNode, uint32_t globalBegin, uint32_t ls,
                          uint32_t bin)
 {
     const uint32_t tid = threadIdx.x, warp = tid >> 5, total = s.binCount;
@@ -989,15 +1012,16 @@ AG_D void sub_split_bins(SubSmem& s, BinNode* __restrict__ bnodes, uint32_t root
 
 // levels: the binary levels that the big-task kernels ran; big tasks left
 // after them mean that the tree cannot be finished here (kCntFailed).
-__global__ void __launch_bounds__(kSubThreads, 2) k_subtree(const SmallTask* __restrict__ small,
-                                                            const uint32_t* __restrict__ refs0,
-                                                            const uint32_t* __restrict__ refs1,
-                                                            const float4* __restrict__ boxes,
-                                                            BinNode* __restrict__ bnodes, uint32_t* __restrict__ order,
-                                                            float* __restrict__ cost, uint32_t* __restrict__ choice,
-                                                            float triCost, bool sah, uint32_t* __restrict__ cnt,
+__global__ void __launch_bounds__(kSubThreads, 2) k_subtree(const SmallTask* small,
+                                                            const uint32_t* refs0,
+                                                            const uint32_t* refs1,
+                                                            const float4* boxes,
+                                                            BinNode* bnodes, uint32_t* order,
+                                                            float* cost, uint32_t* choice,
+                                                            float triCost, bool sah, uint32_t* cnt,
                                                             uint32_t levels, uint32_t capPrims)
 {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     SubSmem& s = *reinterpret_cast<SubSmem*>(smem);
     const uint32_t tid = threadIdx.x;
@@ -1217,11 +1241,12 @@ AG_D float bn_area(const BinNode& b) { return area_of(b.lo.x, b.lo.y, b.lo.z, b.
 // maxLevels, leaves the collapse without items (the previous tree stays in
 // place); status (may be null) then gets kErrBuildDepth.
 constexpr int kTopThreads = 1024;
-__global__ void __launch_bounds__(kTopThreads) k_top(const BinNode* __restrict__ bnodes, float* __restrict__ cost,
-                                                     uint32_t* __restrict__ choice, float triCost, bool sah,
-                                                     uint2* __restrict__ items, uint32_t* __restrict__ cnt,
-                                                     uint32_t levels, uint32_t maxLevels, uint32_t* __restrict__ status)
+__global__ void __launch_bounds__(kTopThreads) k_top(const BinNode* bnodes, float* cost,
+                                                     uint32_t* choice, float triCost, bool sah,
+                                                     uint2* items, uint32_t* cnt,
+                                                     uint32_t levels, uint32_t maxLevels, uint32_t* status)
 {
+    chain_wait();
     if (cnt[kCntFailed] != 0u || cnt[kCntLevels] > maxLevels) {
         if (threadIdx.x == 0) {
             cnt[kCntFailed] |= kFailLevels;
@@ -1267,13 +1292,14 @@ constexpr uint32_t kWideItemsPerBlock = kWideThreads / 8;
 // program's decisions) selects the SAH-optimal distribution; null selects the
 // greedy rule. The entries are then assigned to octants, and the block's
 // counts kept for k_wide_emit's prefix sums.
-__global__ void __launch_bounds__(kWideThreads) k_wide_decide(const uint2* __restrict__ items,
-                                                              const BinNode* __restrict__ bnodes,
-                                                              const uint32_t* __restrict__ choice,
-                                                              int32_t* __restrict__ slots, uint2* __restrict__ itemOff,
-                                                              uint2* __restrict__ blockSum, uint32_t* __restrict__ cnt,
+__global__ void __launch_bounds__(kWideThreads) k_wide_decide(const uint2* items,
+                                                              const BinNode* bnodes,
+                                                              const uint32_t* choice,
+                                                              int32_t* slots, uint2* itemOff,
+                                                              uint2* blockSum, uint32_t* cnt,
                                                               uint32_t level, uint32_t capItems)
 {
+    chain_wait();
     __shared__ uint32_t sInt[kWideItemsPerBlock], sTri[kWideItemsPerBlock], sSlots[kWideItemsPerBlock];
     const uint32_t n = min(cnt[kWideItems + level], capItems);
     const uint32_t g = threadIdx.x & 7u, gshift = lane_id() & 24u;
@@ -1474,20 +1500,21 @@ AG_D uint32_t plane_word(float lo, float hi, float origin)
 // triangle records and the next level's items. The places of a block's items
 // follow from the sums of the blocks before it, so the layout is breadth
 // first and does not depend on scheduling.
-__global__ void __launch_bounds__(kWideThreads) k_wide_emit(const uint2* __restrict__ items,
-                                                            const BinNode* __restrict__ bnodes,
-                                                            const int32_t* __restrict__ slots,
-                                                            const uint2* __restrict__ itemOff,
-                                                            const uint2* __restrict__ blockSum,
-                                                            const uint32_t* __restrict__ order,
-                                                            const float* __restrict__ verts,
-                                                            const uint32_t* __restrict__ idx, uint32_t ntris,
-                                                            const float4* __restrict__ spheres,
-                                                            WideNode* __restrict__ nodes, TriRecord* __restrict__ tris,
-                                                            uint2* __restrict__ itemsNext, uint32_t* __restrict__ cnt,
+__global__ void __launch_bounds__(kWideThreads) k_wide_emit(const uint2* items,
+                                                            const BinNode* bnodes,
+                                                            const int32_t* slots,
+                                                            const uint2* itemOff,
+                                                            const uint2* blockSum,
+                                                            const uint32_t* order,
+                                                            const float* verts,
+                                                            const uint32_t* idx, uint32_t ntris,
+                                                            const float4* spheres,
+                                                            WideNode* nodes, TriRecord* tris,
+                                                            uint2* itemsNext, uint32_t* cnt,
                                                             uint32_t level, uint32_t nodeCap, uint32_t triCap,
-                                                            uint32_t* __restrict__ status)
+                                                            uint32_t* status)
 {
+    chain_wait();
     __shared__ __align__(16) uint8_t rec[kWideItemsPerBlock][sizeof(WideNode)];
     __shared__ uint32_t sums[2][kWideThreads / 32];
     __shared__ float sahSums[kWideThreads / 32];
@@ -1617,7 +1644,7 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_emit(const uint2* __restr
 
 // End of a device-driven build: a tree that needed more collapse levels than
 // were enqueued, or is deeper than the traversal stack, is reported.
-__global__ void k_end(const uint32_t* __restrict__ cnt, uint32_t n, uint32_t wideLevels, uint32_t* __restrict__ status)
+__global__ void k_end(const uint32_t* cnt, uint32_t n, uint32_t wideLevels, uint32_t* status)
 {
     if (cnt[kCntFailed] != 0u) return;  // reported by k_top
     uint32_t depth = 0, tris = 0;
@@ -1647,6 +1674,23 @@ inline unsigned blocks_for(size_t n, int threads, size_t cap = 0x7fffffff)
 {
     const size_t b = (n + threads - 1) / threads;
     return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
+}
+
+// A launch that may overlap the end of the kernel before it on the stream.
+template <typename... P, typename... A>
+void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 // Capacities of the big-task lists: at most N / (kSmallMax + 1) tasks on a
@@ -1739,11 +1783,11 @@ void Builder::launch_begin(const Input& in, cudaStream_t st)
 {
     const uint32_t n = in.ntris + in.nspheres;
     k_begin<<<4, 1024, 0, st>>>(counters_);
-    k_prep_prims<<<blocks_for(n, kPrepThreads, 148 * 8), kPrepThreads, 0, st>>>(
-        in.verts, in.idx, in.ntris, in.spheres, n, boxes_, refs_[0], counters_ + kCntBounds);
+    launch_chained(k_prep_prims, blocks_for(n, kPrepThreads, 148 * 8), kPrepThreads, 0, st, in.verts, in.idx, in.ntris,
+                   in.spheres, n, boxes_, refs_[0], counters_ + kCntBounds);
     const size_t rootThreads = std::max<size_t>(n > kSmallMax ? (n + kChunk - 1) / kChunk : 1, kTaskBinWords);
-    k_root<<<blocks_for(rootThreads, 256), 256, 0, st>>>(n, counters_, static_cast<BigTask*>(tasks_[0]), bnodes_,
-                                                         static_cast<SmallTask*>(small_), chunkTask_[0], bins_[0]);
+    launch_chained(k_root, blocks_for(rootThreads, 256), 256, 0, st, n, counters_, static_cast<BigTask*>(tasks_[0]),
+                   bnodes_, static_cast<SmallTask*>(small_), chunkTask_[0], bins_[0]);
 }
 
 // Binary levels [first, last) of the big tasks.
@@ -1758,13 +1802,13 @@ void Builder::launch_big_levels(const Input& in, uint32_t first, uint32_t last, 
         // level L has at most 2^L tasks; the kernels loop, so any grid covers them
         const size_t tasks = std::min<size_t>(L < 20 ? size_t(1) << L : capBig, n / (kSmallMax + 1) + 1);
         const unsigned gTasks = blocks_for(tasks, 1, 148 * 8), gChunks = blocks_for(n / kChunk + tasks, 1, 148 * 8);
-        k_bin<<<gChunks, kChunkThreads, 0, st>>>(cur, refs_[a], boxes_, chunkTask_[a], bins_[a], chunkCnt_, counters_, L,
-                                                 capChunks);
-        k_split<<<gTasks, kSplitThreads, 0, st>>>(cur, bins_[a], chunkCnt_, chunkLeft_, splits, bnodes_, next,
-                                                  chunkTask_[b], bins_[b], static_cast<SmallTask*>(small_), counters_, L,
-                                                  capBig, capChunks, n, in.status);
-        k_scatter<<<gChunks, kChunkThreads, 0, st>>>(next, cur, refs_[a], refs_[b], boxes_, chunkTask_[a], splits,
-                                                     chunkLeft_, counters_, L, capChunks, in.status);
+        launch_chained(k_bin, gChunks, kChunkThreads, 0, st, cur, refs_[a], boxes_, chunkTask_[a], bins_[a], chunkCnt_,
+                       counters_, L, capChunks);
+        launch_chained(k_split, gTasks, kSplitThreads, 0, st, cur, bins_[a], chunkCnt_, chunkLeft_, splits, bnodes_,
+                       next, chunkTask_[b], bins_[b], static_cast<SmallTask*>(small_), counters_, L, capBig, capChunks,
+                       n, in.status);
+        launch_chained(k_scatter, gChunks, kChunkThreads, 0, st, next, cur, refs_[a], refs_[b], boxes_, chunkTask_[a],
+                       splits, chunkLeft_, counters_, L, capChunks, in.status);
     }
 }
 
@@ -1774,12 +1818,11 @@ void Builder::launch_subtrees(const Input& in, uint32_t levels, uint32_t maxLeve
     const uint32_t n = in.ntris + in.nspheres;
     const bool sah = collapse_ == kCollapseSah;
     cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SubSmem));
-    k_subtree<<<blocks_for(n, 64, 148 * 2), kSubThreads, sizeof(SubSmem), st>>>(
-        static_cast<const SmallTask*>(small_), refs_[0], refs_[1], boxes_, bnodes_, order_, collapseCost_,
-        collapseChoice_, triCost_, sah, counters_, levels, n);
-    k_top<<<1, kTopThreads, 0, st>>>(bnodes_, collapseCost_, collapseChoice_, triCost_, sah,
-                                     reinterpret_cast<uint2*>(items_[0]), counters_, levels, maxLevels,
-                                     report ? in.status : nullptr);
+    launch_chained(k_subtree, blocks_for(n, 64, 148 * 2), kSubThreads, sizeof(SubSmem), st,
+                   static_cast<const SmallTask*>(small_), refs_[0], refs_[1], boxes_, bnodes_, order_, collapseCost_,
+                   collapseChoice_, triCost_, sah, counters_, levels, n);
+    launch_chained(k_top, 1, kTopThreads, 0, st, bnodes_, collapseCost_, collapseChoice_, triCost_, sah,
+                   reinterpret_cast<uint2*>(items_[0]), counters_, levels, maxLevels, report ? in.status : nullptr);
 }
 
 // Collapse levels [first, last).
@@ -1792,10 +1835,10 @@ void Builder::launch_wide_levels(const Input& in, uint32_t first, uint32_t last,
         // level D has at most 8^D wide nodes
         const size_t items = std::min<size_t>(D < 7 ? size_t(1) << (3 * D) : n + 1, n + 1);
         const unsigned grid = blocks_for(items, (int)kWideItemsPerBlock, 148 * 8);
-        k_wide_decide<<<grid, kWideThreads, 0, st>>>(cur, bnodes_, collapse_ == kCollapseSah ? collapseChoice_ : nullptr,
-                                                     slots_, off, sums, counters_, D, n + 1);
-        k_wide_emit<<<grid, kWideThreads, 0, st>>>(cur, bnodes_, slots_, off, sums, order_, in.verts, in.idx, in.ntris,
-                                                   in.spheres, in.nodes, in.tris, next, counters_, D, n + 1, n, in.status);
+        launch_chained(k_wide_decide, grid, kWideThreads, 0, st, cur, bnodes_,
+                       collapse_ == kCollapseSah ? collapseChoice_ : nullptr, slots_, off, sums, counters_, D, n + 1);
+        launch_chained(k_wide_emit, grid, kWideThreads, 0, st, cur, bnodes_, slots_, off, sums, order_, in.verts, in.idx,
+                       in.ntris, in.spheres, in.nodes, in.tris, next, counters_, D, n + 1, n, in.status);
     }
 }
 
