@@ -1,6 +1,6 @@
 // GPU BVH builder: binned SAH (32 bins) binary build, then a collapse
 // (SAH-optimal by default, or the reference's greedy rule) to the 8-wide
-// quantised layout of bvh.cuh. Replaces the reference's CPU build
+// layout of bvh.cuh. Replaces the reference's CPU build
 // (src/accelerators/bvh_common.cpp:185-391 binned SAH with 9 bins and
 // src/accelerators/wide_bvh.cpp:200-243 collapse + 290-356 flatten).
 #pragma once

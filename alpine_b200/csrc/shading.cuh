@@ -622,8 +622,9 @@ AG_HD int32_t float_bits(float f)
 
 // Out of line in the shading kernels: the descent is a loop that their
 // registers and the code around it slowed down (12.6 of the stall cycles per
-// instruction were instruction fetch). Measured on B200, city of 20,000
-// lights, 1M paths: 5,288 to 4,449 us a render.
+// instruction were instruction fetch, 4.7 now). Measured on B200, city of
+// 20,000 lights, 1M paths: 5,288 to 4,449 us a render, and 4,030 with the
+// records above.
 // The light BVH (bvh_light_sampler.cpp:267-319): stochastic descent by
 // importance with u remapping. Returns the light index or -1.
 static __host__ __device__ __noinline__ int light_descent(const LightSamplerView& ls, float u, float3 hit, float3 ns,

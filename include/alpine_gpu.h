@@ -78,8 +78,8 @@ typedef struct alpine_gpu_bvh_stats {
     float build_ms;      /* device time of the last build */
     uint32_t spheres;    /* analytic spheres in the BVH */
     uint32_t child_slots; /* filled child slots over all wide nodes (of 8 each) */
-    uint32_t big_levels;  /* leading binary levels with a node of more than 512 primitives (split by the
-                             block-wide kernels; the rest are split one warp per node) */
+    uint32_t big_levels;  /* leading binary levels with a node of more than 512 primitives (split level
+                             by level; one block finishes each of the others) */
 } alpine_gpu_bvh_stats;
 
 /* Creates a context on cfg->device (replaces alpine::initialize,
@@ -176,7 +176,7 @@ ALPINE_GPU_API int alpine_gpu_build(alpine_gpu_ctx* ctx, alpine_gpu_bvh_stats* s
  *   of the last alpine_gpu_build_async from device memory (build_ms: its
  *   device time; triangles, spheres and big_levels: those of the last
  *   alpine_gpu_build); graph_captures / graph_launches (either may be NULL)
- *   count the captures and replays of its graph. The block-wide kernels for
+ *   count the captures and replays of its graph. The kernels that split
  *   nodes of more than 512 primitives run on the first big_levels + 2 levels
  *   only; a larger node met below them is reported like a level cap. */
 ALPINE_GPU_API int alpine_gpu_build_async(alpine_gpu_ctx* ctx, uint32_t max_binary_levels, uint32_t max_wide_levels);
