@@ -1,7 +1,7 @@
 """GPU builds at the sizes where the builder changes kernels: leaves (1 to 3
-primitives), nodes split one thread per reference (up to 32), by one warp
-(up to 512) and by blocks of 1,024 references, each side of the limit, and
-nodes whose centroids coincide (split by position). Both drivers; hits against
+primitives), nodes whose references each try their own plane (up to 32), nodes
+binned in one block (up to 512) and by blocks of 1,024 references, each side of
+the limit, and nodes whose centroids coincide (split by position). Both drivers; hits against
 the brute-force oracle, bit for bit but for exact ties."""
 import numpy as np
 import pytest
