@@ -218,3 +218,62 @@ def test_training_learns_a_target_distribution(ctx):
     assert loss < first - 1.0
     assert np.median(p_mode) > 10 / (4 * math.pi)
     assert np.median(p_anti) < 1 / (4 * math.pi)
+
+
+def _samples(n, seed):
+    rng = np.random.default_rng(seed)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    return np.concatenate([_queries(n, seed), d, rng.uniform(0.2, 3.0, (n, 1))], axis=1).astype(np.float32)
+
+
+def test_gradients_finish_before_they_return(ctx):
+    """Nothing of guide_gradients is left running on the GPU when it returns:
+    its gradient buffers (67 MB of grid, at least 8.4 us to clear at the HBM's
+    nominal 8 TB/s) are clean by then. Waiting for the device right after the
+    call takes no longer than waiting for it 200 us later."""
+    import time
+
+    import torch
+
+    s = _samples(256, 41)
+    dW = np.empty(G.WEIGHT_COUNT, np.float32)
+    args = (ctx.h, gpu._ptr(s), len(s), gpu._ptr(dW), None, 0, None, None)
+
+    def wait_us(later):  # median wait for the device, `later` seconds after the call
+        t = []
+        for _ in range(200):
+            assert ctx.L.alpine_gpu_guide_gradients(*args) == 0
+            a = time.perf_counter()
+            while time.perf_counter() < a + later:
+                pass
+            a = time.perf_counter()
+            torch.cuda.synchronize()
+            t.append(1e6 * (time.perf_counter() - a))
+        return float(np.median(t))
+
+    wait_us(0.0)
+    busy, idle = wait_us(0.0), wait_us(2e-4)
+    print(f"wait after guide_gradients {busy:.1f} us, idle {idle:.1f} us")
+    assert busy - idle < 4.0
+
+
+def test_gradients_do_not_see_the_call_before(ctx):
+    """The second of two calls with other samples answers as the first call of
+    a new context: weights bit for bit, the grid's to the rounding of its float
+    atomics (at most a few hundred terms an entry, 2^-24 each)."""
+    res = G.resolutions()
+    a, b = _samples(4096, 42), _samples(3000, 43)
+    idx = G.grid_flat_indices(np.concatenate([a[:64, :12], b[:64, :12]]), LO, HI, res)
+    _randomise(ctx, np.concatenate([a, b])[:, :12], 44)
+    ctx.guide_gradients(a, idx)
+    dw, dg = ctx.guide_gradients(b, idx)
+    fresh = gpu.Context(0)
+    try:
+        fresh.guide_reset(7, LO, HI)
+        _randomise(fresh, np.concatenate([a, b])[:, :12], 44)
+        fw, fg = fresh.guide_gradients(b, idx)
+    finally:
+        fresh.close()
+    assert dw.tobytes() == fw.tobytes()
+    assert np.linalg.norm(dg - fg) <= 1e-4 * np.linalg.norm(fg) and np.linalg.norm(fg) > 0
