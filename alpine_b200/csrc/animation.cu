@@ -26,24 +26,36 @@ struct Piece {
 };
 constexpr int kMorphThreads = 256;
 
+// The pieces of one launch and their weights, passed as the kernel's argument:
+// the driver takes a copy at the launch, so that calls may be enqueued ahead
+// without waiting on the host. (A copy from pageable memory may wait for the
+// stream: ten updates of 1,000 meshes behind 200 ms of work did.) 64 meshes with
+// normals and up to 8 targets each fit; more take further launches.
+constexpr uint32_t kMorphPieces = 128, kMorphWeights = 512;
+struct MorphBatch {
+    uint32_t pieces, weights, blocks;
+    Piece piece[kMorphPieces];
+    float weight[kMorphWeights];
+};
+static_assert(kMorphWeights >= kMaxTargets, "any mesh fits a batch of its own");
+
 // out[i] = base[i] + sum_j deltas[j][i] * w_j over the floats of every piece.
-// One launch for all meshes of a scene: at 3 us a launch the 35 meshes of an
+// One launch for the meshes of a scene: at 3 us a launch the 35 meshes of an
 // 8k-triangle scene took longer than the largest part of their BVH's rebuild.
-__global__ void __launch_bounds__(kMorphThreads) k_morph(const Piece* __restrict__ pieces, uint32_t count,
-                                                         const float* __restrict__ weights)
+__global__ void __launch_bounds__(kMorphThreads) k_morph(const __grid_constant__ MorphBatch batch)
 {
-    uint32_t lo = 0, hi = count;  // the last piece that starts at or before this block
+    uint32_t lo = 0, hi = batch.pieces;  // the last piece that starts at or before this block
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) / 2;
-        if (pieces[mid].firstBlock <= blockIdx.x) lo = mid;
+        if (batch.piece[mid].firstBlock <= blockIdx.x) lo = mid;
         else hi = mid;
     }
-    const Piece p = pieces[lo];
+    const Piece& p = batch.piece[lo];
     const uint32_t i = (blockIdx.x - p.firstBlock) * kMorphThreads + threadIdx.x;
     if (i >= p.n) return;
     float v = p.base[i];
     for (uint32_t j = 0; j < p.targets; ++j)
-        v = __fadd_rn(v, __fmul_rn(p.deltas[(uint64_t)j * p.n + i], weights[p.firstWeight + j]));
+        v = __fadd_rn(v, __fmul_rn(p.deltas[(uint64_t)j * p.n + i], batch.weight[p.firstWeight + j]));
     p.out[i] = v;
 }
 
@@ -77,39 +89,38 @@ void channel_weights(const alpine_gpu_ctx::Channel& ch, uint32_t targets, float 
         out[j] = lerp_c20(ch.weights[(size_t)index * targets + j], ch.weights[(size_t)(index + 1) * targets + j], t);
 }
 
-// Morphs the marked meshes with their current weights, in one launch.
+// Morphs the marked meshes with their current weights, as many to a launch as
+// fit its argument.
 int morph_shapes(alpine_gpu_ctx* c, const std::vector<char>& marked)
 {
-    std::vector<Piece> pieces;
-    std::vector<float> weights;
-    uint32_t blocks = 0;
+    MorphBatch batch;
+    batch.pieces = batch.weights = batch.blocks = 0;
+    cudaError_t e = cudaSuccess;
+    auto flush = [&]() {
+        if (batch.blocks && e == cudaSuccess) {
+            k_morph<<<batch.blocks, kMorphThreads, 0, c->stream>>>(batch);
+            e = cudaGetLastError();
+        }
+        batch.pieces = batch.weights = batch.blocks = 0;
+    };
     for (size_t k = 0; k < c->morphs.size(); ++k) {
         if (!marked[k]) continue;
         const alpine_gpu_ctx::Morph& m = *c->morphs[k];
         const uint32_t n = 3 * c->shapeVertCount[m.shape];
         if (n == 0) continue;
+        if (batch.pieces + 2 > kMorphPieces || batch.weights + m.targets > kMorphWeights) flush();
         const size_t off = 3ull * c->shapeVertBase[m.shape];
         auto add = [&](const ag::DeviceBuffer& base, const ag::DeviceBuffer& deltas, float* out) {
-            pieces.push_back({base.as<float>(), deltas.as<float>(), out + off, n, m.targets, (uint32_t)weights.size(), blocks});
-            blocks += (n + kMorphThreads - 1) / kMorphThreads;
+            batch.piece[batch.pieces++] = {base.as<float>(), deltas.as<float>(), out + off, n, m.targets, batch.weights,
+                                           batch.blocks};
+            batch.blocks += (n + kMorphThreads - 1) / kMorphThreads;
         };
         add(m.dBase, m.dDeltas, c->dVerts.as<float>());
         if (m.normals) add(m.dBaseN, m.dDeltasN, c->dNormals.as<float>());
-        weights.insert(weights.end(), m.weights.begin(), m.weights.begin() + m.targets);
+        std::copy(m.weights.begin(), m.weights.begin() + m.targets, batch.weight + batch.weights);
+        batch.weights += m.targets;
     }
-    if (blocks == 0) return ALPINE_GPU_OK;
-    // pieces and weights in one copy; the host memory is free again when the call returns
-    const size_t pb = pieces.size() * sizeof(Piece), wb = weights.size() * sizeof(float);
-    std::vector<char> host(pb + wb);
-    std::memcpy(host.data(), pieces.data(), pb);
-    std::memcpy(host.data() + pb, weights.data(), wb);
-    if (!c->dMorphWork.reserve(host.size())) return c->fail(ALPINE_GPU_ERR_OUT_OF_MEMORY, "morph: cudaMalloc failed");
-    cudaError_t e = cudaMemcpyAsync(c->dMorphWork.ptr, host.data(), host.size(), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) {
-        k_morph<<<blocks, kMorphThreads, 0, c->stream>>>(c->dMorphWork.as<Piece>(), (uint32_t)pieces.size(),
-                                                         reinterpret_cast<const float*>(c->dMorphWork.as<char>() + pb));
-        e = cudaGetLastError();
-    }
+    flush();
     return e == cudaSuccess ? ALPINE_GPU_OK : c->fail(ALPINE_GPU_ERR_CUDA, std::string("morph: ") + cudaGetErrorString(e));
 }
 

@@ -192,7 +192,6 @@ struct alpine_gpu_ctx {
     };
     std::vector<std::unique_ptr<Morph>> morphs;
     std::vector<Channel> channels;
-    ag::DeviceBuffer dMorphWork;          // the meshes and weights of the last morph launch
     bool hostVertsStale = false, hostNormalsStale = false;
 
     // learned path guiding

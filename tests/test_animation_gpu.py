@@ -166,3 +166,54 @@ def test_many_meshes_morph_in_one_launch():
                     assert gn.tobytes() == en.tobytes()
     finally:
         ctx.close()
+
+
+def test_async_update_of_many_meshes_does_not_wait():
+    """1,000 meshes with normals (2,000 arrays to morph, more than one launch's
+    argument holds): ten calls of update_scene_async return while the stream is
+    still busy with what was enqueued before them, and the vertices are those of
+    the last one, bit for bit."""
+    import time
+
+    import torch
+
+    rng = np.random.default_rng(6)
+    ctx = gpu.Context(0)
+    try:
+        last = None
+        for _ in range(1000):
+            v = rng.normal(size=(3, 3)).astype(np.float32)
+            sid = ctx.add_mesh(v, np.arange(3, dtype=np.uint32).reshape(1, 3))
+            nrm = rng.normal(size=(3, 3)).astype(np.float32)
+            ctx.set_triangle_attributes(sid, nrm, np.zeros(1, np.uint32))
+            d = rng.normal(size=(2, 3, 3)).astype(np.float32)
+            ctx.set_morph_targets(sid, d, d)
+            w = rng.normal(size=(2, 2)).astype(np.float32)
+            ctx.add_animation_channel(sid, [0.0, 1.0], w)
+            last = (sid, v + d[0] * w[1, 0] + d[1] * w[1, 1], nrm + d[0] * w[1, 0] + d[1] * w[1, 1])
+        ctx.update_scene(1.0)
+        ctx.update_scene_async(0.5)  # captures the rebuild's graph
+        ctx.synchronize()
+        rays = torch.zeros(1 << 22, 8, device="cuda")
+        rays[:, 4:7] = torch.randn(1 << 22, 3, device="cuda")
+        rays[:, 7] = 3.4e38
+        out = torch.empty(1 << 22, 4, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        ctx.trace_device(rays.data_ptr(), 1 << 22, out.data_ptr())
+        ctx.synchronize()
+        t = [time.perf_counter()]
+        for _ in range(10):  # about 200 ms on the context's stream
+            ctx.trace_device(rays.data_ptr(), 1 << 22, out.data_ptr())
+        t.append(time.perf_counter())
+        for k in range(1, 11):
+            ctx.update_scene_async(k / 10)
+        t.append(time.perf_counter())
+        ctx.synchronize()
+        t.append(time.perf_counter())
+        enqueue, update, wait = np.diff(t) * 1e3
+        print(f"enqueue {enqueue:.2f} ms, ten updates {update:.2f} ms, wait {wait:.2f} ms")
+        assert update < wait
+        gv, gn = ctx.get_vertices(last[0], 3)
+        assert gv.tobytes() == last[1].tobytes() and gn.tobytes() == last[2].tobytes()
+    finally:
+        ctx.close()
