@@ -1489,18 +1489,21 @@ __global__ void __launch_bounds__(kWideThreads, 8) k_wide_decide(const uint2* it
 }
 
 // A plane word of bvh.cuh: the box [lo, hi] of one axis as offsets from the
-// node's origin, rounded outwards to the top 16 bits of a float.
+// node's origin, rounded outwards to the top 16 bits of a float. A maximum that
+// no finite word reaches (infinite, NaN, or next to FLT_MAX) gets the top half
+// of +inf: with a lower half of 0 the word is +inf, with any other a NaN, which
+// the traversal's minimum and maximum over the axes pass over.
+constexpr uint32_t kNoBound = 0x7f800000u;
 AG_D uint32_t plane_word(float lo, float hi, float origin)
 {
     float dl = __fsub_rd(lo, origin), dh = __fsub_ru(hi, origin);
     dl = dl >= 0.0f ? dl : 0.0f;                      // (NaN: the origin)
-    constexpr float kNoBound = 1.7014118346046923e38f;  // 2^127: finite with any lower half
-    dh = dh <= kNoBound ? fmaxf(dh, 0.0f) : kNoBound;   // (infinite or NaN: no bound)
+    dh = dh <= 0.0f ? 0.0f : dh;
     const uint32_t l16 = __float_as_uint(dl) >> 16;   // truncated: rounded down
     const uint32_t hb = __float_as_uint(dh);
     uint32_t h16 = hb >> 16;                          // read with the lower half below it
     if (((h16 << 16) | l16) < hb) ++h16;
-    return (h16 << 16) | l16;
+    return min(h16 << 16, kNoBound) | l16;
 }
 
 // Writes one wide node per group of eight lanes, a lane per slot, with its
@@ -1589,9 +1592,16 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_emit(const uint2* items,
         uint32_t* u = reinterpret_cast<uint32_t*>(r);
         // an empty slot's box is inside out: minimum 1e30, maximum -1e30
         constexpr uint32_t kEmptyPlanes = 0xf1497149u;
-        u[8 + g] = e >= 0 ? plane_word(c.lo.x, c.hi.x, p[0]) : kEmptyPlanes;
-        u[16 + g] = e >= 0 ? plane_word(c.lo.y, c.hi.y, p[1]) : kEmptyPlanes;
-        u[24 + g] = e >= 0 ? plane_word(c.lo.z, c.hi.z, p[2]) : kEmptyPlanes;
+        uint32_t planes[3] = {kEmptyPlanes, kEmptyPlanes, kEmptyPlanes};
+        if (e >= 0) {
+            planes[0] = plane_word(c.lo.x, c.hi.x, p[0]);
+            planes[1] = plane_word(c.lo.y, c.hi.y, p[1]);
+            planes[2] = plane_word(c.lo.z, c.hi.z, p[2]);
+            // unbounded on every axis: one must not be a NaN
+            if (min(planes[0], min(planes[1], planes[2])) >= kNoBound) planes[0] = kNoBound;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) u[8 * (k + 1) + g] = planes[k];
         if (g == 0) {
             float* f = reinterpret_cast<float*>(r);
             f[0] = p[0];

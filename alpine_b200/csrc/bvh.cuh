@@ -14,6 +14,13 @@
 //                                    maximum in the upper. The maximum is read as
 //                                    the whole word, so the lower half is part of
 //                                    its value; it is rounded up with that counted.
+//                                    A maximum too large for that is +inf or a NaN
+//                                    (not on every axis): no bound.
+// The planes never lie inside a child's box. The traversal takes |d| for at
+// least 1e-20 on every axis (with the byte planes before it did too), so a hit
+// is missed where a plane's distance overflows (a node's minimum is -inf, or
+// further than FLT_MAX * |d| from the ray's origin), or where it lies further
+// along an axis-parallel ray than 1e20 times the box's extent beside it.
 // A word becomes the near or the far plane by one integer multiplication (by
 // 65536 or 1, chosen per ray and axis by the direction's sign). The 80-byte
 // node before it held the planes as bytes of a per-axis quantum, which took

@@ -301,3 +301,34 @@ def test_child_box_planes(ctx, kind):
     tris = oracle.make_tris(verts, idx)
     compare_closest(rays, tris, ctx.trace(rays), *oracle.closest_brute(rays, tris)[:4])
     assert (ctx.occluded(rays) == oracle.any_brute(rays, tris)).all()
+
+
+@pytest.mark.parametrize("lo,hi", [(-1.0e38, 0.5e38), (-1.6e38, 1.3e38), (0.0, 3.3e38), (-1.7e38, 1.7e38)])
+def test_child_box_planes_of_the_largest_boxes(ctx, lo, hi):
+    """Two leaves as far apart on x as floats go (the last extent passes the
+    largest finite plane): rays along x meet the small triangle of each. Its two
+    neighbours, lines that no ray meets, widen its box to 6e18: along an axis
+    that a ray does not move on, the traversal takes |d| for 1e-20, so a box
+    ends 1e20 times its distance away, and 3e18 is the most that keeps the
+    product finite."""
+    s, tri = np.float32(3e18), [[0.2, 0.1], [0.9, 0.3], [0.4, 0.8]]
+    v = np.empty((6, 3, 3), np.float32)
+    for k, x in enumerate((lo, hi)):
+        v[3 * k:3 * k + 3, :, 0] = np.float32(x)
+        v[3 * k, :, 1:] = tri
+        v[3 * k + 1:3 * k + 3, 0, 1:], v[3 * k + 1:3 * k + 3, 1:, 1:] = -s, s
+    verts, idx = v.reshape(-1, 3), np.arange(18, dtype=np.uint32).reshape(-1, 3)
+    st = _load(ctx, verts, idx)
+    assert st["binary_nodes"] == 3 and st["wide_nodes"] == 1
+    tris = oracle.make_tris(verts, idx)
+    rng = np.random.default_rng(94)
+    rays = np.zeros((2000, 8), np.float32)
+    rays[:, 1:3] = rng.random((2000, 2))
+    rays[:, 7] = FLT_MAX
+    rays[::2, 0], rays[::2, 4] = np.float32(0.75 * lo + 0.25 * hi), 1.0
+    rays[1::2, 0], rays[1::2, 4] = np.float32(0.25 * lo + 0.75 * hi), -1.0
+    ref = oracle.closest_brute(rays, tris)
+    hit = ref[0] != MISS
+    assert hit[::2].sum() > 100 and hit[1::2].sum() > 100
+    compare_closest(rays, tris, ctx.trace(rays), *ref[:4])
+    assert (ctx.occluded(rays) == oracle.any_brute(rays, tris)).all()
