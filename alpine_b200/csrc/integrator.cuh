@@ -449,11 +449,13 @@ __global__ void __launch_bounds__(kThreads) k_guide_query(SceneView sc, WaveView
     if (guided) w.guideQuery[slot] = gq;
     if (q < n) w.guideSlot[q] = guided ? (int)slot : -1;
     if (!sk.keys) return;
+    uint32_t key = kShadeBins;
     if (q < n) {
-        const uint32_t key = shade_key(sk, h.x, guided && w.guideLobes);
+        key = shade_key(sk, h.x, guided && w.guideLobes);
         sk.keys[q] = (uint8_t)key;
-        bin_rank(hist, key);
     }
+    __syncwarp();
+    bin_rank(hist, key);
     __syncthreads();
     if (threadIdx.x < kShadeBins && hist[threadIdx.x]) atomicAdd(sk.counts + threadIdx.x, hist[threadIdx.x]);
 }
@@ -647,11 +649,10 @@ __global__ void __launch_bounds__(kThreads) k_shade_scatter(WaveView w, uint32_t
     __syncthreads();
     const uint32_t n = *w.queueCount;
     const uint32_t q = blockIdx.x * kThreads + threadIdx.x;
-    uint32_t key = 0, rank = 0;
-    if (q < n) {
-        key = keys[q];
-        rank = bin_rank(hist, key);
-    }
+    uint32_t key = kShadeBins;
+    if (q < n) key = keys[q];
+    __syncwarp();
+    const uint32_t rank = bin_rank(hist, key);
     __syncthreads();
     if (threadIdx.x < kShadeBins && hist[threadIdx.x]) {
         uint32_t start = 0;

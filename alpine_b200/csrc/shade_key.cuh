@@ -36,17 +36,16 @@ AG_D uint32_t shade_key(const ShadeKeys& s, uint32_t prim, bool guided)
     return guided ? key | kShadeGuided : key;
 }
 
-// Warp-aggregated rank of this thread among the block's threads with the
-// same key, added to hist[key] (shared memory). Called by the active threads
-// of a warp together.
+// Warp-aggregated rank of this lane's entry among the block's entries with the
+// same key, added to hist[key] (shared memory). The whole warp calls it
+// together; a lane without an entry passes kShadeBins, which is not counted.
 AG_D uint32_t bin_rank(uint32_t* hist, uint32_t key)
 {
-    const uint32_t am = __activemask();
-    const uint32_t peers = __match_any_sync(am, key);
+    const uint32_t peers = __match_any_sync(0xffffffffu, key);
     const int leader = __ffs(peers) - 1;
     uint32_t base = 0;
-    if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(hist + key, __popc(peers));
-    base = __shfl_sync(am, base, leader);
+    if ((int)(threadIdx.x & 31) == leader && key < kShadeBins) base = atomicAdd(hist + key, __popc(peers));
+    base = __shfl_sync(0xffffffffu, base, leader);
     return base + __popc(peers & lanemask_lt());
 }
 

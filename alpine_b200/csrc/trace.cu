@@ -94,20 +94,24 @@ __global__ void __launch_bounds__(kBlock, kTraceThreads / kBlock)
     uint32_t err = 0, nv = 0, tv = 0;
     for (uint32_t base = blockIdx.x * kBlock + (threadIdx.x & ~31u); base < n;) {
         const uint32_t i = base + lane_id();
+        TraceResult r;
         if (i < n) {
             const float4 a = rays[2ull * i], b = rays[2ull * i + 1];
-            TraceResult r;
             const bool hit = trace<kAny, kBinary>(bvh, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), a.w, b.w, r,
                                                   stack + threadIdx.x, kBlock, err, nv, tv);
             if (kAny) static_cast<uint8_t*>(out)[i] = hit ? 1 : 0;
             else static_cast<uint4*>(out)[i] = make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.b1), __float_as_uint(r.b2));
-            if (!kAny && sk.keys) {
-                const uint32_t key = shade_key(sk, r.prim, false);
-                sk.keys[i] = (uint8_t)key;
-                bin_rank(hist, key);
-            }
         }
-        __syncwarp();
+        __syncwarp();  // the lanes' traversals have ended: the warp counts its keys together
+        if (!kAny && sk.keys) {
+            uint32_t key = kShadeBins;
+            if (i < n) {
+                key = shade_key(sk, r.prim, false);
+                sk.keys[i] = (uint8_t)key;
+            }
+            __syncwarp();
+            bin_rank(hist, key);
+        }
         uint32_t taken = 0;
         if (lane_id() == 0) taken = atomicAdd(ticket, 32u);
         base = first + __shfl_sync(0xffffffffu, taken, 0);

@@ -53,3 +53,17 @@ def test_shade_order_guided_identical():
                     guide_train=False, guide_spp_per_wave=8)
             for order in (gpu.SHADE_ORDER_QUEUE, gpu.SHADE_ORDER_BY_MATERIAL)]
     assert imgs[0].tobytes() == imgs[1].tobytes()
+
+
+@pytest.mark.parametrize("guide", [False, True])
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (5, 1, 3), (31, 1, 1), (33, 31, 3)])
+def test_shade_order_of_queues_that_end_within_a_warp(w, h, spp, guide):
+    """Queues whose last warp has idle lanes, down to one path, and shorter from
+    bounce to bounce by roulette: every entry gets its place in the order (an
+    image differs where one is lost or shaded twice), and the image is the same
+    on a second render."""
+    scene = scenes.room_scene(seed=5)
+    imgs = [_render(scene, w, h, 6, gpu.SAMPLER_POWER, order, spp, sampler=gpu.RNG_COUNTER, seed=9, guide=guide,
+                    guide_train=False, russian_roulette_depth=1)
+            for order in (gpu.SHADE_ORDER_QUEUE, gpu.SHADE_ORDER_BY_MATERIAL, gpu.SHADE_ORDER_BY_MATERIAL)]
+    assert imgs[0].tobytes() == imgs[1].tobytes() == imgs[2].tobytes()
