@@ -507,8 +507,11 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* tasks, c
     chain_wait();
     __shared__ SplitChoice axisBest[3];
     __shared__ BigSplit split;
-    __shared__ uint32_t childChunk0[2], childChunks[2], warpSums[kSplitThreads / 32];
-    const uint32_t nb = cnt[kCntFailed] & kFailCapacity ? 0u : min(cnt[kLevelBig + level], capBig);
+    __shared__ uint32_t childChunk0[2], childChunks[2], warpSums[kSplitThreads / 32], failed;
+    // (read by one thread: another block may set the flag, and the threads of a block stay together)
+    if (threadIdx.x == 0) failed = cnt[kCntFailed] & kFailCapacity;
+    __syncthreads();
+    const uint32_t nb = failed ? 0u : min(cnt[kLevelBig + level], capBig);
     const uint32_t warp = threadIdx.x >> 5;
     for (uint32_t bi = blockIdx.x; bi < nb; bi += gridDim.x) {
         const BigTask task = tasks[bi];
@@ -1029,9 +1032,10 @@ __global__ void __launch_bounds__(kSubThreads, 2) k_subtree(const SmallTask* sma
         if (blockIdx.x == 0 && tid == 0) atomicOr(cnt + kCntFailed, kFailLevels);
         return;
     }
-    const uint32_t numSmall = cnt[kCntFailed] & kFailCapacity ? 0u : min(cnt[kCntSmall], capPrims);
+    const uint32_t numSmall = min(cnt[kCntSmall], capPrims);
     for (;;) {
-        if (tid == 0) s.ticket = atomicAdd(cnt + kCntTicket, 1u);
+        // (one thread reads the flag, which another block may set: the threads of a block stay together)
+        if (tid == 0) s.ticket = cnt[kCntFailed] & kFailCapacity ? kNoTask : atomicAdd(cnt + kCntTicket, 1u);
         __syncthreads();
         const uint32_t ticket = s.ticket;
         if (ticket >= numSmall) break;
