@@ -148,7 +148,7 @@ struct alpine_gpu_ctx {
     // lights and the light sampler
     std::vector<ag::Light> lights;
     bool lightsDirty = true;
-    ag::DeviceBuffer dLights, dAlias, dLightNodes, dLightPairs;
+    ag::DeviceBuffer dLights, dAlias, dLightNodes;
     ag::DeviceBuffer dLightRecords[2];  // [0] integrator_fast's, [1] integrator_exact's
     uint32_t samplerKind = ag::kSamplerNone;
     uint32_t samplerLightCount = 0;

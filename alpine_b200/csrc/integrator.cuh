@@ -131,7 +131,7 @@ struct IntegratorKernels {
     // caller); shadeOrderBuf: the queue entries grouped by bin
     void (*sort)(const WaveView&, uint32_t maxQueue, cudaStream_t);
     // the light BVH's records for this integrator's descent
-    void (*light_records)(const LightPair* pairs, uint32_t count, LightRecord* out, cudaStream_t);
+    void (*light_records)(const LightNode* nodes, uint32_t count, LightRecord* out, cudaStream_t);
 };
 
 const IntegratorKernels& integrator_fast();
@@ -239,11 +239,13 @@ AG_D bool sample_material(const Material& m, float3 wo, float u0, float u1, Bsdf
 }
 #endif
 
-__global__ void __launch_bounds__(kThreads) k_light_records(const LightPair* __restrict__ pairs, uint32_t count,
+__global__ void __launch_bounds__(kThreads) k_light_records(const LightNode* __restrict__ nodes, uint32_t count,
                                                             LightRecord* __restrict__ out)
 {
     const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < count) out[i] = light_record(pairs[i]);
+    if (i >= count) return;
+    const int32_t left = nodes[i].left, right = nodes[i].right;
+    if (left >= 0 && right >= 0) out[i] = light_record(nodes, left, right);
 }
 
 __global__ void __launch_bounds__(kThreads) k_generate(SceneView sc, WaveView w, bool streamRng)
@@ -807,9 +809,9 @@ void sort(const WaveView& w, uint32_t maxQueue, cudaStream_t st)
 {
     if (maxQueue) k_shade_scatter<<<grid(maxQueue), kThreads, 0, st>>>(w, w.shadeBins, w.shadeKeys, w.shadeOrderBuf);
 }
-void light_records(const LightPair* pairs, uint32_t count, LightRecord* out, cudaStream_t st)
+void light_records(const LightNode* nodes, uint32_t count, LightRecord* out, cudaStream_t st)
 {
-    if (count) k_light_records<<<grid(count), kThreads, 0, st>>>(pairs, count, out);
+    if (count) k_light_records<<<grid(count), kThreads, 0, st>>>(nodes, count, out);
 }
 
 }  // namespace AG_INTEGRATOR_NS

@@ -682,34 +682,14 @@ int alpine_gpu_build_light_sampler(alpine_gpu_ctx* c, int type)
         std::vector<ag::LightNode> nodes;
         nodes.reserve(2 * all.size());
         create_light_node(c->lights, all, nodes);
-        // the descent's packed records: both children of every interior node
-        std::vector<ag::LightPair> pairs(nodes.size());
-        auto ref = [&](int32_t i) {
-            const ag::LightNode& n = nodes[i];
-            const int32_t r = (n.left >= 0 && n.right >= 0) ? i : -(n.light + 1);
-            float f;
-            std::memcpy(&f, &r, sizeof f);
-            return f;
-        };
-        for (size_t i = 0; i < nodes.size(); ++i) {
-            const ag::LightNode& n = nodes[i];
-            if (n.left < 0 || n.right < 0) continue;
-            const ag::LightNode& a = nodes[n.left];
-            const ag::LightNode& b = nodes[n.right];
-            pairs[i].lo0 = make_float4(a.bmin.x, a.bmin.y, a.bmin.z, a.power);
-            pairs[i].hi0 = make_float4(a.bmax.x, a.bmax.y, a.bmax.z, ref(n.left));
-            pairs[i].lo1 = make_float4(b.bmin.x, b.bmin.y, b.bmin.z, b.power);
-            pairs[i].hi1 = make_float4(b.bmax.x, b.bmax.y, b.bmax.z, ref(n.right));
-        }
-        const size_t rb = pairs.size() * sizeof(ag::LightRecord);
-        if (!upload(c->dLightNodes, nodes, c->stream) || !upload(c->dLightPairs, pairs, c->stream) ||
-            !c->dLightRecords[0].reserve(rb) || !c->dLightRecords[1].reserve(rb))
+        const uint32_t count = (uint32_t)nodes.size();
+        if (!upload(c->dLightNodes, nodes, c->stream) || !c->dLightRecords[0].reserve(count * sizeof(ag::LightRecord)) ||
+            !c->dLightRecords[1].reserve(count * sizeof(ag::LightRecord)))
             return c->fail(ALPINE_GPU_ERR_CUDA, "light BVH upload failed");
-        const uint32_t count = (uint32_t)pairs.size();
-        ag::integrator_fast().light_records(c->dLightPairs.as<ag::LightPair>(), count,
-                                            c->dLightRecords[0].as<ag::LightRecord>(), c->stream);
-        ag::integrator_exact().light_records(c->dLightPairs.as<ag::LightPair>(), count,
-                                             c->dLightRecords[1].as<ag::LightRecord>(), c->stream);
+        const ag::LightNode* dNodes = c->dLightNodes.as<ag::LightNode>();
+        ag::integrator_fast().light_records(dNodes, count, c->dLightRecords[0].as<ag::LightRecord>(), c->stream);
+        ag::integrator_exact().light_records(dNodes, count, c->dLightRecords[1].as<ag::LightRecord>(), c->stream);
+        if (cudaGetLastError() != cudaSuccess) return c->fail(ALPINE_GPU_ERR_CUDA, "light BVH records: launch failed");
         c->lightNodeCount = (uint32_t)nodes.size();
     }
     if (cudaStreamSynchronize(c->stream) != cudaSuccess)

@@ -568,19 +568,11 @@ AG_HD float light_importance(float3 c, float br, float power, float3 p, float3 n
 AG_HD float3 light_centre(float3 bmin, float3 bmax) { return 0.5f * (bmin + bmax); }
 AG_HD float light_half_diagonal(float3 bmin, float3 bmax) { return 0.5f * len3(bmax - bmin); }
 
-// The light BVH as it is uploaded: per interior node, both children's bounds
-// and power. ref: the child's interior node index, or -(light + 1) for a leaf.
-struct LightPair {
-    float4 lo0;  // child 0: bmin.xyz, power
-    float4 hi0;  // child 0: bmax.xyz, ref (int bits)
-    float4 lo1;  // child 1
-    float4 hi1;
-};
-static_assert(sizeof(LightPair) == 64, "LightPair layout");
-
-// The same as the sampler descends it, three aligned loads per level: what
-// the importance takes from a child's bounds is computed once per sampler
-// build (by the integrator's own arithmetic, see light_records there).
+// An interior node of the light BVH as the sampler descends it, three aligned
+// loads per level: both children's power, and what the importance takes from
+// their bounds, computed once per sampler build (by the integrator's own
+// arithmetic, see light_records there). A child's ref is its node index, or
+// -(light + 1) for a leaf.
 struct LightRecord {
     float4 c0;  // child 0: centre, power
     float4 c1;  // child 1
@@ -588,15 +580,16 @@ struct LightRecord {
 };
 static_assert(sizeof(LightRecord) == 48, "LightRecord layout");
 
-AG_HD LightRecord light_record(const LightPair& p)
+AG_D LightRecord light_record(const LightNode* nodes, int32_t left, int32_t right)
 {
-    const float3 lo0 = mk3(p.lo0.x, p.lo0.y, p.lo0.z), hi0 = mk3(p.hi0.x, p.hi0.y, p.hi0.z);
-    const float3 lo1 = mk3(p.lo1.x, p.lo1.y, p.lo1.z), hi1 = mk3(p.hi1.x, p.hi1.y, p.hi1.z);
-    const float3 a = light_centre(lo0, hi0), b = light_centre(lo1, hi1);
+    const LightNode a = nodes[left], b = nodes[right];
+    const float3 ca = light_centre(a.bmin, a.bmax), cb = light_centre(b.bmin, b.bmax);
     LightRecord r;
-    r.c0 = make_float4(a.x, a.y, a.z, p.lo0.w);
-    r.c1 = make_float4(b.x, b.y, b.z, p.lo1.w);
-    r.m = make_float4(light_half_diagonal(lo0, hi0), light_half_diagonal(lo1, hi1), p.hi0.w, p.hi1.w);
+    r.c0 = make_float4(ca.x, ca.y, ca.z, a.power);
+    r.c1 = make_float4(cb.x, cb.y, cb.z, b.power);
+    r.m = make_float4(light_half_diagonal(a.bmin, a.bmax), light_half_diagonal(b.bmin, b.bmax),
+                      __int_as_float(a.left >= 0 && a.right >= 0 ? left : -(a.light + 1)),
+                      __int_as_float(b.left >= 0 && b.right >= 0 ? right : -(b.light + 1)));
     return r;
 }
 

@@ -295,3 +295,27 @@ def test_textured_scene_counter_mode_unbiased_vs_reference():
     plain = ctx.read_accumulation(w, h)[0][..., :3] / 64
     ctx.close()
     assert abs(plain.mean() - gmean.mean()) > 0.1 * gmean.mean()
+
+
+def test_light_bvh_sampler_holds_nodes_and_records_only():
+    """A light-BVH sampler of 100,000 lights keeps its nodes (40 bytes) and one
+    record (48 bytes) a node for each random-number mode on the device, in
+    allocations of at most 2 MiB more each."""
+    import torch
+
+    n = 100_000
+    rng = np.random.default_rng(8)
+    ctx = gpu.Context(0)
+    try:
+        c = rng.uniform(-100, 100, (n, 3)).astype(np.float32)
+        for k, p in enumerate(c):
+            ctx.add_point_light(1.0, (1.0, 1.0, 1.0), p.tolist())
+            if k == 1:  # loads what a build needs once
+                ctx.build_light_sampler(gpu.SAMPLER_BVH)
+        before = torch.cuda.mem_get_info()[0]
+        ctx.build_light_sampler(gpu.SAMPLER_BVH)
+        held = before - torch.cuda.mem_get_info()[0]
+        print(f"{held / 2**20:.1f} MiB")
+        assert held <= (2 * n - 1) * (40 + 2 * 48) + 3 * (2 << 20)
+    finally:
+        ctx.close()
