@@ -332,3 +332,35 @@ def test_child_box_planes_of_the_largest_boxes(ctx, lo, hi):
     assert hit[::2].sum() > 100 and hit[1::2].sum() > 100
     compare_closest(rays, tris, ctx.trace(rays), *ref[:4])
     assert (ctx.occluded(rays) == oracle.any_brute(rays, tris)).all()
+
+
+@pytest.mark.parametrize("n", [1, 31, 4095, 4096, 4097])
+def test_host_queries_on_each_side_of_the_copies(ctx, n):
+    """Host queries of up to 4,096 rays go through page-locked memory that the
+    kernel reads and writes itself, larger ones through copies (page-locked and
+    pageable ones differ): each gives the device query's bytes, and nothing is
+    written past the last result."""
+    import torch
+
+    verts, idx = scenes.triangle_soup(20000, seed=95, mu=np.log(0.02))
+    _load(ctx, verts, idx)
+    rays = np.concatenate([scenes.primary_rays(64, 32), scenes.incoherent_rays(4097, seed=96)])[-n:]
+    dr = torch.from_numpy(rays).cuda()
+    dh = torch.empty(n, 4, dtype=torch.int32, device="cuda")
+    do = torch.empty(n, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    ctx.trace_device(dr.data_ptr(), n, dh.data_ptr())
+    ctx.occluded_device(dr.data_ptr(), n, do.data_ptr())
+    ctx.synchronize()
+    for pinned in (False, True):
+        def host(shape, dtype):
+            t = torch.full(shape, 0x5A, dtype=dtype)
+            return (t.pin_memory() if pinned else t).numpy()
+
+        r = host((n, 8), torch.float32)
+        r[:] = rays
+        hits, occ = host((n + 1, 16), torch.uint8), host((n + 1,), torch.uint8)
+        ctx.trace(r, hits[:n].reshape(-1).view(gpu.HIT_DTYPE))
+        ctx.occluded(r, occ[:n])
+        assert hits[:n].tobytes() == dh.cpu().numpy().tobytes() and (hits[n] == 0x5A).all()
+        assert occ[:n].tobytes() == do.cpu().numpy().tobytes() and occ[n] == 0x5A

@@ -155,3 +155,24 @@ def test_invalid_traversal_options(ctx):
         with pytest.raises(gpu.GpuError) as e:
             ctx.set_traversal_options(**kw)
         assert e.value.code == gpu.ERR_INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize("n,pinned", [(4096, False), (4097, False), (4097, True), (200_000, True)])
+def test_device_limit_is_reported_on_every_way_to_the_kernel(ctx, n, pinned):
+    """A limit that runs out is reported by host queries through page-locked
+    memory, through copies and through chunks of page-locked buffers, and the
+    next query of the same kind answers."""
+    import torch
+
+    verts, idx = scenes.triangle_soup(20000, seed=21, mu=np.log(0.01))
+    _load(ctx, verts, idx, gpu.TRIANGLE_TEST_WIDE_BVH)
+    t = torch.from_numpy(scenes.incoherent_rays(n, seed=23))
+    rays = (t.pin_memory() if pinned else t).numpy()
+    occ = torch.empty(n, dtype=torch.uint8, pin_memory=pinned).numpy()
+    want = ctx.occluded(rays, occ).copy()
+    ctx.set_traversal_options(gpu.TRIANGLE_TEST_WIDE_BVH, max_visits=1)
+    with pytest.raises(gpu.GpuError) as e:
+        ctx.occluded(rays, occ)
+    assert e.value.code == gpu.ERR_LIMIT and "visit cap" in str(e.value)
+    ctx.set_traversal_options(gpu.TRIANGLE_TEST_WIDE_BVH)
+    assert ctx.occluded(rays, occ).tobytes() == want.tobytes()
