@@ -82,8 +82,12 @@ int host_query(alpine_gpu_ctx* c, const alpine_gpu_ray* rays, uint64_t n, void* 
         // A small batch is all latency: the rays are copied by the host into
         // page-locked memory that the kernel reads over the link, the results
         // come back the same way, and one wait covers them and the status word.
-        // With copies and two waits 256 rays took 57 us, so 43 us; 4,096 rays
-        // 154 and 110 us (B200). Larger batches use the link's copy engines.
+        // Closest hits with copies and so, us (B200; room of 4,036 triangles,
+        // soup of 262,144): 256 rays 51 and 43, 123 and 105; 4,096 rays 70 and
+        // 50, 142 and 122; page-locked buffers 60 and 49, 134 and 122. At 8,192
+        // page-locked rays the two are level in the room (67 and 63), at 16,384
+        // the copies are ahead (71 and 87; pageable rays at 65,536), so the line
+        // lies where both kinds of buffer gain.
         char* hits = c->hDirect + ag::kDirectRays * sizeof(alpine_gpu_ray);
         std::memcpy(c->hDirect, rays, n * sizeof(alpine_gpu_ray));
         if (kAny) ag::launch_occluded(view(c), c->hDirect, n, reinterpret_cast<uint8_t*>(hits), c->dStatus, c->stream);

@@ -1726,8 +1726,8 @@ void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t 
 inline size_t max_big(size_t N) { return N / kSmallMax + 2; }
 inline size_t max_chunks(size_t N) { return N / kChunk + max_big(N) + 2; }
 
-// Collapse levels enqueued before the depth is known: log8 of the primitives,
-// doubled for uneven trees. A level without items costs two empty launches.
+// Halvings until at most `per` of n primitives are left: the binary depth of a
+// balanced tree over them.
 inline uint32_t expected_levels(uint32_t n, uint32_t per)
 {
     uint32_t bits = 0;
@@ -1899,8 +1899,10 @@ int Builder::build(const float* verts, const uint32_t* idx, uint32_t ntris, cons
     }
     if (int rc = reserve(n, err, errLen)) return rc;
     const Input in{verts, idx, ntris, spheres, nspheres, nodes, tris, deviceStatus};
-    // levels enqueued at first: the last build's with a margin, or those of a
-    // balanced tree with one
+    // levels enqueued at first: the last build's and one more, or those of a
+    // balanced tree (three binary levels to a collapse level) with a margin of 3
+    // and 4 for uneven ones. A big level without tasks costs three empty
+    // launches, a collapse level without items two; one too few costs a wait.
     uint32_t levels = n > kSmallMax ? (bigLevels_ ? bigLevels_ + 1u : expected_levels(n, kSmallMax) + 3u) : 0u;
     uint32_t wide = wideLevels_ ? wideLevels_ + 1u : 4u + expected_levels(n, 1) / 3u;
     levels = std::min(levels, kMaxLevels);

@@ -851,8 +851,9 @@ __global__ void __launch_bounds__(32 * kTrainRowWarps) k_train_rows(Params g, co
 }
 
 // One warp: rows 16 mt .. 16 mt + 15 of dW_l over the samples of its split
-// (k-steps of 16 samples; the slice's last partial 32-sample chunk is zero
-// padded by k_train_rows), written to partial[split].
+// (k-steps of 16 samples; the slice's last partial step is zero padded by
+// k_train_rows), written to partial[split].
+static_assert(kTrainRows % 16 == 0, "k_train_rows pads whole k-steps");
 __global__ void __launch_bounds__(32) k_dw(const __nv_bfloat16* __restrict__ XT, const __nv_bfloat16* __restrict__ DT,
                                           uint32_t n, float* __restrict__ partial)
 {

@@ -8,8 +8,10 @@ namespace ag {
 namespace {
 
 // Resident threads per SM: 1,024 leave 64 registers, which hold a node's 32
-// words beside the ray. With 896 (72 registers) the 1M-triangle soup took 6 %
-// longer, with 1,152 (56 registers, spills) 40 %.
+// words beside the ray: k_trace spills at most 4 bytes, k_trace_dyn, whose loop
+// keeps its place in the queue besides, 64 (closest hit) and 36 (any hit). With
+// 896 (72 registers) the 1M-triangle soup took 6 % longer, with 1,152 (56
+// registers, spills) 40 %.
 constexpr int kTraceThreads = 1024;
 
 template <bool kAny, bool kBinary>

@@ -772,13 +772,17 @@ def run_ours(args):
     bytes_closest = n * (RAY_BYTES + HIT_BYTES) + nv_c * NODE_BYTES + tv_c * TRI_BYTES
     bytes_any = n * (RAY_BYTES + 1) + nv_s * NODE_BYTES + tv_s * TRI_BYTES
     achieved = bytes_closest / (closest_ms / 1e3) / 1e9
+    traffic = traffic_from_profile()
     roofline = {
         "bound": "hbm", "kernel": "k_trace<closest>", "achieved": achieved, "peak": peak, "unit": "GB/s",
-        "frac": achieved / peak, "peak_source": peak_kind, "traffic": traffic_from_profile(),
+        "frac": achieved / peak, "peak_source": peak_kind, "traffic": traffic,
         "traffic_source": "DRAM bytes of one full-size launch from the committed ncu summary of this workload "
                           "(profiles/trace_closest_soup1M.md); not captured in this run",
-        "limiter": "instruction issue and SIMD divergence: the BVH (about 65 MB) is served from L2, so DRAM "
-                   "traffic is a small fraction of the algorithmic bytes",
+        "limiter": f"instruction issue and SIMD divergence, not HBM: a node visit counts its {NODE_BYTES} bytes as "
+                   f"laid out (so that the fraction is not comparable with another node size), and the BVH "
+                   f"({(stats['wide_nodes'] * NODE_BYTES + stats['triangles'] * TRI_BYTES) / 1e6:.0f} MB) is served "
+                   "from L2; dram_frac is the DRAM traffic's own share of the HBM copy rate",
+        "dram_frac": traffic / (closest_ms / 1e3) / 1e9 / peak if traffic else None,
         "l2": {"achieved": achieved, "peak": l2_gbs, "frac": achieved / l2_gbs if l2_gbs else None,
                "peak_source": "L2-resident device copy (best of 4-24 MiB buffers) measured in this run"},
         "algorithmic_bytes_per_launch": bytes_closest,
