@@ -1496,14 +1496,15 @@ __global__ void __launch_bounds__(kWideThreads, 8) k_wide_decide(const uint2* it
 // node's origin, rounded outwards to the top 16 bits of a float. A maximum that
 // no finite word reaches (infinite, NaN, or next to FLT_MAX) gets the top half
 // of +inf: with a lower half of 0 the word is +inf, with any other a NaN, which
-// the traversal's minimum and maximum over the axes pass over.
-constexpr uint32_t kNoBound = 0x7f800000u;
+// the traversal's minimum and maximum over the axes pass over. A minimum below
+// the origin, which is 0 where a node's minimum is infinite, is stored as -inf.
+constexpr uint32_t kNoBound = 0x7f800000u, kBelow16 = 0xff80u;
 AG_D uint32_t plane_word(float lo, float hi, float origin)
 {
-    float dl = __fsub_rd(lo, origin), dh = __fsub_ru(hi, origin);
-    dl = dl >= 0.0f ? dl : 0.0f;                      // (NaN: the origin)
+    float dh = __fsub_ru(hi, origin);
     dh = dh <= 0.0f ? 0.0f : dh;
-    const uint32_t l16 = __float_as_uint(dl) >> 16;   // truncated: rounded down
+    // truncated: rounded down
+    const uint32_t l16 = lo >= origin ? __float_as_uint(__fsub_rd(lo, origin)) >> 16 : kBelow16;
     const uint32_t hb = __float_as_uint(dh);
     uint32_t h16 = hb >> 16;                          // read with the lower half below it
     if (((h16 << 16) | l16) < hb) ++h16;
@@ -1573,7 +1574,8 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_emit(const uint2* items,
         const uint2 off = valid ? itemOff[i] : make_uint2(0u, 0u);
         const int32_t e = valid ? slots[size_t(i) * kWidth + g] : -1;
         const BinNode nb = bnodes[it.x];
-        const float p[3] = {nb.lo.x, nb.lo.y, nb.lo.z};
+        const float p[3] = {isinf(nb.lo.x) ? 0.0f : nb.lo.x, isinf(nb.lo.y) ? 0.0f : nb.lo.y,
+                            isinf(nb.lo.z) ? 0.0f : nb.lo.z};
         BinNode c = nb;
         if (e >= 0) c = bnodes[e];
         const bool leaf = e >= 0 && c.count <= (uint32_t)kMaxLeafTris, inner = e >= 0 && !leaf;
@@ -1596,16 +1598,14 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_emit(const uint2* items,
         uint32_t* u = reinterpret_cast<uint32_t*>(r);
         // an empty slot's box is inside out: minimum 1e30, maximum -1e30
         constexpr uint32_t kEmptyPlanes = 0xf1497149u;
-        uint32_t planes[3] = {kEmptyPlanes, kEmptyPlanes, kEmptyPlanes};
-        if (e >= 0) {
-            planes[0] = plane_word(c.lo.x, c.hi.x, p[0]);
-            planes[1] = plane_word(c.lo.y, c.hi.y, p[1]);
-            planes[2] = plane_word(c.lo.z, c.hi.z, p[2]);
-            // unbounded on every axis: one must not be a NaN
-            if (min(planes[0], min(planes[1], planes[2])) >= kNoBound) planes[0] = kNoBound;
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) u[8 * (k + 1) + g] = planes[k];
+        const uint32_t wy = plane_word(c.lo.y, c.hi.y, p[1]), wz = plane_word(c.lo.z, c.hi.z, p[2]);
+        uint32_t wx = plane_word(c.lo.x, c.hi.x, p[0]);
+        // unbounded on every axis: one must not be a NaN (a minimum of -inf
+        // leaves the largest finite word, 2^-17 below FLT_MAX)
+        if (min(wx, min(wy, wz)) >= kNoBound) wx = (wx & 0xffffu) == kBelow16 ? 0x7f7f0000u | kBelow16 : kNoBound;
+        u[8 + g] = e >= 0 ? wx : kEmptyPlanes;
+        u[16 + g] = e >= 0 ? wy : kEmptyPlanes;
+        u[24 + g] = e >= 0 ? wz : kEmptyPlanes;
         if (g == 0) {
             float* f = reinterpret_cast<float*>(r);
             f[0] = p[0];

@@ -1,7 +1,7 @@
 // BVH layouts in HBM.
 //
 // Wide node (128 bytes, one cache line, read with four 256-bit loads):
-//   words 0-7:   float px, py, pz    origin = node box minimum
+//   words 0-7:   float px, py, pz    origin = node box minimum (0 where that is infinite)
 //                u32 imask           bit s set <=> slot s holds an internal child
 //                u32 childBase       index of the first internal child node
 //                u32 triBase         index of the first triangle record
@@ -10,17 +10,18 @@
 //                                    leaf = (unary count << 5) | triangle offset
 //   words 8-31:  u32 planes[3][8]    per axis and slot the child's box, as offsets
 //                                    from the origin in the top 16 bits of a float:
-//                                    minimum (rounded down) in the lower half,
+//                                    minimum (rounded down; -inf if below the
+//                                    origin) in the lower half,
 //                                    maximum in the upper. The maximum is read as
 //                                    the whole word, so the lower half is part of
 //                                    its value; it is rounded up with that counted.
 //                                    A maximum too large for that is +inf or a NaN
 //                                    (not on every axis): no bound.
-// The planes never lie inside a child's box. The traversal takes |d| for at
-// least 1e-20 on every axis (with the byte planes before it did too), so a hit
-// is missed where a plane's distance overflows (a node's minimum is -inf, or
-// further than FLT_MAX * |d| from the ray's origin), or where it lies further
-// along an axis-parallel ray than 1e20 times the box's extent beside it.
+// The planes never lie inside a child's box, infinite boxes included. The
+// traversal takes |d| for at least 1e-20 on every axis (with the byte planes
+// before it did too), so a hit is missed where a plane's distance overflows (a
+// node's origin is further than FLT_MAX * |d| from the ray's), or where it lies
+// further along an axis-parallel ray than 1e20 times the box's extent beside it.
 // A word becomes the near or the far plane by one integer multiplication (by
 // 65536 or 1, chosen per ray and axis by the direction's sign). The 80-byte
 // node before it held the planes as bytes of a per-axis quantum, which took

@@ -364,3 +364,22 @@ def test_host_queries_on_each_side_of_the_copies(ctx, n):
         ctx.occluded(r, occ[:n])
         assert hits[:n].tobytes() == dh.cpu().numpy().tobytes() and (hits[n] == 0x5A).all()
         assert occ[:n].tobytes() == do.cpu().numpy().tobytes() and occ[n] == 0x5A
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf])
+@pytest.mark.parametrize("axes", [(0,), (1, 2), (0, 1, 2)])
+def test_infinite_vertices_hide_nothing(ctx, value, axes):
+    """A triangle with an infinite vertex, on one to three axes, and another with
+    both infinities: every hit on the finite triangles beside them is found."""
+    verts, idx = scenes.triangle_soup(700, seed=97, mu=np.log(0.05))
+    for a in axes:
+        verts[33, a] = value
+        verts[600, a], verts[601, a] = value, -value
+    _load(ctx, verts, idx)
+    rays = np.concatenate([scenes.primary_rays(64, 32), scenes.incoherent_rays(4000, seed=98)])
+    rays[::4, 4:7] = -rays[::4, 4:7]
+    tris = oracle.make_tris(verts, idx)
+    ref = oracle.closest_brute(rays, tris)[:4]
+    assert (ref[0] != MISS).sum() > 500
+    compare_closest(rays, tris, ctx.trace(rays), *ref)
+    assert (ctx.occluded(rays) == oracle.any_brute(rays, tris)).all()
