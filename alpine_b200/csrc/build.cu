@@ -68,7 +68,7 @@ struct alignas(16) BigTask {
 struct BigSplit {
     int axis;
     int bin;
-    int mode;  // 0 = SAH bin split, 1 = median (all centroids coincide)
+    int mode;  // 0 = SAH bin split, 1 = median (all centroids coincide, or every cost overflows)
     uint32_t nL;
     uint32_t child[2];  // big-task index of each child in the next level, kNoTask for a small one
 };
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* tasks, c
             float box[6];
 #pragma unroll
             for (int j = 0; j < 6; ++j) box[j] = k ? best.R[j] : best.L[j];
-            if (median) {  // all centroids coincide: split by position, the children keep the parent's box
+            if (median) {  // no plane with a finite cost (all centroids coincide): split by position, the children keep the parent's box
                 const BinNode parent = bnodes[task.node];
                 box[0] = parent.lo.x; box[1] = parent.lo.y; box[2] = parent.lo.z;
                 box[3] = parent.hi.x; box[4] = parent.hi.y; box[5] = parent.hi.z;
@@ -572,9 +572,16 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const BigTask* tasks, c
             if (nodes && listed) {
                 if (chunks) {
                     BigTask t{};
+                    // gathered by k_scatter; a split by position of finite
+                    // centroids starts from the parent's bounds, so that where
+                    // the costs overflow (boxes beyond about 1e18) the halves
+                    // are halved again, and the depth stays a balanced tree's
+                    bool inherit = median;
+                    for (int a = 0; a < 3; ++a)
+                        inherit = inherit && isfinite(ord2f(task.clo[a])) && isfinite(ord2f(task.chi[a]));
                     for (int a = 0; a < 3; ++a) {
-                        t.clo[a] = 0xffffffffu;  // gathered by k_scatter
-                        t.chi[a] = 0u;
+                        t.clo[a] = inherit ? task.clo[a] : 0xffffffffu;
+                        t.chi[a] = inherit ? task.chi[a] : 0u;
                     }
                     t.node = id + k;
                     t.begin = begin;

@@ -50,3 +50,29 @@ def test_sizes_around_the_builders_limits(n, kind):
             assert ctx.trace(rays).tobytes() == hits.tobytes()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("growth", [1.03, 1.04, 1.05])
+def test_boxes_whose_areas_overflow(growth):
+    """Nested triangles up to 1.05^1500 across: where the SAH costs overflow,
+    nodes are halved by position, and the tree stays within the traversal's
+    stack under both collapse rules."""
+    n = 60000
+    base = np.array([[0, 0, 0], [1, 0, 0.1], [0.2, 1, 0.3]], np.float32) - np.float32(0.4)
+    v = (base[None] * (growth ** (np.arange(n) % 1500))[:, None, None]).astype(np.float32)
+    verts, idx = v.reshape(-1, 3), np.arange(3 * n, dtype=np.uint32).reshape(-1, 3)
+    rays = scenes.incoherent_rays(300, seed=12)
+    tris = oracle.make_tris(verts, idx)
+    ref = oracle.closest_brute(rays, tris)[:4]
+    ctx = gpu.Context(0)
+    try:
+        ctx.add_mesh(verts, idx)
+        for rule in (gpu.COLLAPSE_SAH, gpu.COLLAPSE_GREEDY):
+            ctx.set_build_options(rule)
+            ctx.build()
+            compare_closest(rays, tris, ctx.trace(rays), *ref)
+            ctx.build_async()
+            ctx.synchronize()
+            compare_closest(rays, tris, ctx.trace(rays), *ref)
+    finally:
+        ctx.close()
